@@ -1,6 +1,7 @@
-"""Builds libvsparse_b200.so (CUDA kernels + C ABI + host builder) and the C++ benchmark drivers in-tree.
+"""Builds libvsparse_b200.so (CUDA kernels + C ABI + host builder), the torch binding and the C++ benchmark drivers
+in-tree.
 
-    python -m vectorsparse_b200.build            # library + drivers
+    python -m vectorsparse_b200.build            # library + binding + drivers
 """
 from __future__ import annotations
 
@@ -12,6 +13,7 @@ import sys
 HERE = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(HERE)
 LIB = os.path.join(HERE, "libvsparse_b200.so")
+BINDING = os.path.join(HERE, "_binding.so")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 
 
@@ -52,6 +54,27 @@ def build_library(force: bool = False, verbose: bool = False) -> str:
     return LIB
 
 
+def build_binding(force: bool = False) -> str:
+    """The CPython module between torch tensors and the C ABI (host code only; the library is bound by address)."""
+    src = os.path.join(HERE, "csrc", "binding.cpp")
+    if not force and not _stale(BINDING, [src, os.path.join(ROOT, "include", "vsparse_b200.h")]):
+        return BINDING
+    import sysconfig
+
+    import torch
+    from torch.utils import cpp_extension
+
+    cuda_home = os.path.dirname(os.path.dirname(_nvcc()))
+    cmd = ["g++", "-O2", "-std=c++17", "-shared", "-fPIC", "-fvisibility=hidden", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}"]
+    for d in [*cpp_extension.include_paths(), sysconfig.get_paths()["include"], os.path.join(cuda_home, "include")]:
+        cmd += ["-isystem", d]
+    cmd += ["-I", os.path.join(ROOT, "include"), "-o", BINDING, src]
+    for d in cpp_extension.library_paths():
+        cmd += ["-L", d, f"-Wl,-rpath,{d}"]
+    subprocess.run([*cmd, "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"], check=True)
+    return BINDING
+
+
 def build_drivers(force: bool = False):
     """spmm_benchmark / sddmm_benchmark: same positional command line as the reference drivers; compat_check: every
     overload of include/vsparse_compat.h against a host product."""
@@ -70,5 +93,6 @@ def build_drivers(force: bool = False):
 
 if __name__ == "__main__":
     build_library(force="--force" in sys.argv, verbose="-v" in sys.argv)
+    build_binding(force="--force" in sys.argv)
     build_drivers(force="--force" in sys.argv)
     print(LIB)

@@ -1,0 +1,311 @@
+// CPython extension module `_binding`: the fast way from torch tensors to the C ABI.
+//
+// A call of one small product costs the host more than the GPU: through ctypes and Python-side checks the operators took
+// 17-28 us per call on a B200 host, against 13-16 us of GPU time.  Each function here takes the operator's arguments as
+// they stand, checks them without creating Python objects, finds the current stream and calls the library.  It answers
+//     an int   the library's return code (0, VS_ERR_* or a cudaError_t)
+//     None     some argument is not what the fast path takes (wrong type, device, layout or size): the Python operator
+//              then makes its own checks, which raise the error that belongs to the argument
+// so there is one set of error messages.  The library's functions are handed over by address (bind), so that the library
+// that vectorsparse_b200._lib has loaded is the one that is called.
+#include <Python.h>
+
+#include <ATen/core/Tensor.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include <climits>
+#include <cstdint>
+
+#include "vsparse_b200.h"
+
+namespace {
+
+struct Library {
+    decltype(&vs_spmm_batched) spmm;
+    decltype(&vs_spmm_t_batched) spmm_t;
+    decltype(&vs_sddmm_batched) sddmm;
+    decltype(&vs_softmax_cvse) softmax;
+    decltype(&vs_softmax_cvse_backward) softmax_backward;
+    decltype(&vs_attention_cvse) attention;
+    decltype(&vs_attention_cvse_backward) attention_backward;
+} g_lib;
+
+// The arguments of one call: `ok` turns false at the first one the fast path does not take.
+struct Args {
+    PyObject *const *argv;
+    bool ok = true;
+    int device = -1;
+
+    explicit Args(PyObject *const *a) : argv(a) {}
+
+    int64_t integer64(int i) {
+        const long long v = PyLong_CheckExact(argv[i]) ? PyLong_AsLongLong(argv[i]) : -1;
+        if (!PyLong_CheckExact(argv[i]) || (v == -1 && PyErr_Occurred())) {
+            PyErr_Clear();
+            ok = false;
+        }
+        return v;
+    }
+    int integer(int i) {
+        const int64_t v = integer64(i);
+        if (v < INT_MIN || v > INT_MAX) ok = false;
+        return (int)v;
+    }
+    double number(int i) {
+        if (PyFloat_CheckExact(argv[i])) return PyFloat_AS_DOUBLE(argv[i]);
+        if (PyLong_CheckExact(argv[i])) return (double)integer64(i);
+        ok = false;
+        return 0.0;
+    }
+    bool none(int i) const { return argv[i] == Py_None; }
+    // a contiguous CUDA tensor on the device of the others
+    const at::Tensor *tensor(int i) {
+        if (!ok || !THPVariable_Check(argv[i])) {
+            ok = false;
+            return nullptr;
+        }
+        const at::Tensor &t = THPVariable_Unpack(argv[i]);
+        if (!t.is_cuda() || !t.is_contiguous()) {
+            ok = false;
+            return nullptr;
+        }
+        const int dev = t.get_device();
+        if (device < 0) device = dev;
+        if (dev != device) ok = false;
+        return &t;
+    }
+    void need(const at::Tensor *t, int64_t numel) {
+        if (!ok || t->numel() < numel) ok = false;
+    }
+    void type(const at::Tensor *t, at::ScalarType want) {
+        if (!ok || t->scalar_type() != want) ok = false;
+    }
+    const int32_t *index(int i, int64_t numel) {
+        const at::Tensor *t = tensor(i);
+        need(t, numel);
+        type(t, at::kInt);
+        return ok ? static_cast<const int32_t *>(t->const_data_ptr()) : nullptr;
+    }
+    int dtype(const at::Tensor *t) {
+        if (ok && t->scalar_type() == at::kHalf) return VS_F16;
+        if (ok && t->scalar_type() == at::kFloat) return VS_F32;
+        ok = false;
+        return -1;
+    }
+};
+
+// Element stride between the problems of a batch; 0 for one problem or a shared operand.
+int64_t batch_stride(const at::Tensor *t, int batched_dims, int batch) {
+    return batch > 1 && t->dim() == batched_dims ? t->stride(0) : 0;
+}
+int64_t lead(const at::Tensor *t, int batched_dims, int batch) { return t->dim() == batched_dims ? batch : 1; }
+
+// Makes `device` current for the call (a look at the current one when it already is) and names its current stream.
+template <typename F> PyObject *call(const Args &a, F &&enqueue) {
+    c10::cuda::OptionalCUDAGuard guard;
+    if (c10::cuda::current_device() != a.device) guard.set_index((c10::DeviceIndex)a.device);
+    void *stream = (void *)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)a.device).stream();
+    return PyLong_FromLong(enqueue(stream));
+}
+
+#define VS_FAST_CALL(name, count)                                                       \
+    PyObject *name##_impl(Args &a);                                                     \
+    PyObject *name(PyObject *, PyObject *const *argv, Py_ssize_t n) {                   \
+        if (n != count) {                                                               \
+            PyErr_SetString(PyExc_TypeError, #name ": wrong number of arguments");      \
+            return nullptr;                                                             \
+        }                                                                               \
+        Args a(argv);                                                                   \
+        try {                                                                           \
+            return name##_impl(a);                                                      \
+        } catch (const std::exception &e) {                                             \
+            PyErr_SetString(PyExc_RuntimeError, e.what());                              \
+            return nullptr;                                                             \
+        }                                                                               \
+    }                                                                                   \
+    PyObject *name##_impl(Args &a)
+
+// spmm(path, m_vec, V, k, n, row_indices, row_offsets, column_indices, values, rhs, out, batch, nonzeros_vec | None)
+VS_FAST_CALL(spmm, 13) {
+    const int path = a.integer(0), m_vec = a.integer(1), V = a.integer(2), k = a.integer(3), n = a.integer(4), batch = a.integer(11);
+    const int64_t nnz = a.none(12) ? 0 : a.integer64(12);
+    const int32_t *ri = a.index(5, m_vec), *ro = a.index(6, (int64_t)m_vec + 1), *ci = a.index(7, nnz);
+    const at::Tensor *values = a.tensor(8), *rhs = a.tensor(9), *out = a.tensor(10);
+    if (!a.ok) Py_RETURN_NONE;
+    a.need(values, lead(values, 2, batch) * nnz * V);
+    a.need(rhs, lead(rhs, 3, batch) * (int64_t)n * k);
+    a.need(out, (int64_t)batch * m_vec * V * k);
+    a.type(rhs, values->scalar_type());
+    const int in_t = a.dtype(values), out_t = a.dtype(out);
+    if (!a.ok) Py_RETURN_NONE;
+    return call(a, [&](void *s) {
+        return g_lib.spmm(path, in_t, out_t, m_vec, V, k, n, ri, ro, ci, values->const_data_ptr(), rhs->const_data_ptr(),
+                          out->mutable_data_ptr(), batch, batch_stride(values, 2, batch), batch_stride(rhs, 3, batch),
+                          batch_stride(out, 3, batch), s);
+    });
+}
+
+// spmm_t(m_vec, V, k, n, t_offsets, t_rows, t_src, values, rhs, out, nonzeros_vec | None)
+VS_FAST_CALL(spmm_t, 11) {
+    const int m_vec = a.integer(0), V = a.integer(1), k = a.integer(2), n = a.integer(3);
+    const int64_t nnz = a.none(10) ? 0 : a.integer64(10);
+    const int32_t *off = a.index(4, (int64_t)n + 1), *rows = a.index(5, nnz), *src = a.index(6, nnz);
+    const at::Tensor *values = a.tensor(7), *rhs = a.tensor(8), *out = a.tensor(9);
+    if (!a.ok || THPVariable_Unpack(a.argv[5]).numel() != THPVariable_Unpack(a.argv[6]).numel()) Py_RETURN_NONE;
+    const int64_t lead_out = out->dim() == 3 ? out->size(0) : 1;
+    if (lead_out > INT_MAX) Py_RETURN_NONE;
+    const int batch = (int)lead_out;
+    a.need(values, lead(values, 2, batch) * nnz * V);
+    a.need(rhs, lead(rhs, 3, batch) * (int64_t)m_vec * V * k);
+    a.need(out, (int64_t)batch * n * k);
+    a.type(rhs, values->scalar_type());
+    const int in_t = a.dtype(values), out_t = a.dtype(out);
+    if (!a.ok) Py_RETURN_NONE;
+    return call(a, [&](void *s) {
+        return g_lib.spmm_t(in_t, out_t, m_vec, V, k, n, off, rows, src, values->const_data_ptr(), rhs->const_data_ptr(),
+                            out->mutable_data_ptr(), batch, batch_stride(values, 2, batch), batch_stride(rhs, 3, batch),
+                            batch_stride(out, 3, batch), s);
+    });
+}
+
+// sddmm(path, m_vec, k, n, nonzeros_vec, row_indices, row_offsets, col_indices, lhs, rhs, out, V, algorithm, batch)
+VS_FAST_CALL(sddmm, 14) {
+    const int path = a.integer(0), m_vec = a.integer(1), k = a.integer(2), n = a.integer(3), nnz = a.integer(4);
+    const int V = a.integer(11), algorithm = a.integer(12), batch = a.integer(13);
+    const int32_t *ri = a.index(5, m_vec), *ro = a.index(6, (int64_t)m_vec + 1), *ci = a.index(7, nnz);
+    const at::Tensor *lhs = a.tensor(8), *rhs = a.tensor(9), *out = a.tensor(10);
+    if (!a.ok) Py_RETURN_NONE;
+    a.need(lhs, lead(lhs, 3, batch) * (int64_t)m_vec * V * k);
+    a.need(rhs, lead(rhs, 3, batch) * (int64_t)n * k);
+    a.need(out, (int64_t)batch * nnz * V);
+    a.type(rhs, lhs->scalar_type());
+    const int in_t = a.dtype(lhs), out_t = a.dtype(out);
+    if (!a.ok) Py_RETURN_NONE;
+    return call(a, [&](void *s) {
+        return g_lib.sddmm(path, in_t, out_t, m_vec, k, n, nnz, ri, ro, ci, lhs->const_data_ptr(), rhs->const_data_ptr(),
+                           out->mutable_data_ptr(), V, batch, batch_stride(lhs, 3, batch), batch_stride(rhs, 3, batch),
+                           batch_stride(out, 2, batch), s, algorithm);
+    });
+}
+
+// Number of problems in a score array: [nnz] or [batch, nnz].  False if it cannot be a batch.
+bool score_batch(const at::Tensor *t, int *batch) {
+    const int64_t b = t->dim() == 2 ? t->size(0) : 1;
+    *batch = (int)b;
+    return b <= INT_MAX;
+}
+
+// softmax(m_vec, V, row_indices, row_offsets, scores, probs, scale)
+VS_FAST_CALL(softmax, 7) {
+    const int m_vec = a.integer(0), V = a.integer(1);
+    const double scale = a.number(6);
+    const int32_t *ri = a.index(2, 0), *ro = a.index(3, 0);
+    const at::Tensor *scores = a.tensor(4), *probs = a.tensor(5);
+    int batch = 1;
+    if (!a.ok || !score_batch(scores, &batch)) Py_RETURN_NONE;
+    a.type(probs, scores->scalar_type());
+    const int t = a.dtype(scores);
+    if (!a.ok) Py_RETURN_NONE;
+    return call(a, [&](void *s) {
+        return g_lib.softmax(t, m_vec, V, ri, ro, scores->const_data_ptr(), probs->mutable_data_ptr(), (float)scale, batch,
+                             batch_stride(scores, 2, batch), s);
+    });
+}
+
+// softmax_backward(m_vec, V, row_offsets, probs, grad_probs, grad_scores, scale)
+VS_FAST_CALL(softmax_backward, 7) {
+    const int m_vec = a.integer(0), V = a.integer(1);
+    const double scale = a.number(6);
+    const int32_t *ro = a.index(2, 0);
+    const at::Tensor *probs = a.tensor(3), *gp = a.tensor(4), *gs = a.tensor(5);
+    int batch = 1;
+    if (!a.ok || !score_batch(probs, &batch)) Py_RETURN_NONE;
+    a.type(gp, probs->scalar_type());
+    a.type(gs, probs->scalar_type());
+    const int t = a.dtype(probs);
+    if (!a.ok) Py_RETURN_NONE;
+    return call(a, [&](void *s) {
+        return g_lib.softmax_backward(t, m_vec, V, ro, probs->const_data_ptr(), gp->const_data_ptr(), gs->mutable_data_ptr(),
+                                      (float)scale, batch, batch_stride(probs, 2, batch), s);
+    });
+}
+
+// attention(path, m_vec, V, n, d, nonzeros_vec, row_indices, row_offsets, col_indices, q, k, v, out, workspace, scale)
+VS_FAST_CALL(attention, 15) {
+    const int path = a.integer(0), m_vec = a.integer(1), V = a.integer(2), n = a.integer(3), d = a.integer(4), nnz = a.integer(5);
+    const double scale = a.number(14);
+    const int32_t *ri = a.index(6, 0), *ro = a.index(7, 0), *ci = a.index(8, nnz);
+    const at::Tensor *t[5];
+    for (int i = 0; i < 5; ++i) {
+        t[i] = a.tensor(9 + i);
+        a.type(t[i], at::kHalf);
+    }
+    if (!a.ok) Py_RETURN_NONE;
+    const int64_t batch = t[0]->dim() == 3 ? t[0]->size(0) : 1;
+    if (batch > INT_MAX) Py_RETURN_NONE;
+    a.need(t[4], batch * nnz * V);
+    if (!a.ok) Py_RETURN_NONE;
+    return call(a, [&](void *s) {
+        return g_lib.attention(path, m_vec, V, n, d, nnz, ri, ro, ci, t[0]->const_data_ptr(), t[1]->const_data_ptr(),
+                               t[2]->const_data_ptr(), t[3]->mutable_data_ptr(), t[4]->mutable_data_ptr(), (float)scale, (int)batch, s);
+    });
+}
+
+// attention_backward(path, m_vec, V, n, d, nonzeros_vec, row_indices, row_offsets, col_indices, t_offsets, t_rows, t_src,
+//                    q, k, v, grad_out, grad_q, grad_k, grad_v, probs_workspace, grad_workspace, scale)
+VS_FAST_CALL(attention_backward, 22) {
+    const int path = a.integer(0), m_vec = a.integer(1), V = a.integer(2), n = a.integer(3), d = a.integer(4), nnz = a.integer(5);
+    const double scale = a.number(21);
+    const int32_t *ri = a.index(6, 0), *ro = a.index(7, 0), *ci = a.index(8, nnz);
+    const int32_t *off = a.index(9, 0), *rows = a.index(10, nnz), *src = a.index(11, nnz);
+    const at::Tensor *t[9];
+    for (int i = 0; i < 9; ++i) {
+        t[i] = a.tensor(12 + i);
+        a.type(t[i], at::kHalf);
+    }
+    if (!a.ok) Py_RETURN_NONE;
+    const int64_t batch = t[0]->dim() == 3 ? t[0]->size(0) : 1;
+    if (batch > INT_MAX) Py_RETURN_NONE;
+    a.need(t[7], batch * nnz * V);
+    a.need(t[8], batch * nnz * V);
+    if (!a.ok) Py_RETURN_NONE;
+    return call(a, [&](void *s) {
+        return g_lib.attention_backward(path, m_vec, V, n, d, nnz, ri, ro, ci, off, rows, src, t[0]->const_data_ptr(),
+                                        t[1]->const_data_ptr(), t[2]->const_data_ptr(), t[3]->const_data_ptr(), t[4]->mutable_data_ptr(),
+                                        t[5]->mutable_data_ptr(), t[6]->mutable_data_ptr(), t[7]->mutable_data_ptr(),
+                                        t[8]->mutable_data_ptr(), (float)scale, (int)batch, s);
+    });
+}
+
+// bind(addresses): the library's functions in the order of struct Library
+PyObject *bind(PyObject *, PyObject *const *argv, Py_ssize_t n) {
+    constexpr Py_ssize_t kCount = sizeof(Library) / sizeof(void *);
+    if (n != kCount) {
+        PyErr_SetString(PyExc_TypeError, "bind: wrong number of addresses");
+        return nullptr;
+    }
+    void **slot = reinterpret_cast<void **>(&g_lib);
+    for (Py_ssize_t i = 0; i < n; ++i) {
+        slot[i] = PyLong_AsVoidPtr(argv[i]);
+        if (!slot[i]) {
+            if (!PyErr_Occurred()) PyErr_SetString(PyExc_ValueError, "bind: null address");
+            return nullptr;
+        }
+    }
+    Py_RETURN_NONE;
+}
+
+#define VS_METHOD(name) {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(&name)), METH_FASTCALL, nullptr}
+PyMethodDef g_methods[] = {
+    VS_METHOD(bind), VS_METHOD(spmm), VS_METHOD(spmm_t), VS_METHOD(sddmm), VS_METHOD(softmax), VS_METHOD(softmax_backward),
+    VS_METHOD(attention), VS_METHOD(attention_backward), {nullptr, nullptr, 0, nullptr},
+};
+PyModuleDef g_module = {PyModuleDef_HEAD_INIT, "_binding", "torch tensors to the C ABI of libvsparse_b200", -1, g_methods,
+                        nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__binding() { return PyModule_Create(&g_module); }

@@ -12,6 +12,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <algorithm>
+#include <atomic>
 #include <cstring>
 #include <cmath>
 #include <mutex>
@@ -82,6 +83,15 @@ int device_info(DeviceInfo **out) {
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
     if (dev < 0 || dev >= kMaxDevices) return VS_ERR_ARG;
+    // A thread that has made no runtime call yet (autograd's backward thread, say) has no current context, and the
+    // driver's cuTensorMapEncodeTiled refuses to work without one: its first call would take the kernels that need no
+    // tensor maps.  Setting the device binds the context; once per thread and device.
+    static thread_local uint64_t bound = 0;
+    if (!(bound >> dev & 1u)) {
+        e = cudaSetDevice(dev);
+        if (e != cudaSuccess) return (int)e;
+        bound |= 1ull << dev;
+    }
     std::lock_guard<std::mutex> lock(g_devices_mutex);
     DeviceInfo &d = g_devices[dev];
     if (!d.ready) {
@@ -145,6 +155,19 @@ inline bool stride_ok(int64_t stride, int dtype) { return stride >= 0 && (stride
 template <typename K> int set_smem(K kernel, int bytes) {
     cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     return e == cudaSuccess ? VS_OK : (int)e;
+}
+// The same for a kernel whose shared memory never changes: asked once per device (`done`, one bit per device, belongs
+// to one kernel), not once per call, where it costs about as much as a tensor map.
+typedef std::atomic<uint64_t> DeviceBits;
+static_assert(kMaxDevices <= 64, "one bit per device");
+template <typename K> int set_smem_once(K kernel, int bytes, DeviceBits &done) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return set_smem(kernel, bytes);
+    const uint64_t bit = 1ull << dev;
+    if (done.load(std::memory_order_acquire) & bit) return VS_OK;
+    const int rc = set_smem(kernel, bytes);
+    if (rc == VS_OK) done.fetch_or(bit, std::memory_order_release);
+    return rc;
 }
 
 // Launches `kernel` so that it may start while the kernel ahead of it in the stream is still running (programmatic
@@ -332,7 +355,8 @@ template <typename TIn, typename TOut> int spmm_cc_by_v(int V, const SpmmParams 
 template <typename TOut, int V>
 int launch_spmm_tc_cpasync(const SpmmParams &p, cudaStream_t s, DeviceInfo *d, const int32_t *plan_hdr = nullptr, int plan_checks = 0) {
     auto kernel = tcspmm::spmm_tc_kernel<TOut, V>;
-    int rc = set_smem(kernel, tcspmm::kSmemBytes);
+    static DeviceBits smem_set;
+    int rc = set_smem_once(kernel, tcspmm::kSmemBytes, smem_set);
     if (rc != VS_OK) return rc;
     const int n_tiles = (p.N + tcspmm::kTileN - 1) / tcspmm::kTileN;
     const int64_t items = (int64_t)p.batch * n_tiles * p.m_vec;
@@ -361,7 +385,8 @@ int launch_spmm_gather(const SpmmParams &p, cudaStream_t s, DeviceInfo *d, const
     int rc = make_gather_map(&map, p.rhs, (uint64_t)total_rows, (uint64_t)p.N);
     if (rc != VS_OK) return launch_spmm_tc_cpasync<TOut, V>(p, s, d, plan_hdr, plan_checks);
     auto kernel = tmaspmm::spmm_tma_kernel<TOut, V>;
-    rc = set_smem(kernel, tmaspmm::kSmemBytes);
+    static DeviceBits smem_set;
+    rc = set_smem_once(kernel, tmaspmm::kSmemBytes, smem_set);
     if (rc != VS_OK) return rc;
     const int n_tiles = (p.N + tmaspmm::kTileN - 1) / tmaspmm::kTileN;
     const int64_t items = (int64_t)p.batch * n_tiles * p.m_vec;
@@ -520,7 +545,8 @@ template <typename TOut, int V> int launch_spmm_tc(const SpmmParams &p, cudaStre
     const int use_b4 = (p.N % 64 == 0 && make_blocked_map(&map_b4, p.rhs, (uint64_t)p.K, (uint64_t)p.N, (uint64_t)p.batch,
                                                           (uint64_t)p.stride_rhs, densespmm::kTileN / 64) == VS_OK) ? 1 : 0;
     auto kernel = densespmm::spmm_dense_kernel<TOut, V, false>;
-    rc = set_smem(kernel, densespmm::kSmemBytes);
+    static DeviceBits smem_set;
+    rc = set_smem_once(kernel, densespmm::kSmemBytes, smem_set);
     if (rc != VS_OK) return rc;
     uint8_t *plan = nullptr;
     if (stream_scratch(d, s, (size_t)plan_bytes, reinterpret_cast<void **>(&plan)) != VS_OK)
@@ -599,7 +625,8 @@ template <typename TIn, typename TOut> int sddmm_cc_by_v(int V, const SddmmParam
 // Software (cp.async) gather: works for any batch stride.
 template <typename TOut, int V> int launch_sddmm_tc_cpasync(const SddmmParams &p, cudaStream_t s, DeviceInfo *d) {
     auto kernel = tcsddmm::sddmm_tc_kernel<TOut, V>;
-    int rc = set_smem(kernel, tcsddmm::kSmemBytes);
+    static DeviceBits smem_set;
+    int rc = set_smem_once(kernel, tcsddmm::kSmemBytes, smem_set);
     if (rc != VS_OK) return rc;
     const int64_t items = (int64_t)p.batch * p.m_vec;
     const int64_t cap = 2ll * d->sm_count;
@@ -628,7 +655,8 @@ template <typename TOut, int V> int launch_sddmm_gather(const SddmmParams &p, cu
         make_gather_map(&map_l, p.lhs, (uint64_t)rows_l, (uint64_t)p.k) != VS_OK)
         return launch_sddmm_tc_cpasync<TOut, V>(p, s, d);
     auto kernel = tmasddmm::sddmm_tma_kernel<TOut, V>;
-    int rc = set_smem(kernel, tmasddmm::kSmemBytes);
+    static DeviceBits smem_set;
+    int rc = set_smem_once(kernel, tmasddmm::kSmemBytes, smem_set);
     if (rc != VS_OK) return rc;
     const int64_t items = (int64_t)p.batch * p.m_vec;
     const int64_t cap = (int64_t)tmasddmm::kCtasPerSm * d->sm_count;
@@ -747,7 +775,8 @@ template <typename TOut, int V> int launch_sddmm_tc(const SddmmParams &p, cudaSt
                       densesddmm::kTileN) != VS_OK)
         return launch_sddmm_gather<TOut, V>(p, s, d);
     auto kernel = densesddmm::sddmm_dense_kernel<TOut, V>;
-    rc = set_smem(kernel, densesddmm::kSmemBytes);
+    static DeviceBits smem_set;
+    rc = set_smem_once(kernel, densesddmm::kSmemBytes, smem_set);
     if (rc != VS_OK) return rc;
     uint8_t *plan = nullptr;
     if (stream_scratch(d, s, (size_t)plan_bytes, reinterpret_cast<void **>(&plan)) != VS_OK)
@@ -921,7 +950,8 @@ template <typename TOut, int V> int launch_spmm_t(const spmmt::Params &p, int m_
     const int use_b4 = (q.N % 64 == 0 && make_blocked_map(&map_b4, q.rhs, (uint64_t)q.K, (uint64_t)q.N, (uint64_t)q.batch,
                                                           (uint64_t)q.stride_rhs, densespmm::kTileN / 64) == VS_OK) ? 1 : 0;
     auto kernel = densespmm::spmm_dense_kernel<TOut, V, true>;
-    rc = set_smem(kernel, densespmm::kSmemBytes);
+    static DeviceBits smem_set;
+    rc = set_smem_once(kernel, densespmm::kSmemBytes, smem_set);
     if (rc != VS_OK) return rc;
     uint8_t *plan = nullptr;
     if (stream_scratch(d, s, (size_t)plan_bytes, reinterpret_cast<void **>(&plan)) != VS_OK)

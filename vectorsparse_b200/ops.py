@@ -8,9 +8,15 @@ column_indices, values, rhs_matrix, output_matrix); tensors replace raw device p
 are taken from them, which is what overload resolution does in the reference.  Every call enqueues on the
 current torch CUDA stream and returns 0; rejected arguments raise VsError (the reference prints and returns).
 PyTorch is used for device memory and streams only: the arithmetic is in libvsparse_b200.so.
+
+Every operator goes through the `_binding` extension first, which checks the arguments and calls the library without
+creating Python objects: one small product costs the GPU less than ctypes and the checks below cost the host.  It
+returns None for arguments it does not take, and the operator then makes its own checks, which raise the error that
+belongs to the argument.
 """
 from __future__ import annotations
 
+import ctypes
 import types
 
 import torch
@@ -18,7 +24,23 @@ import torch
 from . import _lib
 from ._lib import VS_F16, VS_F32, VS_PATH_CUDA_CORE, VS_PATH_TENSOR
 
+try:
+    from . import _binding
+except ImportError as e:
+    raise ImportError(f"vectorsparse_b200/_binding.so cannot be loaded ({e}): build it with `python -m vectorsparse_b200.build`. "
+                      "There is no fallback implementation.") from e
+
 _DT = {torch.float16: VS_F16, torch.float32: VS_F32}
+
+
+def _bind() -> None:
+    """Hands the binding the functions of the library that _lib has loaded, in the order of its `Library` struct."""
+    names = ("vs_spmm_batched", "vs_spmm_t_batched", "vs_sddmm_batched", "vs_softmax_cvse", "vs_softmax_cvse_backward",
+             "vs_attention_cvse", "vs_attention_cvse_backward")
+    _binding.bind(*(ctypes.cast(getattr(_lib.lib(), n), ctypes.c_void_p).value for n in names))
+
+
+_bind()
 
 
 def _one_device(**tensors):
@@ -68,6 +90,12 @@ def _need(t: torch.Tensor, numel: int, name: str):
 
 def _spmm(path, m_vec, vec_length, k, n, row_indices, row_offsets, column_indices, values, rhs_matrix,
           output_matrix, batch=1, nonzeros_vec=None):
+    rc = _binding.spmm(path, m_vec, vec_length, k, n, row_indices, row_offsets, column_indices, values, rhs_matrix,
+                       output_matrix, batch, nonzeros_vec)
+    if rc is not None:
+        if rc:
+            _lib.check(rc, "vs_spmm")
+        return 0
     device = _one_device(row_indices=row_indices, row_offsets=row_offsets, column_indices=column_indices, values=values,
                          rhs_matrix=rhs_matrix, output_matrix=output_matrix)
     _need(row_indices, m_vec, "row_indices")
@@ -93,6 +121,12 @@ def _spmm(path, m_vec, vec_length, k, n, row_indices, row_offsets, column_indice
 
 def _sddmm(path, m_vec, k, n, nonzeros_vec, row_indices, row_offsets, col_indices, lhs_matrix, rhs_matrix,
            output_values, vec_length, algorithm, batch=1):
+    rc = _binding.sddmm(path, m_vec, k, n, nonzeros_vec, row_indices, row_offsets, col_indices, lhs_matrix, rhs_matrix,
+                        output_values, vec_length, algorithm, batch)
+    if rc is not None:
+        if rc:
+            _lib.check(rc, "vs_sddmm")
+        return 0
     _need(row_indices, m_vec, "row_indices")
     _need(row_offsets, m_vec + 1, "row_offsets")
     _need(col_indices, nonzeros_vec, "col_indices")
@@ -173,6 +207,11 @@ def spmm_batched(path, m_vec, vec_length, k, n, row_indices, row_offsets, column
 def spmm_t(m_vec, vec_length, k, n, t_offsets, t_rows, t_src, values, rhs_matrix, output_matrix, nonzeros_vec=None):
     """output [n, k] (or [B, n, k]) = A^T @ rhs, rhs [m_vec * V, k] (or [B, ...]), values [nnz] (or [B, nnz]): the
     product with the transposed CVSE matrix; t_offsets / t_rows / t_src come from cvse.transpose (on the device)."""
+    rc = _binding.spmm_t(m_vec, vec_length, k, n, t_offsets, t_rows, t_src, values, rhs_matrix, output_matrix, nonzeros_vec)
+    if rc is not None:
+        if rc:
+            _lib.check(rc, "vs_spmm_t")
+        return 0
     batch = output_matrix.shape[0] if output_matrix.dim() == 3 else 1
     _need(t_offsets, n + 1, "t_offsets")
     _need(rhs_matrix, (batch if rhs_matrix.dim() == 3 else 1) * m_vec * vec_length * k, "rhs_matrix")
@@ -207,6 +246,11 @@ def sddmm_batched(path, m_vec, k, n, nonzeros_vec, row_indices, row_offsets, col
 
 def softmax_cvse(m_vec, vec_length, row_indices, row_offsets, scores, probs, scale=1.0):
     """Row softmax over the CVSE values; scores/probs [nnz] or [B, nnz]; probs may be scores."""
+    rc = _binding.softmax(m_vec, vec_length, row_indices, row_offsets, scores, probs, scale)
+    if rc is not None:
+        if rc:
+            _lib.check(rc, "vs_softmax_cvse")
+        return 0
     batch = scores.shape[0] if scores.dim() == 2 else 1
     stride = scores.stride(0) if scores.dim() == 2 and batch > 1 else 0
     device = _one_device(row_indices=row_indices, row_offsets=row_offsets, scores=scores, probs=probs)
@@ -222,6 +266,12 @@ def softmax_cvse(m_vec, vec_length, row_indices, row_offsets, scores, probs, sca
 def attention_cvse(path, m_vec, vec_length, n, d, nonzeros_vec, row_indices, row_offsets, col_indices, q, kmat,
                    vmat, out, workspace, scale):
     """softmax(scale * SDDMM(q, k)) @ v for [B, ., d] fp16 tensors sharing one mask; workspace [B, nnz] fp16."""
+    rc = _binding.attention(path, m_vec, vec_length, n, d, nonzeros_vec, row_indices, row_offsets, col_indices, q, kmat, vmat,
+                            out, workspace, scale)
+    if rc is not None:
+        if rc:
+            _lib.check(rc, "vs_attention_cvse")
+        return 0
     batch = q.shape[0] if q.dim() == 3 else 1
     _need(workspace, batch * nonzeros_vec * vec_length, "workspace")
     _need(col_indices, nonzeros_vec, "col_indices")
@@ -241,6 +291,11 @@ def attention_cvse(path, m_vec, vec_length, n, d, nonzeros_vec, row_indices, row
 
 def softmax_cvse_backward(m_vec, vec_length, row_offsets, probs, grad_probs, grad_scores, scale=1.0):
     """Gradient of softmax_cvse with respect to its scores; all three [nnz] or [B, nnz]; grad_scores may be grad_probs."""
+    rc = _binding.softmax_backward(m_vec, vec_length, row_offsets, probs, grad_probs, grad_scores, scale)
+    if rc is not None:
+        if rc:
+            _lib.check(rc, "vs_softmax_cvse_backward")
+        return 0
     batch = probs.shape[0] if probs.dim() == 2 else 1
     stride = probs.stride(0) if probs.dim() == 2 and batch > 1 else 0
     device = _one_device(row_offsets=row_offsets, probs=probs, grad_probs=grad_probs, grad_scores=grad_scores)
@@ -258,6 +313,13 @@ def attention_cvse_backward(path, m_vec, vec_length, n, d, nonzeros_vec, row_ind
                             t_rows, t_src, q, kmat, vmat, grad_out, grad_q, grad_k, grad_v, probs_workspace, grad_workspace,
                             scale):
     """Gradients of attention_cvse for [B, ., d] fp16 tensors sharing one mask; both workspaces [B, nnz] fp16."""
+    rc = _binding.attention_backward(path, m_vec, vec_length, n, d, nonzeros_vec, row_indices, row_offsets, col_indices,
+                                     t_offsets, t_rows, t_src, q, kmat, vmat, grad_out, grad_q, grad_k, grad_v,
+                                     probs_workspace, grad_workspace, scale)
+    if rc is not None:
+        if rc:
+            _lib.check(rc, "vs_attention_cvse_backward")
+        return 0
     batch = q.shape[0] if q.dim() == 3 else 1
     for w, name in ((probs_workspace, "probs_workspace"), (grad_workspace, "grad_workspace")):
         _need(w, batch * nonzeros_vec * vec_length, name)

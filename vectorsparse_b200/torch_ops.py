@@ -97,8 +97,9 @@ class FixedMaskAttention(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, mask: AttentionMask, scale: float, path: int = VS_PATH_TENSOR):
         q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-        out = torch.ops.vsparse.attention(path, mask.m_vec, mask.V, mask.nnz_vec, mask.row_indices, mask.row_offsets,
-                                          mask.col_indices, q, k, v, float(scale))
+        # the functions behind torch.ops.vsparse.*: the dispatcher's way to them and back costs the host ~10 us a call
+        out = _attention(path, mask.m_vec, mask.V, mask.nnz_vec, mask.row_indices, mask.row_offsets, mask.col_indices, q, k, v,
+                         float(scale))
         ctx.save_for_backward(q, k, v)
         ctx.mask, ctx.scale, ctx.path = mask, float(scale), path
         return out
@@ -128,7 +129,7 @@ class SparseDenseProduct(torch.autograd.Function):
     @staticmethod
     def forward(ctx, values, b, mask: AttentionMask, path: int = VS_PATH_TENSOR):
         values, b = values.contiguous(), b.contiguous()
-        c = torch.ops.vsparse.spmm(path, mask.m_vec, mask.V, mask.row_indices, mask.row_offsets, mask.col_indices, values, b)
+        c = _spmm(path, mask.m_vec, mask.V, mask.row_indices, mask.row_offsets, mask.col_indices, values, b)
         ctx.save_for_backward(values, b)
         ctx.mask, ctx.path = mask, path
         return c
@@ -143,7 +144,7 @@ class SparseDenseProduct(torch.autograd.Function):
             grad_b = torch.empty_like(b)
             ops.spmm_t(m.m_vec, m.V, b.shape[-1], m.n, m.t_offsets, m.t_rows, m.t_src, values, grad_c, grad_b, m.nnz_vec)
         if ctx.needs_input_grad[0]:
-            g = torch.ops.vsparse.sddmm(ctx.path, m.m_vec, m.V, m.nnz_vec, m.row_indices, m.row_offsets, m.col_indices, grad_c, b)
+            g = _sddmm(ctx.path, m.m_vec, m.V, m.nnz_vec, m.row_indices, m.row_offsets, m.col_indices, grad_c, b)
             grad_values = g.sum(0) if (g.dim() == 2 and values.dim() == 1) else g
         return grad_values, grad_b, None, None
 
