@@ -1,0 +1,85 @@
+"""The one-kernel forms of the tensor-core products (small problems), forced at the sizes where their tiles, chunks and
+windows end, and on the inputs they hand to their entry-by-entry path; against the fp64 oracle, conftest tolerance."""
+import numpy as np
+import pytest
+import torch
+
+import oracle
+from conftest import assert_close
+from gpu_util import DEV, custom, dev, problem, spmm_oracle, structure
+from vectorsparse_b200 import VS_PATH_TENSOR, cvse, ops
+
+pytestmark = pytest.mark.gpu
+
+
+def spmm_forced(monkeypatch, a, N, vals, B, out_t, mode):
+    monkeypatch.setenv("VSPARSE_B200_SPMM", mode)
+    out = torch.full((a.m, N), float("nan"), dtype=out_t, device=DEV)
+    ops.spmm.wmmaSpmm(a.m_vec, a.V, N, a.n, *structure(a), dev(vals), dev(B), out)
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    return out.float().cpu().numpy()
+
+
+# rows around the 128-row tile, columns around the 128-column chunk and the three-chunk ring, an empty matrix and full
+# rows (a chunk holds more than two windows of a row)
+@pytest.mark.parametrize("V,m_vec,K,N,sparsity", [(8, 1, 1, 64, 0.0), (8, 16, 128, 64, 0.5), (8, 17, 129, 128, 0.9), (8, 33, 700, 192, 0.95),
+                                                  (4, 31, 127, 64, 0.0), (4, 33, 513, 64, 0.8), (2, 63, 64, 64, 0.7), (2, 65, 385, 128, 0.1),
+                                                  (8, 20, 300, 64, 1.0)])
+@pytest.mark.parametrize("out_t", [torch.float16, torch.float32])
+def test_direct_spmm_at_the_edges_of_its_tiles(monkeypatch, V, m_vec, K, N, sparsity, out_t):
+    a = problem(cvse.GEN_UNIFORM, 3, m_vec, K, V, sparsity)
+    vals = cvse.fill_random((max(a.nnz_vec, 1) * V,), np.float16, cvse.DIST_NORMAL, 1, 0.25)
+    B = cvse.fill_random((K, N), np.float16, cvse.DIST_NORMAL, 2, 0.5)
+    got = spmm_forced(monkeypatch, a, N, vals, B, out_t, "direct")
+    assert_close(got, spmm_oracle(a, N, vals[:a.nnz_vec * V], B), "direct")
+    if sparsity < 1.0:   # the same K order, so the same bits as the kernels that work from a plan
+        assert np.array_equal(got, spmm_forced(monkeypatch, a, N, vals, B, out_t, "dense"))
+
+
+@pytest.mark.parametrize("V", [2, 8])
+@pytest.mark.parametrize("what", ["unsorted", "repeated", "non-finite"])
+def test_direct_spmm_tiles_computed_entry_by_entry(monkeypatch, V, what):
+    """Unsorted columns, a column named twice, and an Inf in a row of B that one vector-row names: only that row may
+    become non-finite."""
+    K, N = 200, 128
+    a = custom([40] * (300 // V), K, V, seed=5)
+    vals = cvse.fill_random((a.nnz_vec * V,), np.float16, cvse.DIST_NORMAL, 1, 0.25)
+    B = cvse.fill_random((K, N), np.float16, cvse.DIST_NORMAL, 2, 0.5)
+    if what == "unsorted":
+        ci = a.col_indices.reshape(-1, 40)
+        ci[3] = ci[3, ::-1]
+    elif what == "repeated":
+        a.col_indices[40 * 7 + 11] = a.col_indices[40 * 7 + 10]
+    else:
+        B[a.col_indices[0], 5] = np.inf
+    want = spmm_oracle(a, N, vals, B)
+    got = spmm_forced(monkeypatch, a, N, vals, B, torch.float32, "direct")
+    finite = np.isfinite(want)
+    assert np.array_equal(np.isfinite(got), finite)
+    assert_close(got[finite], want[finite], what)
+
+
+@pytest.mark.parametrize("V,m_vec,n,k,lens", [(8, 1, 1, 64, [1]), (8, 17, 129, 192, None), (4, 33, 63, 64, None), (2, 65, 257, 320, None),
+                                              (8, 16, 2000, 64, [1500] * 16), (2, 64, 128, 128, [0, 128] * 32)])
+@pytest.mark.parametrize("out_t", [torch.float16, torch.float32])
+def test_direct_sddmm_at_the_edges_of_its_tiles(monkeypatch, V, m_vec, n, k, lens, out_t):
+    """Rows around the 128-row tile, mask columns around the 64-column one, more contraction blocks than ring stages, rows with
+    more entries than are looked up ahead, unsorted and repeated columns."""
+    lens = lens or [(7 * i) % min(n, 40) for i in range(m_vec)]
+    a = custom(lens, n, V, seed=9)
+    rng = np.random.default_rng(1)
+    if a.nnz_vec > 4:   # any order, any repetition
+        first = slice(int(a.row_offsets[m_vec - 1]), int(a.row_offsets[m_vec]))
+        a.col_indices[first] = rng.permutation(a.col_indices[first])
+        a.col_indices[a.nnz_vec // 2] = a.col_indices[a.nnz_vec // 2 - 1]
+    lhs = cvse.fill_random((a.m, k), np.float16, cvse.DIST_NORMAL, 3, 0.25)
+    rhs = cvse.fill_random((n, k), np.float16, cvse.DIST_NORMAL, 4, 0.25)
+    monkeypatch.setenv("VSPARSE_B200_SDDMM", "direct")
+    out = torch.full((a.nnz_vec * V + 8,), float("nan"), dtype=out_t, device=DEV)
+    ops._sddmm(VS_PATH_TENSOR, m_vec, k, n, a.nnz_vec, *structure(a), dev(lhs), dev(rhs), out, V, 1)
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    want = oracle.sddmm(m_vec, k, V, a.row_offsets, a.col_indices, lhs.astype(np.float32), rhs.astype(np.float32), acc="f64")
+    assert_close(out[:a.nnz_vec * V].float().cpu().numpy(), want, "direct")
+    assert torch.isnan(out[a.nnz_vec * V:]).all()

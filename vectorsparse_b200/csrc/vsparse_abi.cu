@@ -28,12 +28,14 @@
 #include "spmm_tc.cuh"
 #include "spmm_tma.cuh"
 #include "spmm_dense.cuh"
+#include "spmm_direct.cuh"
 #include "sddmm_pair.cuh"
 #include "spmm_pair.cuh"
 #include "spmm_t.cuh"
 #include "sddmm_tc.cuh"
 #include "sddmm_tma.cuh"
 #include "sddmm_dense.cuh"
+#include "sddmm_direct.cuh"
 #include "tc_selftest.cuh"
 
 #define VS_EXPORT extern "C" __attribute__((visibility("default")))
@@ -407,11 +409,12 @@ int launch_spmm_gather(const SpmmParams &p, cudaStream_t s, DeviceInfo *d, const
 // leaves a flag that one of the two kernels, both enqueued, finds set against it and returns at once.  The
 // densifying kernel clears the flag again if it produced a non-finite sum, so that the gather kernel redoes the
 // call with the reference's semantics for Inf / NaN in rows of B that no nonzero names.
-enum class SpmmMode { kAuto, kDense, kGather };
+enum class SpmmMode { kAuto, kDense, kGather, kDirect };
 SpmmMode spmm_mode() {   // read at every call, so that a test can switch kernels inside one process
     const char *e = std::getenv("VSPARSE_B200_SPMM");
     if (e && !std::strcmp(e, "dense")) return SpmmMode::kDense;
     if (e && !std::strcmp(e, "gather")) return SpmmMode::kGather;
+    if (e && !std::strcmp(e, "direct")) return SpmmMode::kDirect;
     return SpmmMode::kAuto;
 }
 constexpr int64_t kMaxPlanBytes = 512ll << 20;
@@ -514,11 +517,57 @@ bool launch_spmm_pair(const SpmmParams &q, cudaStream_t s, DeviceInfo *d, const 
     return true;
 }
 
+// Costs of the two formulations in SM-cycles per 128 columns of B, as the plan kernel compares them (see there).
+struct SpmmCosts {
+    float dense_per_stage, dense_per_entry, gather_per_row, gather_per_entry;
+};
+constexpr SpmmCosts kGatherCosts = {1100.0f, 0.0f, 370.0f, 4.7f};
+
+// Small products in one kernel (spmm_direct.cuh); false if this call or this device cannot take it.  When the densified
+// product is the cheaper one whatever the number of nonzeros, nothing else is enqueued; otherwise the kernel leaves its
+// verdict where the gather kernel behind it looks for the plan kernel's.
+template <typename TOut, int V> bool launch_spmm_direct(const SpmmParams &p, cudaStream_t s, DeviceInfo *d, const SpmmCosts &cost,
+                                                        bool forced, int *rc_out) {
+    const int m_tiles = (int)(((int64_t)p.m_vec * V + directspmm::kTileM - 1) / directspmm::kTileM);
+    const int n_tiles = (p.N + directspmm::kTileN - 1) / directspmm::kTileN;
+    const int64_t tiles = (int64_t)p.batch * m_tiles * n_tiles;
+    if (tiles > 0x7fffffffll || p.K <= 0 || p.N % 8 != 0) return false;
+    const float stages = std::ceil((float)p.m_vec * V / densespmm::kTileM) * std::ceil((float)p.K / densespmm::kBlockK);
+    const bool always = forced || (cost.dense_per_entry == 0.0f && cost.dense_per_stage * stages < cost.gather_per_row * (float)p.m_vec);
+    CUtensorMap map;
+    static DeviceBits smem_set;
+    auto kernel = directspmm::spmm_direct_kernel<TOut, V>;
+    if (make_tile_map(&map, p.rhs, false, (uint64_t)p.K, (uint64_t)p.N, (uint64_t)p.batch, (uint64_t)p.stride_rhs, 64, 64) != VS_OK ||
+        set_smem_once(kernel, directspmm::kSmemBytes, smem_set) != VS_OK)
+        return false;
+    void *verdict = nullptr;
+    if (!always && (t_no_scratch || stream_scratch(d, s, 16, &verdict) != VS_OK)) return false;
+    *rc_out = (int)launch_overlapped(kernel, (unsigned)tiles, directspmm::kThreads, directspmm::kSmemBytes, s, p, map, m_tiles, n_tiles,
+                                     cost.dense_per_stage * stages, cost.dense_per_entry, cost.gather_per_row, cost.gather_per_entry,
+                                     static_cast<int32_t *>(verdict), d->status);
+    if (*rc_out == VS_OK && !always) *rc_out = launch_spmm_gather<TOut, V>(p, s, d, static_cast<const int32_t *>(verdict), 0);
+    return true;
+}
+// Which products are small: up to one wave of 128 x 64 tiles at two per SM the one-kernel form saves the ~9 us of the other
+// launches and loses nothing (2048 x 512 x 256, V = 8: 15.4 -> 6.5 us; 512 x 2048 x 256: 22.3 -> 13.3), up to two waves while
+// K is short.  Shorter vectors mean more entries per tile, which it scatters again for every 64 columns of B, so there
+// the line lies at a smaller K (V = 2, 1024 x 1024 x 256, four of them: 26.6 -> 24.6; 4096 x 4608 x 256: 74 -> 88).
+bool spmm_direct_wanted(const SpmmParams &p, int V, const DeviceInfo *d) {
+    const int64_t m_tiles = ((int64_t)p.m_vec * V + directspmm::kTileM - 1) / directspmm::kTileM;
+    const int64_t tiles = m_tiles * ((p.N + directspmm::kTileN - 1) / directspmm::kTileN) * p.batch;
+    const int chunks = (p.K + directspmm::kChunkK - 1) / directspmm::kChunkK;
+    if (tiles <= 2 * d->sm_count) return chunks <= (V == 8 ? 64 : V == 4 ? 16 : V == 2 ? 8 : 4);
+    return tiles <= 4 * d->sm_count && chunks <= (V == 8 ? 4 : V == 4 ? 2 : 1);
+}
+
 template <typename TOut, int V> int launch_spmm_tc(const SpmmParams &p, cudaStream_t s) {
     DeviceInfo *d;
     int rc = device_info(&d);
     if (rc != VS_OK) return rc;
     const SpmmMode mode = spmm_mode();
+    if ((mode == SpmmMode::kDirect || (mode == SpmmMode::kAuto && spmm_direct_wanted(p, V, d))) &&
+        launch_spmm_direct<TOut, V>(p, s, d, kGatherCosts, mode == SpmmMode::kDirect, &rc))
+        return rc;
     const int k_blocks = (p.K + densespmm::kBlockK - 1) / densespmm::kBlockK;
     const int m_tiles = (p.m_vec * V + densespmm::kTileM - 1) / densespmm::kTileM;
     const int n_tiles = (p.N + densespmm::kTileN - 1) / densespmm::kTileN;
@@ -559,7 +608,8 @@ template <typename TOut, int V> int launch_spmm_tc(const SpmmParams &p, cudaStre
     // a dependent launch as well: in a stream of calls the plan kernel queues up behind the previous call's last kernel
     rc = (int)launch_overlapped(densespmm::dense_plan_kernel<false>, (unsigned)(groups + checks), densespmm::kPlanThreads, plan_smem, s,
                                 p.row_offsets, p.col_indices, (const int32_t *)nullptr, 0, p.m_vec, p.K, groups, rows_per_group,
-                                plan_blocks, blk_offsets, blk_entries, capacity, force_dense, 370.0f, 4.7f, 0.0f, flag);
+                                plan_blocks, blk_offsets, blk_entries, capacity, force_dense, kGatherCosts.gather_per_row,
+                                kGatherCosts.gather_per_entry, kGatherCosts.dense_per_entry, flag);
     if (rc != VS_OK) return rc;
     const int64_t items = (int64_t)p.batch * n_tiles * m_tiles;
     const unsigned grid = (unsigned)(items < d->sm_count ? items : d->sm_count);   // one persistent CTA per SM
@@ -677,7 +727,7 @@ bool sddmm_use_dense(const SddmmParams &p, int V) {
     const char *e = std::getenv("VSPARSE_B200_SDDMM");
     if (e && !std::strcmp(e, "dense")) return true;
     if (e && !std::strcmp(e, "gather")) return false;
-    const double k_blocks = (double)(p.k / densesddmm::kBlockK);
+    const double k_blocks = std::ceil((double)p.k / densesddmm::kBlockK);
     const double tiles = std::ceil((double)p.m_vec * V / 256.0) * std::ceil((double)p.n / 256.0);
     const double gather = (double)p.m_vec * 306.0 * k_blocks + (double)p.nnz_vec * 4.0;
     const double dense = tiles * std::max(2230.0 * k_blocks, 4250.0);
@@ -754,10 +804,54 @@ template <typename TOut, int V> bool launch_sddmm_pair(const SddmmParams &p, cud
     return true;
 }
 
+// Small problems in one kernel (sddmm_direct.cuh); false if this call or this device cannot take it.
+template <typename TOut, int V> bool launch_sddmm_direct(const SddmmParams &p, cudaStream_t s, DeviceInfo *d, int *rc_out) {
+    const int m_tiles = (int)(((int64_t)p.m_vec * V + directsddmm::kTileM - 1) / directsddmm::kTileM);
+    // 64-column tiles while 128-column ones would leave SMs without a tile
+    const int tn = (int64_t)p.batch * m_tiles * ((p.n + 127) / 128) >= d->sm_count ? 128 : 64;
+    const int n_tiles = (p.n + tn - 1) / tn;
+    const int64_t tiles = (int64_t)p.batch * m_tiles * n_tiles;
+    if (tiles > 0x7fffffffll || p.n <= 0 || p.k <= 0 || p.k % 8 != 0) return false;
+    CUtensorMap map_l, map_r;
+    static DeviceBits smem_set;
+    auto kernel = directsddmm::sddmm_direct_kernel<TOut, V>;
+    if (make_tile_map(&map_l, p.lhs, false, (uint64_t)p.m_vec * V, (uint64_t)p.k, (uint64_t)p.batch, (uint64_t)p.stride_lhs, 64,
+                      directsddmm::kTileM) != VS_OK ||
+        make_tile_map(&map_r, p.rhs, false, (uint64_t)p.n, (uint64_t)p.k, (uint64_t)p.batch, (uint64_t)p.stride_rhs, 64, (uint32_t)tn) != VS_OK ||
+        set_smem_once(kernel, directsddmm::kSmemBytes, smem_set) != VS_OK)
+        return false;
+    *rc_out = (int)launch_overlapped(kernel, (unsigned)tiles, directsddmm::kThreads, directsddmm::kSmemBytes, s, p, map_l, map_r, tn, m_tiles,
+                                     n_tiles, d->status);
+    return true;
+}
+// Which sampled products are small, from the time each form takes (us, fitted to B200 at V = 2 and 8, 64 to 4096 rows and
+// columns, contraction lengths 64 to 1984, batches of 1 to 32).  Direct: waves of 128 x 128 tiles at two per SM, each paying
+// for its contraction and for looking at every entry of its rows.  Planned: the launches, the plan of 32 vector-rows per
+// CTA, the dense tiles; or the gather kernel by the costs sddmm_use_dense() knows.  lhs 512 x 256, rhs 2048 x 256, V = 4:
+// 17.0 -> 7.8 us; 2048 x 512 x 256, V = 8, 90 % sparse: one 11.1 -> 5.1, eight 14.4 -> 10.2, sixteen 18.9 -> 18.4.
+bool sddmm_direct_wanted(const SddmmParams &p, int V, const DeviceInfo *d) {
+    const char *e = std::getenv("VSPARSE_B200_SDDMM");   // "dense" and "gather" force those, "direct" this one
+    if (e) return !std::strcmp(e, "direct");
+    if (p.m_vec <= 0 || p.n <= 0) return true;
+    const double cycles_per_us = 1900.0 * d->sm_count;
+    const double k_blocks = std::ceil(p.k / 64.0), per_row = (double)p.nnz_vec / p.m_vec;
+    const double tiles = std::ceil((double)p.m_vec * V / 128.0) * std::ceil(p.n / 128.0) * p.batch;
+    const double direct = 2.0 + std::max(1.0, tiles / (2.0 * d->sm_count)) * (1.5 + 0.3 * k_blocks + 0.14 * (128.0 / V) * per_row / 256.0);
+    double planned;
+    if (sddmm_use_dense(p, V)) {
+        const double dense_tiles = std::ceil((double)p.m_vec * V / 256.0) * std::ceil(p.n / 256.0) * p.batch;
+        planned = 8.0 + 1.1e-3 * 32.0 * per_row + dense_tiles * std::max(2230.0 * k_blocks, 4250.0) / cycles_per_us;
+    } else {
+        planned = 4.5 + ((double)p.m_vec * 306.0 * k_blocks + (double)p.nnz_vec * 4.0) * p.batch / cycles_per_us;
+    }
+    return direct < planned;
+}
+
 template <typename TOut, int V> int launch_sddmm_tc(const SddmmParams &p, cudaStream_t s) {
     DeviceInfo *d;
     int rc = device_info(&d);
     if (rc != VS_OK) return rc;
+    if (sddmm_direct_wanted(p, V, d) && launch_sddmm_direct<TOut, V>(p, s, d, &rc)) return rc;
     const int chunks = (p.n + densesddmm::kChunk - 1) / densesddmm::kChunk;
     int64_t offsets_bytes = 0;
     const int64_t plan_bytes = sddmm_plan_bytes(p.m_vec, p.n, p.nnz_vec, &offsets_bytes);
