@@ -110,9 +110,11 @@ def kernels_per_step(w, a=None):
             return ["spmm_tma_kernel"]
         return ["dense_plan_kernel", dense,
                 "spmm_tma_kernel (returns at once unless the plan kernel chose it)"]
-    if w["op"] == "spmm":
-        return ["spmm_cc_kernel"]
-    if not tensor:
+    if w["op"] == "spmm":   # the CUDA-core entry point: fp16 results come from the tensor cores where that is quicker
+        if w.get("dtype") == "f32" or os.environ.get("VSPARSE_B200_SPMM") == "gather":
+            return ["spmm_cc_kernel"]
+        return ["dense_plan_kernel", dense, "spmm_cc_standby_kernel (returns at once unless the plan kernel chose it)"]
+    if not tensor and os.environ.get("VSPARSE_B200_SDDMM") == "gather":
         # a group of lanes per vector-row while the contraction length fits 32 chunks of 16 bytes, per mask entry beyond
         by_row = w["N"] // 8 <= 32 and os.environ.get("VSPARSE_B200_SDDMM_CC") != "entry"
         return ["sddmm_cc_row_kernel" if by_row else "sddmm_cc_kernel"]

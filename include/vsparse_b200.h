@@ -32,7 +32,10 @@ extern "C" {
 #define VS_F16 0
 #define VS_F32 1
 
-/* kernel families: the reference's wmma* entry points map to TENSOR, its cuda* entry points to CUDA_CORE */
+/* kernel families: the reference's wmma* entry points map to TENSOR, its cuda* entry points to CUDA_CORE.  CUDA_CORE takes what
+ * the cuda* entry points take (V = 1, widths that are multiples of 8 or 4, fp32); its products of fp16 operands with fp16
+ * results are computed on the tensor cores where that is quicker (exact products, fp32 sums in another order, one rounding to
+ * fp16), everything else on CUDA cores. */
 #define VS_PATH_TENSOR 0
 #define VS_PATH_CUDA_CORE 1
 

@@ -7,7 +7,7 @@ import torch
 import oracle
 from conftest import assert_close
 from gpu_util import DEV, custom, dev, problem, spmm_oracle, structure
-from vectorsparse_b200 import VS_PATH_TENSOR, cvse, ops
+from vectorsparse_b200 import VS_PATH_CUDA_CORE, VS_PATH_TENSOR, cvse, ops
 
 pytestmark = pytest.mark.gpu
 
@@ -83,3 +83,41 @@ def test_direct_sddmm_at_the_edges_of_its_tiles(monkeypatch, V, m_vec, n, k, len
     want = oracle.sddmm(m_vec, k, V, a.row_offsets, a.col_indices, lhs.astype(np.float32), rhs.astype(np.float32), acc="f64")
     assert_close(out[:a.nnz_vec * V].float().cpu().numpy(), want, "direct")
     assert torch.isnan(out[a.nnz_vec * V:]).all()
+
+
+@pytest.mark.parametrize("mode", ["direct", "dense", "gather"])
+@pytest.mark.parametrize("V,m_vec,K,N", [(1, 130, 200, 72), (2, 70, 129, 136), (4, 40, 300, 8), (8, 33, 64, 264)])
+def test_cuda_core_spmm_with_fp16_results_in_every_form(monkeypatch, mode, V, m_vec, K, N):
+    """The entry point that takes V = 1 and dense widths that are multiples of 8: its one-kernel form, its planned form (widths of
+    both multiplying kernels) and the CUDA-core kernel; a column named twice on top of each."""
+    monkeypatch.setenv("VSPARSE_B200_SPMM", mode)
+    a = problem(cvse.GEN_BETA, 8, m_vec, K, V, 0.7)
+    for repeat in (False, True):
+        if repeat:
+            j = int(a.row_offsets[np.argmax(np.diff(a.row_offsets))])
+            a.col_indices[j + 1] = a.col_indices[j]
+        vals = cvse.fill_random((a.nnz_vec * V,), np.float16, cvse.DIST_NORMAL, 1, 0.25)
+        B = cvse.fill_random((K, N), np.float16, cvse.DIST_NORMAL, 2, 0.5)
+        out = torch.full((a.m, N), float("nan"), dtype=torch.float16, device=DEV)
+        ops.spmm.cudaSpmm(m_vec, V, N, K, *structure(a), dev(vals), dev(B), out)
+        torch.cuda.synchronize()
+        assert ops.device_status() == 0
+        assert_close(out.float().cpu().numpy(), spmm_oracle(a, N, vals, B), f"{mode}, repeated column: {repeat}")
+
+
+@pytest.mark.parametrize("mode", ["direct", "dense", "gather"])
+@pytest.mark.parametrize("V,m_vec,n,k", [(1, 130, 130, 8), (2, 70, 257, 72), (4, 33, 100, 200), (8, 40, 300, 456)])
+def test_cuda_core_sddmm_with_fp16_results_in_every_form(monkeypatch, mode, V, m_vec, n, k):
+    """Contraction lengths that are multiples of 8 and not of 64: the last block of the tiles is filled up with zeros."""
+    monkeypatch.setenv("VSPARSE_B200_SDDMM", mode)
+    a = problem(cvse.GEN_BETA, 8, m_vec, n, V, 0.7)
+    lhs = cvse.fill_random((2, a.m, k), np.float16, cvse.DIST_NORMAL, 3, 0.25)
+    rhs = cvse.fill_random((2, n, k), np.float16, cvse.DIST_NORMAL, 4, 0.25)
+    row = (a.nnz_vec * V + 7) // 8 * 8
+    out = torch.full((2, row), float("nan"), dtype=torch.float16, device=DEV)
+    ops.sddmm_batched(VS_PATH_CUDA_CORE, m_vec, k, n, a.nnz_vec, *structure(a), dev(lhs), dev(rhs), out, V)
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    for b in range(2):
+        want = oracle.sddmm(m_vec, k, V, a.row_offsets, a.col_indices, lhs[b].astype(np.float32), rhs[b].astype(np.float32), acc="f64")
+        assert_close(out[b, :a.nnz_vec * V].float().cpu().numpy(), want, f"{mode}, entry {b}")

@@ -19,18 +19,15 @@ constexpr int kCcThreads = 128;
 // flight.  With two or four chunks per thread the warp-uniform loads of an entry (column index, value vector) feed
 // that many times the FMAs; it needs the dense width to be a multiple of 32 kChunks chunks.
 template <typename TIn, typename TOut, int V, int kChunks>
-__global__ void __launch_bounds__(kCcThreads) spmm_cc_kernel(const SpmmParams p) {
+__device__ __forceinline__ void spmm_cc_item(const SpmmParams &p, int b, int64_t item) {
     constexpr int E = Chunk<TIn>::kElems;
     constexpr int U = kChunks == 1 ? 4 : (kChunks == 2 ? 2 : 1);
     const int chunks = p.N / (E * kChunks);            // items per vector-row
-    const int64_t item = (int64_t)blockIdx.x * kCcThreads + threadIdx.x;
-    if (item >= (int64_t)p.m_vec * chunks) return;
     const int order = (int)(item / chunks);
     const int piece = (int)(item - (int64_t)order * chunks);
     // kChunks > 1: warp-sized groups of items take chunks 32 kChunks g + lane, + 32 + lane, ...
     const int chunk = kChunks == 1 ? piece : (piece / 32) * (32 * kChunks) + (piece % 32);
     const int row = __ldg(p.row_indices + order);
-    const int b = blockIdx.y;
 
     const TIn *values = static_cast<const TIn *>(p.values) + (int64_t)b * p.stride_values;
     const TIn *rhs = static_cast<const TIn *>(p.rhs) + (int64_t)b * p.stride_rhs + (int64_t)chunk * E;
@@ -87,6 +84,25 @@ __global__ void __launch_bounds__(kCcThreads) spmm_cc_kernel(const SpmmParams p)
     for (int q = 0; q < kChunks; ++q)
 #pragma unroll
         for (int v = 0; v < V; ++v) store_chunk(out + ((int64_t)row * V + v) * p.N + q * 32 * E, acc[q][v]);
+}
+
+template <typename TIn, typename TOut, int V, int kChunks>
+__global__ void __launch_bounds__(kCcThreads) spmm_cc_kernel(const SpmmParams p) {
+    const int64_t item = (int64_t)blockIdx.x * kCcThreads + threadIdx.x;
+    if (item < (int64_t)p.m_vec * (p.N / (Chunk<TIn>::kElems * kChunks))) spmm_cc_item<TIn, TOut, V, kChunks>(p, blockIdx.y, item);
+}
+
+// The same work enqueued behind a densifying kernel that usually has taken the call: returns at once unless the plan
+// header says otherwise, and walks its items in strides, because a grid of one thread per item takes longer to start and
+// return than the rest of a small call.
+template <typename TIn, typename TOut, int V>
+__global__ void __launch_bounds__(kCcThreads) spmm_cc_standby_kernel(const SpmmParams p, const int32_t *plan_hdr, int plan_checks) {
+    pdl_launch_dependents();
+    pdl_wait();
+    if (plan_dense_chosen(plan_hdr, plan_checks)) return;
+    const int64_t per = (int64_t)p.m_vec * (p.N / Chunk<TIn>::kElems), total = per * p.batch;
+    for (int64_t i = (int64_t)blockIdx.x * kCcThreads + threadIdx.x; i < total; i += (int64_t)gridDim.x * kCcThreads)
+        spmm_cc_item<TIn, TOut, V, 1>(p, (int)(i / per), i % per);
 }
 
 // ---- SDDMM --------------------------------------------------------------------------------------------------

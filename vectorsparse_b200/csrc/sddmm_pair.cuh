@@ -286,7 +286,7 @@ sddmm_pair_kernel(const SddmmParams p, const __grid_constant__ CUtensorMap map_l
 
     pdl_launch_dependents();
     pdl_wait();   // the set-up above may have run beside the plan kernel; its cells are read from here on
-    const int k_blocks = p.k / kBlockK;
+    const int k_blocks = (p.k + kBlockK - 1) / kBlockK;   // the last one may be filled up with zeros by TMA
     const int64_t total_items = (int64_t)p.batch * n_tiles * m_tiles;
     // this pair's items: a contiguous run with a resident rhs, every pairs-th item otherwise
     const int64_t item0 = resident ? total_items * pair / pairs : (int64_t)pair;

@@ -119,14 +119,14 @@ static_assert(kBStages == kAStages || kBStages == 2 * kAStages,
 // never straddle a 16-column block (V divides 16).  The entry keeps the vector's first column and its index in the caller's
 // `values` array (t_src), so the multiplying kernel reads the values where the forward operators keep them and
 // drops the V of them side by side into one row of its tile.  Groups are 128 rows of A^T.
-// Costs: `gather_per_row`, `gather_per_entry` for the kernel that takes the call otherwise, `dense_per_entry` for
+// Costs: `dense_per_stage` for the multiplying kernel; `gather_per_row`, `gather_per_entry` for the kernel that takes the call otherwise, `dense_per_entry` for
 // the fill work of the dense kernel where that matters (V stores per vector instead of one).
 template <bool kTransposed>
 __global__ void __launch_bounds__(kPlanThreads)
 dense_plan_kernel(const int32_t *__restrict__ row_offsets, const int32_t *__restrict__ cols, const int32_t *__restrict__ src,
                   int shift, int m_vec, int K, int groups, int rows_per_group, int plan_blocks,
                   int32_t *__restrict__ blk_offsets, uint2 *__restrict__ blk_entries, int64_t entry_capacity, int force_dense,
-                  float gather_per_row, float gather_per_entry, float dense_per_entry, int32_t *use_dense) {
+                  float dense_per_stage, float gather_per_row, float gather_per_entry, float dense_per_entry, int32_t *use_dense) {
     auto offset_of = [&](int i) { return __ldg(row_offsets + i); };
     auto column_of = [&](int j) { return kTransposed ? __ldg(cols + j) << shift : __ldg(cols + j); };
     auto value_of = [&](int j) { return kTransposed ? __ldg(src + j) : j; };
@@ -136,7 +136,7 @@ dense_plan_kernel(const int32_t *__restrict__ row_offsets, const int32_t *__rest
     {
         const int64_t nnz = __ldg(row_offsets + m_vec);
         const float stages = (float)(groups / (kTileM / kGroupRows)) * (float)(plan_blocks / (kBlockK / kPlanCols));
-        const float dense_cost = stages * 1100.0f + dense_per_entry * (float)nnz;
+        const float dense_cost = stages * dense_per_stage + dense_per_entry * (float)nnz;
         const float gather_cost = (float)m_vec * gather_per_row + gather_per_entry * (float)nnz;
         const bool dense = nnz <= entry_capacity && (force_dense || dense_cost < gather_cost);
         if (blockIdx.x == 0 && threadIdx.x == 0) *use_dense = dense ? 1 : 0;

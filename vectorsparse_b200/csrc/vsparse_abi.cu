@@ -352,6 +352,12 @@ template <typename TIn, typename TOut> int spmm_cc_by_v(int V, const SpmmParams 
     }
     return VS_ERR_VEC_LENGTH;
 }
+template <typename TOut, int V> int launch_spmm_cc_standby(const SpmmParams &p, cudaStream_t s, DeviceInfo *d, const int32_t *plan_hdr, int plan_checks) {
+    const int64_t blocks = ((int64_t)p.m_vec * (p.N / Chunk<__half>::kElems) * p.batch + kCcThreads - 1) / kCcThreads;
+    const int64_t cap = (int64_t)d->sm_count * 8;
+    return (int)launch_overlapped(spmm_cc_standby_kernel<__half, TOut, V>, (unsigned)(blocks < cap ? blocks : cap), kCcThreads, 0, s, p, plan_hdr,
+                                  plan_checks);
+}
 
 // Software (cp.async) gather: works for any batch stride.
 template <typename TOut, int V>
@@ -522,18 +528,35 @@ struct SpmmCosts {
     float dense_per_stage, dense_per_entry, gather_per_row, gather_per_entry;
 };
 constexpr SpmmCosts kGatherCosts = {1100.0f, 0.0f, 370.0f, 4.7f};
+// The same with the CUDA-core kernel as the other formulation.
+constexpr SpmmCosts cores_costs(int V) {
+    return {700.0f, V == 1 ? 1.0f : V == 2 ? 0.5f : 0.0f, 100.0f, V == 1 ? 5.2f : V == 2 ? 8.0f : V == 4 ? 13.0f : 20.0f};
+}
+
+// What takes a call that the densified product does not: the gather kernels (wmmaSpmm) or the CUDA-core kernel (cudaSpmm
+// with fp16 results).  With a plan header: as a stand-by behind a densifying kernel.
+template <typename TOut, int V, bool kCores>
+int launch_spmm_other(const SpmmParams &p, cudaStream_t s, DeviceInfo *d, const int32_t *plan_hdr, int plan_checks) {
+    if constexpr (kCores) {
+        return plan_hdr ? launch_spmm_cc_standby<TOut, V>(p, s, d, plan_hdr, plan_checks) : launch_spmm_cc<__half, TOut, V>(p, s);
+    } else {
+        return launch_spmm_gather<TOut, V>(p, s, d, plan_hdr, plan_checks);
+    }
+}
 
 // Small products in one kernel (spmm_direct.cuh); false if this call or this device cannot take it.  When the densified
 // product is the cheaper one whatever the number of nonzeros, nothing else is enqueued; otherwise the kernel leaves its
 // verdict where the gather kernel behind it looks for the plan kernel's.
-template <typename TOut, int V> bool launch_spmm_direct(const SpmmParams &p, cudaStream_t s, DeviceInfo *d, const SpmmCosts &cost,
-                                                        bool forced, int *rc_out) {
+template <typename TOut, int V, bool kCores> bool launch_spmm_direct(const SpmmParams &p, cudaStream_t s, DeviceInfo *d, const SpmmCosts &cost,
+                                                                     bool forced, int *rc_out) {
     const int m_tiles = (int)(((int64_t)p.m_vec * V + directspmm::kTileM - 1) / directspmm::kTileM);
     const int n_tiles = (p.N + directspmm::kTileN - 1) / directspmm::kTileN;
     const int64_t tiles = (int64_t)p.batch * m_tiles * n_tiles;
     if (tiles > 0x7fffffffll || p.K <= 0 || p.N % 8 != 0) return false;
     const float stages = std::ceil((float)p.m_vec * V / densespmm::kTileM) * std::ceil((float)p.K / densespmm::kBlockK);
-    const bool always = forced || (cost.dense_per_entry == 0.0f && cost.dense_per_stage * stages < cost.gather_per_row * (float)p.m_vec);
+    // (against the CUDA-core kernel it is the quicker form of a small product down to ~5 % of the vectors: a stand-by behind
+    // every call would cost more than it saves on the few below)
+    const bool always = forced || kCores || (cost.dense_per_entry == 0.0f && cost.dense_per_stage * stages < cost.gather_per_row * (float)p.m_vec);
     CUtensorMap map;
     static DeviceBits smem_set;
     auto kernel = directspmm::spmm_direct_kernel<TOut, V>;
@@ -545,28 +568,29 @@ template <typename TOut, int V> bool launch_spmm_direct(const SpmmParams &p, cud
     *rc_out = (int)launch_overlapped(kernel, (unsigned)tiles, directspmm::kThreads, directspmm::kSmemBytes, s, p, map, m_tiles, n_tiles,
                                      cost.dense_per_stage * stages, cost.dense_per_entry, cost.gather_per_row, cost.gather_per_entry,
                                      static_cast<int32_t *>(verdict), d->status);
-    if (*rc_out == VS_OK && !always) *rc_out = launch_spmm_gather<TOut, V>(p, s, d, static_cast<const int32_t *>(verdict), 0);
+    if (*rc_out == VS_OK && !always) *rc_out = launch_spmm_other<TOut, V, kCores>(p, s, d, static_cast<const int32_t *>(verdict), 0);
     return true;
 }
 // Which products are small: up to one wave of 128 x 64 tiles at two per SM the one-kernel form saves the ~9 us of the other
-// launches and loses nothing (2048 x 512 x 256, V = 8: 15.4 -> 6.5 us; 512 x 2048 x 256: 22.3 -> 13.3), up to two waves while
-// K is short.  Shorter vectors mean more entries per tile, which it scatters again for every 64 columns of B, so there
-// the line lies at a smaller K (V = 2, 1024 x 1024 x 256, four of them: 26.6 -> 24.6; 4096 x 4608 x 256: 74 -> 88).
+// launches (2048 x 512 x 256, V = 8: 15.4 -> 6.5 us; 512 x 2048 x 256: 22.3 -> 13.3), up to two waves while K is short.  Shorter
+// vectors mean more entries per tile, which it scatters again for every 64 columns of B, so there the line lies at a smaller
+// K (V = 2, 2048 x 2048 x 256, 60 and 95 % sparse: 85 -> 68 and 28 -> 30; 4096 x 4608 x 256, 85 % sparse: 74 -> 88).
 bool spmm_direct_wanted(const SpmmParams &p, int V, const DeviceInfo *d) {
     const int64_t m_tiles = ((int64_t)p.m_vec * V + directspmm::kTileM - 1) / directspmm::kTileM;
     const int64_t tiles = m_tiles * ((p.N + directspmm::kTileN - 1) / directspmm::kTileN) * p.batch;
     const int chunks = (p.K + directspmm::kChunkK - 1) / directspmm::kChunkK;
-    if (tiles <= 2 * d->sm_count) return chunks <= (V == 8 ? 64 : V == 4 ? 16 : V == 2 ? 8 : 4);
-    return tiles <= 4 * d->sm_count && chunks <= (V == 8 ? 4 : V == 4 ? 2 : 1);
+    if (tiles <= 2 * d->sm_count) return chunks <= (V == 8 ? 64 : V == 4 ? 32 : 16);
+    return tiles <= 4 * d->sm_count && chunks <= (V >= 4 ? 4 : 1);
 }
 
-template <typename TOut, int V> int launch_spmm_tc(const SpmmParams &p, cudaStream_t s) {
+template <typename TOut, int V, bool kCores> int launch_spmm_tc(const SpmmParams &p, cudaStream_t s) {
     DeviceInfo *d;
     int rc = device_info(&d);
     if (rc != VS_OK) return rc;
     const SpmmMode mode = spmm_mode();
+    constexpr SpmmCosts cost = kCores ? cores_costs(V) : kGatherCosts;
     if ((mode == SpmmMode::kDirect || (mode == SpmmMode::kAuto && spmm_direct_wanted(p, V, d))) &&
-        launch_spmm_direct<TOut, V>(p, s, d, kGatherCosts, mode == SpmmMode::kDirect, &rc))
+        launch_spmm_direct<TOut, V, kCores>(p, s, d, cost, mode == SpmmMode::kDirect, &rc))
         return rc;
     const int k_blocks = (p.K + densespmm::kBlockK - 1) / densespmm::kBlockK;
     const int m_tiles = (p.m_vec * V + densespmm::kTileM - 1) / densespmm::kTileM;
@@ -582,14 +606,14 @@ template <typename TOut, int V> int launch_spmm_tc(const SpmmParams &p, cudaStre
     const bool dense_ok = !t_no_scratch && mode != SpmmMode::kGather && p.K > 0 && p.m_vec > 0 && p.N % 8 == 0 && plan_bytes <= kMaxPlanBytes &&
                           plan_smem <= 40 * 1024 && (p.batch == 1 || (p.stride_rhs * 2) % 16 == 0) &&
                           (p.batch == 1 || (p.stride_out * sizeof(TOut)) % 16 == 0) && aligned16(p.rhs) && aligned16(p.out);
-    if (!dense_ok) return launch_spmm_gather<TOut, V>(p, s, d, nullptr, 0);
+    if (!dense_ok) return launch_spmm_other<TOut, V, kCores>(p, s, d, nullptr, 0);
 
     constexpr bool kOutF32 = sizeof(TOut) == 4;
     CUtensorMap map, map_out;
     if (make_tile_map(&map, p.rhs, false, (uint64_t)p.K, (uint64_t)p.N, (uint64_t)p.batch, (uint64_t)p.stride_rhs, 64, 64) != VS_OK ||
         make_tile_map(&map_out, p.out, kOutF32, (uint64_t)p.m_vec * V, (uint64_t)p.N, (uint64_t)p.batch,
                       (uint64_t)p.stride_out, densespmm::kStoreCols, 32) != VS_OK)
-        return launch_spmm_gather<TOut, V>(p, s, d, nullptr, 0);
+        return launch_spmm_other<TOut, V, kCores>(p, s, d, nullptr, 0);
     CUtensorMap map_b4 = map;
     const int use_b4 = (p.N % 64 == 0 && make_blocked_map(&map_b4, p.rhs, (uint64_t)p.K, (uint64_t)p.N, (uint64_t)p.batch,
                                                           (uint64_t)p.stride_rhs, densespmm::kTileN / 64) == VS_OK) ? 1 : 0;
@@ -599,7 +623,7 @@ template <typename TOut, int V> int launch_spmm_tc(const SpmmParams &p, cudaStre
     if (rc != VS_OK) return rc;
     uint8_t *plan = nullptr;
     if (stream_scratch(d, s, (size_t)plan_bytes, reinterpret_cast<void **>(&plan)) != VS_OK)
-        return launch_spmm_gather<TOut, V>(p, s, d, nullptr, 0);
+        return launch_spmm_other<TOut, V, kCores>(p, s, d, nullptr, 0);
     int32_t *flag = reinterpret_cast<int32_t *>(plan);
     const int64_t header_bytes = spmm_plan_header_bytes(checks);
     int32_t *blk_offsets = reinterpret_cast<int32_t *>(plan + header_bytes);
@@ -608,8 +632,8 @@ template <typename TOut, int V> int launch_spmm_tc(const SpmmParams &p, cudaStre
     // a dependent launch as well: in a stream of calls the plan kernel queues up behind the previous call's last kernel
     rc = (int)launch_overlapped(densespmm::dense_plan_kernel<false>, (unsigned)(groups + checks), densespmm::kPlanThreads, plan_smem, s,
                                 p.row_offsets, p.col_indices, (const int32_t *)nullptr, 0, p.m_vec, p.K, groups, rows_per_group,
-                                plan_blocks, blk_offsets, blk_entries, capacity, force_dense, kGatherCosts.gather_per_row,
-                                kGatherCosts.gather_per_entry, kGatherCosts.dense_per_entry, flag);
+                                plan_blocks, blk_offsets, blk_entries, capacity, force_dense, cost.dense_per_stage,
+                                cost.gather_per_row, cost.gather_per_entry, cost.dense_per_entry, flag);
     if (rc != VS_OK) return rc;
     const int64_t items = (int64_t)p.batch * n_tiles * m_tiles;
     const unsigned grid = (unsigned)(items < d->sm_count ? items : d->sm_count);   // one persistent CTA per SM
@@ -623,15 +647,28 @@ template <typename TOut, int V> int launch_spmm_tc(const SpmmParams &p, cudaStre
             rc = (int)launch_overlapped(kernel, grid, densespmm::kThreads, densespmm::kSmemBytes, s, p, map, map_out, map_b4, use_b4,
                                         blk_offsets, blk_entries, m_tiles, n_tiles, k_blocks, d->status, flag, checks);
     }
-    if (rc == VS_OK) rc = launch_spmm_gather<TOut, V>(p, s, d, flag, checks);
+    if (rc == VS_OK) rc = launch_spmm_other<TOut, V, kCores>(p, s, d, flag, checks);
     return rc;
 }
 
 template <typename TOut> int spmm_tc_by_v(int V, const SpmmParams &p, cudaStream_t s) {
     switch (V) {
-        case 2: return launch_spmm_tc<TOut, 2>(p, s);
-        case 4: return launch_spmm_tc<TOut, 4>(p, s);
-        case 8: return launch_spmm_tc<TOut, 8>(p, s);
+        case 2: return launch_spmm_tc<TOut, 2, false>(p, s);
+        case 4: return launch_spmm_tc<TOut, 4, false>(p, s);
+        case 8: return launch_spmm_tc<TOut, 8, false>(p, s);
+    }
+    return VS_ERR_VEC_LENGTH;
+}
+// cudaSpmm with fp16 operands and results.  The results are rounded to fp16 (2^-11 of their size), so the fp32 sums may be taken
+// in any order and on the tensor cores, whose products of fp16 values are exact and whose sums are fp32 too; what the densified
+// product cannot do (repeated columns, non-finite values, few nonzeros) stays with the CUDA-core kernel.  fp32 results keep it
+// throughout: there the order of the sums shows.  VSPARSE_B200_SPMM=gather forces the CUDA-core kernel.
+int spmm_cores_by_v(int V, const SpmmParams &p, cudaStream_t s) {
+    switch (V) {
+        case 1: return launch_spmm_tc<__half, 1, true>(p, s);
+        case 2: return launch_spmm_tc<__half, 2, true>(p, s);
+        case 4: return launch_spmm_tc<__half, 4, true>(p, s);
+        case 8: return launch_spmm_tc<__half, 8, true>(p, s);
     }
     return VS_ERR_VEC_LENGTH;
 }
@@ -792,7 +829,7 @@ template <typename TOut, int V> bool launch_sddmm_pair(const SddmmParams &p, cud
         const unsigned pairs = (unsigned)(items < resident[dev] ? items : resident[dev]);
         // rhs of a batch entry fits the resident slots (VSPARSE_B200_SDDMM_RESIDENT=0: stream both operands anyway)
         const char *res_env = std::getenv("VSPARSE_B200_SDDMM_RESIDENT");
-        const int resident = (n_tiles * (p.k / densesddmm::kBlockK) <= pairsddmm::kMaxResident && !(res_env && !std::strcmp(res_env, "0"))) ? 1 : 0;
+        const int resident = (n_tiles * ((p.k + densesddmm::kBlockK - 1) / densesddmm::kBlockK) <= pairsddmm::kMaxResident && !(res_env && !std::strcmp(res_env, "0"))) ? 1 : 0;
         TimedLaunch timed(s);
         rc = (int)launch_pairs(kernel, pairs, pairsddmm::kThreads, (size_t)pairsddmm::kSmemBytes, s, true, p, map_l, map_r, cells, order,
                                blocks, m_tiles, n_tiles, resident, d->status);
@@ -824,27 +861,33 @@ template <typename TOut, int V> bool launch_sddmm_direct(const SddmmParams &p, c
                                      n_tiles, d->status);
     return true;
 }
-// Which sampled products are small, from the time each form takes (us, fitted to B200 at V = 2 and 8, 64 to 4096 rows and
-// columns, contraction lengths 64 to 1984, batches of 1 to 32).  Direct: waves of 128 x 128 tiles at two per SM, each paying
-// for its contraction and for looking at every entry of its rows.  Planned: the launches, the plan of 32 vector-rows per
-// CTA, the dense tiles; or the gather kernel by the costs sddmm_use_dense() knows.  lhs 512 x 256, rhs 2048 x 256, V = 4:
-// 17.0 -> 7.8 us; 2048 x 512 x 256, V = 8, 90 % sparse: one 11.1 -> 5.1, eight 14.4 -> 10.2, sixteen 18.9 -> 18.4.
-bool sddmm_direct_wanted(const SddmmParams &p, int V, const DeviceInfo *d) {
-    const char *e = std::getenv("VSPARSE_B200_SDDMM");   // "dense" and "gather" force those, "direct" this one
-    if (e) return !std::strcmp(e, "direct");
-    if (p.m_vec <= 0 || p.n <= 0) return true;
+// Time each form of a sampled product takes (us, fitted to B200 at V = 1 to 8, 64 to 4096 rows and columns, contraction
+// lengths 64 to 1984, batches of 1 to 64).  Direct: waves of 128 x 128 tiles at two per SM, each paying for its contraction
+// (three times as much per block once both CTAs of an SM draw on L2) and for looking at every entry of its rows.  Dense:
+// the launches, the plan of 32 vector-rows per CTA, the tiles.  Gather: by the costs sddmm_use_dense() knows.
+struct SddmmTimes {
+    double direct, dense, gather;
+};
+SddmmTimes sddmm_times(const SddmmParams &p, int V, const DeviceInfo *d) {
     const double cycles_per_us = 1900.0 * d->sm_count;
-    const double k_blocks = std::ceil(p.k / 64.0), per_row = (double)p.nnz_vec / p.m_vec;
+    const double k_blocks = std::ceil(p.k / 64.0), per_row = (double)p.nnz_vec / std::max(p.m_vec, 1);
     const double tiles = std::ceil((double)p.m_vec * V / 128.0) * std::ceil(p.n / 128.0) * p.batch;
-    const double direct = 2.0 + std::max(1.0, tiles / (2.0 * d->sm_count)) * (1.5 + 0.3 * k_blocks + 0.14 * (128.0 / V) * per_row / 256.0);
-    double planned;
-    if (sddmm_use_dense(p, V)) {
-        const double dense_tiles = std::ceil((double)p.m_vec * V / 256.0) * std::ceil(p.n / 256.0) * p.batch;
-        planned = 8.0 + 1.1e-3 * 32.0 * per_row + dense_tiles * std::max(2230.0 * k_blocks, 4250.0) / cycles_per_us;
-    } else {
-        planned = 4.5 + ((double)p.m_vec * 306.0 * k_blocks + (double)p.nnz_vec * 4.0) * p.batch / cycles_per_us;
-    }
-    return direct < planned;
+    const double dense_tiles = std::ceil((double)p.m_vec * V / 256.0) * std::ceil(p.n / 256.0) * p.batch;
+    const double shared = std::min(1.0, std::max(0.0, tiles / d->sm_count - 1.0));
+    SddmmTimes t;
+    t.direct = 2.0 + std::max(1.0, tiles / (2.0 * d->sm_count)) * (1.5 + (0.3 + 0.6 * shared) * k_blocks + 0.14 * (128.0 / V) * per_row / 256.0);
+    t.dense = 8.0 + 1.1e-3 * 32.0 * per_row + dense_tiles * std::max(2230.0 * k_blocks, 4250.0) / cycles_per_us;
+    t.gather = 4.5 + ((double)p.m_vec * 306.0 * k_blocks + (double)p.nnz_vec * 4.0) * p.batch / cycles_per_us;
+    return t;
+}
+// Small sampled products go to the one-kernel form.  lhs 512 x 256, rhs 2048 x 256, V = 4: 17.0 -> 7.8 us; 2048 x 512 x 256, V = 8,
+// 90 % sparse: one 11.1 -> 5.1, eight 14.4 -> 10.2, sixteen 18.9 -> 18.4.  VSPARSE_B200_SDDMM = "dense" and "gather" force those,
+// "direct" this one.
+bool sddmm_direct_wanted(const SddmmParams &p, int V, const DeviceInfo *d) {
+    const char *e = std::getenv("VSPARSE_B200_SDDMM");
+    if (e) return !std::strcmp(e, "direct");
+    const SddmmTimes t = sddmm_times(p, V, d);
+    return t.direct < (sddmm_use_dense(p, V) ? t.dense : t.gather);
 }
 
 template <typename TOut, int V> int launch_sddmm_tc(const SddmmParams &p, cudaStream_t s) {
@@ -887,6 +930,38 @@ template <typename TOut, int V> int launch_sddmm_tc(const SddmmParams &p, cudaSt
     if (rc != VS_OK) return rc;
     return (int)launch_overlapped(kernel, grid, densesddmm::kThreads, densesddmm::kSmemBytes, s, p, map_l, map_r, chunk_offsets,
                                   chunk_entries, m_tiles, n_tiles, chunks, d->status);
+}
+
+// cudaSddmm with fp16 results: on the tensor cores like cudaSpmm's (spmm_cores_by_v), any contraction length that is a
+// multiple of 8 (the tiles' last block is filled up with zeros by TMA).  The CUDA-core kernel, a group of lanes per
+// vector-row, is never the quicker one (64 x 64 to 4096 x 2048, 60 and 95 % sparse: by 1.1 to 19 times at V > 1, 0.95 to 4.7
+// at V = 1, where only the one-kernel form exists); it takes the strides that tensor maps cannot address.
+// 159 x 577, 115 entries per row, k = 200, V = 8, 16 of them: 65 -> 18.5 us.
+template <int V> int launch_sddmm_cores(const SddmmParams &p, cudaStream_t s) {
+    DeviceInfo *d;
+    int rc = device_info(&d);
+    if (rc != VS_OK) return rc;
+    const char *e = std::getenv("VSPARSE_B200_SDDMM");
+    const bool force_cores = e && !std::strcmp(e, "gather"), force_dense = e && !std::strcmp(e, "dense"), force_direct = e && !std::strcmp(e, "direct");
+    const bool strides = p.batch == 1 || ((p.stride_lhs * 2) % 16 == 0 && (p.stride_rhs * 2) % 16 == 0);
+    if (!force_cores && strides && p.n > 0 && p.m_vec > 0) {
+        if constexpr (V > 1) {
+            const SddmmTimes t = sddmm_times(p, V, d);
+            if ((force_dense || (!force_direct && t.dense < t.direct)) && !t_no_scratch && sddmm_pair_enabled() && launch_sddmm_pair<__half, V>(p, s, d, &rc))
+                return rc;
+        }
+        if (!force_dense && launch_sddmm_direct<__half, V>(p, s, d, &rc)) return rc;
+    }
+    return launch_sddmm_cc<__half, __half, V>(p, s);
+}
+int sddmm_cores_by_v(int V, const SddmmParams &p, cudaStream_t s) {
+    switch (V) {
+        case 1: return launch_sddmm_cores<1>(p, s);
+        case 2: return launch_sddmm_cores<2>(p, s);
+        case 4: return launch_sddmm_cores<4>(p, s);
+        case 8: return launch_sddmm_cores<8>(p, s);
+    }
+    return VS_ERR_VEC_LENGTH;
 }
 
 template <typename TOut> int sddmm_tc_by_v(int V, const SddmmParams &p, cudaStream_t s) {
@@ -962,8 +1037,7 @@ VS_EXPORT int vs_spmm_batched(int path, int in_dtype, int out_dtype, int m_vec, 
         return out_dtype == VS_F16 ? spmm_tc_by_v<__half>(vec_length, p, s) : spmm_tc_by_v<float>(vec_length, p, s);
     }
     if (in_dtype == VS_F32) return spmm_cc_by_v<float, float>(vec_length, p, s);
-    return out_dtype == VS_F16 ? spmm_cc_by_v<__half, __half>(vec_length, p, s)
-                               : spmm_cc_by_v<__half, float>(vec_length, p, s);
+    return out_dtype == VS_F16 ? spmm_cores_by_v(vec_length, p, s) : spmm_cc_by_v<__half, float>(vec_length, p, s);
 }
 
 VS_EXPORT int vs_spmm(int path, int in_dtype, int out_dtype, int m_vec, int vec_length, int k, int n,
@@ -1056,7 +1130,7 @@ template <typename TOut, int V> int launch_spmm_t(const spmmt::Params &p, int m_
     uint2 *blk_entries = reinterpret_cast<uint2 *>(plan + header_bytes + offsets_bytes);
     rc = (int)launch_overlapped(densespmm::dense_plan_kernel<true>, (unsigned)(groups + checks), densespmm::kPlanThreads, plan_smem, s,
                                 p.t_offsets, p.t_rows, p.t_src, shift, q.m_vec, q.K, groups, rows_per_group, plan_blocks, blk_offsets,
-                                blk_entries, capacity, mode == SpmmTMode::kDense ? 1 : 0, 0.0f, 5.0f * V, 1.5f, flag);
+                                blk_entries, capacity, mode == SpmmTMode::kDense ? 1 : 0, 1100.0f, 0.0f, 5.0f * V, 1.5f, flag);
     const int64_t items = (int64_t)q.batch * n_tiles * m_tiles;
     const unsigned grid = (unsigned)(items < d->sm_count ? items : d->sm_count);   // one persistent CTA per SM
     if (rc == VS_OK) {
@@ -1153,8 +1227,7 @@ VS_EXPORT int vs_sddmm_batched(int path, int in_dtype, int out_dtype, int m_vec,
     if (path == VS_PATH_TENSOR) {
         return out_dtype == VS_F16 ? sddmm_tc_by_v<__half>(vec_length, p, s) : sddmm_tc_by_v<float>(vec_length, p, s);
     }
-    return out_dtype == VS_F16 ? sddmm_cc_by_v<__half, __half>(vec_length, p, s)
-                               : sddmm_cc_by_v<__half, float>(vec_length, p, s);
+    return out_dtype == VS_F16 ? sddmm_cores_by_v(vec_length, p, s) : sddmm_cc_by_v<__half, float>(vec_length, p, s);
 }
 
 VS_EXPORT int vs_sddmm(int path, int in_dtype, int out_dtype, int m_vec, int k, int n, int nonzeros_vec,

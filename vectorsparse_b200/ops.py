@@ -162,8 +162,9 @@ def _wmmaSpmm(m_vec, vec_length, k, n, row_indices, row_offsets, column_indices,
 
 def _cudaSpmm(m_vec, vec_length, k, n, row_indices, row_offsets, column_indices, values, rhs_matrix, output_matrix,
               nonzeros_vec=None):
-    """CUDA-core SpMM, V in {1,2,4,8}; fp16 or fp32 (src/cuda_spmm.cu:304-338; fp32 is a stub there).  nonzeros_vec:
-    as for wmmaSpmm."""
+    """SpMM for V in {1,2,4,8}; fp16 or fp32 (src/cuda_spmm.cu:304-338; fp32 is a stub there), on CUDA cores except for
+    fp16 results of fp16 operands, which come from the tensor cores where that is quicker.  nonzeros_vec: as for
+    wmmaSpmm."""
     return _spmm(VS_PATH_CUDA_CORE, m_vec, vec_length, k, n, row_indices, row_offsets, column_indices, values,
                  rhs_matrix, output_matrix, nonzeros_vec=nonzeros_vec)
 
@@ -181,7 +182,8 @@ def _wmmaSddmm(m_vec, k, n, nonzeros_vec, row_indices, row_offsets, col_indices,
 
 def _cudaSddmm(m_vec, k, n, nonzeros_vec, row_indices, row_offsets, col_indices, lhs_matrix, rhs_matrix,
                output_values, vec_length, stream=None):
-    """CUDA-core SDDMM (src/cuda_sddmm.cu:1257-1331)."""
+    """SDDMM for V in {1,2,4,8} (src/cuda_sddmm.cu:1257-1331); fp32 results from CUDA cores, fp16 ones from the tensor cores
+    where that is quicker."""
     if stream is not None:
         with torch.cuda.stream(stream):
             return _sddmm(VS_PATH_CUDA_CORE, m_vec, k, n, nonzeros_vec, row_indices, row_offsets, col_indices,
