@@ -121,3 +121,56 @@ def test_cuda_core_sddmm_with_fp16_results_in_every_form(monkeypatch, mode, V, m
     for b in range(2):
         want = oracle.sddmm(m_vec, k, V, a.row_offsets, a.col_indices, lhs[b].astype(np.float32), rhs[b].astype(np.float32), acc="f64")
         assert_close(out[b, :a.nnz_vec * V].float().cpu().numpy(), want, f"{mode}, entry {b}")
+
+
+# rows around the 16 of a CTA, columns around the 128 of a tile and the three-tile ring, dense widths around the 128-column slab, full
+# rows (more than one batch of entries per tile), rows with few entries (gathered instead of staged) and an empty matrix
+@pytest.mark.parametrize("V", [1, 2, 4, 8])
+@pytest.mark.parametrize("m_vec,K,N,sparsity", [(1, 1, 4, 0.0), (16, 128, 128, 0.0), (17, 129, 132, 0.5), (33, 513, 260, 0.3), (40, 700, 124, 0.97),
+                                                (20, 640, 64, 1.0)])
+@pytest.mark.parametrize("order", ["ascending", "mixed"])
+def test_fp32_spmm_on_staged_tiles(monkeypatch, V, m_vec, K, N, sparsity, order):
+    """The same bits as the kernel without staged tiles, whose sums are formed in the same order, and the oracle's values."""
+    a = problem(cvse.GEN_UNIFORM, 3, m_vec, K, V, sparsity)
+    if order == "mixed":   # every other row in any order, one of them with a column named twice
+        rng = np.random.default_rng(1)
+        for r in range(0, m_vec, 2):
+            part = slice(int(a.row_offsets[r]), int(a.row_offsets[r + 1]))
+            a.col_indices[part] = rng.permutation(a.col_indices[part])
+        if a.row_offsets[1] > 1:
+            a.col_indices[1] = a.col_indices[0]
+    row = (max(a.nnz_vec, 1) * V + 3) // 4 * 4
+    vals = cvse.fill_random((2, row), np.float32, cvse.DIST_UNIFORM, 1)
+    B = cvse.fill_random((2, K, N), np.float32, cvse.DIST_UNIFORM, 2)
+    got = {}
+    for mode in ("rows", "tiles"):
+        monkeypatch.setenv("VSPARSE_B200_SPMM_CC", mode)
+        out = torch.full((2, a.m, N), float("nan"), dtype=torch.float32, device=DEV)
+        ops.spmm_batched(VS_PATH_CUDA_CORE, m_vec, V, N, K, *structure(a), dev(vals), dev(B), out)
+        torch.cuda.synchronize()
+        assert ops.device_status() == 0
+        got[mode] = out.cpu().numpy()
+    assert np.array_equal(got["rows"], got["tiles"])
+    for b in range(2):
+        assert_close(got["tiles"][b], spmm_oracle(a, N, vals[b, :a.nnz_vec * V], B[b]), f"entry {b}")
+
+
+@pytest.mark.parametrize("shared", [False, True])
+def test_fp32_spmm_on_staged_tiles_with_non_finite_operands(monkeypatch, shared):
+    """Inf and NaN reach the rows that name them and no others; one dense operand for the whole batch."""
+    a = problem(cvse.GEN_UNIFORM, 4, 20, 200, 4, 0.5)
+    row = (a.nnz_vec * 4 + 3) // 4 * 4
+    vals = dev(cvse.fill_random((2, row), np.float32, cvse.DIST_UNIFORM, 1))
+    B = cvse.fill_random((1 if shared else 2, 200, 132), np.float32, cvse.DIST_UNIFORM, 2)
+    B[0, a.col_indices[0], 3] = np.inf
+    B[0, a.col_indices[1], 130] = np.nan
+    rhs = dev(B[0]) if shared else dev(B)
+    got = {}
+    for mode in ("rows", "tiles"):
+        monkeypatch.setenv("VSPARSE_B200_SPMM_CC", mode)
+        out = torch.zeros((2, a.m, 132), dtype=torch.float32, device=DEV)
+        ops.spmm_batched(VS_PATH_CUDA_CORE, 20, 4, 132, 200, *structure(a), vals, rhs, out)
+        torch.cuda.synchronize()
+        got[mode] = out.cpu().numpy()
+    assert not np.isfinite(got["rows"]).all()
+    assert np.array_equal(got["rows"], got["tiles"], equal_nan=True)

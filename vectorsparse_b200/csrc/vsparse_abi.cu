@@ -26,6 +26,7 @@
 #include "common.cuh"
 #include "cuda_core.cuh"
 #include "spmm_tc.cuh"
+#include "spmm_cc_tile.cuh"
 #include "spmm_tma.cuh"
 #include "spmm_dense.cuh"
 #include "spmm_direct.cuh"
@@ -283,7 +284,7 @@ int make_gather_map(CUtensorMap *map, const void *ptr, uint64_t rows, uint64_t c
 // box_cols x box_rows elements, swizzled over the bytes of a box row (128 or 64); loads read zeros outside the
 // matrix, stores are clipped there.
 int make_tile_map(CUtensorMap *map, const void *ptr, bool f32, uint64_t rows, uint64_t cols, uint64_t batch,
-                  uint64_t batch_stride, uint32_t box_cols, uint32_t box_rows) {
+                  uint64_t batch_stride, uint32_t box_cols, uint32_t box_rows, bool swizzled = true) {
     EncodeTiledFn fn = encode_tiled_fn();
     if (!fn) return VS_ERR_DEVICE;
     const uint64_t es = f32 ? 4 : 2;
@@ -291,7 +292,7 @@ int make_tile_map(CUtensorMap *map, const void *ptr, bool f32, uint64_t rows, ui
     const cuuint64_t strides[2] = {cols * es, (batch > 1 ? batch_stride : rows * cols) * es};
     const cuuint32_t box[3] = {box_cols, box_rows, 1};
     const cuuint32_t estr[3] = {1, 1, 1};
-    const CUtensorMapSwizzle swizzle = box_cols * es == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
+    const CUtensorMapSwizzle swizzle = !swizzled ? CU_TENSOR_MAP_SWIZZLE_NONE : box_cols * es == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B;
     CUresult r = fn(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, const_cast<void *>(ptr), dims,
                     strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, swizzle, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                     CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -316,13 +317,62 @@ int make_blocked_map(CUtensorMap *map, const void *ptr, uint64_t rows, uint64_t 
 }
 
 // ---- SpMM dispatch ----------------------------------------------------------------------------------------
-template <typename TIn, typename TOut, int V> int launch_spmm_cc(const SpmmParams &p, cudaStream_t s) {
-    constexpr int E = Chunk<TIn>::kElems;
-    // several 16-byte chunks per thread where the dense width allows it and the accumulators stay in registers (64 at
-    // most); VSPARSE_B200_SPMM_CC_CHUNKS=1|2|4 caps them
+// 16-byte chunks of the dense width per thread of spmm_cc_kernel: several where the width allows it and the accumulators
+// stay in registers (64 at most); VSPARSE_B200_SPMM_CC_CHUNKS=1|2|4 caps them.
+int spmm_cc_chunks(int VE, int E, int N) {
     const char *e = std::getenv("VSPARSE_B200_SPMM_CC_CHUNKS");
     const int cap = e ? std::atoi(e) : 4;
-    const int want = (V * E <= 16 && cap >= 4 && p.N % (128 * E) == 0) ? 4 : (V * E <= 32 && cap >= 2 && p.N % (64 * E) == 0) ? 2 : 1;
+    return (VE <= 16 && cap >= 4 && N % (128 * E) == 0) ? 4 : (VE <= 32 && cap >= 2 && N % (64 * E) == 0) ? 2 : 1;
+}
+// Whether the fp32 product goes to the kernel that stages tiles of B.  Its CTAs take an SM each: where one wave of them
+// holds the product it won or drew at every V, size and sparsity measured from 128 columns up (up to 4x; with 64 columns
+// and a few entries per vector-row it lost, 5.5 against 4.3 us).  With two waves it still wins where the other kernel is
+// left with under eight warps per SM (1024 x 1024 x 1024 at V = 2, 50 / 90 / 98 % sparse: 60 / 23 / 12.5 against 131 / 39 / 12.5 us), and
+// loses where that has more (2048 x 512 x 256 at V = 1: 31 / 12.6 / 8.5 against 29 / 11.5 / 6.4).
+// VSPARSE_B200_SPMM_CC=rows|tiles chooses one.
+bool spmm_cc_tiles_chosen(int V, const SpmmParams &p, const DeviceInfo *d) {
+    if (p.K < 1 || p.K > 1 << 30) return false;   // tile coordinates and column sums in 32 bits
+    const int64_t ctas = (((int64_t)p.m_vec + cctile::kWarps - 1) / cctile::kWarps) * (((int64_t)p.N + cctile::kCols - 1) / cctile::kCols) * p.batch;
+    if (ctas > 0x7fffffffll) return false;
+    const char *e = std::getenv("VSPARSE_B200_SPMM_CC");
+    if (e && !std::strcmp(e, "rows")) return false;
+    if (e && !std::strcmp(e, "tiles")) return true;
+    const int64_t threads = (int64_t)p.m_vec * (p.N / 4) / spmm_cc_chunks(4 * V, 4, p.N) * p.batch;
+    return p.K >= 128 && (ctas <= d->sm_count || (ctas <= 2 * d->sm_count && threads <= (int64_t)d->sm_count * 256));
+}
+// Leaves *taken false where no tensor map can be made.
+template <int V> int launch_spmm_cc_tile(const SpmmParams &p, DeviceInfo *d, cudaStream_t s, bool *taken) {
+    using L = cctile::Layout<V>;
+    const int groups = (int)(((int64_t)p.m_vec + cctile::kWarps - 1) / cctile::kWarps), slabs = (int)(((int64_t)p.N + cctile::kCols - 1) / cctile::kCols);
+    CUtensorMap map;
+    if (make_tile_map(&map, p.rhs, true, (uint64_t)p.K, (uint64_t)p.N, p.stride_rhs ? (uint64_t)p.batch : 1, (uint64_t)p.stride_rhs, cctile::kCols,
+                      cctile::kTile, false) != VS_OK)
+        return VS_OK;
+    auto kernel = cctile::spmm_cc_tile_kernel<V>;
+    static DeviceBits done;
+    const int rc = set_smem_once(kernel, L::kSmemBytes, done);
+    if (rc != VS_OK) return rc;
+    *taken = true;
+    kernel<<<(unsigned)groups * slabs * p.batch, cctile::kThreads, L::kSmemBytes, s>>>(p, map, groups, slabs, d->status);
+    return (int)cudaGetLastError();
+}
+int spmm_cc_tile(int V, const SpmmParams &p, cudaStream_t s, bool *taken) {
+    DeviceInfo *d = nullptr;
+    const int rc = device_info(&d);
+    if (rc != VS_OK) return rc;
+    if (!spmm_cc_tiles_chosen(V, p, d)) return VS_OK;
+    switch (V) {
+        case 1: return launch_spmm_cc_tile<1>(p, d, s, taken);
+        case 2: return launch_spmm_cc_tile<2>(p, d, s, taken);
+        case 4: return launch_spmm_cc_tile<4>(p, d, s, taken);
+        case 8: return launch_spmm_cc_tile<8>(p, d, s, taken);
+    }
+    return VS_OK;
+}
+
+template <typename TIn, typename TOut, int V> int launch_spmm_cc(const SpmmParams &p, cudaStream_t s) {
+    constexpr int E = Chunk<TIn>::kElems;
+    const int want = spmm_cc_chunks(V * E, E, p.N);
     const int64_t items = (int64_t)p.m_vec * (p.N / E) / want;
     const int64_t blocks = (items + kCcThreads - 1) / kCcThreads;
     if (blocks > 0x7fffffffll) return VS_ERR_SHAPE;
@@ -344,6 +394,11 @@ template <typename TIn, typename TOut, int V> int launch_spmm_cc(const SpmmParam
 }
 
 template <typename TIn, typename TOut> int spmm_cc_by_v(int V, const SpmmParams &p, cudaStream_t s) {
+    if constexpr (sizeof(TIn) == 4) {
+        bool taken = false;
+        const int rc = spmm_cc_tile(V, p, s, &taken);
+        if (rc != VS_OK || taken) return rc;
+    }
     switch (V) {
         case 1: return launch_spmm_cc<TIn, TOut, 1>(p, s);
         case 2: return launch_spmm_cc<TIn, TOut, 2>(p, s);
