@@ -174,3 +174,19 @@ def test_fp32_spmm_on_staged_tiles_with_non_finite_operands(monkeypatch, shared)
         got[mode] = out.cpu().numpy()
     assert not np.isfinite(got["rows"]).all()
     assert np.array_equal(got["rows"], got["tiles"], equal_nan=True)
+
+
+@pytest.mark.parametrize("V,m_vec,K,sparsity", [(1, 200, 1100, 0.99), (1, 200, 1100, 0.7), (2, 90, 1300, 0.99), (2, 90, 1300, 0.8), (1, 1040, 1025, 0.95)])
+def test_cuda_core_spmm_chooses_by_density(V, m_vec, K, sparsity):
+    """More than 1024 columns at V <= 2: the device takes the one-kernel form or the CUDA-core kernel behind it, on either side of its line;
+    two calls in a row on one stream."""
+    N = 200
+    a = problem(cvse.GEN_BETA, 8, m_vec, K, V, sparsity)
+    for seed in (1, 2):
+        vals = cvse.fill_random((a.nnz_vec * V,), np.float16, cvse.DIST_NORMAL, seed, 0.25)
+        B = cvse.fill_random((K, N), np.float16, cvse.DIST_NORMAL, seed + 2, 0.5)
+        out = torch.full((a.m, N), float("nan"), dtype=torch.float16, device=DEV)
+        ops.spmm.cudaSpmm(m_vec, V, N, K, *structure(a), dev(vals), dev(B), out)
+        torch.cuda.synchronize()
+        assert ops.device_status() == 0
+        assert_close(out.float().cpu().numpy(), spmm_oracle(a, N, vals, B), f"seed {seed}")

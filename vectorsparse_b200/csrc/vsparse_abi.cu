@@ -407,11 +407,16 @@ template <typename TIn, typename TOut> int spmm_cc_by_v(int V, const SpmmParams 
     }
     return VS_ERR_VEC_LENGTH;
 }
-template <typename TOut, int V> int launch_spmm_cc_standby(const SpmmParams &p, cudaStream_t s, DeviceInfo *d, const int32_t *plan_hdr, int plan_checks) {
+template <typename TOut, int V> int launch_spmm_cc_standby(const SpmmParams &p, cudaStream_t s, DeviceInfo *d, const int32_t *plan_hdr, int plan_checks,
+                                                          bool overlapped = true) {
     const int64_t blocks = ((int64_t)p.m_vec * (p.N / Chunk<__half>::kElems) * p.batch + kCcThreads - 1) / kCcThreads;
     const int64_t cap = (int64_t)d->sm_count * 8;
-    return (int)launch_overlapped(spmm_cc_standby_kernel<__half, TOut, V>, (unsigned)(blocks < cap ? blocks : cap), kCcThreads, 0, s, p, plan_hdr,
-                                  plan_checks);
+    const unsigned grid = (unsigned)(blocks < cap ? blocks : cap);
+    if (!overlapped) {
+        spmm_cc_standby_kernel<__half, TOut, V><<<grid, kCcThreads, 0, s>>>(p, plan_hdr, plan_checks);
+        return (int)cudaGetLastError();
+    }
+    return (int)launch_overlapped(spmm_cc_standby_kernel<__half, TOut, V>, grid, kCcThreads, 0, s, p, plan_hdr, plan_checks);
 }
 
 // Software (cp.async) gather: works for any batch stride.
@@ -602,16 +607,21 @@ int launch_spmm_other(const SpmmParams &p, cudaStream_t s, DeviceInfo *d, const 
 // Small products in one kernel (spmm_direct.cuh); false if this call or this device cannot take it.  When the densified
 // product is the cheaper one whatever the number of nonzeros, nothing else is enqueued; otherwise the kernel leaves its
 // verdict where the gather kernel behind it looks for the plan kernel's.
-template <typename TOut, int V, bool kCores> bool launch_spmm_direct(const SpmmParams &p, cudaStream_t s, DeviceInfo *d, const SpmmCosts &cost,
+template <typename TOut, int V, bool kCores> bool launch_spmm_direct(const SpmmParams &p, cudaStream_t s, DeviceInfo *d, SpmmCosts cost,
                                                                      bool forced, int *rc_out) {
     const int m_tiles = (int)(((int64_t)p.m_vec * V + directspmm::kTileM - 1) / directspmm::kTileM);
     const int n_tiles = (p.N + directspmm::kTileN - 1) / directspmm::kTileN;
     const int64_t tiles = (int64_t)p.batch * m_tiles * n_tiles;
     if (tiles > 0x7fffffffll || p.K <= 0 || p.N % 8 != 0) return false;
     const float stages = std::ceil((float)p.m_vec * V / densespmm::kTileM) * std::ceil((float)p.K / densespmm::kBlockK);
-    // (against the CUDA-core kernel it is the quicker form of a small product down to ~5 % of the vectors: a stand-by behind
-    // every call would cost more than it saves on the few below)
-    const bool always = forced || kCores || (cost.dense_per_entry == 0.0f && cost.dense_per_stage * stages < cost.gather_per_row * (float)p.m_vec);
+    // Against the CUDA-core kernel it is the quicker form of a small product down to a few per cent of the vectors.  Up to 1024
+    // columns, and at V > 2, a stand-by behind every call would cost more than it saves on the few below; with short vectors
+    // and more columns the line is a density, which the device knows.  Forced / CUDA-core kernel, us, 90 / 95 / 98 % sparse: V = 1,
+    // 2048 x 2048 x 256 53 / 37 / 28 against 53 / 31 / 17, 419 x 2665 x 64 49 / 35 / 29 against 80 / 43 / 25; V = 2, 209 vector-rows of that
+    // with 256 dense columns 34 / 31 / 25 against 72 / 41 / 23.
+    const bool by_density = kCores && V <= 2 && !forced && p.K > 1024;
+    if (by_density) cost = {(V == 2 ? 0.03f : tiles > 48 ? 0.045f : 0.035f) * (float)p.K * (float)p.m_vec / stages, 0.0f, 0.0f, 1.0f};
+    const bool always = forced || (kCores && !by_density) || (!kCores && cost.dense_per_entry == 0.0f && cost.dense_per_stage * stages < cost.gather_per_row * (float)p.m_vec);
     CUtensorMap map;
     static DeviceBits smem_set;
     auto kernel = directspmm::spmm_direct_kernel<TOut, V>;
@@ -623,17 +633,27 @@ template <typename TOut, int V, bool kCores> bool launch_spmm_direct(const SpmmP
     *rc_out = (int)launch_overlapped(kernel, (unsigned)tiles, directspmm::kThreads, directspmm::kSmemBytes, s, p, map, m_tiles, n_tiles,
                                      cost.dense_per_stage * stages, cost.dense_per_entry, cost.gather_per_row, cost.gather_per_entry,
                                      static_cast<int32_t *>(verdict), d->status);
-    if (*rc_out == VS_OK && !always) *rc_out = launch_spmm_other<TOut, V, kCores>(p, s, d, static_cast<const int32_t *>(verdict), 0);
+    if (*rc_out == VS_OK && !always) {
+        // Not overlapped: CTAs that become resident beside a grid of under one wave crowd onto the SMs it leaves free, and where the
+        // CUDA-core kernel then does the work that cost it half its speed (V = 1, 4096 x 4096 x 256, 98 % sparse: 31 -> 46 us).
+        if constexpr (kCores) *rc_out = launch_spmm_cc_standby<TOut, V>(p, s, d, static_cast<const int32_t *>(verdict), 0, false);
+        else *rc_out = launch_spmm_other<TOut, V, kCores>(p, s, d, static_cast<const int32_t *>(verdict), 0);
+    }
     return true;
 }
 // Which products are small: up to one wave of 128 x 64 tiles at two per SM the one-kernel form saves the ~9 us of the other
 // launches (2048 x 512 x 256, V = 8: 15.4 -> 6.5 us; 512 x 2048 x 256: 22.3 -> 13.3), up to two waves while K is short.  Shorter
 // vectors mean more entries per tile, which it scatters again for every 64 columns of B, so there the line lies at a smaller
 // K (V = 2, 2048 x 2048 x 256, 60 and 95 % sparse: 85 -> 68 and 28 -> 30; 4096 x 4608 x 256, 85 % sparse: 74 -> 88).
-bool spmm_direct_wanted(const SpmmParams &p, int V, const DeviceInfo *d) {
+// The entry point with the CUDA-core kernel behind it takes it at any K where short vectors meet a narrow B: the planned
+// kernels' 256-row tiles leave most SMs idle there (V = 1, 4096 x 4096 x 64, 80 / 95 % sparse: 272 -> 114 and 94 -> 53 us; 128 x 4096 x
+// 256: 136 -> 109 and 51 -> 50), at V = 2 up to 64 tiles (2048 vector-rows x 4096 x 64: 143 -> 71 and 58 -> 46; with 256 dense columns
+// 82 -> 93 and 47 -> 60).
+bool spmm_direct_wanted(const SpmmParams &p, int V, bool cores, const DeviceInfo *d) {
     const int64_t m_tiles = ((int64_t)p.m_vec * V + directspmm::kTileM - 1) / directspmm::kTileM;
     const int64_t tiles = m_tiles * ((p.N + directspmm::kTileN - 1) / directspmm::kTileN) * p.batch;
     const int chunks = (p.K + directspmm::kChunkK - 1) / directspmm::kChunkK;
+    if (cores && p.N <= 256 && ((V == 1 && tiles <= 2 * d->sm_count) || (V == 2 && tiles <= 64))) return true;
     if (tiles <= 2 * d->sm_count) return chunks <= (V == 8 ? 64 : V == 4 ? 32 : 16);
     return tiles <= 4 * d->sm_count && chunks <= (V >= 4 ? 4 : 1);
 }
@@ -644,7 +664,7 @@ template <typename TOut, int V, bool kCores> int launch_spmm_tc(const SpmmParams
     if (rc != VS_OK) return rc;
     const SpmmMode mode = spmm_mode();
     constexpr SpmmCosts cost = kCores ? cores_costs(V) : kGatherCosts;
-    if ((mode == SpmmMode::kDirect || (mode == SpmmMode::kAuto && spmm_direct_wanted(p, V, d))) &&
+    if ((mode == SpmmMode::kDirect || (mode == SpmmMode::kAuto && spmm_direct_wanted(p, V, kCores, d))) &&
         launch_spmm_direct<TOut, V, kCores>(p, s, d, cost, mode == SpmmMode::kDirect, &rc))
         return rc;
     const int k_blocks = (p.K + densespmm::kBlockK - 1) / densespmm::kBlockK;
@@ -989,9 +1009,19 @@ template <typename TOut, int V> int launch_sddmm_tc(const SddmmParams &p, cudaSt
 
 // cudaSddmm with fp16 results: on the tensor cores like cudaSpmm's (spmm_cores_by_v), any contraction length that is a
 // multiple of 8 (the tiles' last block is filled up with zeros by TMA).  The CUDA-core kernel, a group of lanes per
-// vector-row, is never the quicker one (64 x 64 to 4096 x 2048, 60 and 95 % sparse: by 1.1 to 19 times at V > 1, 0.95 to 4.7
-// at V = 1, where only the one-kernel form exists); it takes the strides that tensor maps cannot address.
+// vector-row or mask entry, is slower by 1.1 to 19 times at V > 1 (64 x 64 to 4096 x 2048, 60 and 95 % sparse); it takes the
+// strides that tensor maps cannot address, and what sddmm_cores_wanted names.
 // 159 x 577, 115 entries per row, k = 200, V = 8, 16 of them: 65 -> 18.5 us.
+//
+// Where the tensor cores do not pay, for V <= 2, whose tiles sample one or two values per look-up.  One 128-byte line per entry
+// is little to gather: V = 1, 4096 x 4096, k = 64, 80 / 95 / 98 % sparse 144 / 44 / 21 us against 170 / 75 / 51; V = 2 at 98 % 23 against 26.
+// Past k = 256 the CUDA-core kernel takes single entries and is not held up by long rows: 303 x 982, k = 296, V = 1, 80 %
+// sparse 10.4 against 22.3, up to some 100 MB of gathered rows (1024 x 1024, k = 512, 54 / 107 / 215 MB: 12.5 / 18.7 / 31.9 against 13.1 /
+// 16.9 / 23).
+bool sddmm_cores_wanted(const SddmmParams &p, int V) {
+    if (V == 1) return p.k <= 64 || (p.k > 256 && 2.0 * p.k * p.nnz_vec * p.batch < 1e8);
+    return V == 2 && p.k <= 64 && p.nnz_vec < 0.03 * p.m_vec * p.n;
+}
 template <int V> int launch_sddmm_cores(const SddmmParams &p, cudaStream_t s) {
     DeviceInfo *d;
     int rc = device_info(&d);
@@ -999,7 +1029,8 @@ template <int V> int launch_sddmm_cores(const SddmmParams &p, cudaStream_t s) {
     const char *e = std::getenv("VSPARSE_B200_SDDMM");
     const bool force_cores = e && !std::strcmp(e, "gather"), force_dense = e && !std::strcmp(e, "dense"), force_direct = e && !std::strcmp(e, "direct");
     const bool strides = p.batch == 1 || ((p.stride_lhs * 2) % 16 == 0 && (p.stride_rhs * 2) % 16 == 0);
-    if (!force_cores && strides && p.n > 0 && p.m_vec > 0) {
+    const bool by_rule = !force_dense && !force_direct && sddmm_cores_wanted(p, V);
+    if (!force_cores && !by_rule && strides && p.n > 0 && p.m_vec > 0) {
         if constexpr (V > 1) {
             const SddmmTimes t = sddmm_times(p, V, d);
             if ((force_dense || (!force_direct && t.dense < t.direct)) && !t_no_scratch && sddmm_pair_enabled() && launch_sddmm_pair<__half, V>(p, s, d, &rc))
