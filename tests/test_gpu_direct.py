@@ -190,3 +190,47 @@ def test_cuda_core_spmm_chooses_by_density(V, m_vec, K, sparsity):
         torch.cuda.synchronize()
         assert ops.device_status() == 0
         assert_close(out.float().cpu().numpy(), spmm_oracle(a, N, vals, B), f"seed {seed}")
+
+
+@pytest.mark.parametrize("V,m_vec,K,N", [(1, 600, 2100, 512), (1, 300, 1200, 64), (8, 128, 8300, 128)])
+def test_cuda_core_products_in_a_graph(V, m_vec, K, N):
+    """Captured on a stream that has made no call yet, replayed twice with other values, then called on that stream: sizes of the planned,
+    the density-dependent and the pair form, which keep scratch outside a graph."""
+    a = problem(cvse.GEN_UNIFORM, 3, m_vec, K, V, 0.9)
+    st = structure(a)
+    vals = [cvse.fill_random((a.nnz_vec * V,), np.float16, cvse.DIST_NORMAL, seed, 0.25) for seed in (1, 2, 3)]
+    B = cvse.fill_random((K, N), np.float16, cvse.DIST_NORMAL, 4, 0.5)
+    lhs = cvse.fill_random((a.m, N), np.float16, cvse.DIST_NORMAL, 5, 0.25)
+    v, b, l = dev(vals[0]), dev(B), dev(lhs)
+    out = torch.empty((a.m, N), dtype=torch.float16, device=DEV)
+    sampled = torch.empty((a.nnz_vec * V,), dtype=torch.float16, device=DEV)
+
+    def products():
+        ops.spmm.cudaSpmm(m_vec, V, N, K, *st, v, b, out)
+        ops.sddmm.cudaSddmm(m_vec, N, K, a.nnz_vec, *st, l, b, sampled, V)
+
+    def check(values, what):
+        torch.cuda.synchronize()
+        assert ops.device_status() == 0
+        assert_close(out.float().cpu().numpy(), spmm_oracle(a, N, values, B), what)
+        want = oracle.sddmm(m_vec, N, V, a.row_offsets, a.col_indices, lhs.astype(np.float32), B.astype(np.float32), acc="f64")
+        got = sampled.float().cpu().numpy()
+        assert np.linalg.norm(got - want) <= 2e-3 * np.linalg.norm(want)   # fp16 results, 2^-11 each
+
+    stream = torch.cuda.Stream()
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        products()
+    for values in vals[:2]:
+        v.copy_(dev(values))
+        out.fill_(float("nan"))
+        sampled.fill_(float("nan"))
+        torch.cuda.synchronize()
+        graph.replay()
+        check(values, "replay")
+    v.copy_(dev(vals[2]))
+    torch.cuda.synchronize()
+    with torch.cuda.stream(stream):
+        products()
+    check(vals[2], "after the graph")

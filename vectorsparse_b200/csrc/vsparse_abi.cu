@@ -122,7 +122,17 @@ thread_local bool t_ws_set = false;
 thread_local void *t_ws_ptr = nullptr;
 thread_local int64_t t_ws_bytes = 0;
 
-// Scratch of at least `bytes` for work enqueued on `stream`.  Grows by stream-ordered allocation (the old buffer
+bool stream_capturing(cudaStream_t s) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return false;
+    }
+    return st != cudaStreamCaptureStatusNone;
+}
+
+// Scratch of at least `bytes` for work enqueued on `stream`.  Does not grow while the stream is being captured: memory
+// allocated there belongs to the graph, and the buffer kept for later calls would be gone between its launches.  Grows by stream-ordered allocation (the old buffer
 // is released behind the work already enqueued); in the steady state this makes no CUDA call.  Buffers live
 // until vs_release_scratch or the end of the process.
 int stream_scratch(DeviceInfo *d, cudaStream_t stream, size_t bytes, void **out) {
@@ -134,6 +144,7 @@ int stream_scratch(DeviceInfo *d, cudaStream_t stream, size_t bytes, void **out)
     std::lock_guard<std::mutex> lock(g_devices_mutex);
     Scratch &sc = d->scratch[DeviceInfo::key_of(stream)];
     if (sc.bytes < bytes) {
+        if (stream_capturing(stream)) return VS_ERR_ARG;
         size_t want = 1u << 20;
         while (want < bytes) want <<= 1;
         void *fresh = nullptr;
@@ -662,6 +673,13 @@ template <typename TOut, int V, bool kCores> int launch_spmm_tc(const SpmmParams
     DeviceInfo *d;
     int rc = device_info(&d);
     if (rc != VS_OK) return rc;
+    if constexpr (kCores) {
+        // A captured cudaSpmm holds no pointer to the library's scratch, which a later, larger call replaces.
+        if (!t_ws_set && !t_no_scratch && stream_capturing(s)) {
+            NoScratchScope scope;
+            return launch_spmm_tc<TOut, V, kCores>(p, s);
+        }
+    }
     const SpmmMode mode = spmm_mode();
     constexpr SpmmCosts cost = kCores ? cores_costs(V) : kGatherCosts;
     if ((mode == SpmmMode::kDirect || (mode == SpmmMode::kAuto && spmm_direct_wanted(p, V, kCores, d))) &&
@@ -1026,6 +1044,10 @@ template <int V> int launch_sddmm_cores(const SddmmParams &p, cudaStream_t s) {
     DeviceInfo *d;
     int rc = device_info(&d);
     if (rc != VS_OK) return rc;
+    if (!t_ws_set && !t_no_scratch && stream_capturing(s)) {   // as in launch_spmm_tc
+        NoScratchScope scope;
+        return launch_sddmm_cores<V>(p, s);
+    }
     const char *e = std::getenv("VSPARSE_B200_SDDMM");
     const bool force_cores = e && !std::strcmp(e, "gather"), force_dense = e && !std::strcmp(e, "dense"), force_direct = e && !std::strcmp(e, "direct");
     const bool strides = p.batch == 1 || ((p.stride_lhs * 2) % 16 == 0 && (p.stride_rhs * 2) % 16 == 0);
