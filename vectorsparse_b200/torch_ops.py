@@ -20,6 +20,7 @@ of fixed-mask sparse attention into torch.autograd, so that the pair can sit ins
 from __future__ import annotations
 
 import torch
+from torch._ops import _len_torch_dispatch_stack_pre_dispatch as _len_pre_dispatch
 
 from . import cvse as _cvse
 from . import ops
@@ -74,6 +75,17 @@ def _attention(path, m_vec, V, nonzeros_vec, row_indices, row_offsets, col_indic
     return out
 
 
+def _through(kernel, op, operands, *args):
+    """The registered operator `op`, whose CUDA kernel is `kernel`.  The dispatcher's way there and back costs the host ~10 us
+    a call, so plain CUDA tensors with nobody listening go to the kernel at once; modes of either kind (tracers, fake tensors, user
+    modes), torch.jit.trace, a running profiler, tensor subclasses and a backward pass that is itself differentiated see the operator."""
+    heard = (torch._C._len_torch_dispatch_stack() or _len_pre_dispatch() or torch._C._len_torch_function_stack()
+             or torch._C._get_tracing_state() is not None or torch.autograd.profiler._is_profiler_enabled or torch.is_grad_enabled())
+    if not heard and all((type(t) is torch.Tensor or type(t) is torch.nn.Parameter) and t.is_cuda for t in operands):
+        return kernel(*args)
+    return op(*args)
+
+
 _LIB.impl("spmm", _spmm, "CUDA")
 _LIB.impl("sddmm", _sddmm, "CUDA")
 _LIB.impl("softmax", _softmax, "CUDA")
@@ -97,9 +109,8 @@ class FixedMaskAttention(torch.autograd.Function):
     @staticmethod
     def forward(ctx, q, k, v, mask: AttentionMask, scale: float, path: int = VS_PATH_TENSOR):
         q, k, v = q.contiguous(), k.contiguous(), v.contiguous()
-        # the functions behind torch.ops.vsparse.*: the dispatcher's way to them and back costs the host ~10 us a call
-        out = _attention(path, mask.m_vec, mask.V, mask.nnz_vec, mask.row_indices, mask.row_offsets, mask.col_indices, q, k, v,
-                         float(scale))
+        out = _through(_attention, torch.ops.vsparse.attention, (q, k, v), path, mask.m_vec, mask.V, mask.nnz_vec,
+                       mask.row_indices, mask.row_offsets, mask.col_indices, q, k, v, float(scale))
         ctx.save_for_backward(q, k, v)
         ctx.mask, ctx.scale, ctx.path = mask, float(scale), path
         return out
@@ -129,7 +140,8 @@ class SparseDenseProduct(torch.autograd.Function):
     @staticmethod
     def forward(ctx, values, b, mask: AttentionMask, path: int = VS_PATH_TENSOR):
         values, b = values.contiguous(), b.contiguous()
-        c = _spmm(path, mask.m_vec, mask.V, mask.row_indices, mask.row_offsets, mask.col_indices, values, b)
+        c = _through(_spmm, torch.ops.vsparse.spmm, (values, b), path, mask.m_vec, mask.V, mask.row_indices, mask.row_offsets,
+                     mask.col_indices, values, b)
         ctx.save_for_backward(values, b)
         ctx.mask, ctx.path = mask, path
         return c
@@ -144,7 +156,8 @@ class SparseDenseProduct(torch.autograd.Function):
             grad_b = torch.empty_like(b)
             ops.spmm_t(m.m_vec, m.V, b.shape[-1], m.n, m.t_offsets, m.t_rows, m.t_src, values, grad_c, grad_b, m.nnz_vec)
         if ctx.needs_input_grad[0]:
-            g = _sddmm(ctx.path, m.m_vec, m.V, m.nnz_vec, m.row_indices, m.row_offsets, m.col_indices, grad_c, b)
+            g = _through(_sddmm, torch.ops.vsparse.sddmm, (grad_c, b), ctx.path, m.m_vec, m.V, m.nnz_vec, m.row_indices, m.row_offsets,
+                         m.col_indices, grad_c, b)
             grad_values = g.sum(0) if (g.dim() == 2 and values.dim() == 1) else g
         return grad_values, grad_b, None, None
 
