@@ -103,12 +103,19 @@ int64_t batch_stride(const at::Tensor *t, int batched_dims, int batch) {
 }
 int64_t lead(const at::Tensor *t, int batched_dims, int batch) { return t->dim() == batched_dims ? batch : 1; }
 
-// Makes `device` current for the call (a look at the current one when it already is) and names its current stream.
+// Makes `device` current for the call (a look at the current one when it already is) and names its current stream.  Other
+// Python threads run while the library is in the call: it can block (a full launch queue, an allocation, a kernel's first
+// load), and what it waits for may be a callback of one of them.  `enqueue` therefore holds addresses and numbers only: a
+// tensor's may change as soon as other threads run, and reading them may throw.
 template <typename F> PyObject *call(const Args &a, F &&enqueue) {
     c10::cuda::OptionalCUDAGuard guard;
     if (c10::cuda::current_device() != a.device) guard.set_index((c10::DeviceIndex)a.device);
     void *stream = (void *)c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)a.device).stream();
-    return PyLong_FromLong(enqueue(stream));
+    int rc;
+    Py_BEGIN_ALLOW_THREADS
+    rc = enqueue(stream);
+    Py_END_ALLOW_THREADS
+    return PyLong_FromLong(rc);
 }
 
 #define VS_FAST_CALL(name, count)                                                       \
@@ -141,10 +148,11 @@ VS_FAST_CALL(spmm, 13) {
     a.type(rhs, values->scalar_type());
     const int in_t = a.dtype(values), out_t = a.dtype(out);
     if (!a.ok) Py_RETURN_NONE;
+    const void *pv = values->const_data_ptr(), *pr = rhs->const_data_ptr();
+    void *po = out->mutable_data_ptr();
+    const int64_t sv = batch_stride(values, 2, batch), sr = batch_stride(rhs, 3, batch), so = batch_stride(out, 3, batch);
     return call(a, [&](void *s) {
-        return g_lib.spmm(path, in_t, out_t, m_vec, V, k, n, ri, ro, ci, values->const_data_ptr(), rhs->const_data_ptr(),
-                          out->mutable_data_ptr(), batch, batch_stride(values, 2, batch), batch_stride(rhs, 3, batch),
-                          batch_stride(out, 3, batch), s);
+        return g_lib.spmm(path, in_t, out_t, m_vec, V, k, n, ri, ro, ci, pv, pr, po, batch, sv, sr, so, s);
     });
 }
 
@@ -164,10 +172,11 @@ VS_FAST_CALL(spmm_t, 11) {
     a.type(rhs, values->scalar_type());
     const int in_t = a.dtype(values), out_t = a.dtype(out);
     if (!a.ok) Py_RETURN_NONE;
+    const void *pv = values->const_data_ptr(), *pr = rhs->const_data_ptr();
+    void *po = out->mutable_data_ptr();
+    const int64_t sv = batch_stride(values, 2, batch), sr = batch_stride(rhs, 3, batch), so = batch_stride(out, 3, batch);
     return call(a, [&](void *s) {
-        return g_lib.spmm_t(in_t, out_t, m_vec, V, k, n, off, rows, src, values->const_data_ptr(), rhs->const_data_ptr(),
-                            out->mutable_data_ptr(), batch, batch_stride(values, 2, batch), batch_stride(rhs, 3, batch),
-                            batch_stride(out, 3, batch), s);
+        return g_lib.spmm_t(in_t, out_t, m_vec, V, k, n, off, rows, src, pv, pr, po, batch, sv, sr, so, s);
     });
 }
 
@@ -184,10 +193,11 @@ VS_FAST_CALL(sddmm, 14) {
     a.type(rhs, lhs->scalar_type());
     const int in_t = a.dtype(lhs), out_t = a.dtype(out);
     if (!a.ok) Py_RETURN_NONE;
+    const void *pl = lhs->const_data_ptr(), *pr = rhs->const_data_ptr();
+    void *po = out->mutable_data_ptr();
+    const int64_t sl = batch_stride(lhs, 3, batch), sr = batch_stride(rhs, 3, batch), so = batch_stride(out, 2, batch);
     return call(a, [&](void *s) {
-        return g_lib.sddmm(path, in_t, out_t, m_vec, k, n, nnz, ri, ro, ci, lhs->const_data_ptr(), rhs->const_data_ptr(),
-                           out->mutable_data_ptr(), V, batch, batch_stride(lhs, 3, batch), batch_stride(rhs, 3, batch),
-                           batch_stride(out, 2, batch), s, algorithm);
+        return g_lib.sddmm(path, in_t, out_t, m_vec, k, n, nnz, ri, ro, ci, pl, pr, po, V, batch, sl, sr, so, s, algorithm);
     });
 }
 
@@ -209,9 +219,11 @@ VS_FAST_CALL(softmax, 7) {
     a.type(probs, scores->scalar_type());
     const int t = a.dtype(scores);
     if (!a.ok) Py_RETURN_NONE;
+    const void *in = scores->const_data_ptr();
+    void *out = probs->mutable_data_ptr();
+    const int64_t stride = batch_stride(scores, 2, batch);
     return call(a, [&](void *s) {
-        return g_lib.softmax(t, m_vec, V, ri, ro, scores->const_data_ptr(), probs->mutable_data_ptr(), (float)scale, batch,
-                             batch_stride(scores, 2, batch), s);
+        return g_lib.softmax(t, m_vec, V, ri, ro, in, out, (float)scale, batch, stride, s);
     });
 }
 
@@ -227,9 +239,11 @@ VS_FAST_CALL(softmax_backward, 7) {
     a.type(gs, probs->scalar_type());
     const int t = a.dtype(probs);
     if (!a.ok) Py_RETURN_NONE;
+    const void *pp = probs->const_data_ptr(), *pg = gp->const_data_ptr();
+    void *po = gs->mutable_data_ptr();
+    const int64_t stride = batch_stride(probs, 2, batch);
     return call(a, [&](void *s) {
-        return g_lib.softmax_backward(t, m_vec, V, ro, probs->const_data_ptr(), gp->const_data_ptr(), gs->mutable_data_ptr(),
-                                      (float)scale, batch, batch_stride(probs, 2, batch), s);
+        return g_lib.softmax_backward(t, m_vec, V, ro, pp, pg, po, (float)scale, batch, stride, s);
     });
 }
 
@@ -248,9 +262,12 @@ VS_FAST_CALL(attention, 15) {
     if (batch > INT_MAX) Py_RETURN_NONE;
     a.need(t[4], batch * nnz * V);
     if (!a.ok) Py_RETURN_NONE;
+    const void *in[3];
+    void *out[2];
+    for (int i = 0; i < 3; ++i) in[i] = t[i]->const_data_ptr();
+    for (int i = 0; i < 2; ++i) out[i] = t[3 + i]->mutable_data_ptr();
     return call(a, [&](void *s) {
-        return g_lib.attention(path, m_vec, V, n, d, nnz, ri, ro, ci, t[0]->const_data_ptr(), t[1]->const_data_ptr(),
-                               t[2]->const_data_ptr(), t[3]->mutable_data_ptr(), t[4]->mutable_data_ptr(), (float)scale, (int)batch, s);
+        return g_lib.attention(path, m_vec, V, n, d, nnz, ri, ro, ci, in[0], in[1], in[2], out[0], out[1], (float)scale, (int)batch, s);
     });
 }
 
@@ -272,11 +289,13 @@ VS_FAST_CALL(attention_backward, 22) {
     a.need(t[7], batch * nnz * V);
     a.need(t[8], batch * nnz * V);
     if (!a.ok) Py_RETURN_NONE;
+    const void *in[4];
+    void *out[5];
+    for (int i = 0; i < 4; ++i) in[i] = t[i]->const_data_ptr();
+    for (int i = 0; i < 5; ++i) out[i] = t[4 + i]->mutable_data_ptr();
     return call(a, [&](void *s) {
-        return g_lib.attention_backward(path, m_vec, V, n, d, nnz, ri, ro, ci, off, rows, src, t[0]->const_data_ptr(),
-                                        t[1]->const_data_ptr(), t[2]->const_data_ptr(), t[3]->const_data_ptr(), t[4]->mutable_data_ptr(),
-                                        t[5]->mutable_data_ptr(), t[6]->mutable_data_ptr(), t[7]->mutable_data_ptr(),
-                                        t[8]->mutable_data_ptr(), (float)scale, (int)batch, s);
+        return g_lib.attention_backward(path, m_vec, V, n, d, nnz, ri, ro, ci, off, rows, src, in[0], in[1], in[2], in[3], out[0],
+                                        out[1], out[2], out[3], out[4], (float)scale, (int)batch, s);
     });
 }
 
