@@ -81,6 +81,19 @@ struct DeviceInfo {
 DeviceInfo g_devices[kMaxDevices];
 std::mutex g_devices_mutex;
 
+// Whether the calling thread has a current context (cuCtxGetCurrent, fetched from the driver at first use).
+bool context_is_current() {
+    typedef CUresult (*GetCurrentFn)(CUcontext *);
+    static const GetCurrentFn fn = []() -> GetCurrentFn {
+        void *p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &p, cudaEnableDefault, &q) != cudaSuccess) return nullptr;
+        return q == cudaDriverEntryPointSuccess ? reinterpret_cast<GetCurrentFn>(p) : nullptr;
+    }();
+    CUcontext current = nullptr;
+    return fn && fn(&current) == CUDA_SUCCESS && current;
+}
+
 int device_info(DeviceInfo **out) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -88,12 +101,10 @@ int device_info(DeviceInfo **out) {
     if (dev < 0 || dev >= kMaxDevices) return VS_ERR_ARG;
     // A thread that has made no runtime call yet (autograd's backward thread, say) has no current context, and the
     // driver's cuTensorMapEncodeTiled refuses to work without one: its first call would take the kernels that need no
-    // tensor maps.  Setting the device binds the context; once per thread and device.
-    static thread_local uint64_t bound = 0;
-    if (!(bound >> dev & 1u)) {
+    // tensor maps.  Setting the device binds the device's primary context; a context that the caller has made current stays.
+    if (!context_is_current()) {
         e = cudaSetDevice(dev);
         if (e != cudaSuccess) return (int)e;
-        bound |= 1ull << dev;
     }
     std::lock_guard<std::mutex> lock(g_devices_mutex);
     DeviceInfo &d = g_devices[dev];
