@@ -260,6 +260,8 @@ int vs_device_status(int clear, uint32_t *status);
  *                                                        thread put their plan in [ptr, ptr + bytes) when it
  *                                                        fits and run the row-gather formulation when it does
  *                                                        not: with a workspace set the library never allocates.
+ *                                                        Calls with VS_PATH_CUDA_CORE neither use it nor keep a
+ *                                                        plan while one is set: they take the forms without.
  *                                                        (NULL, 0) returns to the library's own buffers.
  *
  * ptr must be 16-byte aligned device memory and stay valid until the work enqueued with it has completed; calls

@@ -120,11 +120,11 @@ int device_info(DeviceInfo **out) {
 }
 
 // Set for the duration of an entry point that promises not to allocate: the tensor-core formulations that need
-// plan scratch are skipped on this thread, the gather kernels (which need none) take the call.
+// plan scratch are skipped on this thread, the kernels that need none take the call.
 thread_local bool t_no_scratch = false;
 struct NoScratchScope {
     bool saved;
-    NoScratchScope() : saved(t_no_scratch) { t_no_scratch = true; }
+    explicit NoScratchScope(bool on = true) : saved(t_no_scratch) { t_no_scratch |= on; }
     ~NoScratchScope() { t_no_scratch = saved; }
 };
 
@@ -686,7 +686,7 @@ template <typename TOut, int V, bool kCores> int launch_spmm_tc(const SpmmParams
     if (rc != VS_OK) return rc;
     if constexpr (kCores) {
         // A captured cudaSpmm holds no pointer to the library's scratch, which a later, larger call replaces.
-        if (!t_ws_set && !t_no_scratch && stream_capturing(s)) {
+        if (!t_no_scratch && stream_capturing(s)) {
             NoScratchScope scope;
             return launch_spmm_tc<TOut, V, kCores>(p, s);
         }
@@ -767,7 +767,10 @@ template <typename TOut> int spmm_tc_by_v(int V, const SpmmParams &p, cudaStream
 // in any order and on the tensor cores, whose products of fp16 values are exact and whose sums are fp32 too; what the densified
 // product cannot do (repeated columns, non-finite values, few nonzeros) stays with the CUDA-core kernel.  fp32 results keep it
 // throughout: there the order of the sums shows.  VSPARSE_B200_SPMM=gather forces the CUDA-core kernel.
+// The workspace of vs_set_workspace is the tensor path's: a thread may make cuda* calls beside those, on streams of their own, so
+// while one is set these take the forms without scratch.
 int spmm_cores_by_v(int V, const SpmmParams &p, cudaStream_t s) {
+    NoScratchScope scope(t_ws_set);
     switch (V) {
         case 1: return launch_spmm_tc<__half, 1, true>(p, s);
         case 2: return launch_spmm_tc<__half, 2, true>(p, s);
@@ -1055,7 +1058,7 @@ template <int V> int launch_sddmm_cores(const SddmmParams &p, cudaStream_t s) {
     DeviceInfo *d;
     int rc = device_info(&d);
     if (rc != VS_OK) return rc;
-    if (!t_ws_set && !t_no_scratch && stream_capturing(s)) {   // as in launch_spmm_tc
+    if (!t_no_scratch && stream_capturing(s)) {   // as in launch_spmm_tc
         NoScratchScope scope;
         return launch_sddmm_cores<V>(p, s);
     }
@@ -1074,6 +1077,7 @@ template <int V> int launch_sddmm_cores(const SddmmParams &p, cudaStream_t s) {
     return launch_sddmm_cc<__half, __half, V>(p, s);
 }
 int sddmm_cores_by_v(int V, const SddmmParams &p, cudaStream_t s) {
+    NoScratchScope scope(t_ws_set);   // as in spmm_cores_by_v
     switch (V) {
         case 1: return launch_sddmm_cores<1>(p, s);
         case 2: return launch_sddmm_cores<2>(p, s);
