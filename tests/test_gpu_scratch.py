@@ -1,4 +1,7 @@
-"""Whose memory the library's plans live in: the caller's workspace is the tensor path's alone."""
+"""Whose memory the library's plans live in: the caller's workspace is the tensor path's alone, and a
+stream's buffer belongs to one call at a time."""
+import threading
+
 import numpy as np
 import pytest
 import torch
@@ -6,7 +9,7 @@ import torch
 import oracle
 from conftest import assert_close
 from gpu_util import DEV, dev, problem, spmm_oracle, structure
-from vectorsparse_b200 import cvse, ops
+from vectorsparse_b200 import _lib, cvse, ops
 
 pytestmark = pytest.mark.gpu
 
@@ -14,8 +17,8 @@ pytestmark = pytest.mark.gpu
 class Products:
     """One structure with an SpMM and an SDDMM on it, their operands and oracle results."""
 
-    def __init__(self, V, m_vec, K, N, sparsity, seed=1):
-        self.a = a = problem(cvse.GEN_UNIFORM, seed, m_vec, K, V, sparsity)
+    def __init__(self, V, m_vec, K, N, sparsity, seed=1, kind=cvse.GEN_UNIFORM):
+        self.a = a = problem(kind, seed, m_vec, K, V, sparsity)
         self.st, self.N = structure(a), N
         vals = cvse.fill_random((a.nnz_vec * V,), np.float16, cvse.DIST_NORMAL, seed, 0.25)
         B = cvse.fill_random((K, N), np.float16, cvse.DIST_NORMAL, seed + 1, 0.25)
@@ -58,3 +61,35 @@ def test_cuda_core_calls_leave_the_callers_workspace_alone(V, m_vec):
     finally:
         ops.set_workspace(None)
     assert bool((workspace == 0x5A).all())
+
+
+@pytest.mark.parametrize("names", [("cudaSpmm", "cudaSddmm"), ("wmmaSpmm", "wmmaSddmm")])
+def test_host_threads_can_share_a_stream(names):
+    """Each call plans, multiplies and cleans up in several launches: those of another thread's call must not come between them."""
+    problems = [Products(8, 1200, 1024, 512, 0.9, seed, cvse.GEN_FIXED) for seed in (1, 5)]   # of one size, so that a plan that is mixed up stays in bounds
+    assert problems[0].a.nnz_vec == problems[1].a.nnz_vec
+    stream, failures = torch.cuda.Stream(), []
+    torch.cuda.synchronize()
+
+    def calls(p):
+        try:
+            with torch.cuda.stream(stream):
+                for i in range(200):
+                    p.spmm(getattr(ops.spmm, names[0]))
+                    p.sddmm(getattr(ops.sddmm, names[1]))
+                    if i % 50 == 49:   # given up while the other thread works with it
+                        _lib.lib().vs_release_scratch(stream.cuda_stream, 0)
+        except Exception as e:
+            failures.append(e)
+
+    for p in problems:
+        p.poison()
+    torch.cuda.synchronize()
+    threads = [threading.Thread(target=calls, args=(p,)) for p in problems]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failures
+    for i, p in enumerate(problems):
+        p.check(f"thread {i}")

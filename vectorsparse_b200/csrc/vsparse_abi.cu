@@ -15,6 +15,7 @@
 #include <atomic>
 #include <cstring>
 #include <cmath>
+#include <memory>
 #include <mutex>
 #include <thread>
 #include <functional>
@@ -55,6 +56,8 @@ __device__ uint32_t g_device_status = 0;
 
 constexpr int kMaxDevices = 64;
 struct Scratch {
+    std::mutex use;         // held by a call from the look at `ptr` to its last launch
+    bool retired = false;   // no longer in the table
     void *ptr = nullptr;
     size_t bytes = 0;
 };
@@ -75,7 +78,7 @@ struct DeviceInfo {
             return std::hash<const void *>()(static_cast<const void *>(k.stream)) ^ (std::hash<std::thread::id>()(k.thread) * 0x9e3779b97f4a7c15ull);
         }
     };
-    std::unordered_map<Key, Scratch, KeyHash> scratch;
+    std::unordered_map<Key, std::shared_ptr<Scratch>, KeyHash> scratch;
     static Key key_of(cudaStream_t s) { return Key{s, s == cudaStreamPerThread ? std::this_thread::get_id() : std::thread::id()}; }
 };
 DeviceInfo g_devices[kMaxDevices];
@@ -142,35 +145,53 @@ bool stream_capturing(cudaStream_t s) {
     return st != cudaStreamCaptureStatusNone;
 }
 
-// Scratch of at least `bytes` for work enqueued on `stream`.  Does not grow while the stream is being captured: memory
-// allocated there belongs to the graph, and the buffer kept for later calls would be gone between its launches.  Grows by stream-ordered allocation (the old buffer
-// is released behind the work already enqueued); in the steady state this makes no CUDA call.  Buffers live
-// until vs_release_scratch or the end of the process.
-int stream_scratch(DeviceInfo *d, cudaStream_t stream, size_t bytes, void **out) {
-    if (t_ws_set) {   // the caller's buffer or nothing: never allocate behind a caller that manages memory itself
-        if ((int64_t)bytes > t_ws_bytes) return VS_ERR_SHAPE;
-        *out = t_ws_ptr;
+// The plan scratch of one call.  The call's kernels share it, so nothing else may be enqueued on the stream between them that
+// uses it too: the object holds the stream's buffer against other host threads until it goes out of scope behind the last
+// launch.
+class PlanScratch {
+public:
+    // At least `bytes` for work enqueued on `stream`.  Does not grow while the stream is being captured: memory allocated there
+    // belongs to the graph, and the buffer kept for later calls would be gone between its launches.  Grows by stream-ordered
+    // allocation (the old buffer is released behind the work already enqueued); in the steady state this makes no CUDA call.
+    // Buffers live until vs_release_scratch or the end of the process.
+    int take(DeviceInfo *d, cudaStream_t stream, size_t bytes, void **out) {
+        if (t_ws_set) {   // the caller's buffer or nothing: never allocate behind a caller that manages memory itself
+            if ((int64_t)bytes > t_ws_bytes) return VS_ERR_SHAPE;
+            *out = t_ws_ptr;
+            return VS_OK;
+        }
+        do {
+            lock_ = {};
+            {
+                std::lock_guard<std::mutex> table(g_devices_mutex);
+                std::shared_ptr<Scratch> &entry = d->scratch[DeviceInfo::key_of(stream)];
+                if (!entry) entry = std::make_shared<Scratch>();
+                held_ = entry;
+            }
+            lock_ = std::unique_lock<std::mutex>(held_->use);
+        } while (held_->retired);   // released while this thread waited for it
+        if (held_->bytes < bytes) {
+            if (stream_capturing(stream)) return VS_ERR_ARG;
+            size_t want = 1u << 20;
+            while (want < bytes) want <<= 1;
+            void *fresh = nullptr;
+            cudaError_t e = cudaMallocAsync(&fresh, want, stream);
+            if (e != cudaSuccess) {
+                (void)cudaGetLastError();
+                return (int)e;
+            }
+            if (held_->ptr) (void)cudaFreeAsync(held_->ptr, stream);
+            held_->ptr = fresh;
+            held_->bytes = want;
+        }
+        *out = held_->ptr;
         return VS_OK;
     }
-    std::lock_guard<std::mutex> lock(g_devices_mutex);
-    Scratch &sc = d->scratch[DeviceInfo::key_of(stream)];
-    if (sc.bytes < bytes) {
-        if (stream_capturing(stream)) return VS_ERR_ARG;
-        size_t want = 1u << 20;
-        while (want < bytes) want <<= 1;
-        void *fresh = nullptr;
-        cudaError_t e = cudaMallocAsync(&fresh, want, stream);
-        if (e != cudaSuccess) {
-            (void)cudaGetLastError();
-            return (int)e;
-        }
-        if (sc.ptr) (void)cudaFreeAsync(sc.ptr, stream);
-        sc.ptr = fresh;
-        sc.bytes = want;
-    }
-    *out = sc.ptr;
-    return VS_OK;
-}
+
+private:
+    std::shared_ptr<Scratch> held_;   // outlives the lock on it
+    std::unique_lock<std::mutex> lock_;
+};
 
 inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 inline bool valid_v(int v) { return v == 1 || v == 2 || v == 4 || v == 8; }
@@ -651,7 +672,8 @@ template <typename TOut, int V, bool kCores> bool launch_spmm_direct(const SpmmP
         set_smem_once(kernel, directspmm::kSmemBytes, smem_set) != VS_OK)
         return false;
     void *verdict = nullptr;
-    if (!always && (t_no_scratch || stream_scratch(d, s, 16, &verdict) != VS_OK)) return false;
+    PlanScratch scratch;
+    if (!always && (t_no_scratch || scratch.take(d, s, 16, &verdict) != VS_OK)) return false;
     *rc_out = (int)launch_overlapped(kernel, (unsigned)tiles, directspmm::kThreads, directspmm::kSmemBytes, s, p, map, m_tiles, n_tiles,
                                      cost.dense_per_stage * stages, cost.dense_per_entry, cost.gather_per_row, cost.gather_per_entry,
                                      static_cast<int32_t *>(verdict), d->status);
@@ -726,7 +748,8 @@ template <typename TOut, int V, bool kCores> int launch_spmm_tc(const SpmmParams
     rc = set_smem_once(kernel, densespmm::kSmemBytes, smem_set);
     if (rc != VS_OK) return rc;
     uint8_t *plan = nullptr;
-    if (stream_scratch(d, s, (size_t)plan_bytes, reinterpret_cast<void **>(&plan)) != VS_OK)
+    PlanScratch scratch;
+    if (scratch.take(d, s, (size_t)plan_bytes, reinterpret_cast<void **>(&plan)) != VS_OK)
         return launch_spmm_other<TOut, V, kCores>(p, s, d, nullptr, 0);
     int32_t *flag = reinterpret_cast<int32_t *>(plan);
     const int64_t header_bytes = spmm_plan_header_bytes(checks);
@@ -921,7 +944,8 @@ template <typename TOut, int V> bool launch_sddmm_pair(const SddmmParams &p, cud
                       pairsddmm::kCtaRows) != VS_OK)
         return false;
     uint8_t *plan = nullptr;
-    if (stream_scratch(d, s, (size_t)plan_bytes, reinterpret_cast<void **>(&plan)) != VS_OK) return false;
+    PlanScratch scratch;
+    if (scratch.take(d, s, (size_t)plan_bytes, reinterpret_cast<void **>(&plan)) != VS_OK) return false;
     uint2 *cells = reinterpret_cast<uint2 *>(plan);
     int32_t *order = reinterpret_cast<int32_t *>(plan + cells_bytes);
     int32_t *twins = reinterpret_cast<int32_t *>(plan + cells_bytes + order_bytes);
@@ -1023,7 +1047,8 @@ template <typename TOut, int V> int launch_sddmm_tc(const SddmmParams &p, cudaSt
     rc = set_smem_once(kernel, densesddmm::kSmemBytes, smem_set);
     if (rc != VS_OK) return rc;
     uint8_t *plan = nullptr;
-    if (stream_scratch(d, s, (size_t)plan_bytes, reinterpret_cast<void **>(&plan)) != VS_OK)
+    PlanScratch scratch;
+    if (scratch.take(d, s, (size_t)plan_bytes, reinterpret_cast<void **>(&plan)) != VS_OK)
         return launch_sddmm_gather<TOut, V>(p, s, d);
     int32_t *chunk_offsets = reinterpret_cast<int32_t *>(plan);
     uint2 *chunk_entries = reinterpret_cast<uint2 *>(plan + offsets_bytes);
@@ -1245,7 +1270,8 @@ template <typename TOut, int V> int launch_spmm_t(const spmmt::Params &p, int m_
     rc = set_smem_once(kernel, densespmm::kSmemBytes, smem_set);
     if (rc != VS_OK) return rc;
     uint8_t *plan = nullptr;
-    if (stream_scratch(d, s, (size_t)plan_bytes, reinterpret_cast<void **>(&plan)) != VS_OK)
+    PlanScratch scratch;
+    if (scratch.take(d, s, (size_t)plan_bytes, reinterpret_cast<void **>(&plan)) != VS_OK)
         return launch_spmm_t_cc<TOut, V>(p, s, d, nullptr, 0);
     int32_t *flag = reinterpret_cast<int32_t *>(plan);
     const int64_t header_bytes = spmm_plan_header_bytes(checks);
@@ -1657,17 +1683,24 @@ VS_EXPORT int vs_release_scratch(void *stream, int every_stream) {
     DeviceInfo *d;
     int rc = device_info(&d);
     if (rc != VS_OK) return rc;
-    std::lock_guard<std::mutex> lock(g_devices_mutex);
-    if (every_stream) {
-        for (auto &kv : d->scratch)
-            if (kv.second.ptr) (void)cudaFreeAsync(kv.second.ptr, kv.first.stream);
-        d->scratch.clear();
-        return VS_OK;
+    std::vector<std::pair<cudaStream_t, std::shared_ptr<Scratch>>> released;
+    {
+        std::lock_guard<std::mutex> table(g_devices_mutex);
+        if (every_stream) {
+            for (auto &kv : d->scratch) released.emplace_back(kv.first.stream, std::move(kv.second));
+            d->scratch.clear();
+        } else {
+            auto it = d->scratch.find(DeviceInfo::key_of(static_cast<cudaStream_t>(stream)));
+            if (it != d->scratch.end()) {
+                released.emplace_back(it->first.stream, std::move(it->second));
+                d->scratch.erase(it);
+            }
+        }
     }
-    auto it = d->scratch.find(DeviceInfo::key_of(static_cast<cudaStream_t>(stream)));
-    if (it != d->scratch.end()) {
-        if (it->second.ptr) (void)cudaFreeAsync(it->second.ptr, it->first.stream);
-        d->scratch.erase(it);
+    for (auto &r : released) {
+        std::lock_guard<std::mutex> use(r.second->use);   // behind the launches of a call in progress
+        r.second->retired = true;
+        if (r.second->ptr) (void)cudaFreeAsync(r.second->ptr, r.first);
     }
     return VS_OK;
 }
