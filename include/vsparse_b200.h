@@ -78,10 +78,13 @@ const char *vs_version(void);
  * reference.  A matrix that names a column twice in one vector-row (the reference's generator pads rows that
  * way, include/bm_test_utils.h:110-124, and its kernels add both values) is recognised on the device and goes
  * to the gather kernel, which adds them too.
- * Environment variable VSPARSE_B200_SPMM = "dense" | "gather" forces one formulation.  The first tensor-path
- * call on a stream allocates a plan scratch buffer with cudaMallocAsync on that stream (8 bytes per nonzero
- * vector, bounded by m_vec * n and by 512 MB; reused and grown by later calls on the stream, never freed): make
- * that call outside stream capture.  Everything else about the call is asynchronous and allocation-free.
+ * Environment variable VSPARSE_B200_SPMM = "dense" | "gather" forces one formulation.  The first call with a plan on a
+ * stream allocates a scratch buffer with cudaMallocAsync on that stream (8 bytes per possible nonzero vector, m_vec * n
+ * of them, at most 512 MB; reused and grown by later calls on the stream, freed by vs_release_scratch).  Under stream
+ * capture a call's scratch belongs to the graph: it is allocated with cudaMalloc while the call is captured, shared by the
+ * calls of one capture on one stream, and given back to the library when the graph and all that was instantiated from
+ * it are gone.  Two executable graphs of one captured graph share it and must not run at the same time.  Everything else about
+ * the call is asynchronous and allocation-free.
  * ---------------------------------------------------------------------------------------------------- */
 int vs_spmm(int path, int in_dtype, int out_dtype, int m_vec, int vec_length, int k, int n,
             const int32_t *row_indices, const int32_t *row_offsets, const int32_t *col_indices,
@@ -112,8 +115,8 @@ int vs_spmm_batched(int path, int in_dtype, int out_dtype, int m_vec, int vec_le
  * (in_dtype, out_dtype): (F16,F16), (F16,F32); fp32 accumulation in the listed order (reproducible).
  * vec_length in {1,2,4,8}; k % 8 == 0; values, rhs, out 16-byte aligned.  Two kernels, chosen on the device from
  * their measured costs: A^T through the densifying tensor-core kernel of vs_spmm
- * (plan built from the transposed structure, the V values of a vector side by side in one row of the tile; same plan scratch rules as vs_spmm: per-stream buffer or
- * vs_set_workspace, first call on a stream outside capture), or CUDA cores (one warp per 256 columns of an
+ * (plan built from the transposed structure, the V values of a vector side by side in one row of the tile; same plan scratch
+ * rules as vs_spmm), or CUDA cores (one warp per 256 columns of an
  * output row: very sparse matrices, a column named twice by one vector-row, non-finite sums, no scratch).
  * VSPARSE_B200_SPMM_T = "dense" | "gather" forces one.  The batched form shares the structure and strides
  * values / rhs / out as vs_spmm_batched.
@@ -273,7 +276,8 @@ int64_t vs_spmm_t_workspace_bytes(int m_vec, int vec_length, int n, int batch, i
 int vs_set_workspace(void *workspace, int64_t bytes);
 
 /* Frees the plan scratch the library keeps on the current device for `stream` (stream-ordered: behind the work
- * already enqueued there), or for every stream when every_stream != 0.  The next tensor-path call on such a
+ * already enqueued there), or for every stream when every_stream != 0, and what graphs that no longer exist have given
+ * back (with cudaFree).  The next tensor-path call on such a
  * stream allocates again.  With the per-thread default stream handle (cudaStreamPerThread) the buffer of the
  * calling thread is meant: each host thread has its own.  No counterpart in the reference. */
 int vs_release_scratch(void *stream, int every_stream);

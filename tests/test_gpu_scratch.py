@@ -1,5 +1,5 @@
 """Whose memory the library's plans live in: the caller's workspace is the tensor path's alone, and a
-stream's buffer belongs to one call at a time."""
+stream's buffer belongs to one call at a time, and a graph's to the graph."""
 import threading
 
 import numpy as np
@@ -93,3 +93,67 @@ def test_host_threads_can_share_a_stream(names):
     assert not failures
     for i, p in enumerate(problems):
         p.check(f"thread {i}")
+
+
+def captured(stream, *calls):
+    graph = torch.cuda.CUDAGraph()
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph, stream=stream):
+        for call in calls:
+            call()
+    return graph
+
+
+@pytest.mark.parametrize("warm", [False, True])
+def test_a_graph_keeps_its_scratch(warm):
+    """Products with a plan, captured on a stream with and without earlier calls; a larger call on that stream, then replays beside calls there."""
+    small, large = Products(8, 1200, 1024, 512, 0.9), Products(8, 2500, 2048, 256, 0.9, 4)
+    a = small.a
+    transposed = [dev(x) for x in cvse.transpose(a)]
+    out_t = torch.empty((a.n, small.N), dtype=torch.float16, device=DEV)
+    want_t = oracle.spmm_t(a.m_vec, a.V, small.N, a.n, a.row_offsets, a.col_indices, small.vals.float().cpu().numpy(),
+                           small.lhs.float().cpu().numpy())
+
+    def products():
+        small.spmm(ops.spmm.wmmaSpmm)
+        small.sddmm(ops.sddmm.wmmaSddmm)
+        ops.spmm_t(a.m_vec, a.V, small.N, a.n, *transposed, small.vals, small.lhs, out_t)
+
+    stream, other = torch.cuda.Stream(), torch.cuda.Stream()
+    if warm:
+        with torch.cuda.stream(stream):
+            products()
+    graph = captured(stream, products)
+    with torch.cuda.stream(stream):
+        large.spmm(ops.spmm.wmmaSpmm)   # grows the stream's buffer
+    torch.cuda.synchronize()
+    for i in range(3):
+        small.poison()
+        out_t.fill_(float("nan"))
+        large.poison()
+        torch.cuda.synchronize()
+        with torch.cuda.stream(other):
+            graph.replay()
+        with torch.cuda.stream(stream):   # beside the replay
+            large.spmm(ops.spmm.wmmaSpmm)
+            large.sddmm(ops.sddmm.wmmaSddmm)
+        small.check(f"replay {i}")
+        large.check(f"beside replay {i}")
+        assert_close(out_t.float().cpu().numpy(), want_t, f"transposed, replay {i}")
+
+
+def test_graphs_give_their_scratch_back():
+    """Captured again and again: what an earlier graph held serves a later one."""
+    p, stream = Products(8, 1200, 2048, 512, 0.9), torch.cuda.Stream()   # a plan of 20 MB
+    free = []
+    for _ in range(12):
+        graph = captured(stream, lambda: p.spmm(ops.spmm.wmmaSpmm))
+        graph.replay()
+        torch.cuda.synchronize()
+        del graph
+        torch.cuda.synchronize()
+        free.append(torch.cuda.mem_get_info()[0])
+    p.sddmm(ops.sddmm.wmmaSddmm)
+    p.check("after the graphs")
+    assert free[1] - free[-1] < 64 << 20
+    assert _lib.lib().vs_release_scratch(stream.cuda_stream, 0) == 0

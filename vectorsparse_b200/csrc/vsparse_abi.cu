@@ -60,6 +60,10 @@ struct Scratch {
     bool retired = false;   // no longer in the table
     void *ptr = nullptr;
     size_t bytes = 0;
+    // the capture that last asked for scratch on this stream, and what it was given (memory of the graph, see graph_scratch)
+    unsigned long long capture = 0;
+    void *capture_ptr = nullptr;
+    size_t capture_bytes = 0;
 };
 struct DeviceInfo {
     bool ready = false;
@@ -136,13 +140,110 @@ thread_local bool t_ws_set = false;
 thread_local void *t_ws_ptr = nullptr;
 thread_local int64_t t_ws_bytes = 0;
 
-bool stream_capturing(cudaStream_t s) {
-    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(s, &st) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return false;
+// Scratch for captured work belongs to the graph: a buffer that the library keeps for a stream is replaced by a later, larger
+// call and used by other calls beside a replay.  The graph and whatever is instantiated from it hold a reference (a CUDA user
+// object); when the last one goes, the buffer comes back to this list and serves another capture, or is freed: by
+// vs_release_scratch, or here when the list holds more than kMaxReturnedBytes.
+struct GraphScratch {
+    int device;
+    void *ptr;
+    size_t bytes;
+};
+constexpr size_t kMaxReturnedBytes = 256u << 20;
+struct ReturnedScratch {
+    std::mutex lock;   // nothing else is locked and no CUDA call made under it: the driver calls returned() from a thread of its own
+    std::vector<GraphScratch *> list;
+};
+ReturnedScratch &returned_scratch() {
+    static ReturnedScratch *r = new ReturnedScratch;   // never destroyed: graphs may outlive the library's static objects
+    return *r;
+}
+void CUDART_CB graph_scratch_returned(void *buffer) {
+    ReturnedScratch &r = returned_scratch();
+    std::lock_guard<std::mutex> guard(r.lock);
+    r.list.push_back(static_cast<GraphScratch *>(buffer));
+}
+// Allocating and freeing beside a capture, which forbids them unless the thread says that it knows what it does.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { (void)cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+// Frees returned buffers of `device` until those left hold at most `keep` bytes.
+void free_returned_scratch(int device, size_t keep) {
+    std::vector<GraphScratch *> gone;
+    {
+        ReturnedScratch &r = returned_scratch();
+        std::lock_guard<std::mutex> guard(r.lock);
+        size_t held = 0;
+        for (size_t i = 0; i < r.list.size();) {
+            if (r.list[i]->device == device && (held += r.list[i]->bytes) > keep) {
+                gone.push_back(r.list[i]);
+                r.list.erase(r.list.begin() + i);
+            } else {
+                ++i;
+            }
+        }
     }
-    return st != cudaStreamCaptureStatusNone;
+    RelaxedCapture relaxed;
+    for (GraphScratch *g : gone) {
+        (void)cudaFree(g->ptr);
+        delete g;
+    }
+}
+int graph_scratch(cudaGraph_t graph, size_t bytes, void **out) {
+    int device = 0;
+    cudaError_t e = cudaGetDevice(&device);
+    if (e != cudaSuccess) return (int)e;
+    RelaxedCapture relaxed;
+    GraphScratch *buffer = nullptr;
+    {
+        ReturnedScratch &r = returned_scratch();
+        std::lock_guard<std::mutex> guard(r.lock);
+        auto best = r.list.end();   // the smallest that is large enough
+        for (auto it = r.list.begin(); it != r.list.end(); ++it)
+            if ((*it)->device == device && (*it)->bytes >= bytes && (best == r.list.end() || (*it)->bytes < (*best)->bytes)) best = it;
+        if (best != r.list.end()) {
+            buffer = *best;
+            r.list.erase(best);
+        }
+    }
+    if (!buffer) {
+        free_returned_scratch(device, kMaxReturnedBytes);
+        void *ptr = nullptr;
+        e = cudaMalloc(&ptr, bytes);
+        if (e != cudaSuccess) {
+            (void)cudaGetLastError();
+            return (int)e;
+        }
+        buffer = new GraphScratch{device, ptr, bytes};
+    }
+    cudaUserObject_t owner = nullptr;
+    e = cudaUserObjectCreate(&owner, buffer, graph_scratch_returned, 1, cudaUserObjectNoDestructorSync);
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        graph_scratch_returned(buffer);
+        return (int)e;
+    }
+    *out = buffer->ptr;
+    e = cudaGraphRetainUserObject(graph, owner, 1, cudaGraphUserObjectMove);
+    if (e != cudaSuccess) {
+        (void)cudaGetLastError();
+        (void)cudaUserObjectRelease(owner, 1);   // the buffer goes back to the list
+        return (int)e;
+    }
+    return VS_OK;
+}
+
+// The graph that `s` is being captured into and the capture's number, unique in the process; null without a capture.
+cudaGraph_t capture_graph(cudaStream_t s, unsigned long long *id) {
+    cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+    cudaGraph_t graph = nullptr;
+    if (cudaStreamGetCaptureInfo(s, &st, id, &graph) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return nullptr;
+    }
+    return st == cudaStreamCaptureStatusActive ? graph : nullptr;
 }
 
 // The plan scratch of one call.  The call's kernels share it, so nothing else may be enqueued on the stream between them that
@@ -150,10 +251,9 @@ bool stream_capturing(cudaStream_t s) {
 // launch.
 class PlanScratch {
 public:
-    // At least `bytes` for work enqueued on `stream`.  Does not grow while the stream is being captured: memory allocated there
-    // belongs to the graph, and the buffer kept for later calls would be gone between its launches.  Grows by stream-ordered
-    // allocation (the old buffer is released behind the work already enqueued); in the steady state this makes no CUDA call.
-    // Buffers live until vs_release_scratch or the end of the process.
+    // At least `bytes` for work enqueued on `stream`.  Grows by stream-ordered allocation (the old buffer is released behind the
+    // work already enqueued) and lives until vs_release_scratch or the end of the process.  While the stream is being captured
+    // the buffer is the graph's; the calls that one capture makes on one stream follow one another in the graph too, so they share one.
     int take(DeviceInfo *d, cudaStream_t stream, size_t bytes, void **out) {
         if (t_ws_set) {   // the caller's buffer or nothing: never allocate behind a caller that manages memory itself
             if ((int64_t)bytes > t_ws_bytes) return VS_ERR_SHAPE;
@@ -170,8 +270,19 @@ public:
             }
             lock_ = std::unique_lock<std::mutex>(held_->use);
         } while (held_->retired);   // released while this thread waited for it
+        unsigned long long capture = 0;
+        if (cudaGraph_t graph = capture_graph(stream, &capture)) {
+            if (held_->capture != capture || held_->capture_bytes < bytes) {
+                const size_t want = held_->capture == capture ? std::max(bytes, 2 * held_->capture_bytes) : bytes;
+                const int rc = graph_scratch(graph, want, &held_->capture_ptr);
+                held_->capture = rc == VS_OK ? capture : 0;
+                held_->capture_bytes = want;
+                if (rc != VS_OK) return rc;
+            }
+            *out = held_->capture_ptr;
+            return VS_OK;
+        }
         if (held_->bytes < bytes) {
-            if (stream_capturing(stream)) return VS_ERR_ARG;
             size_t want = 1u << 20;
             while (want < bytes) want <<= 1;
             void *fresh = nullptr;
@@ -706,13 +817,6 @@ template <typename TOut, int V, bool kCores> int launch_spmm_tc(const SpmmParams
     DeviceInfo *d;
     int rc = device_info(&d);
     if (rc != VS_OK) return rc;
-    if constexpr (kCores) {
-        // A captured cudaSpmm holds no pointer to the library's scratch, which a later, larger call replaces.
-        if (!t_no_scratch && stream_capturing(s)) {
-            NoScratchScope scope;
-            return launch_spmm_tc<TOut, V, kCores>(p, s);
-        }
-    }
     const SpmmMode mode = spmm_mode();
     constexpr SpmmCosts cost = kCores ? cores_costs(V) : kGatherCosts;
     if ((mode == SpmmMode::kDirect || (mode == SpmmMode::kAuto && spmm_direct_wanted(p, V, kCores, d))) &&
@@ -1083,10 +1187,6 @@ template <int V> int launch_sddmm_cores(const SddmmParams &p, cudaStream_t s) {
     DeviceInfo *d;
     int rc = device_info(&d);
     if (rc != VS_OK) return rc;
-    if (!t_no_scratch && stream_capturing(s)) {   // as in launch_spmm_tc
-        NoScratchScope scope;
-        return launch_sddmm_cores<V>(p, s);
-    }
     const char *e = std::getenv("VSPARSE_B200_SDDMM");
     const bool force_cores = e && !std::strcmp(e, "gather"), force_dense = e && !std::strcmp(e, "dense"), force_direct = e && !std::strcmp(e, "direct");
     const bool strides = p.batch == 1 || ((p.stride_lhs * 2) % 16 == 0 && (p.stride_rhs * 2) % 16 == 0);
@@ -1702,6 +1802,8 @@ VS_EXPORT int vs_release_scratch(void *stream, int every_stream) {
         r.second->retired = true;
         if (r.second->ptr) (void)cudaFreeAsync(r.second->ptr, r.first);
     }
+    int dev = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess) free_returned_scratch(dev, 0);   // what graphs that are gone have left
     return VS_OK;
 }
 
