@@ -234,3 +234,46 @@ def test_cuda_core_products_in_a_graph(V, m_vec, K, N):
     with torch.cuda.stream(stream):
         products()
     check(vals[2], "after the graph")
+
+
+@pytest.mark.parametrize("V", [1, 2, 4, 8])
+@pytest.mark.parametrize("N", [64, 72])
+def test_direct_spmm_computes_only_the_odd_rows_entry_by_entry(monkeypatch, V, N):
+    """A tile with columns in any order, columns named twice, columns outside the matrix and a non-finite sum, each in some of its
+    vector-rows, which hold more entries than the lanes of a row fetch at a time, or none: the other rows keep their bits."""
+    K = 300
+    a = custom([70, 0, 33, 100, 1] * (180 // V // 5 + 1), K, V, seed=5)
+    rows = lambda i: slice(int(a.row_offsets[i]), int(a.row_offsets[i + 1]))
+    vals = cvse.fill_random((a.nnz_vec * V,), np.float16, cvse.DIST_NORMAL, 1, 0.25)
+    B = cvse.fill_random((K, N), np.float16, cvse.DIST_NORMAL, 2, 0.5)
+    monkeypatch.setenv("VSPARSE_B200_SPMM", "direct")
+
+    def product(ci, B):
+        st = structure(a)
+        out = torch.full((a.m, N), float("nan"), dtype=torch.float16, device=DEV)
+        ops.spmm.cudaSpmm(a.m_vec, V, N, K, st[0], st[1], dev(ci), dev(vals), dev(B), out)
+        torch.cuda.synchronize()
+        assert ops.device_status() == 0
+        return out.float().cpu().numpy()
+
+    plain = product(a.col_indices, B)
+    ci = a.col_indices.copy()
+    ci[rows(0)] = ci[rows(0)][::-1]
+    ci[rows(7)] = np.random.default_rng(1).permutation(ci[rows(7)])
+    ci[rows(13)][40] = ci[rows(13)][39]
+    ci[rows(12)][-1] = K + 5
+    ci[rows(5)][0] = -3
+    odd = [0, 7, 13, 12, 5]
+    entries = vals.astype(np.float32).reshape(-1, V).copy()
+    entries[(ci < 0) | (ci >= K)] = 0   # no entries
+    a2 = cvse.CVSE(a.m_vec, K, V, a.row_offsets, np.clip(ci, 0, K - 1), a.row_indices)
+    want = spmm_oracle(a2, N, entries.ravel(), B)
+    got = product(ci, B)
+    assert_close(got, want, "odd rows")
+    untouched = np.repeat(~np.isin(np.arange(a.m_vec), odd), V)
+    assert np.array_equal(got[untouched], plain[untouched])
+    B[ci[rows(3)][50], 5] = np.inf   # named by some rows
+    got, want = product(a.col_indices, B), spmm_oracle(a, N, vals, B)
+    assert np.array_equal(np.isfinite(got), np.isfinite(want)) and not np.isfinite(want).all()
+    assert np.array_equal(got[:, :5], plain[:, :5]) or np.allclose(got[:, :5], plain[:, :5], rtol=2e-3, atol=2e-3)
+    assert_close(got[np.isfinite(want)], want[np.isfinite(want)], "non-finite operand")

@@ -14,7 +14,7 @@
 // How a CTA finds its entries without a plan.  Each of eight fill warps owns 16 rows of the tile (16 / V vector-rows)
 // and walks their entries in windows, one being scattered and the next one on its way: the entries below the chunk's last
 // column are scattered, a window that is used up makes room for the next.  That needs columns that ascend strictly
-// within a vector-row, which is checked on every entry.  A tile with a row that does not (unsorted, or a column named twice), and a tile with
+// within a vector-row, which is checked on every entry.  A row that does not (unsorted, or a column named twice), and a row with
 // a non-finite sum (0 x Inf of the densified tile, see spmm_dense.cuh), is computed again by the same CTA from the
 // CVSE arrays on CUDA cores, entry by entry as the reference does.
 //
@@ -64,39 +64,107 @@ struct Smem {   // offsets from the 1024-byte aligned base
     static constexpr int kBarDone = kBarFull + kBBuffers * 8;
     static constexpr int kTmemHolder = kBarDone + kBBuffers * 8;
     static constexpr int kAbort = kTmemHolder + 8;
-    static constexpr int kTotal = kAbort + 8;
+    static constexpr int kRedo = kAbort + 8;              // vector-rows of the tile to be computed entry by entry, a bit each
+    static constexpr int kTotal = kRedo + kTileM / 8;
 };
 constexpr int kSmemBytes = Smem::kTotal;   // the dynamic segment is 1024-byte aligned (nothing static lies ahead of it)
 static_assert(2 * (kSmemBytes + 1024) <= 228 * 1024, "two CTAs per SM");
 
-// One tile from the CVSE arrays on CUDA cores: a thread per (vector-row, 8 columns), fp32 sums in list order.
+// Vector-rows of one tile (a bit each in `which`) from the CVSE arrays on CUDA cores, fp32 sums in list order (the sums of
+// spmm_cc_kernel, bit for bit).  kLanes lanes share a vector-row, each with E columns of the tile.  They fetch the indices and
+// values of kLanes entries at a time, one each and a batch ahead, and pass them round; the rows of B of kAhead entries are in
+// flight together.  What bounds it: the latency of a gather, on the few SMs that the call's tiles occupy.  512 x 1024 x 256, V = 2, 90 %
+// sparse, every row with a column named twice: one entry at a time 84 us beside the 14 of the product, eight in flight 30, passed round 27.
 template <typename TOut, int V>
-__device__ __noinline__ void tile_by_entries(const SpmmParams &p, int b, int row0, int rows, int n0) {
+__device__ __noinline__ void rows_by_entries(const SpmmParams &p, int b, int row0, int rows, int n0, const uint32_t *which) {
+    constexpr int E = V >= 4 ? 4 : 8, kWords = E / 2;
+    constexpr int kLanes = kTileN / E, kWarpVecRows = 32 / kLanes;
+    constexpr int kAhead = V >= 4 ? 16 : 8;
+    constexpr int kValueWords = V >= 2 ? V / 2 : 1;
     const __half *values = static_cast<const __half *>(p.values) + (int64_t)b * p.stride_values;
-    const __half *rhs = static_cast<const __half *>(p.rhs) + (int64_t)b * p.stride_rhs;
     TOut *out = static_cast<TOut *>(p.out) + (int64_t)b * p.stride_out;
-    const int chunks = min(kTileN, p.N - n0) / 8;
-    for (int item = threadIdx.x; item < rows * chunks; item += kThreads) {
-        const int r = row0 + item / chunks, n = n0 + 8 * (item % chunks);
-        float acc[V][8];
+    const int lane = threadIdx.x & 31, l = lane % kLanes;
+    const int n = n0 + E * l;
+    const bool stored = n < p.N;   // lanes past the last column take part with the columns of the first lane
+    const __half *rhs = static_cast<const __half *>(p.rhs) + (int64_t)b * p.stride_rhs + (stored ? n : n0);
+    for (int base = (threadIdx.x >> 5) * kWarpVecRows; base < rows; base += kThreads / 32 * kWarpVecRows) {
+        const int i = base + lane / kLanes, r = row0 + i;
+        const bool live = i < rows && (which[i >> 5] >> (i & 31) & 1u);
+        if (!__any_sync(0xffffffffu, live)) continue;
+        int j = live ? __ldg(p.row_offsets + r) : 0;
+        const int end = live ? __ldg(p.row_offsets + r + 1) : 0;
+        float acc[V][E];
 #pragma unroll
         for (int v = 0; v < V; ++v)
 #pragma unroll
-            for (int e = 0; e < 8; ++e) acc[v][e] = 0.f;
-        for (int j = __ldg(p.row_offsets + r), end = __ldg(p.row_offsets + r + 1); j < end; ++j) {
-            const int c = __ldg(p.col_indices + j);
-            if ((unsigned)c >= (unsigned)p.K) continue;
-            float a[V];
-            VecLoad<__half, V>::load(values + (int64_t)j * V, a);
-            Chunk<__half> x;
-            x.load(rhs + (int64_t)c * p.N + n);
+            for (int e = 0; e < E; ++e) acc[v][e] = 0.f;
+        int col;
+        uint32_t val[kValueWords];
+        auto look_up = [&](int at) {   // a column outside the matrix counts as no entry: column -1
+            col = at < end ? __ldg(p.col_indices + at) : -1;
+            if ((unsigned)col >= (unsigned)p.K) col = -1;
+            ValueVec<V> a;
+            a.raw = typename ValueVec<V>::Raw{};
+            if (col >= 0) a.load(values + (int64_t)at * V);
+            if constexpr (V == 8) {
+                val[0] = a.raw.x; val[1] = a.raw.y; val[2] = a.raw.z; val[3] = a.raw.w;
+            } else if constexpr (V == 4) {
+                val[0] = a.raw.x; val[1] = a.raw.y;
+            } else {
+                val[0] = a.raw;
+            }
+        };
+        look_up(j + l);
+        while (__any_sync(0xffffffffu, j < end)) {
+            const int batch_col = col;
+            uint32_t batch_val[kValueWords];
 #pragma unroll
-            for (int v = 0; v < V; ++v)
+            for (int w = 0; w < kValueWords; ++w) batch_val[w] = val[w];
+            j += kLanes;
+            look_up(j + l);
 #pragma unroll
-                for (int e = 0; e < 8; ++e) acc[v][e] = fmaf(a[v], x.f[e], acc[v][e]);
+            for (int u0 = 0; u0 < kLanes; u0 += kAhead) {
+                uint32_t x[kAhead][kWords];
+                int c[kAhead];
+#pragma unroll
+                for (int u = 0; u < kAhead; ++u) {   // no entry: a row of zeros, whose values are zeros too
+                    c[u] = __shfl_sync(0xffffffffu, batch_col, u0 + u, kLanes);
+                    const __half *from = rhs + (int64_t)max(c[u], 0) * p.N;
+                    if constexpr (E == 8) {
+                        const uint4 q = __ldg(reinterpret_cast<const uint4 *>(from));
+                        x[u][0] = q.x; x[u][1] = q.y; x[u][2] = q.z; x[u][3] = q.w;
+                    } else {
+                        const uint2 q = __ldg(reinterpret_cast<const uint2 *>(from));
+                        x[u][0] = q.x; x[u][1] = q.y;
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < kAhead; ++u) {
+                    uint32_t av[kValueWords];
+                    float value[V];
+#pragma unroll
+                    for (int w = 0; w < kValueWords; ++w) {
+                        av[w] = __shfl_sync(0xffffffffu, batch_val[w], u0 + u, kLanes);
+                        const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&av[w]));
+                        value[2 * w] = f.x;
+                        if constexpr (V >= 2) value[2 * w + 1] = f.y;
+                    }
+#pragma unroll
+                    for (int w = 0; w < kWords; ++w) {
+                        if (c[u] < 0) x[u][w] = 0;
+                        const float2 f = __half22float2(*reinterpret_cast<const __half2 *>(&x[u][w]));
+#pragma unroll
+                        for (int v = 0; v < V; ++v) {
+                            acc[v][2 * w] = fmaf(value[v], f.x, acc[v][2 * w]);
+                            acc[v][2 * w + 1] = fmaf(value[v], f.y, acc[v][2 * w + 1]);
+                        }
+                    }
+                }
+            }
         }
+        if (live && stored)
 #pragma unroll
-        for (int v = 0; v < V; ++v) store_chunk(out + ((int64_t)r * V + v) * p.N + n, acc[v]);
+            for (int v = 0; v < V; ++v) store_chunk(out + ((int64_t)r * V + v) * p.N + n, acc[v]);
     }
 }
 
@@ -115,6 +183,7 @@ spmm_direct_kernel(const __grid_constant__ SpmmParams p, const __grid_constant__
     const uint32_t base = tc::smem_u32(sm);
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     volatile int *abort_flag = reinterpret_cast<volatile int *>(sm + Smem::kAbort);
+    uint32_t *redo_rows = reinterpret_cast<uint32_t *>(sm + Smem::kRedo);
     const uint32_t bar_full = base + Smem::kBarFull, bar_done = base + Smem::kBarDone;
 
     pdl_launch_dependents();
@@ -126,6 +195,7 @@ spmm_direct_kernel(const __grid_constant__ SpmmParams p, const __grid_constant__
         *abort_flag = 0;
         tc::fence_mbar_init();
     }
+    if (t < kTileM / 32) redo_rows[t] = 0;
     if (warp == kMmaWarp) {
         tc::tmem_alloc(base + Smem::kTmemHolder, kTmemCols);
         tc::tmem_relinquish();
@@ -155,7 +225,7 @@ spmm_direct_kernel(const __grid_constant__ SpmmParams p, const __grid_constant__
         // window 1).  Lanes move on by themselves, without a shuffle.
         const int row = mt * (kTileM / V) + warp * kRows + lane / kGroup;
         int next = 0, begin = 0, end = 0;
-        if (row < p.m_vec) {
+        if (mine && row < p.m_vec) {
             begin = __ldg(p.row_offsets + row);
             end = __ldg(p.row_offsets + row + 1);
         }
@@ -226,9 +296,10 @@ spmm_direct_kernel(const __grid_constant__ SpmmParams p, const __grid_constant__
             if (lane == 0) tc::mbar_arrive(bar_full + 8 * (c % kBBuffers));
             if (used_up) load_window();   // behind the fence, which waits for outstanding loads as well as for stores
         }
-        if (mine)
 #pragma unroll
-            for (int e = 0; e < kWindow; ++e) bad |= cols[0][e] != INT_MAX && cols[0][e] >= p.K;   // columns beyond the matrix
+        for (int e = 0; e < kWindow; ++e) bad |= cols[0][e] != INT_MAX && cols[0][e] >= p.K;   // columns beyond the matrix
+        const int fill_row = warp * kRows + lane / kGroup;
+        if (bad) atomicOr(redo_rows + (fill_row >> 5), 1u << (fill_row & 31));
 
         // =========================== epilogue ============================================================
         if (chunks > 0)   // the last chunk multiplied is the accumulator complete
@@ -253,6 +324,8 @@ spmm_direct_kernel(const __grid_constant__ SpmmParams p, const __grid_constant__
                     }
                     store_chunk(out + 8 * q, f);
                 }
+                const int row = (quarter * 32 + lane) / V;
+                if (probe != 0.0f) atomicOr(redo_rows + (row >> 5), 1u << (row & 31));
                 bad |= probe != 0.0f;
             }
         }
@@ -300,7 +373,7 @@ spmm_direct_kernel(const __grid_constant__ SpmmParams p, const __grid_constant__
     if (warp == kMmaWarp) tc::tmem_dealloc(tmem_base, kTmemCols);
     if (redo) {
         const int row0 = mt * (kTileM / V);
-        tile_by_entries<TOut, V>(p, b, row0, min(kTileM / V, p.m_vec - row0), n0);
+        rows_by_entries<TOut, V>(p, b, row0, min(kTileM / V, p.m_vec - row0), n0, redo_rows);
     }
 }
 
