@@ -1,5 +1,6 @@
 """Whose memory the library's plans live in: the caller's workspace is the tensor path's alone, and a
 stream's buffer belongs to one call at a time, and a graph's to the graph."""
+import ctypes
 import threading
 
 import numpy as np
@@ -157,3 +158,23 @@ def test_graphs_give_their_scratch_back():
     p.check("after the graphs")
     assert free[1] - free[-1] < 64 << 20
     assert _lib.lib().vs_release_scratch(stream.cuda_stream, 0) == 0
+
+
+def test_a_workspace_of_the_stated_size_serves_the_pair_kernel():
+    """A mask of 3 % of the vectors: the plan of the pair kernel is larger than that of the single-CTA kernel."""
+    p = Products(8, 1200, 1024, 512, 0.97)
+    size = _lib.lib().vs_sddmm_workspace_bytes(p.a.m_vec, p.a.n, p.a.nnz_vec)
+    workspace = torch.full((size + 256,), 0x5A, dtype=torch.uint8, device=DEV)
+    p.spmm(ops.spmm.wmmaSpmm)
+    p.sampled.fill_(float("nan"))
+    pairs = ctypes.c_int(0)
+    ops.set_workspace(workspace[:size])
+    _lib.lib().vs_kernel_timing(1, None, None)
+    try:
+        p.sddmm(ops.sddmm.wmmaSddmm)
+    finally:
+        _lib.lib().vs_kernel_timing(0, None, ctypes.byref(pairs))
+        ops.set_workspace(None)
+    p.check("in a workspace of that size")
+    assert pairs.value == 1   # the pair kernels are the ones that are timed
+    assert bool((workspace[size:] == 0x5A).all())

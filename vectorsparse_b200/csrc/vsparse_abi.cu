@@ -1766,8 +1766,10 @@ VS_EXPORT int64_t vs_spmm_t_workspace_bytes(int m_vec, int vec_length, int n, in
 
 VS_EXPORT int64_t vs_sddmm_workspace_bytes(int m_vec, int n, int nonzeros_vec) {
     if (m_vec <= 0 || n <= 0 || nonzeros_vec <= 0) return 0;
-    const int64_t bytes = sddmm_plan_bytes(m_vec, n, nonzeros_vec, nullptr);
-    return bytes <= kMaxPlanBytes ? bytes : 0;
+    int64_t bytes = sddmm_plan_bytes(m_vec, n, nonzeros_vec, nullptr);   // of the single-CTA form
+    if (bytes > kMaxPlanBytes) bytes = 0;
+    const int64_t pair = sddmm_pair_plan_bytes(m_vec, n, nonzeros_vec, nullptr, nullptr);
+    return n <= pairsddmm::kMaxPlanColumns && pair <= kMaxPlanBytes ? std::max(bytes, pair) : bytes;
 }
 
 VS_EXPORT int vs_set_workspace(void *workspace, int64_t bytes) {
