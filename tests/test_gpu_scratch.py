@@ -178,3 +178,18 @@ def test_a_workspace_of_the_stated_size_serves_the_pair_kernel():
     p.check("in a workspace of that size")
     assert pairs.value == 1   # the pair kernels are the ones that are timed
     assert bool((workspace[size:] == 0x5A).all())
+
+
+def test_a_large_plan_takes_about_what_it_needs():
+    """4096 x 4096 at V = 1: 134 MB of entries."""
+    p, stream = Products(1, 4096, 4096, 1024, 0.95), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    _lib.lib().vs_release_scratch(None, 1)
+    torch.cuda.synchronize()
+    before = torch.cuda.mem_get_info()[0]
+    with torch.cuda.stream(stream):
+        p.spmm(ops.spmm.cudaSpmm)
+        p.sddmm(ops.sddmm.cudaSddmm)
+    p.check("with a plan of its own")
+    assert before - torch.cuda.mem_get_info()[0] < 200 << 20
+    assert _lib.lib().vs_release_scratch(stream.cuda_stream, 0) == 0

@@ -285,6 +285,7 @@ public:
         if (held_->bytes < bytes) {
             size_t want = 1u << 20;
             while (want < bytes) want <<= 1;
+            if (bytes > 1u << 20) want = (bytes + want / 16 - 1) / (want / 16) * (want / 16);   // an eighth too much at most
             void *fresh = nullptr;
             cudaError_t e = cudaMallocAsync(&fresh, want, stream);
             if (e != cudaSuccess) {
