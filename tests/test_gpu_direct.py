@@ -277,3 +277,22 @@ def test_direct_spmm_computes_only_the_odd_rows_entry_by_entry(monkeypatch, V, N
     assert np.array_equal(np.isfinite(got), np.isfinite(want)) and not np.isfinite(want).all()
     assert np.array_equal(got[:, :5], plain[:, :5]) or np.allclose(got[:, :5], plain[:, :5], rtol=2e-3, atol=2e-3)
     assert_close(got[np.isfinite(want)], want[np.isfinite(want)], "non-finite operand")
+
+
+@pytest.mark.parametrize("V,m,n,k,density", [(1, 4096, 4096, 128, 0.003), (2, 4096, 4096, 256, 0.001), (4, 4096, 4096, 128, 0.003), (8, 4096, 4096, 256, 0.01),
+                                             (8, 512, 512, 1504, 0.3), (8, 16384, 16384, 64, 0.001)])
+def test_cuda_core_sddmm_of_sparse_masks_keeps_to_the_cuda_cores(monkeypatch, V, m, n, k, density):
+    """A few entries per row: the CUDA-core kernel's bits and not those of the tiles; a denser mask the other way round (0.3)."""
+    a = custom([int(n * density)] * (m // V), n, V, seed=3)
+    lhs = dev(cvse.fill_random((m, k), np.float16, cvse.DIST_NORMAL, 3, 0.25))
+    rhs = dev(cvse.fill_random((n, k), np.float16, cvse.DIST_NORMAL, 4, 0.25))
+    st, got = structure(a), {}
+    for mode in (None, "direct", "gather"):
+        monkeypatch.setenv("VSPARSE_B200_SDDMM", mode) if mode else monkeypatch.delenv("VSPARSE_B200_SDDMM", raising=False)
+        got[mode] = torch.full((a.nnz_vec * V,), float("nan"), dtype=torch.float16, device=DEV)
+        ops.sddmm.cudaSddmm(a.m_vec, k, n, a.nnz_vec, *st, lhs, rhs, got[mode], V)
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    assert torch.equal(got[None], got["gather" if density < 0.1 else "direct"])
+    assert density < 0.1 or not torch.equal(got["direct"], got["gather"])
+    assert torch.allclose(got["direct"].float(), got["gather"].float(), rtol=2e-3, atol=2e-3 * 0.25 * 0.25 * k**0.5)

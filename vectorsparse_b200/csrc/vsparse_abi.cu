@@ -1193,16 +1193,43 @@ template <int V> int launch_sddmm_cores(const SddmmParams &p, cudaStream_t s) {
     const bool strides = p.batch == 1 || ((p.stride_lhs * 2) % 16 == 0 && (p.stride_rhs * 2) % 16 == 0);
     const bool by_rule = !force_dense && !force_direct && sddmm_cores_wanted(p, V);
     if (!force_cores && !by_rule && strides && p.n > 0 && p.m_vec > 0) {
-        if constexpr (V > 1) {
-            const SddmmTimes t = sddmm_times(p, V, d);
-            if ((force_dense || (!force_direct && t.dense < t.direct)) && !t_no_scratch && sddmm_pair_enabled() && launch_sddmm_pair<__half, V>(p, s, d, &rc))
-                return rc;
-        }
-        if (!force_dense && launch_sddmm_direct<__half, V>(p, s, d, &rc)) return rc;
+        const SddmmTimes t = sddmm_times(p, V, d);
+        const bool pair_ok = V > 1 && !t_no_scratch && sddmm_pair_enabled() && p.n <= pairsddmm::kMaxPlanColumns;
+        const double dense = pair_ok ? sddmm_cores_dense_time(p, V, d, t) : 0.0;
+        const bool pair = pair_ok && !force_direct && (force_dense || dense < t.direct);
+        // The tile forms' estimates are up to 1.7 times too high where they are long; below, what the CUDA-core kernel is taken for is a clear gain.
+        const double tiled = pair ? dense : t.direct;
+        const bool sparse = !force_dense && !force_direct && sddmm_cores_time(p, V) + 1.2 < (tiled < 30.0 ? 1.0 : V == 1 ? 0.9 : 0.6) * tiled;
+        if constexpr (V > 1)
+            if (!sparse && pair && launch_sddmm_pair<__half, V>(p, s, d, &rc)) return rc;
+        if (!sparse && !force_dense && launch_sddmm_direct<__half, V>(p, s, d, &rc)) return rc;
     }
     return launch_sddmm_cc<__half, __half, V>(p, s);
 }
 int sddmm_cores_by_v(int V, const SddmmParams &p, cudaStream_t s) {
+// And where the mask is sparse: the tensor-core forms multiply every tile, the CUDA-core kernels read a row per entry.  Their time (us, fitted
+// to 64 x 64 to 16384 x 16384, k = 64 to 1504, 60 to 99.9 % sparse: 0.85 to 1.2 times the measured one): a launch, the bytes of
+// the gathered rows, and up to k = 256 the longest chain, a row's entries one behind the other; beyond, where a group of lanes has one
+// entry, its k.  16384 x 16384, k = 128, V = 4, 99.9 % sparse 182 us on tiles and 6.5 here; 4096 x 4096, k = 256, V = 8, 99 % 18 and 7.
+double sddmm_cores_time(const SddmmParams &p, int V) {
+    const int v = V == 1 ? 0 : V == 2 ? 1 : V == 4 ? 2 : 3;
+    const double gathered = (double)p.nnz_vec * p.k * p.batch;
+    if (p.k <= 256) {
+        constexpr double launch[4] = {2.1, 2.1, 2.1, 3.7}, rows[4] = {2.04e-7, 2.32e-7, 2.84e-7, 3.69e-7}, chain[4] = {0.071, 0.087, 0.093, 0.119};
+        return launch[v] + rows[v] * gathered + chain[v] * p.nnz_vec / std::max(p.m_vec, 1);
+    }
+    constexpr double rows[4] = {2.27e-7, 3.66e-7, 4.90e-7, 8.99e-7}, chain[4] = {2.8e-3, 3.1e-3, 2.9e-3, 1.0e-2};
+    return 2.5 + rows[v] * gathered + chain[v] * p.k;
+}
+// The planned form behind cudaSddmm, beside what sddmm_times() knows: a tile's contraction in series, 0.35 us for each 64 elements
+// (512 x 512, k = 1504: 17 us where the one-kernel form takes 9.6), and the sampling of a tile, which short vectors make the
+// longer part (4096 x 4096, k = 128, V = 2, 98 % sparse: 24.6 us, 14.9 without this).
+double sddmm_cores_dense_time(const SddmmParams &p, int V, const DeviceInfo *d, const SddmmTimes &t) {
+    const double per_row = (double)p.nnz_vec / std::max(p.m_vec, 1), launches = 8.0 + 1.1e-3 * 32.0 * per_row;
+    const double tiles = std::ceil((double)p.m_vec * V / 256.0) * std::ceil(p.n / 256.0) * p.batch;
+    const double sampling = (V == 2 ? 8000.0 : V == 4 ? 4400.0 : 4250.0) * tiles + (V == 2 ? 5.5 : V == 4 ? 2.0 : 1.0) * p.nnz_vec * p.batch;
+    return std::max(t.dense, launches + std::max(sampling / (1900.0 * d->sm_count), 0.35 * std::ceil(p.k / 64.0)));
+}
     NoScratchScope scope(t_ws_set);   // as in spmm_cores_by_v
     switch (V) {
         case 1: return launch_sddmm_cores<1>(p, s);
