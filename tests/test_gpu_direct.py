@@ -1,5 +1,7 @@
 """The one-kernel forms of the tensor-core products (small problems), forced at the sizes where their tiles, chunks and
 windows end, and on the inputs they hand to their entry-by-entry path; against the fp64 oracle, conftest tolerance."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
@@ -7,7 +9,7 @@ import torch
 import oracle
 from conftest import assert_close
 from gpu_util import DEV, custom, dev, problem, spmm_oracle, structure
-from vectorsparse_b200 import VS_PATH_CUDA_CORE, VS_PATH_TENSOR, cvse, ops
+from vectorsparse_b200 import VS_PATH_CUDA_CORE, VS_PATH_TENSOR, _lib, cvse, ops
 
 pytestmark = pytest.mark.gpu
 
@@ -88,8 +90,8 @@ def test_direct_sddmm_at_the_edges_of_its_tiles(monkeypatch, V, m_vec, n, k, len
 @pytest.mark.parametrize("mode", ["direct", "dense", "gather"])
 @pytest.mark.parametrize("V,m_vec,K,N", [(1, 130, 200, 72), (2, 70, 129, 136), (4, 40, 300, 8), (8, 33, 64, 264)])
 def test_cuda_core_spmm_with_fp16_results_in_every_form(monkeypatch, mode, V, m_vec, K, N):
-    """The entry point that takes V = 1 and dense widths that are multiples of 8: its one-kernel form, its planned form (widths of
-    both multiplying kernels) and the CUDA-core kernel; a column named twice on top of each."""
+    """The entry point that takes V = 1 and dense widths that are multiples of 8: its one-kernel form, its planned form on single CTAs
+    and the CUDA-core kernel; a column named twice on top of each."""
     monkeypatch.setenv("VSPARSE_B200_SPMM", mode)
     a = problem(cvse.GEN_BETA, 8, m_vec, K, V, 0.7)
     for repeat in (False, True):
@@ -103,6 +105,49 @@ def test_cuda_core_spmm_with_fp16_results_in_every_form(monkeypatch, mode, V, m_
         torch.cuda.synchronize()
         assert ops.device_status() == 0
         assert_close(out.float().cpu().numpy(), spmm_oracle(a, N, vals, B), f"{mode}, repeated column: {repeat}")
+
+
+@pytest.mark.parametrize("N", [128, 256])
+@pytest.mark.parametrize("V,m_vec,K", [(1, 300, 200), (2, 130, 449), (4, 70, 300), (8, 33, 640)])
+@pytest.mark.parametrize("what", ["plain", "repeated", "non-finite"])
+def test_cuda_core_spmm_behind_the_pair_kernel(monkeypatch, V, m_vec, K, N, what):
+    """Dense widths of the pair kernel, at every vector length; a column named twice, and an Inf in a row of B that some vector-rows name
+    and others do not, send the call to the CUDA-core kernel behind it."""
+    monkeypatch.setenv("VSPARSE_B200_SPMM", "dense")
+    a = problem(cvse.GEN_BETA, 8, m_vec, K, V, 0.7)
+    vals = cvse.fill_random((a.nnz_vec * V,), np.float16, cvse.DIST_NORMAL, 1, 0.25)
+    B = cvse.fill_random((K, N), np.float16, cvse.DIST_NORMAL, 2, 0.5)
+    if what == "repeated":
+        j = int(a.row_offsets[np.argmax(np.diff(a.row_offsets))])
+        a.col_indices[j + 1] = a.col_indices[j]
+    elif what == "non-finite":
+        B[a.col_indices[0], 5] = np.inf
+    out = torch.full((a.m, N), float("nan"), dtype=torch.float16, device=DEV)
+    pairs = ctypes.c_int(0)
+    _lib.lib().vs_kernel_timing(1, None, None)
+    ops.spmm.cudaSpmm(m_vec, V, N, K, *structure(a), dev(vals), dev(B), out)
+    _lib.lib().vs_kernel_timing(0, None, ctypes.byref(pairs))
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0 and pairs.value == 1   # the pair kernels are the ones that are timed
+    got, want = out.float().cpu().numpy(), spmm_oracle(a, N, vals, B)
+    finite = np.isfinite(want)
+    assert np.array_equal(np.isfinite(got), finite) and finite.all() == (what != "non-finite")
+    assert_close(got[finite], want[finite], what)
+
+
+@pytest.mark.parametrize("V", [1, 2, 8])
+def test_one_kernel_spmm_with_one_dense_operand_for_the_batch(monkeypatch, V):
+    monkeypatch.setenv("VSPARSE_B200_SPMM", "direct")
+    a = problem(cvse.GEN_UNIFORM, 4, 200 // V, 300, V, 0.8)
+    row = (a.nnz_vec * V + 7) // 8 * 8
+    vals = cvse.fill_random((3, row), np.float16, cvse.DIST_NORMAL, 1, 0.25)
+    B = cvse.fill_random((300, 72), np.float16, cvse.DIST_NORMAL, 2, 0.5)
+    out = torch.full((3, a.m, 72), float("nan"), dtype=torch.float16, device=DEV)
+    ops.spmm_batched(VS_PATH_CUDA_CORE, a.m_vec, V, 72, 300, *structure(a), dev(vals), dev(B), out)
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    for b in range(3):
+        assert_close(out[b].float().cpu().numpy(), spmm_oracle(a, 72, vals[b, :a.nnz_vec * V], B), f"entry {b}")
 
 
 @pytest.mark.parametrize("mode", ["direct", "dense", "gather"])
@@ -176,20 +221,27 @@ def test_fp32_spmm_on_staged_tiles_with_non_finite_operands(monkeypatch, shared)
     assert np.array_equal(got["rows"], got["tiles"], equal_nan=True)
 
 
-@pytest.mark.parametrize("V,m_vec,K,sparsity", [(1, 200, 1100, 0.99), (1, 200, 1100, 0.7), (2, 90, 1300, 0.99), (2, 90, 1300, 0.8), (1, 1040, 1025, 0.95)])
-def test_cuda_core_spmm_chooses_by_density(V, m_vec, K, sparsity):
-    """More than 1024 columns at V <= 2: the device takes the one-kernel form or the CUDA-core kernel behind it, on either side of its line;
-    two calls in a row on one stream."""
+# far from the line on either side
+@pytest.mark.parametrize("V,m_vec,K,sparsity,route", [(1, 200, 1100, 0.99, "gather"), (1, 200, 1100, 0.7, "direct"), (2, 90, 1300, 0.99, "gather"),
+                                                      (2, 90, 1300, 0.8, "direct"), (1, 1040, 1025, 0.995, "gather"), (8, 24, 4200, 0.997, "gather"), (8, 24, 4200, 0.9, "direct")])
+def test_cuda_core_spmm_chooses_by_density(monkeypatch, V, m_vec, K, sparsity, route):
+    """The device takes the one-kernel form or the CUDA-core kernel behind it, on either side of its line: the bits are those of the form that
+    the line names and not of the other, whose sums are in another order."""
     N = 200
     a = problem(cvse.GEN_BETA, 8, m_vec, K, V, sparsity)
-    for seed in (1, 2):
-        vals = cvse.fill_random((a.nnz_vec * V,), np.float16, cvse.DIST_NORMAL, seed, 0.25)
-        B = cvse.fill_random((K, N), np.float16, cvse.DIST_NORMAL, seed + 2, 0.5)
+    vals = cvse.fill_random((a.nnz_vec * V,), np.float16, cvse.DIST_NORMAL, 1, 0.25)
+    B = cvse.fill_random((K, N), np.float16, cvse.DIST_NORMAL, 3, 0.5)
+    got = {}
+    for mode in (None, "direct", "gather"):
+        monkeypatch.setenv("VSPARSE_B200_SPMM", mode) if mode else monkeypatch.delenv("VSPARSE_B200_SPMM", raising=False)
         out = torch.full((a.m, N), float("nan"), dtype=torch.float16, device=DEV)
         ops.spmm.cudaSpmm(m_vec, V, N, K, *structure(a), dev(vals), dev(B), out)
         torch.cuda.synchronize()
         assert ops.device_status() == 0
-        assert_close(out.float().cpu().numpy(), spmm_oracle(a, N, vals, B), f"seed {seed}")
+        got[mode] = out.float().cpu().numpy()
+    assert_close(got[None], spmm_oracle(a, N, vals, B), route)
+    assert not np.array_equal(got["direct"], got["gather"])
+    assert np.array_equal(got[None], got[route])
 
 
 @pytest.mark.parametrize("V,m_vec,K,N", [(1, 600, 2100, 512), (1, 300, 1200, 64), (8, 128, 8300, 128)])

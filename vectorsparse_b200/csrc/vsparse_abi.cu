@@ -743,9 +743,21 @@ struct SpmmCosts {
     float dense_per_stage, dense_per_entry, gather_per_row, gather_per_entry;
 };
 constexpr SpmmCosts kGatherCosts = {1100.0f, 0.0f, 370.0f, 4.7f};
-// The same with the CUDA-core kernel as the other formulation.
+// The same with the CUDA-core kernel as the other formulation, fitted at V = 1 and 2 to 512 x 4096 to 4096 x 4096, 64 to 1024 dense columns, 60 to
+// 99.7 % sparse.
 constexpr SpmmCosts cores_costs(int V) {
-    return {700.0f, V == 1 ? 1.0f : V == 2 ? 0.5f : 0.0f, 100.0f, V == 1 ? 5.2f : V == 2 ? 8.0f : V == 4 ? 13.0f : 20.0f};
+    return {700.0f, V == 1 ? 1.0f : V == 2 ? 0.5f : 0.0f, V == 1 ? 25.0f : V == 2 ? 50.0f : 100.0f, V == 1 ? 5.6f : V == 2 ? 13.0f : V == 4 ? 13.0f : 20.0f};
+}
+// What they come to where a product leaves SMs idle: the densified one has few tiles, each walking its columns in series; the CUDA-core
+// kernel few rows, with 0.3 us for an entry behind the other.  Without this 4096 x 4096 x 256 at V = 2 and 99 % sparse took 34 us on tiles that the
+// CUDA-core kernel needs 10 for; at 95 % the tiles' 41 against 36.
+SpmmCosts cores_costs_of(const SpmmParams &p, int V, int64_t items, int units, const DeviceInfo *d) {
+    SpmmCosts c = cores_costs(V);
+    const float idle = std::max(1.0f, (float)units / (float)std::max<int64_t>(items, 1));
+    c.dense_per_stage *= idle;
+    c.dense_per_entry *= idle;
+    c.gather_per_entry = std::max(c.gather_per_entry, 0.3f * 1900.0f * (float)d->sm_count * 128.0f / (float)p.N / (float)p.m_vec / (float)p.batch);
+    return c;
 }
 
 // What takes a call that the densified product does not: the gather kernels (wmmaSpmm) or the CUDA-core kernel (cudaSpmm
@@ -774,8 +786,9 @@ template <typename TOut, int V, bool kCores> bool launch_spmm_direct(const SpmmP
     // and more columns the line is a density, which the device knows.  Forced / CUDA-core kernel, us, 90 / 95 / 98 % sparse: V = 1,
     // 2048 x 2048 x 256 53 / 37 / 28 against 53 / 31 / 17, 419 x 2665 x 64 49 / 35 / 29 against 80 / 43 / 25; V = 2, 209 vector-rows of that
     // with 256 dense columns 34 / 31 / 25 against 72 / 41 / 23.
-    const bool by_density = kCores && V <= 2 && !forced && p.K > 1024;
-    if (by_density) cost = {(V == 2 ? 0.03f : tiles > 48 ? 0.045f : 0.035f) * (float)p.K * (float)p.m_vec / stages, 0.0f, 0.0f, 1.0f};
+    // V > 2: only past 4096 columns, where a product whose rows hold a few entries waits for 32 and more chunks, and with scratch.
+    const bool by_density = kCores && !forced && (V <= 2 ? p.K > 1024 : p.K > 4096 && !t_no_scratch);
+    if (by_density) cost = {(V > 2 ? 0.018f : V == 2 ? 0.03f : tiles > 48 ? 0.045f : 0.035f) * (float)p.K * (float)p.m_vec / stages, 0.0f, 0.0f, 1.0f};
     const bool always = forced || (kCores && !by_density) || (!kCores && cost.dense_per_entry == 0.0f && cost.dense_per_stage * stages < cost.gather_per_row * (float)p.m_vec);
     CUtensorMap map;
     static DeviceBits smem_set;
@@ -861,11 +874,17 @@ template <typename TOut, int V, bool kCores> int launch_spmm_tc(const SpmmParams
     int32_t *blk_offsets = reinterpret_cast<int32_t *>(plan + header_bytes);
     uint2 *blk_entries = reinterpret_cast<uint2 *>(plan + header_bytes + offsets_bytes);
     const int force_dense = mode == SpmmMode::kDense ? 1 : 0;
+    SpmmCosts planned = cost;
+    if constexpr (kCores) {
+        const bool pairs = use_b4 && p.N % 128 == 0 && spmm_pair_enabled();
+        const int64_t widths = pairs ? p.N / (p.N % 256 == 0 ? 256 : 128) : n_tiles;
+        planned = cores_costs_of(p, V, (int64_t)p.batch * m_tiles * widths, pairs ? d->sm_count / 2 : d->sm_count, d);
+    }
     // a dependent launch as well: in a stream of calls the plan kernel queues up behind the previous call's last kernel
     rc = (int)launch_overlapped(densespmm::dense_plan_kernel<false>, (unsigned)(groups + checks), densespmm::kPlanThreads, plan_smem, s,
                                 p.row_offsets, p.col_indices, (const int32_t *)nullptr, 0, p.m_vec, p.K, groups, rows_per_group,
-                                plan_blocks, blk_offsets, blk_entries, capacity, force_dense, cost.dense_per_stage,
-                                cost.gather_per_row, cost.gather_per_entry, cost.dense_per_entry, flag);
+                                plan_blocks, blk_offsets, blk_entries, capacity, force_dense, planned.dense_per_stage,
+                                planned.gather_per_row, planned.gather_per_entry, planned.dense_per_entry, flag);
     if (rc != VS_OK) return rc;
     const int64_t items = (int64_t)p.batch * n_tiles * m_tiles;
     const unsigned grid = (unsigned)(items < d->sm_count ? items : d->sm_count);   // one persistent CTA per SM
