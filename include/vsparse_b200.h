@@ -3,9 +3,9 @@
  *
  * Every entry point takes plain pointers and sizes.  Unless a function says "host", pointers are DEVICE
  * pointers owned by the caller; the library enqueues its kernels on `stream` (a cudaStream_t passed as void*)
- * and returns without synchronising.  One piece of device memory is the library's own: the tensor-path
- * operators keep a plan scratch per calling stream (cudaMallocAsync at the first call on a stream, and again
- * when a larger matrix needs more — make those calls outside stream capture; vs_release_scratch frees it).
+ * and returns without synchronising.  One piece of device memory is the library's own: the operators that
+ * multiply on the tensor cores (wmma*, and cuda* with fp16 results) keep a plan scratch per calling stream (cudaMallocAsync at the
+ * first call on a stream that needs one, and again when a larger matrix needs more; vs_release_scratch frees it; under capture, see vs_spmm).
  * A caller that hands over a buffer with vs_set_workspace gets a library that never allocates.
  *
  * Return value of every function: 0 on success, a negative VS_ERR_* code when the arguments are rejected
@@ -78,7 +78,9 @@ const char *vs_version(void);
  * reference.  A matrix that names a column twice in one vector-row (the reference's generator pads rows that
  * way, include/bm_test_utils.h:110-124, and its kernels add both values) is recognised on the device and goes
  * to the gather kernel, which adds them too.
- * Environment variable VSPARSE_B200_SPMM = "dense" | "gather" forces one formulation.  The first call with a plan on a
+ * Products of up to about one wave of tiles do the same in one kernel without a plan.  fp16 results with VS_PATH_CUDA_CORE take
+ * the same formulations, with the CUDA-core kernel in the place of the gather kernels; fp32 results there stay on the CUDA cores.
+ * Environment variable VSPARSE_B200_SPMM = "dense" | "gather" | "direct" (one kernel) forces one formulation.  The first call with a plan on a
  * stream allocates a scratch buffer with cudaMallocAsync on that stream (8 bytes per possible nonzero vector, m_vec * n
  * of them, at most 512 MB; reused and grown by later calls on the stream, freed by vs_release_scratch).  Under stream
  * capture a call's scratch belongs to the graph: it is allocated with cudaMalloc while the call is captured, shared by the
@@ -146,7 +148,9 @@ int vs_spmm_t_batched(int in_dtype, int out_dtype, int m_vec, int vec_length, in
  *
  * Tensor path: two formulations, chosen on the host from nonzeros_vec, the shape and k.  Dense 256 x 128 tiles
  * of lhs . rhs^T sampled at the mask (denser masks, k >= 128), or one gathered row of rhs per mask entry as in
- * the reference.  Environment variable VSPARSE_B200_SDDMM = "dense" | "gather" forces one.  The dense
+ * the reference; small problems do the former in one kernel without a plan ("direct").  fp16 results with VS_PATH_CUDA_CORE
+ * take the dense ones or the CUDA-core kernel ("gather").
+ * Environment variable VSPARSE_B200_SDDMM = "dense" | "gather" | "direct" forces one.  The dense
  * formulation keeps a plan scratch buffer per calling stream exactly as the tensor-path SpMM does (see vs_spmm);
  * with it, a mask entry whose column lies outside [0, n) is skipped instead of written as zero.
  * ---------------------------------------------------------------------------------------------------- */
@@ -217,7 +221,8 @@ int vs_attention_cvse_backward(int path, int m_vec, int vec_length, int n, int d
  *
  *  - Larger requests are refused with VS_ERR_SHAPE and a message on stderr; nothing is launched.
  *  - The call itself, and everything it calls, uses no cudaMalloc, cudaFree or allocating library routine: its
- *    SDDMM and SpMM steps always run the row-gather kernels, never the formulations that keep plan scratch.
+ *    SDDMM and SpMM steps run the one-kernel forms of small products or the row-gather kernels, never the
+ *    formulations that keep plan scratch.
  *  - The first call on each device looks up the array's device address (cudaGetSymbolAddress, with that device
  *    current).  Make that first call outside any stream capture.
  *  - All calls on a device share the one array, and it keeps what the last call left in it.  Nothing in it has
@@ -258,7 +263,8 @@ int vs_device_status(int clear, uint32_t *status);
  *
  *   vs_spmm_workspace_bytes / vs_sddmm_workspace_bytes / vs_spmm_t_workspace_bytes
  *                                                        bytes the dense formulation needs for such a call
- *                                                        (0: it is never used for this problem); no device needed
+ *                                                        (0: it is never used for this problem); no device needed.
+ *                                                        For the tensor path: vec_length 1 answers 0
  *   vs_set_workspace(ptr, bytes)                         from now on the tensor-path calls made by THIS host
  *                                                        thread put their plan in [ptr, ptr + bytes) when it
  *                                                        fits and run the row-gather formulation when it does

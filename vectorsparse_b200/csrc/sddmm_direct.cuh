@@ -5,7 +5,7 @@
 //     D[128 rows of lhs x tn mask columns] = lhs[128 x k] . rhs[tn x k]^T          one CTA per tile, tn = 128 or 64
 //
 // What bounds it.  One sampled product of 512 x 2048 x 256 is a microsecond of work; plan, multiplying kernel and twin
-// kernel took 17 us on the GPU, nearly all of it launches and dependent loads; this kernel takes 7.8 us (64 x 64 x 64: 7.1 ->
+// kernel took 17 us on the GPU, nearly all of it launches and dependent loads; this kernel takes 6.0 us (64 x 64 x 64: 7.1 ->
 // 2.5).  Here everything hangs on two short
 // chains that run side by side: TMA -> MMA -> tensor memory -> shared memory, and row offsets -> mask columns.
 //

@@ -6,7 +6,7 @@
 //
 // What bounds it.  One product of 2048 x 512 x 256 is a microsecond of work; the plan, the multiplying kernel and the
 // gather kernel that returns at once took 15.4 us on the GPU, nearly all of it launches and dependent loads; this kernel
-// takes 6.5 us (64 x 64 x 256: 11.2 -> 2.7).  Its chain is row offsets -> columns and values -> scatter -> MMA -> store, once,
+// takes 6.9 us (64 x 64 x 256: 11.2 -> 3.5).  Its chain is row offsets -> columns and values -> scatter -> MMA -> store, once,
 // and after the first chunk ~0.55 us per chunk: filling it (an MMA of 64 columns takes as long as one of 128, ~61 cycles).  128 x 64 tiles and two CTAs per SM because
 // at these sizes the number of CTAs is what is short; a larger problem re-reads A once per 64 columns and goes to the
 // pair kernel instead.
@@ -18,8 +18,8 @@
 // a non-finite sum (0 x Inf of the densified tile, see spmm_dense.cuh), is computed again by the same CTA from the
 // CVSE arrays on CUDA cores, entry by entry as the reference does.
 //
-// The K order of the MMAs is the one of the other densifying kernels (16 columns of A at a time, ascending), so that a
-// product has the same bits whichever of them multiplies it.
+// The K order of the MMAs is the one of the other densifying kernels (16 columns of A at a time, ascending), so that a product whose
+// columns ascend has the same bits whichever of them multiplies it; a row computed entry by entry has those of spmm_cc_kernel.
 //
 // Roles (320 threads): warps 0-7 fill, then epilogue (TMEM lanes 32 (w % 4) .., columns 32 (w / 4) ..); warp 8 the MMA-issuing
 // thread; warp 9 the thread that loads B by TMA.  Rings: 2 chunks of A (32 KiB each), 3 of B (16 KiB each).  Every

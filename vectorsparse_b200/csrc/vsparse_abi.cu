@@ -1203,29 +1203,6 @@ bool sddmm_cores_wanted(const SddmmParams &p, int V) {
     if (V == 1) return p.k <= 64 || (p.k > 256 && 2.0 * p.k * p.nnz_vec * p.batch < 1e8);
     return V == 2 && p.k <= 64 && p.nnz_vec < 0.03 * p.m_vec * p.n;
 }
-template <int V> int launch_sddmm_cores(const SddmmParams &p, cudaStream_t s) {
-    DeviceInfo *d;
-    int rc = device_info(&d);
-    if (rc != VS_OK) return rc;
-    const char *e = std::getenv("VSPARSE_B200_SDDMM");
-    const bool force_cores = e && !std::strcmp(e, "gather"), force_dense = e && !std::strcmp(e, "dense"), force_direct = e && !std::strcmp(e, "direct");
-    const bool strides = p.batch == 1 || ((p.stride_lhs * 2) % 16 == 0 && (p.stride_rhs * 2) % 16 == 0);
-    const bool by_rule = !force_dense && !force_direct && sddmm_cores_wanted(p, V);
-    if (!force_cores && !by_rule && strides && p.n > 0 && p.m_vec > 0) {
-        const SddmmTimes t = sddmm_times(p, V, d);
-        const bool pair_ok = V > 1 && !t_no_scratch && sddmm_pair_enabled() && p.n <= pairsddmm::kMaxPlanColumns;
-        const double dense = pair_ok ? sddmm_cores_dense_time(p, V, d, t) : 0.0;
-        const bool pair = pair_ok && !force_direct && (force_dense || dense < t.direct);
-        // The tile forms' estimates are up to 1.7 times too high where they are long; below, what the CUDA-core kernel is taken for is a clear gain.
-        const double tiled = pair ? dense : t.direct;
-        const bool sparse = !force_dense && !force_direct && sddmm_cores_time(p, V) + 1.2 < (tiled < 30.0 ? 1.0 : V == 1 ? 0.9 : 0.6) * tiled;
-        if constexpr (V > 1)
-            if (!sparse && pair && launch_sddmm_pair<__half, V>(p, s, d, &rc)) return rc;
-        if (!sparse && !force_dense && launch_sddmm_direct<__half, V>(p, s, d, &rc)) return rc;
-    }
-    return launch_sddmm_cc<__half, __half, V>(p, s);
-}
-int sddmm_cores_by_v(int V, const SddmmParams &p, cudaStream_t s) {
 // And where the mask is sparse: the tensor-core forms multiply every tile, the CUDA-core kernels read a row per entry.  Their time (us, fitted
 // to 64 x 64 to 16384 x 16384, k = 64 to 1504, 60 to 99.9 % sparse: 0.85 to 1.2 times the measured one): a launch, the bytes of
 // the gathered rows, and up to k = 256 the longest chain, a row's entries one behind the other; beyond, where a group of lanes has one
@@ -1249,6 +1226,29 @@ double sddmm_cores_dense_time(const SddmmParams &p, int V, const DeviceInfo *d, 
     const double sampling = (V == 2 ? 8000.0 : V == 4 ? 4400.0 : 4250.0) * tiles + (V == 2 ? 5.5 : V == 4 ? 2.0 : 1.0) * p.nnz_vec * p.batch;
     return std::max(t.dense, launches + std::max(sampling / (1900.0 * d->sm_count), 0.35 * std::ceil(p.k / 64.0)));
 }
+template <int V> int launch_sddmm_cores(const SddmmParams &p, cudaStream_t s) {
+    DeviceInfo *d;
+    int rc = device_info(&d);
+    if (rc != VS_OK) return rc;
+    const char *e = std::getenv("VSPARSE_B200_SDDMM");
+    const bool force_cores = e && !std::strcmp(e, "gather"), force_dense = e && !std::strcmp(e, "dense"), force_direct = e && !std::strcmp(e, "direct");
+    const bool strides = p.batch == 1 || ((p.stride_lhs * 2) % 16 == 0 && (p.stride_rhs * 2) % 16 == 0);
+    const bool by_rule = !force_dense && !force_direct && sddmm_cores_wanted(p, V);
+    if (!force_cores && !by_rule && strides && p.n > 0 && p.m_vec > 0) {
+        const SddmmTimes t = sddmm_times(p, V, d);
+        const bool pair_ok = V > 1 && !t_no_scratch && sddmm_pair_enabled() && p.n <= pairsddmm::kMaxPlanColumns;
+        const double dense = pair_ok ? sddmm_cores_dense_time(p, V, d, t) : 0.0;
+        const bool pair = pair_ok && !force_direct && (force_dense || dense < t.direct);
+        // The tile forms' estimates are up to 1.7 times too high where they are long; below, what the CUDA-core kernel is taken for is a clear gain.
+        const double tiled = pair ? dense : t.direct;
+        const bool sparse = !force_dense && !force_direct && sddmm_cores_time(p, V) + 1.2 < (tiled < 30.0 ? 1.0 : V == 1 ? 0.9 : 0.6) * tiled;
+        if constexpr (V > 1)
+            if (!sparse && pair && launch_sddmm_pair<__half, V>(p, s, d, &rc)) return rc;
+        if (!sparse && !force_dense && launch_sddmm_direct<__half, V>(p, s, d, &rc)) return rc;
+    }
+    return launch_sddmm_cc<__half, __half, V>(p, s);
+}
+int sddmm_cores_by_v(int V, const SddmmParams &p, cudaStream_t s) {
     NoScratchScope scope(t_ws_set);   // as in spmm_cores_by_v
     switch (V) {
         case 1: return launch_sddmm_cores<1>(p, s);
