@@ -90,8 +90,9 @@ NCU_TRAFFIC_BYTES = {
 def kernels_per_step(w, a=None):
     """Names of the library's kernels one step launches (the count is what `gpu_launches` reports)."""
     tensor = w.get("path") != 1
-    # the densified product runs on pairs of CTAs for dense widths that are multiples of 128, on single CTAs otherwise
-    pair = w["N"] % 128 == 0 and os.environ.get("VSPARSE_B200_SPMM_PAIR") != "0"
+    # the densified product runs on pairs of CTAs for dense widths above 128 that are multiples of 64, on single CTAs otherwise (128 itself
+    # on pairs where the products are few, which the streams here are not)
+    pair = w["N"] % 64 == 0 and w["N"] > 128 and os.environ.get("VSPARSE_B200_SPMM_PAIR") != "0"
     dense = "spmm_pair_kernel" if pair else "spmm_dense_kernel"
     if w["op"] == "attention":
         return ["sddmm_tma_kernel", "softmax_cvse_kernel", "dense_plan_kernel", dense,

@@ -1,5 +1,5 @@
 """The densifying tensor-core SpMM computed by pairs of CTAs (clusters of two, tcgen05 cta_group::2), which takes
-dense widths that are multiples of 128, against the fp64 oracle and against the single-CTA kernel it replaces there
+dense widths above 128 that are multiples of 64, against the fp64 oracle and against the single-CTA kernel it replaces there
 (VSPARSE_B200_SPMM_PAIR=0 switches it off).  Tolerance: conftest.assert_close (rel-L2 <= 5e-3, max-abs <= 2e-2)."""
 import numpy as np
 import pytest
@@ -43,6 +43,18 @@ def test_pairs_agree_with_the_oracle_and_the_single_cta_kernel(V, shape, monkeyp
             assert_close(two, want, f"pairs {shape} V={V} s={s}")
             assert_close(one, want, f"single {shape} V={V} s={s}")
             assert np.max(np.abs(two - one)) <= 1e-2
+
+
+@pytest.mark.parametrize("V,M,K,N", [(8, 264, 100, 192), (4, 520, 130, 320), (2, 256, 64, 448), (8, 40, 65, 1984)])
+def test_widths_whose_last_tile_is_partly_empty(V, M, K, N, monkeypatch):
+    """64, 128 and 192 columns left in the last 256-column tile: the second CTA's half past the matrix, or all of it.  The sums are those
+    of the single-CTA kernel, bit for bit (same order of columns)."""
+    a = problem(cvse.GEN_BETA, M + N, M // V, K, V, 0.7)
+    vals, B = spmm_inputs(a, N, np.float16, 5, sigma=0.5)
+    for out_t in (torch.float16, torch.float32):
+        two = run(a, N, vals, B, out_t, True, monkeypatch)
+        assert_close(two, spmm_oracle(a, N, vals, B), f"pairs N={N}")
+        assert np.array_equal(two, run(a, N, vals, B, out_t, False, monkeypatch))
 
 
 def test_many_items_per_pair_and_batch_strides(monkeypatch):

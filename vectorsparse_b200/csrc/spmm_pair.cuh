@@ -1,6 +1,6 @@
 // Tensor-core SpMM on densified tiles of the sparse matrix, computed by PAIRS of CTAs (a cluster of two SMs,
 // tcgen05 cta_group::2): the `wmmaSpmm` entry point of the reference (src/wmma_spmm.cu:388-409) for dense widths
-// that are multiples of 128.  Same formulation, plan and semantics as spmm_dense.cuh next to this file (see there
+// that are multiples of 64.  Same formulation, plan and semantics as spmm_dense.cuh next to this file (see there
 // for why a zero-filled tile of A beats a row gather on this part); what changes is who multiplies what:
 //
 //     C[256 rows x tn cols] += A_dense[256 x 64] * B[64 x tn]        per 64-wide block of A's columns, tn = 256 or 128
@@ -56,7 +56,7 @@ using densespmm::ValueVec;
 
 constexpr int kTileM = 256;                               // rows of A per work item: 128 per CTA of the pair
 constexpr int kCtaRows = 128;
-constexpr int kMaxTileN = 256;                            // columns of B per work item: 256, or 128 when N % 256 != 0
+constexpr int kMaxTileN = 256;                            // columns of B per work item: 256 or 128
 constexpr int kAStages = 6;                               // ring of densified A tiles
 constexpr int kBStages = 6;                               // ring of B tiles: loaded that many stages ahead
 constexpr int kFillCols = 32;                             // columns of a stage one fill warp owns: two plan buckets
@@ -151,7 +151,7 @@ struct Walk {
 // map_b: the dense operand as {N, K, batch}, box {64, 64, 1}; map_b2: the same memory as {64, K, N / 64, batch},
 // box {64, 64, 2, 1} (both 64-column slabs of a CTA's half of a 256-column tile in one copy); map_out: the output
 // as {N, rows, batch}, box {32, 32, 1}.  All with zero fill / clipping outside the matrix; no multicast anywhere.
-// tn: columns per work item (256 or 128), N % tn == 0.
+// tn: columns per work item (256 or 128), N % 64 == 0; the last tile of a row may be wider than what is left of the matrix.
 template <typename TOut, int V, bool kTransposed>
 __global__ void __launch_bounds__(kThreads, 1)
 spmm_pair_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_out,
@@ -447,7 +447,7 @@ spmm_pair_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b, 
             const int row0 = walk.mt * kTileM + (int)rank * kCtaRows + quarter * 32;
             const int col0 = walk.nt * tn + half * half_cols;   // accumulator column c of the item is its output column c
 #pragma unroll 1
-            for (int c0 = 0; c0 < half_cols; c0 += kStoreCols) {
+            for (int c0 = 0; c0 < half_cols && col0 + c0 < p.N; c0 += kStoreCols) {   // the last tile may reach past the matrix
                 uint32_t r[kStoreCols];
                 tc::tmem_ld_x32(lane_taddr + buf * kMaxTileN + (uint32_t)c0, r);
                 if (row0 < m_rows) {   // warp-uniform

@@ -704,11 +704,21 @@ template <typename K> int max_resident_pairs(K kernel, int block, size_t smem, D
     return n;
 }
 
-// The densified product by pairs of CTAs (spmm_pair.cuh) takes dense widths that are multiples of 128; the
-// single-CTA kernel (spmm_dense.cuh) the other widths.  VSPARSE_B200_SPMM_PAIR=0 keeps every width on the latter.
-inline bool spmm_pair_enabled() {
+// The densified product by pairs of CTAs (spmm_pair.cuh) takes dense widths from 128 up that are multiples of 64, the single-CTA
+// kernel (spmm_dense.cuh) the others, and 128 where there are more row tiles than its CTAs.  us, single CTAs / pairs, product with the matrix
+// and with its transpose: 64 x (2048 x 512 x N), V = 8, 90 % sparse: N = 128 28 / 33 and 33 / 39, 192 38 / 35 and 51 / 41, 448 65 / 59 and 85 / 64;
+// 4096 x 4096 x 1984, V = 2, 70 %: 261 / 149 and 281 / 161.  VSPARSE_B200_SPMM_PAIR=0 keeps every width on the former, =1 on the latter.
+inline bool spmm_pair_takes(int N, int64_t row_items, const DeviceInfo *d) {
     const char *e = std::getenv("VSPARSE_B200_SPMM_PAIR");
-    return !(e && !std::strcmp(e, "0"));
+    if (N % 64 != 0 || N < 128 || (e && !std::strcmp(e, "0"))) return false;
+    return N > 128 || row_items <= d->sm_count || e;
+}
+// Columns of B per work item of the pair kernel.  An item of 128 columns costs 0.9 of one of 256 (both fill the same tile of A), so
+// 256 it is, a partly empty last tile included, unless the narrower items need fewer waves of pairs.
+int spmm_pair_width(int N, int64_t row_items, int pairs) {
+    if (N <= 128) return 128;
+    const int64_t wide = row_items * ((N + 255) / 256), narrow = row_items * ((N + 127) / 128);
+    return 9 * ((narrow + pairs - 1) / pairs) < 10 * ((wide + pairs - 1) / pairs) ? 128 : 256;
 }
 // Enqueues the pair kernel for a call whose plan kernel has been enqueued; false if this device cannot hold it.
 template <typename TOut, int V, bool kTransposed>
@@ -728,8 +738,8 @@ bool launch_spmm_pair(const SpmmParams &q, cudaStream_t s, DeviceInfo *d, const 
         }
     }
     if (resident[dev] < 0) return false;
-    const int tn = q.N % 256 == 0 ? 256 : 128;
-    const int n_tiles = q.N / tn;
+    const int tn = spmm_pair_width(q.N, (int64_t)q.batch * m_tiles, resident[dev]);
+    const int n_tiles = (q.N + tn - 1) / tn;
     const int64_t items = (int64_t)q.batch * n_tiles * m_tiles;
     const unsigned pairs = (unsigned)(items < resident[dev] ? items : resident[dev]);
     TimedLaunch timed(s);
@@ -876,8 +886,9 @@ template <typename TOut, int V, bool kCores> int launch_spmm_tc(const SpmmParams
     const int force_dense = mode == SpmmMode::kDense ? 1 : 0;
     SpmmCosts planned = cost;
     if constexpr (kCores) {
-        const bool pairs = use_b4 && p.N % 128 == 0 && spmm_pair_enabled();
-        const int64_t widths = pairs ? p.N / (p.N % 256 == 0 ? 256 : 128) : n_tiles;
+        const bool pairs = use_b4 && spmm_pair_takes(p.N, (int64_t)p.batch * m_tiles, d);
+        const int tn = spmm_pair_width(p.N, (int64_t)p.batch * m_tiles, d->sm_count / 2);
+        const int64_t widths = pairs ? (p.N + tn - 1) / tn : n_tiles;
         planned = cores_costs_of(p, V, (int64_t)p.batch * m_tiles * widths, pairs ? d->sm_count / 2 : d->sm_count, d);
     }
     // a dependent launch as well: in a stream of calls the plan kernel queues up behind the previous call's last kernel
@@ -891,7 +902,7 @@ template <typename TOut, int V, bool kCores> int launch_spmm_tc(const SpmmParams
     rc = (int)cudaGetLastError();
     if (rc == VS_OK) {
         int rc_pair = VS_OK;
-        if (use_b4 && p.N % 128 == 0 && spmm_pair_enabled() &&
+        if (use_b4 && spmm_pair_takes(p.N, (int64_t)p.batch * m_tiles, d) &&
             launch_spmm_pair<TOut, V, false>(p, s, d, map, map_out, map_b4, blk_offsets, blk_entries, m_tiles, k_blocks, flag, checks, &rc_pair))
             rc = rc_pair;
         else
@@ -1431,7 +1442,7 @@ template <typename TOut, int V> int launch_spmm_t(const spmmt::Params &p, int m_
     const unsigned grid = (unsigned)(items < d->sm_count ? items : d->sm_count);   // one persistent CTA per SM
     if (rc == VS_OK) {
         int rc_pair = VS_OK;
-        if (use_b4 && q.N % 128 == 0 && spmm_pair_enabled() &&
+        if (use_b4 && spmm_pair_takes(q.N, (int64_t)q.batch * m_tiles, d) &&
             launch_spmm_pair<TOut, V, true>(q, s, d, map, map_out, map_b4, blk_offsets, blk_entries, m_tiles, k_blocks, flag, checks, &rc_pair))
             rc = rc_pair;
         else
