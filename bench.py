@@ -95,12 +95,11 @@ def kernels_per_step(w, a=None):
     pair = w["N"] % 64 == 0 and w["N"] > 128 and os.environ.get("VSPARSE_B200_SPMM_PAIR") != "0"
     dense = "spmm_pair_kernel" if pair else "spmm_dense_kernel"
     if w["op"] == "attention":
-        return ["sddmm_tma_kernel", "softmax_cvse_kernel", "dense_plan_kernel", dense,
-                "spmm_tma_kernel (returns at once unless the plan kernel chose it)"]
+        return ["attention_kernel"]
     if w["op"] == "attention_bwd":
         plan3 = ["dense_plan_kernel", dense,
                  "fallback kernel (returns at once unless the plan kernel chose it)"]
-        return ["sddmm_tma_kernel", "softmax_cvse_kernel"] + plan3 + ["sddmm_tma_kernel", "softmax_cvse_backward_kernel"] + plan3 + plan3
+        return ["attention_kernel"] + plan3 + plan3
     if w["op"] == "spmm_t":
         if os.environ.get("VSPARSE_B200_SPMM_T") == "gather":
             return ["spmm_t_kernel"]

@@ -26,6 +26,7 @@
 #include "vsparse_b200.h"
 #include "common.cuh"
 #include "cuda_core.cuh"
+#include "attention.cuh"
 #include "spmm_tc.cuh"
 #include "spmm_cc_tile.cuh"
 #include "spmm_tma.cuh"
@@ -1694,6 +1695,46 @@ int attention_scratch(void **out) {
     }
     *out = g_attention_scratch_ptr[dev];
     return VS_OK;
+namespace {
+// Attention in one kernel per direction (attention.cuh).
+template <int D, int W, bool kBackward> int launch_attention(const attention::Params &p, int batch, cudaStream_t s) {
+    constexpr int rows = attention::kThreads / (32 * W);
+    attention::attention_kernel<D, W, kBackward><<<dim3((unsigned)((p.m_vec + rows - 1) / rows), (unsigned)batch), attention::kThreads, 0, s>>>(p);
+    return (int)cudaGetLastError();
+}
+// Warps per vector-row: one where the rows fill the GPU three times over, which spares the exchange between them (128 heads, sequence
+// 4096: 588 / 670 / 793 us with 1 / 2 / 4 warps); more where the rows are few (2 heads, sequence 1024, 154 keys: 12.6 / 9.3 / 8.5 us) and long enough
+// for a chunk each.  VSPARSE_B200_ATTENTION_WARPS chooses.
+template <int D, bool kBackward> int launch_attention_rows(const attention::Params &p, int batch, DeviceInfo *d, cudaStream_t s) {
+    const int64_t rows = (int64_t)p.m_vec * batch, wave = (int64_t)d->sm_count * attention::kCtasPerSm<D, kBackward> * (attention::kThreads / 32);
+    const int keys = p.nnz_vec / p.m_vec;
+    const char *e = std::getenv("VSPARSE_B200_ATTENTION_WARPS");
+    const int warps = e ? std::atoi(e) : rows >= 3 * wave || keys <= 32 ? 1 : 2 * rows >= 3 * wave || keys <= 64 ? 2 : 4;
+    if (warps <= 1) return launch_attention<D, 1, kBackward>(p, batch, s);
+    if (warps == 2) return launch_attention<D, 2, kBackward>(p, batch, s);
+    return launch_attention<D, 4, kBackward>(p, batch, s);
+}
+// Whether the one-kernel form takes a call; what it does not take, and every refusal, is the operators' own.
+// VSPARSE_B200_ATTENTION=steps|fused.
+bool attention_fused(int path, int m_vec, int V, int n, int d, int nnz_vec, int batch, std::initializer_list<const void *> indices,
+                     std::initializer_list<const void *> sources, std::initializer_list<const void *> results) {
+    const char *e = std::getenv("VSPARSE_B200_ATTENTION");
+    if (e && !std::strcmp(e, "steps")) return false;
+    if (path != VS_PATH_TENSOR || !(V == 2 || V == 4 || V == 8) || (d != 64 && d != 128)) return false;
+    if (m_vec < 1 || n < 1 || nnz_vec < 1 || batch < 1 || batch > kMaxBatch || (int64_t)m_vec * V > 0x7fffffffll || (int64_t)nnz_vec * V > 0x7fffffffll) return false;
+    // Gathering costs the same for 2 queries as for 8, the operators' dense tiles do not: at d = 128 and V < 8 they win once there is
+    // enough work (32 heads, sequence 2048, V = 4, 205 keys: 142 against 171 us; one million keys break even).
+    if (d == 128 && V < 8 && (int64_t)nnz_vec * batch > 1000000 && !(e && !std::strcmp(e, "fused"))) return false;
+    for (const void *x : indices)
+        if (!x) return false;
+    for (const void *x : sources)   // read 32 bytes at a time
+        if (!x || reinterpret_cast<uintptr_t>(x) % 32 != 0) return false;
+    for (const void *x : results)
+        if (!x || !aligned16(x)) return false;
+    return (int64_t)nnz_vec * V % 8 == 0;
+}
+}  // namespace
+
 }
 }  // namespace
 
@@ -1716,6 +1757,28 @@ VS_EXPORT int vs_attention_cvse_static(int path, int m_vec, int vec_length, int 
     int rc = attention_scratch(&scratch);
     if (rc != VS_OK) return rc;
     NoScratchScope no_allocation;   // SDDMM and SpMM below: the formulations without plan scratch
+    if (attention_fused(path, m_vec, vec_length, n, d, nonzeros_vec, batch, {row_indices, row_offsets, col_indices, t_offsets, t_rows, t_src},
+                        {q, kmat, vmat, grad_out}, {grad_q, grad_k, grad_v, probs_workspace, grad_workspace})) {
+        DeviceInfo *info = nullptr;
+        int rc = device_info(&info);
+        if (rc != VS_OK) return rc;
+        attention::Params p;
+        p.m_vec = m_vec; p.V = vec_length; p.n = n; p.nnz_vec = nonzeros_vec;
+        p.row_offsets = row_offsets; p.col_indices = col_indices;
+        p.q = static_cast<const __half *>(q); p.k = static_cast<const __half *>(kmat); p.v = static_cast<const __half *>(vmat);
+        p.out = static_cast<__half *>(grad_q); p.probs = static_cast<__half *>(probs_workspace);
+        p.grad_out = static_cast<const __half *>(grad_out); p.grad_scores = static_cast<__half *>(grad_workspace);
+        p.scale = scale;
+        cudaStream_t st = static_cast<cudaStream_t>(stream);
+        rc = d == 64 ? launch_attention_rows<64, true>(p, batch, info, st) : launch_attention_rows<128, true>(p, batch, info, st);
+        if (rc != VS_OK) return rc;
+        // dV = P^T dO,  dK = dS^T Q
+        rc = vs_spmm_t_batched(VS_F16, VS_F16, m_vec, vec_length, d, n, t_offsets, t_rows, t_src, probs_workspace, grad_out, grad_v,
+                               batch, s_ws, s_q, s_k, stream);
+        if (rc != VS_OK) return rc;
+        return vs_spmm_t_batched(VS_F16, VS_F16, m_vec, vec_length, d, n, t_offsets, t_rows, t_src, grad_workspace, q, grad_k, batch,
+                                 s_ws, s_q, s_k, stream);
+    }
     return vs_attention_cvse(path, m_vec, vec_length, n, d, nonzeros_vec, row_indices, row_offsets, col_indices, q, kmat,
                              vmat, out, scratch, scale, batch, stream);
 }
@@ -1756,6 +1819,19 @@ VS_EXPORT int vs_spmm_host(int path, int in_dtype, int out_dtype, int m_vec, int
     int32_t *d_idx, *d_off, *d_col;
     void *d_val, *d_rhs, *d_out;
     VS_CUDA_TRY(bufs.alloc((void **)&d_idx, b_idx));
+    if (attention_fused(path, m_vec, vec_length, n, d, nonzeros_vec, batch, {row_indices, row_offsets, col_indices}, {q, kmat, vmat}, {out, workspace})) {
+        DeviceInfo *info = nullptr;
+        const int rc = device_info(&info);
+        if (rc != VS_OK) return rc;
+        attention::Params p;
+        p.m_vec = m_vec; p.V = vec_length; p.n = n; p.nnz_vec = nonzeros_vec;
+        p.row_offsets = row_offsets; p.col_indices = col_indices;
+        p.q = static_cast<const __half *>(q); p.k = static_cast<const __half *>(kmat); p.v = static_cast<const __half *>(vmat);
+        p.out = static_cast<__half *>(out); p.probs = static_cast<__half *>(workspace);
+        p.grad_out = nullptr; p.grad_scores = nullptr; p.scale = scale;
+        cudaStream_t st = static_cast<cudaStream_t>(stream);
+        return d == 64 ? launch_attention_rows<64, false>(p, batch, info, st) : launch_attention_rows<128, false>(p, batch, info, st);
+    }
     VS_CUDA_TRY(bufs.alloc((void **)&d_off, b_off));
     VS_CUDA_TRY(bufs.alloc((void **)&d_col, b_col));
     VS_CUDA_TRY(bufs.alloc(&d_val, b_val));
