@@ -111,6 +111,8 @@ def kernels_per_step(w, a=None):
         return ["dense_plan_kernel", dense,
                 "spmm_tma_kernel (returns at once unless the plan kernel chose it)"]
     if w["op"] == "spmm":   # the CUDA-core entry point: fp16 results come from the tensor cores where that is quicker
+        if w.get("dtype") == "f32" and w["N"] >= 256 and 1 - w["s"] > {1: 0.102, 2: 0.11, 4: 0.205, 8: 0.13}[w["V"]]:
+            return ["spmm_split_prepare", "spmm_split_kernel", "spmm_cc_standby_kernel (returns at once unless the others left it the call)"]
         if w.get("dtype") == "f32" or os.environ.get("VSPARSE_B200_SPMM") == "gather":
             return ["spmm_cc_kernel"]
         return ["dense_plan_kernel", dense, "spmm_cc_standby_kernel (returns at once unless the plan kernel chose it)"]

@@ -150,7 +150,9 @@ VS_FAST_CALL(spmm, 13) {
     if (!a.ok) Py_RETURN_NONE;
     const void *pv = values->const_data_ptr(), *pr = rhs->const_data_ptr();
     void *po = out->mutable_data_ptr();
-    const int64_t sv = batch_stride(values, 2, batch), sr = batch_stride(rhs, 3, batch), so = batch_stride(out, 3, batch);
+    int64_t sv = batch_stride(values, 2, batch);
+    const int64_t sr = batch_stride(rhs, 3, batch), so = batch_stride(out, 3, batch);
+    if (batch == 1) sv = (values->numel() + 7) / 8 * 8;   // no stride: how many values there are at most
     return call(a, [&](void *s) {
         return g_lib.spmm(path, in_t, out_t, m_vec, V, k, n, ri, ro, ci, pv, pr, po, batch, sv, sr, so, s);
     });

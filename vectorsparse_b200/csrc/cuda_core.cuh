@@ -95,14 +95,14 @@ __global__ void __launch_bounds__(kCcThreads) spmm_cc_kernel(const SpmmParams p)
 // The same work enqueued behind a densifying kernel that usually has taken the call: returns at once unless the plan
 // header says otherwise, and walks its items in strides, because a grid of one thread per item takes longer to start and
 // return than the rest of a small call.
-template <typename TIn, typename TOut, int V>
+template <typename TIn, typename TOut, int V, int kChunks = 1>
 __global__ void __launch_bounds__(kCcThreads) spmm_cc_standby_kernel(const SpmmParams p, const int32_t *plan_hdr, int plan_checks) {
     pdl_launch_dependents();
     pdl_wait();
     if (plan_dense_chosen(plan_hdr, plan_checks)) return;
-    const int64_t per = (int64_t)p.m_vec * (p.N / Chunk<TIn>::kElems), total = per * p.batch;
+    const int64_t per = (int64_t)p.m_vec * (p.N / (Chunk<TIn>::kElems * kChunks)), total = per * p.batch;
     for (int64_t i = (int64_t)blockIdx.x * kCcThreads + threadIdx.x; i < total; i += (int64_t)gridDim.x * kCcThreads)
-        spmm_cc_item<TIn, TOut, V, 1>(p, (int)(i / per), i % per);
+        spmm_cc_item<TIn, TOut, V, kChunks>(p, (int)(i / per), i % per);
 }
 
 // ---- SDDMM --------------------------------------------------------------------------------------------------

@@ -34,6 +34,7 @@
 #include "spmm_direct.cuh"
 #include "sddmm_pair.cuh"
 #include "spmm_pair.cuh"
+#include "spmm_split.cuh"
 #include "spmm_t.cuh"
 #include "sddmm_tc.cuh"
 #include "sddmm_tma.cuh"
@@ -472,6 +473,20 @@ int make_blocked_map(CUtensorMap *map, const void *ptr, uint64_t rows, uint64_t 
     return r == CUDA_SUCCESS ? VS_OK : VS_ERR_ARG;
 }
 
+// Tiles of cols x rows fp16 (or bf16) values, `parts` of them side by side, one after another: {cols, rows, parts, tiles}, a copy takes
+// all parts of `box_tiles` tiles.  128-byte swizzle (cols = 64).
+int make_packed_map(CUtensorMap *map, const void *ptr, uint64_t cols, uint64_t rows, uint64_t parts, uint64_t tiles, uint32_t box_tiles) {
+    EncodeTiledFn fn = encode_tiled_fn();
+    if (!fn || tiles > 0x7fffffffull) return VS_ERR_DEVICE;
+    const cuuint64_t dims[4] = {cols, rows, parts, tiles};
+    const cuuint64_t strides[3] = {cols * 2, cols * rows * 2, cols * rows * parts * 2};
+    const cuuint32_t box[4] = {(cuuint32_t)cols, (cuuint32_t)rows, (cuuint32_t)parts, box_tiles};
+    const cuuint32_t estr[4] = {1, 1, 1, 1};
+    CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, const_cast<void *>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                    CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+    return r == CUDA_SUCCESS ? VS_OK : VS_ERR_ARG;
+}
+
 // ---- SpMM dispatch ----------------------------------------------------------------------------------------
 // 16-byte chunks of the dense width per thread of spmm_cc_kernel: several where the width allows it and the accumulators
 // stay in registers (64 at most); VSPARSE_B200_SPMM_CC_CHUNKS=1|2|4 caps them.
@@ -549,10 +564,13 @@ template <typename TIn, typename TOut, int V> int launch_spmm_cc(const SpmmParam
     return (int)cudaGetLastError();
 }
 
+int spmm_split(int V, const SpmmParams &p, cudaStream_t s, bool *taken);
 template <typename TIn, typename TOut> int spmm_cc_by_v(int V, const SpmmParams &p, cudaStream_t s) {
     if constexpr (sizeof(TIn) == 4) {
         bool taken = false;
-        const int rc = spmm_cc_tile(V, p, s, &taken);
+        int rc = spmm_split(V, p, s, &taken);
+        if (rc != VS_OK || taken) return rc;
+        rc = spmm_cc_tile(V, p, s, &taken);
         if (rc != VS_OK || taken) return rc;
     }
     switch (V) {
@@ -937,6 +955,88 @@ int spmm_cores_by_v(int V, const SpmmParams &p, cudaStream_t s) {
         case 8: return launch_spmm_tc<__half, 8, true>(p, s);
     }
     return VS_ERR_VEC_LENGTH;
+}
+
+// ---- fp32 SpMM from bf16 parts ------------------------------------------------------------------------------
+template <int V, int kChunks> int launch_spmm_f32_standby(const SpmmParams &p, cudaStream_t s, DeviceInfo *d, const int32_t *verdict, int checks) {
+    const int64_t blocks = ((int64_t)p.m_vec * (p.N / (4 * kChunks)) * p.batch + kCcThreads - 1) / kCcThreads, cap = (int64_t)d->sm_count * 8;
+    return (int)launch_overlapped(spmm_cc_standby_kernel<float, float, V, kChunks>, (unsigned)(blocks < cap ? blocks : cap), kCcThreads, 0, s, p, verdict, checks);
+}
+// Leaves *taken false where the call is not one for it.
+template <int V> int launch_spmm_split(const SpmmParams &p, int64_t vectors, cudaStream_t s, bool forced, DeviceInfo *d, bool *taken) {
+    static int resident[kMaxDevices];   // 0 = not asked yet, -1 = the kernel cannot run here
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return VS_OK;
+    if (resident[dev] == 0) {
+        const int n = set_smem(splitspmm::spmm_split_kernel, splitspmm::kSmemBytes) == VS_OK
+                          ? max_resident_pairs(splitspmm::spmm_split_kernel, splitspmm::kThreads, splitspmm::kSmemBytes, d) : 0;
+        resident[dev] = n > 0 ? n : -1;
+    }
+    if (resident[dev] < 0) return VS_OK;
+    const int64_t M = (int64_t)p.m_vec * V;
+    splitspmm::PrepParams q;
+    q.batch_a = p.batch > 1 && p.stride_values ? p.batch : 1;
+    q.batch_b = p.batch > 1 && p.stride_rhs ? p.batch : 1;
+    q.Kp = (p.K + 63) / 64 * 64;
+    q.Np = (p.N + 63) / 64 * 64;
+    const int k_blocks = q.Kp / 64, m_tiles = (int)((M + splitspmm::kTileM - 1) / splitspmm::kTileM);
+    const int64_t row_items = (int64_t)p.batch * m_tiles, wide = (p.N + 255) / 256, narrow = (p.N + 127) / 128;
+    auto waves = [&](int64_t items) { return (double)((items + resident[dev] - 1) / resident[dev]); };
+    const double t_wide = 2.2 * waves(row_items * wide), t_narrow = 1.2 * waves(row_items * narrow);
+    const int tn = t_narrow < t_wide ? 128 : 256, n_tiles = (int)(tn == 256 ? wide : narrow);
+    const int row_tiles = (int)((M + 127) / 128), slabs = q.Np / 64;
+    const int64_t a_elems = (int64_t)q.batch_a * row_tiles * 128 * q.Kp, b_elems = (int64_t)q.batch_b * q.Kp * q.Np;
+    // us: 64 columns of an item by a pair, the preparation at 4 TB/s, launches; against the CUDA-core kernel per vector and column
+    const double split_us = k_blocks * std::min(t_wide, t_narrow) + (double)(6 * a_elems + 10 * b_elems) / 4e6 + 10.0;
+    constexpr double kCoresPs = V == 1 ? 0.195 : V == 2 ? 0.23 : V == 4 ? 0.29 : 0.45, kMinDensity = V == 1 ? 0.102 : V == 2 ? 0.11 : V == 4 ? 0.205 : 0.13;
+    q.min_vectors = forced ? 0 : (int64_t)std::max(1.1 * split_us / (kCoresPs * 1e-6 * p.N * p.batch), kMinDensity * p.m_vec * (double)p.K);
+    if (!forced && (vectors < q.min_vectors || p.N < 256)) return VS_OK;
+    const int64_t units = (int64_t)q.batch_a * p.m_vec + b_elems / (8 * splitspmm::kPrepThreads) + 1;
+    const int checks = (int)std::min<int64_t>(units, 8 * d->sm_count);
+    const int64_t header = ((4 + checks) * 4 + 255) / 256 * 256, a_bytes = (a_elems * 6 + 255) / 256 * 256, bytes = header + a_bytes + b_elems * 6;
+    if (bytes > kMaxPlanBytes || row_items * n_tiles * k_blocks > 0x7fffffffll) return VS_OK;
+    CUtensorMap map_out;
+    if (make_tile_map(&map_out, p.out, true, (uint64_t)M, (uint64_t)p.N, (uint64_t)p.batch, (uint64_t)p.stride_out, splitspmm::kStoreCols, 32) != VS_OK) return VS_OK;
+    uint8_t *mem = nullptr;
+    PlanScratch scratch;
+    if (scratch.take(d, s, (size_t)bytes, reinterpret_cast<void **>(&mem)) != VS_OK) return VS_OK;
+    q.verdict = reinterpret_cast<int32_t *>(mem);
+    q.a = reinterpret_cast<__nv_bfloat16 *>(mem + header);
+    q.b = reinterpret_cast<__nv_bfloat16 *>(mem + header + a_bytes);
+    CUtensorMap map_a, map_b;
+    if (make_packed_map(&map_a, q.a, 64, 128, 3, (uint64_t)q.batch_a * row_tiles * k_blocks, 1) != VS_OK ||
+        make_packed_map(&map_b, q.b, 64, 64, 3, (uint64_t)q.batch_b * k_blocks * slabs, (uint32_t)(tn / 128)) != VS_OK)
+        return VS_OK;
+    *taken = true;
+    int rc = (int)launch_overlapped(splitspmm::spmm_split_prepare<V>, (unsigned)checks, splitspmm::kPrepThreads, 0, s, p, q);
+    if (rc != VS_OK) return rc;
+    const int64_t items = row_items * n_tiles;
+    rc = (int)launch_pairs(splitspmm::spmm_split_kernel, (unsigned)std::min<int64_t>(items, resident[dev]), splitspmm::kThreads, (size_t)splitspmm::kSmemBytes, s, true,
+                           p, V, map_a, map_b, map_out, tn, q.batch_a, q.batch_b, m_tiles, n_tiles, k_blocks, row_tiles, slabs, d->status, q.verdict, checks);
+    if (rc != VS_OK) return rc;
+    const int chunks = spmm_cc_chunks(4 * V, 4, p.N);
+    if constexpr (V <= 4) {
+        if (chunks == 4) return launch_spmm_f32_standby<V, 4>(p, s, d, q.verdict, checks);
+    }
+    if (chunks == 2) return launch_spmm_f32_standby<V, 2>(p, s, d, q.verdict, checks);
+    return launch_spmm_f32_standby<V, 1>(p, s, d, q.verdict, checks);
+}
+// VSPARSE_B200_SPMM_F32=cores|split chooses one.
+int spmm_split(int V, const SpmmParams &p, cudaStream_t s, bool *taken) {
+    const char *e = std::getenv("VSPARSE_B200_SPMM_F32");
+    const bool forced = e && !std::strcmp(e, "split");
+    if ((e && !std::strcmp(e, "cores")) || t_no_scratch || t_ws_set || p.K < 1) return VS_OK;
+    DeviceInfo *d = nullptr;
+    const int rc = device_info(&d);
+    if (rc != VS_OK) return rc;
+    const int64_t vectors = p.stride_values > 0 ? p.stride_values / V : (int64_t)p.m_vec * p.K;
+    switch (V) {
+        case 1: return launch_spmm_split<1>(p, vectors, s, forced, d, taken);
+        case 2: return launch_spmm_split<2>(p, vectors, s, forced, d, taken);
+        case 4: return launch_spmm_split<4>(p, vectors, s, forced, d, taken);
+        case 8: return launch_spmm_split<8>(p, vectors, s, forced, d, taken);
+    }
+    return VS_OK;
 }
 
 // ---- SDDMM dispatch ---------------------------------------------------------------------------------------
@@ -1595,6 +1695,46 @@ VS_EXPORT int vs_softmax_cvse_backward(int dtype, int m_vec, int vec_length, con
                            : softmax_backward_by_v<float>(vec_length, p, batch, s);
 }
 
+namespace {
+// Attention in one kernel per direction (attention.cuh).
+template <int D, int W, bool kBackward> int launch_attention(const attention::Params &p, int batch, cudaStream_t s) {
+    constexpr int rows = attention::kThreads / (32 * W);
+    attention::attention_kernel<D, W, kBackward><<<dim3((unsigned)((p.m_vec + rows - 1) / rows), (unsigned)batch), attention::kThreads, 0, s>>>(p);
+    return (int)cudaGetLastError();
+}
+// Warps per vector-row: one where the rows fill the GPU three times over, which spares the exchange between them (128 heads, sequence
+// 4096: 588 / 670 / 793 us with 1 / 2 / 4 warps); more where the rows are few (2 heads, sequence 1024, 154 keys: 12.6 / 9.3 / 8.5 us) and long enough
+// for a chunk each.  VSPARSE_B200_ATTENTION_WARPS chooses.
+template <int D, bool kBackward> int launch_attention_rows(const attention::Params &p, int batch, DeviceInfo *d, cudaStream_t s) {
+    const int64_t rows = (int64_t)p.m_vec * batch, wave = (int64_t)d->sm_count * attention::kCtasPerSm<D, kBackward> * (attention::kThreads / 32);
+    const int keys = p.nnz_vec / p.m_vec;
+    const char *e = std::getenv("VSPARSE_B200_ATTENTION_WARPS");
+    const int warps = e ? std::atoi(e) : rows >= 3 * wave || keys <= 32 ? 1 : 2 * rows >= 3 * wave || keys <= 64 ? 2 : 4;
+    if (warps <= 1) return launch_attention<D, 1, kBackward>(p, batch, s);
+    if (warps == 2) return launch_attention<D, 2, kBackward>(p, batch, s);
+    return launch_attention<D, 4, kBackward>(p, batch, s);
+}
+// Whether the one-kernel form takes a call; what it does not take, and every refusal, is the operators' own.
+// VSPARSE_B200_ATTENTION=steps|fused.
+bool attention_fused(int path, int m_vec, int V, int n, int d, int nnz_vec, int batch, std::initializer_list<const void *> indices,
+                     std::initializer_list<const void *> sources, std::initializer_list<const void *> results) {
+    const char *e = std::getenv("VSPARSE_B200_ATTENTION");
+    if (e && !std::strcmp(e, "steps")) return false;
+    if (path != VS_PATH_TENSOR || !(V == 2 || V == 4 || V == 8) || (d != 64 && d != 128)) return false;
+    if (m_vec < 1 || n < 1 || nnz_vec < 1 || batch < 1 || batch > kMaxBatch || (int64_t)m_vec * V > 0x7fffffffll || (int64_t)nnz_vec * V > 0x7fffffffll) return false;
+    // Gathering costs the same for 2 queries as for 8, the operators' dense tiles do not: at d = 128 and V < 8 they win once there is
+    // enough work (32 heads, sequence 2048, V = 4, 205 keys: 142 against 171 us; one million keys break even).
+    if (d == 128 && V < 8 && (int64_t)nnz_vec * batch > 1000000 && !(e && !std::strcmp(e, "fused"))) return false;
+    for (const void *x : indices)
+        if (!x) return false;
+    for (const void *x : sources)   // read 32 bytes at a time
+        if (!x || reinterpret_cast<uintptr_t>(x) % 32 != 0) return false;
+    for (const void *x : results)
+        if (!x || !aligned16(x)) return false;
+    return (int64_t)nnz_vec * V % 8 == 0;
+}
+}  // namespace
+
 VS_EXPORT int vs_attention_cvse_backward(int path, int m_vec, int vec_length, int n, int d, int nonzeros_vec,
                                          const int32_t *row_indices, const int32_t *row_offsets, const int32_t *col_indices,
                                          const int32_t *t_offsets, const int32_t *t_rows, const int32_t *t_src, const void *q,
@@ -1616,6 +1756,28 @@ VS_EXPORT int vs_attention_cvse_backward(int path, int m_vec, int vec_length, in
         if (s_k > 0) VS_CUDA_TRY(cudaMemsetAsync(grad_k, 0, (size_t)batch * s_k * 2, st));
         if (s_k > 0) VS_CUDA_TRY(cudaMemsetAsync(grad_v, 0, (size_t)batch * s_k * 2, st));
         return VS_OK;
+    }
+    if (attention_fused(path, m_vec, vec_length, n, d, nonzeros_vec, batch, {row_indices, row_offsets, col_indices, t_offsets, t_rows, t_src},
+                        {q, kmat, vmat, grad_out}, {grad_q, grad_k, grad_v, probs_workspace, grad_workspace})) {
+        DeviceInfo *info = nullptr;
+        int rc = device_info(&info);
+        if (rc != VS_OK) return rc;
+        attention::Params p;
+        p.m_vec = m_vec; p.V = vec_length; p.n = n; p.nnz_vec = nonzeros_vec;
+        p.row_offsets = row_offsets; p.col_indices = col_indices;
+        p.q = static_cast<const __half *>(q); p.k = static_cast<const __half *>(kmat); p.v = static_cast<const __half *>(vmat);
+        p.out = static_cast<__half *>(grad_q); p.probs = static_cast<__half *>(probs_workspace);
+        p.grad_out = static_cast<const __half *>(grad_out); p.grad_scores = static_cast<__half *>(grad_workspace);
+        p.scale = scale;
+        cudaStream_t st = static_cast<cudaStream_t>(stream);
+        rc = d == 64 ? launch_attention_rows<64, true>(p, batch, info, st) : launch_attention_rows<128, true>(p, batch, info, st);
+        if (rc != VS_OK) return rc;
+        // dV = P^T dO,  dK = dS^T Q
+        rc = vs_spmm_t_batched(VS_F16, VS_F16, m_vec, vec_length, d, n, t_offsets, t_rows, t_src, probs_workspace, grad_out, grad_v,
+                               batch, s_ws, s_q, s_k, stream);
+        if (rc != VS_OK) return rc;
+        return vs_spmm_t_batched(VS_F16, VS_F16, m_vec, vec_length, d, n, t_offsets, t_rows, t_src, grad_workspace, q, grad_k, batch,
+                                 s_ws, s_q, s_k, stream);
     }
     // P = softmax(scale * Q K^T) at the mask, recomputed rather than kept from the forward pass
     int rc = vs_sddmm_batched(path, VS_F16, VS_F16, m_vec, d, n, nonzeros_vec, row_indices, row_offsets, col_indices, q, kmat,
@@ -1657,6 +1819,19 @@ VS_EXPORT int vs_attention_cvse(int path, int m_vec, int vec_length, int n, int 
         if (!out) return VS_ERR_NULL;
         return (int)cudaMemsetAsync(out, 0, (size_t)batch * m * d * 2, static_cast<cudaStream_t>(stream));
     }
+    if (attention_fused(path, m_vec, vec_length, n, d, nonzeros_vec, batch, {row_indices, row_offsets, col_indices}, {q, kmat, vmat}, {out, workspace})) {
+        DeviceInfo *info = nullptr;
+        const int rc = device_info(&info);
+        if (rc != VS_OK) return rc;
+        attention::Params p;
+        p.m_vec = m_vec; p.V = vec_length; p.n = n; p.nnz_vec = nonzeros_vec;
+        p.row_offsets = row_offsets; p.col_indices = col_indices;
+        p.q = static_cast<const __half *>(q); p.k = static_cast<const __half *>(kmat); p.v = static_cast<const __half *>(vmat);
+        p.out = static_cast<__half *>(out); p.probs = static_cast<__half *>(workspace);
+        p.grad_out = nullptr; p.grad_scores = nullptr; p.scale = scale;
+        cudaStream_t st = static_cast<cudaStream_t>(stream);
+        return d == 64 ? launch_attention_rows<64, false>(p, batch, info, st) : launch_attention_rows<128, false>(p, batch, info, st);
+    }
     int rc = vs_sddmm_batched(path, VS_F16, VS_F16, m_vec, d, n, nonzeros_vec, row_indices, row_offsets,
                               col_indices, q, kmat, workspace, vec_length, batch, m * d, (int64_t)n * d, s_ws,
                               stream, 0);
@@ -1695,46 +1870,6 @@ int attention_scratch(void **out) {
     }
     *out = g_attention_scratch_ptr[dev];
     return VS_OK;
-namespace {
-// Attention in one kernel per direction (attention.cuh).
-template <int D, int W, bool kBackward> int launch_attention(const attention::Params &p, int batch, cudaStream_t s) {
-    constexpr int rows = attention::kThreads / (32 * W);
-    attention::attention_kernel<D, W, kBackward><<<dim3((unsigned)((p.m_vec + rows - 1) / rows), (unsigned)batch), attention::kThreads, 0, s>>>(p);
-    return (int)cudaGetLastError();
-}
-// Warps per vector-row: one where the rows fill the GPU three times over, which spares the exchange between them (128 heads, sequence
-// 4096: 588 / 670 / 793 us with 1 / 2 / 4 warps); more where the rows are few (2 heads, sequence 1024, 154 keys: 12.6 / 9.3 / 8.5 us) and long enough
-// for a chunk each.  VSPARSE_B200_ATTENTION_WARPS chooses.
-template <int D, bool kBackward> int launch_attention_rows(const attention::Params &p, int batch, DeviceInfo *d, cudaStream_t s) {
-    const int64_t rows = (int64_t)p.m_vec * batch, wave = (int64_t)d->sm_count * attention::kCtasPerSm<D, kBackward> * (attention::kThreads / 32);
-    const int keys = p.nnz_vec / p.m_vec;
-    const char *e = std::getenv("VSPARSE_B200_ATTENTION_WARPS");
-    const int warps = e ? std::atoi(e) : rows >= 3 * wave || keys <= 32 ? 1 : 2 * rows >= 3 * wave || keys <= 64 ? 2 : 4;
-    if (warps <= 1) return launch_attention<D, 1, kBackward>(p, batch, s);
-    if (warps == 2) return launch_attention<D, 2, kBackward>(p, batch, s);
-    return launch_attention<D, 4, kBackward>(p, batch, s);
-}
-// Whether the one-kernel form takes a call; what it does not take, and every refusal, is the operators' own.
-// VSPARSE_B200_ATTENTION=steps|fused.
-bool attention_fused(int path, int m_vec, int V, int n, int d, int nnz_vec, int batch, std::initializer_list<const void *> indices,
-                     std::initializer_list<const void *> sources, std::initializer_list<const void *> results) {
-    const char *e = std::getenv("VSPARSE_B200_ATTENTION");
-    if (e && !std::strcmp(e, "steps")) return false;
-    if (path != VS_PATH_TENSOR || !(V == 2 || V == 4 || V == 8) || (d != 64 && d != 128)) return false;
-    if (m_vec < 1 || n < 1 || nnz_vec < 1 || batch < 1 || batch > kMaxBatch || (int64_t)m_vec * V > 0x7fffffffll || (int64_t)nnz_vec * V > 0x7fffffffll) return false;
-    // Gathering costs the same for 2 queries as for 8, the operators' dense tiles do not: at d = 128 and V < 8 they win once there is
-    // enough work (32 heads, sequence 2048, V = 4, 205 keys: 142 against 171 us; one million keys break even).
-    if (d == 128 && V < 8 && (int64_t)nnz_vec * batch > 1000000 && !(e && !std::strcmp(e, "fused"))) return false;
-    for (const void *x : indices)
-        if (!x) return false;
-    for (const void *x : sources)   // read 32 bytes at a time
-        if (!x || reinterpret_cast<uintptr_t>(x) % 32 != 0) return false;
-    for (const void *x : results)
-        if (!x || !aligned16(x)) return false;
-    return (int64_t)nnz_vec * V % 8 == 0;
-}
-}  // namespace
-
 }
 }  // namespace
 
@@ -1757,28 +1892,6 @@ VS_EXPORT int vs_attention_cvse_static(int path, int m_vec, int vec_length, int 
     int rc = attention_scratch(&scratch);
     if (rc != VS_OK) return rc;
     NoScratchScope no_allocation;   // SDDMM and SpMM below: the formulations without plan scratch
-    if (attention_fused(path, m_vec, vec_length, n, d, nonzeros_vec, batch, {row_indices, row_offsets, col_indices, t_offsets, t_rows, t_src},
-                        {q, kmat, vmat, grad_out}, {grad_q, grad_k, grad_v, probs_workspace, grad_workspace})) {
-        DeviceInfo *info = nullptr;
-        int rc = device_info(&info);
-        if (rc != VS_OK) return rc;
-        attention::Params p;
-        p.m_vec = m_vec; p.V = vec_length; p.n = n; p.nnz_vec = nonzeros_vec;
-        p.row_offsets = row_offsets; p.col_indices = col_indices;
-        p.q = static_cast<const __half *>(q); p.k = static_cast<const __half *>(kmat); p.v = static_cast<const __half *>(vmat);
-        p.out = static_cast<__half *>(grad_q); p.probs = static_cast<__half *>(probs_workspace);
-        p.grad_out = static_cast<const __half *>(grad_out); p.grad_scores = static_cast<__half *>(grad_workspace);
-        p.scale = scale;
-        cudaStream_t st = static_cast<cudaStream_t>(stream);
-        rc = d == 64 ? launch_attention_rows<64, true>(p, batch, info, st) : launch_attention_rows<128, true>(p, batch, info, st);
-        if (rc != VS_OK) return rc;
-        // dV = P^T dO,  dK = dS^T Q
-        rc = vs_spmm_t_batched(VS_F16, VS_F16, m_vec, vec_length, d, n, t_offsets, t_rows, t_src, probs_workspace, grad_out, grad_v,
-                               batch, s_ws, s_q, s_k, stream);
-        if (rc != VS_OK) return rc;
-        return vs_spmm_t_batched(VS_F16, VS_F16, m_vec, vec_length, d, n, t_offsets, t_rows, t_src, grad_workspace, q, grad_k, batch,
-                                 s_ws, s_q, s_k, stream);
-    }
     return vs_attention_cvse(path, m_vec, vec_length, n, d, nonzeros_vec, row_indices, row_offsets, col_indices, q, kmat,
                              vmat, out, scratch, scale, batch, stream);
 }
@@ -1819,19 +1932,6 @@ VS_EXPORT int vs_spmm_host(int path, int in_dtype, int out_dtype, int m_vec, int
     int32_t *d_idx, *d_off, *d_col;
     void *d_val, *d_rhs, *d_out;
     VS_CUDA_TRY(bufs.alloc((void **)&d_idx, b_idx));
-    if (attention_fused(path, m_vec, vec_length, n, d, nonzeros_vec, batch, {row_indices, row_offsets, col_indices}, {q, kmat, vmat}, {out, workspace})) {
-        DeviceInfo *info = nullptr;
-        const int rc = device_info(&info);
-        if (rc != VS_OK) return rc;
-        attention::Params p;
-        p.m_vec = m_vec; p.V = vec_length; p.n = n; p.nnz_vec = nonzeros_vec;
-        p.row_offsets = row_offsets; p.col_indices = col_indices;
-        p.q = static_cast<const __half *>(q); p.k = static_cast<const __half *>(kmat); p.v = static_cast<const __half *>(vmat);
-        p.out = static_cast<__half *>(out); p.probs = static_cast<__half *>(workspace);
-        p.grad_out = nullptr; p.grad_scores = nullptr; p.scale = scale;
-        cudaStream_t st = static_cast<cudaStream_t>(stream);
-        return d == 64 ? launch_attention_rows<64, false>(p, batch, info, st) : launch_attention_rows<128, false>(p, batch, info, st);
-    }
     VS_CUDA_TRY(bufs.alloc((void **)&d_off, b_off));
     VS_CUDA_TRY(bufs.alloc((void **)&d_col, b_col));
     VS_CUDA_TRY(bufs.alloc(&d_val, b_val));
