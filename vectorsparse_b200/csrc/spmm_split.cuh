@@ -20,9 +20,8 @@
 // Bound by the tensor pipe: 6 x the dense flops.
 #pragma once
 #include <cuda.h>
-#include <cuda_bf16.h>
-
 #include "common.cuh"
+#include "densify.cuh"
 #include "spmm_pair.cuh"
 #include "tc_ptx.cuh"
 
@@ -34,20 +33,24 @@ using pairspmm::wait_or_abort;
 using pairspmm::Walk;
 
 constexpr int kTileM = 256, kMaxTileN = 256, kCtaRows = 128, kBlockK = 64, kParts = 3;
-constexpr int kStages = 2;
 constexpr int kPartBytes = 128 * kBlockK * 2;                  // 16 KiB: 128 rows of A or columns of B of one part
-constexpr int kStageBytes = 2 * kParts * kPartBytes;           // 96 KiB
+// Operands of a stage (64 columns of A): 96 KiB for 256-column items, 72 KiB for 128-column ones, two resp. three of them in flight.
+template <int kTn> struct Stage {
+    static constexpr int kBytes = kParts * (kPartBytes + kTn / 2 * kBlockK * 2), kCount = kTn == 256 ? 2 : 3;
+};
+constexpr int kMaxStages = 3, kOperandBytes = 3 * Stage<128>::kBytes;
+static_assert(2 * Stage<256>::kBytes <= kOperandBytes, "operand slots");
 constexpr int kEpiWarps = 8, kLoadWarp = 8, kMmaWarp = 9, kThreads = 320;
-constexpr int kStoreCols = 32, kBoxBytes = 32 * kStoreCols * 4;
-constexpr uint32_t kTinyInput = (127u - 100u) << 23, kTinyResult = (127u - 96u) << 23;
+constexpr int kStoreCols = 8, kBoxBytes = 32 * kStoreCols * 4;   // 1 KiB of staging per epilogue warp: once per item, and the operands need the room
+constexpr uint32_t kTinyResult = (127u - 96u) << 23;
 
 struct Smem {
     static constexpr int kOperands = 0;
-    static constexpr int kStaging = kStages * kStageBytes;
+    static constexpr int kStaging = kOperandBytes;
     static constexpr int kBarFull = kStaging + kEpiWarps * kBoxBytes;
-    static constexpr int kBarDone = kBarFull + kStages * 8;
-    static constexpr int kBarEmpty = kBarDone + kStages * 8;
-    static constexpr int kTmemHolder = kBarEmpty + kStages * 8;
+    static constexpr int kBarDone = kBarFull + kMaxStages * 8;
+    static constexpr int kBarAccEmpty = kBarDone + kMaxStages * 8;
+    static constexpr int kTmemHolder = kBarAccEmpty + 2 * 8;
     static constexpr int kAbort = kTmemHolder + 8;
     static constexpr int kTotal = kAbort + 8;
 };
@@ -55,90 +58,28 @@ constexpr int kSmemBytes = Smem::kTotal + 1024;
 static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
 
 // ---- preparation ------------------------------------------------------------------------------------------
-constexpr int kPrepThreads = 256, kPrepFloats = 8192;          // 32 KiB of a vector-row at a time
-
-// Eight values as three groups of eight bf16.  Returns whether one of them is too small to be split exactly.
-__device__ __forceinline__ bool split8(const float (&x)[8], uint4 (&part)[kParts]) {
-    uint32_t w[kParts][4];
-    bool tiny = false;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        float a = x[2 * i], b = x[2 * i + 1];
-        tiny |= (__float_as_uint(a) & 0x7fffffffu) - 1u < kTinyInput - 1u || (__float_as_uint(b) & 0x7fffffffu) - 1u < kTinyInput - 1u;
-#pragma unroll
-        for (int p = 0; p < kParts; ++p) {
-            const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
-            w[p][i] = *reinterpret_cast<const uint32_t *>(&h);
-            a -= __uint_as_float(w[p][i] << 16);
-            b -= __uint_as_float(w[p][i] & 0xffff0000u);
-        }
-    }
-#pragma unroll
-    for (int p = 0; p < kParts; ++p) part[p] = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
-    return tiny;
-}
+using densify::kPrepThreads;
 
 struct PrepParams {
     int batch_a, batch_b;       // problems with values / a dense operand of their own
     int Kp, Np;                 // K and N rounded up to 64
     int64_t min_vectors;        // nonzero vectors from which the split product is the quicker one
-    __nv_bfloat16 *a;           // [batch][M / 128, rounded up][Kp / 64][part][128 rows][64 columns]
-    __nv_bfloat16 *b;           // [batch][Kp / 64][Np / 64][part][64 rows][64 columns]
+    uint16_t *a;                // bf16 [batch][M / 128, rounded up][Kp / 64][part][128 rows][64 columns]
+    uint16_t *b;                // bf16 [batch][Kp / 64][Np / 64][part][64 rows][64 columns]
     int32_t *verdict;           // word 0: taken; words 4 ..: one per CTA of this kernel, nonzero if it met what the product cannot do
 };
 
 template <int V> __global__ void __launch_bounds__(kPrepThreads) spmm_split_prepare(const SpmmParams p, const PrepParams q) {
     pdl_launch_dependents();
     pdl_wait();
-    __shared__ __align__(16) float rows[kPrepFloats];
-    __shared__ uint32_t named[kPrepFloats / V / 32];
+    __shared__ __align__(16) densify::Shared<float> sh;
     const int t = threadIdx.x;
     const int64_t vectors = (int64_t)__ldg(p.row_offsets + p.m_vec) - __ldg(p.row_offsets);
     const bool taken = vectors >= q.min_vectors;
     if (blockIdx.x == 0 && t == 0) q.verdict[0] = taken ? 1 : 0;
     if (!taken) return;
-    bool bad = false;
-    constexpr int kCols = kPrepFloats / V;
-    const int pieces = (q.Kp + kCols - 1) / kCols;
-    const int k_blocks = q.Kp / kBlockK, row_tiles = (int)(((int64_t)p.m_vec * V + 127) / 128);
-    const int64_t units = (int64_t)q.batch_a * p.m_vec * pieces;
-    for (int64_t u = blockIdx.x; u < units; u += gridDim.x) {
-        const int c0 = (int)(u % pieces) * kCols, cols = min(kCols, q.Kp - c0);
-        const int64_t r = u / pieces;
-        const int row = (int)(r % p.m_vec), b = (int)(r / p.m_vec);
-        for (int i = t; i < V * cols / 4; i += kPrepThreads)
-            *reinterpret_cast<float4 *>(rows + (i / (cols / 4)) * kCols + (i % (cols / 4)) * 4) = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int i = t; i < cols / 32; i += kPrepThreads) named[i] = 0u;
-        __syncthreads();
-        const float *values = static_cast<const float *>(p.values) + (int64_t)b * p.stride_values;
-        const int end = __ldg(p.row_offsets + row + 1);
-        for (int j = __ldg(p.row_offsets + row) + t; j < end; j += kPrepThreads) {
-            const int c = __ldg(p.col_indices + j) - c0;
-            if ((unsigned)c >= (unsigned)cols || c + c0 >= p.K) continue;
-            const uint32_t bit = 1u << (c & 31);
-            bad |= (atomicOr(&named[c >> 5], bit) & bit) != 0u;
-            float a[V];
-            VecLoad<float, V>::load(values + (int64_t)j * V, a);
-#pragma unroll
-            for (int v = 0; v < V; ++v) rows[v * kCols + c] = a[v];
-        }
-        __syncthreads();
-        for (int i = t; i < V * (cols / 8); i += kPrepThreads) {
-            const int v = i / (cols / 8), c = (i % (cols / 8)) * 8;
-            float x[8];
-            const float4 lo = *reinterpret_cast<const float4 *>(rows + v * kCols + c), hi = *reinterpret_cast<const float4 *>(rows + v * kCols + c + 4);
-            x[0] = lo.x; x[1] = lo.y; x[2] = lo.z; x[3] = lo.w; x[4] = hi.x; x[5] = hi.y; x[6] = hi.z; x[7] = hi.w;
-            uint4 part[kParts];
-            bad |= split8(x, part);
-#pragma unroll
-            for (int s = 0; s < kParts; ++s) {
-                const int64_t r = (int64_t)row * V + v;
-                const int64_t tile = (((int64_t)b * row_tiles + r / 128) * k_blocks + (c0 + c) / kBlockK) * kParts + s;
-                *reinterpret_cast<uint4 *>(q.a + tile * (128 * kBlockK) + (r % 128) * kBlockK + c % kBlockK) = part[s];
-            }
-        }
-        __syncthreads();
-    }
+    bool bad = densify::lay_out_rows<float, V, kParts>(p, q.batch_a, q.Kp, q.a, sh);
+    const int k_blocks = q.Kp / kBlockK;
     const int chunks = q.Np / 8;
     const int64_t total = (int64_t)q.batch_b * q.Kp * chunks;
     for (int64_t i = (int64_t)blockIdx.x * kPrepThreads + t; i < total; i += (int64_t)gridDim.x * kPrepThreads) {
@@ -151,7 +92,7 @@ template <int V> __global__ void __launch_bounds__(kPrepThreads) spmm_split_prep
         const float4 lo = k < p.K && c < p.N ? __ldg(reinterpret_cast<const float4 *>(src)) : zero, hi = k < p.K && c + 4 < p.N ? __ldg(reinterpret_cast<const float4 *>(src) + 1) : zero;
         x[0] = lo.x; x[1] = lo.y; x[2] = lo.z; x[3] = lo.w; x[4] = hi.x; x[5] = hi.y; x[6] = hi.z; x[7] = hi.w;
         uint4 part[kParts];
-        bad |= split8(x, part);
+        bad |= densify::split8(x, part);
 #pragma unroll
         for (int s = 0; s < kParts; ++s) {
             const int64_t tile = (((int64_t)b * k_blocks + k / kBlockK) * (q.Np / 64) + c / 64) * kParts + s;
@@ -164,12 +105,13 @@ template <int V> __global__ void __launch_bounds__(kPrepThreads) spmm_split_prep
 
 // ---- product ----------------------------------------------------------------------------------------------
 // map_a: the tiles of A as {64 columns, 128 rows, parts, tiles}, box {64, 128, 3, 1}; map_b: those of B as {64 columns, 64 rows, parts,
-// tiles}, box {64, 64, 3, tn / 128}: a CTA's operands of a stage are two copies.  map_out: {N, M, batch} fp32, box {32, 32, 1}; what lies
+// tiles}, box {64, 64, 3, kTn / 128}: a CTA's operands of a stage are two copies.  map_out: {N, M, batch} fp32, box {8, 32, 1}; what lies
 // outside is not written.  Rows and columns past the matrix are multiplied with whatever the scratch holds there, zeros within the
-// last 64 columns and rows of K, and go nowhere.  tn: columns per work item, 256 or 128.  No multicast anywhere.
+// last 64 columns and rows of K, and go nowhere.  kTn: columns per work item, 256 or 128.  No multicast anywhere.
+template <int kTn>
 __global__ void __launch_bounds__(kThreads, 1)
 spmm_split_kernel(const SpmmParams p, int V, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
-                  const __grid_constant__ CUtensorMap map_out, int tn, int batch_a, int batch_b, int m_tiles, int n_tiles, int k_blocks, int row_tiles, int slabs,
+                  const __grid_constant__ CUtensorMap map_out, int batch_a, int batch_b, int m_tiles, int n_tiles, int k_blocks, int row_tiles, int slabs,
                   uint32_t *status, int32_t *verdict, int checks) {
     pdl_launch_dependents();
     pdl_wait();
@@ -183,13 +125,16 @@ spmm_split_kernel(const SpmmParams p, int V, const __grid_constant__ CUtensorMap
     const uint32_t pair = tc::cluster_id_x(), pairs = tc::cluster_count_x();
     volatile int *abort_flag = reinterpret_cast<volatile int *>(sm + Smem::kAbort);
     const uint32_t abort_addr = base + Smem::kAbort;
-    const uint32_t bar_full = base + Smem::kBarFull, bar_done = base + Smem::kBarDone, bar_empty = base + Smem::kBarEmpty;
+    const uint32_t bar_full = base + Smem::kBarFull, bar_done = base + Smem::kBarDone, bar_acc_empty = base + Smem::kBarAccEmpty;
+    constexpr int kStages = Stage<kTn>::kCount, kStageBytes = Stage<kTn>::kBytes, kHalfCols = kTn / 2;   // columns of B each CTA holds
 
     if (t == 0) {
         for (int s = 0; s < kStages; ++s) {
             tc::mbar_init(bar_full + 8 * s, 1);                     // first CTA: its loader's arrival + the bytes of both CTAs
-            tc::mbar_init(bar_done + 8 * s, 1);                     // both: "stage multiplied", operands free and accumulator complete
-            tc::mbar_init(bar_empty + 8 * s, 2 * kEpiWarps * 32);   // first CTA: accumulator read out by every epilogue thread of both
+            tc::mbar_init(bar_done + 8 * s, 1);                     // both: "stage multiplied": its operands are free, its accumulator complete
+        }
+        for (int s = 0; s < 2; ++s) {
+            tc::mbar_init(bar_acc_empty + 8 * s, 2 * kEpiWarps);   // first CTA: read out by every epilogue warp of both
         }
         *abort_flag = 0;
         tc::fence_mbar_init();
@@ -206,9 +151,9 @@ spmm_split_kernel(const SpmmParams p, int V, const __grid_constant__ CUtensorMap
     const int64_t total_items = chosen ? (int64_t)p.batch * n_tiles * m_tiles : 0;
     const uint32_t my_items = (total_items > pair) ? (uint32_t)((total_items - pair + pairs - 1) / pairs) : 0u;
     const uint32_t total_stages = my_items * (uint32_t)k_blocks;
-    const int m_rows = p.m_vec * V, half_cols = tn >> 1;   // columns of B each CTA holds
+    const int m_rows = p.m_vec * V;
 
-    // stage g of the pair uses operand slot, accumulator buffer and barriers g % 2
+    // stage g of the pair uses operand slot g % kStages and accumulator g % 2
     if (warp == kLoadWarp) {
         if (lane == 0) {
             bool ok_run = true;
@@ -222,8 +167,8 @@ spmm_split_kernel(const SpmmParams p, int V, const __grid_constant__ CUtensorMap
                 if (!ok_run) break;
                 const uint32_t bar = full_first + 8 * slot, a_dst = base + Smem::kOperands + slot * kStageBytes, b_dst = a_dst + kParts * kPartBytes;
                 const int za = ((batch_a == 1 ? 0 : walk.b) * row_tiles + 2 * walk.mt + (int)rank) * k_blocks + walk.kb;
-                const int zb = ((batch_b == 1 ? 0 : walk.b) * k_blocks + walk.kb) * slabs + ((walk.nt * tn + (int)rank * half_cols) >> 6);
-                if (rank == 0) tc::mbar_expect_tx(bar_full + 8 * slot, 2u * kParts * (kPartBytes + (uint32_t)half_cols * kBlockK * 2));
+                const int zb = ((batch_b == 1 ? 0 : walk.b) * k_blocks + walk.kb) * slabs + ((walk.nt * kTn + (int)rank * kHalfCols) >> 6);
+                if (rank == 0) tc::mbar_expect_tx(bar_full + 8 * slot, 2u * kStageBytes);
                 tc::tma_load_4d_pair(a_dst, &map_a, bar, 0, 0, 0, za);
                 tc::tma_load_4d_pair(b_dst, &map_b, bar, 0, 0, 0, zb);
             }
@@ -237,83 +182,92 @@ spmm_split_kernel(const SpmmParams p, int V, const __grid_constant__ CUtensorMap
             const uint32_t a_lo0 = tc::smem_desc_lo(base + Smem::kOperands, 16);                                  // K-major, 8-row groups 1 KiB apart
             const uint32_t b_lo0 = tc::smem_desc_lo(base + Smem::kOperands + kParts * kPartBytes, kParts * kPartBytes / 2);   // 64-column slabs, three parts of 8 KiB each
             const uint32_t hi = tc::smem_desc_hi(1024, (uint32_t)tc::kSwizzle128B);
-            const uint32_t idesc = tc::make_idesc_f16(kTileM, tn, 0, 1) | (1u << 7) | (1u << 10);             // both operands bf16
+            const uint32_t idesc = tc::make_idesc_f16(kTileM, kTn, 0, 1) | (1u << 7) | (1u << 10);             // both operands bf16
             const int steps_last = ((p.K - 1) & (kBlockK - 1)) / 16 + 1;
             bool ok_run = true;
             uint32_t g = 0;
             for (uint32_t i = 0; i < my_items && ok_run; ++i) {
                 for (int kb = 0; kb < k_blocks; ++kb, ++g) {
-                    const uint32_t slot = g % kStages, parity = (g / kStages) & 1u;
-                    ok_run = wait_or_abort<0>(bar_empty + 8 * slot, parity, abort_flag, abort_addr, peer) &&
-                             wait_or_abort<0>(bar_full + 8 * slot, parity, abort_flag, abort_addr, peer);
+                    const uint32_t slot = g % kStages, buf = g & 1u;
+                    ok_run = wait_or_abort<0>(bar_acc_empty + 8 * buf, (g >> 1) & 1u, abort_flag, abort_addr, peer) &&
+                             wait_or_abort<0>(bar_full + 8 * slot, (g / kStages) & 1u, abort_flag, abort_addr, peer);
                     if (!ok_run) break;
                     tc::tc_fence_after_sync();
-                    const uint32_t d = tmem_base + slot * kMaxTileN;
+                    const uint32_t d = tmem_base + buf * kMaxTileN;
                     const uint32_t a_lo = a_lo0 + slot * (kStageBytes >> 4), b_lo = b_lo0 + slot * (kStageBytes >> 4);
                     const int steps = kb + 1 < k_blocks ? kBlockK / 16 : steps_last;
                     // parts of A and B, smallest products first
                     constexpr int kA[6] = {2, 0, 1, 1, 0, 0}, kB[6] = {0, 2, 1, 0, 1, 0};
+                    auto product = [&](int s, int kk) {   // 16 columns of A: 32 bytes on in A, 2 KiB in B
+                        tc::mma_f16_ss_pair(d, tc::desc64(a_lo + kA[s] * (kPartBytes >> 4) + 2 * kk, hi),
+                                            tc::desc64(b_lo + kB[s] * (kPartBytes >> 5) + 128 * kk, hi), idesc, (s | kk) ? 1u : 0u);
+                    };
+                    if (steps == kBlockK / 16) {   // written out: a loop issues them more slowly than 128 columns of B multiply
 #pragma unroll
-                    for (int s = 0; s < 6; ++s)
-                        for (int kk = 0; kk < steps; ++kk)   // 16 columns of A: 32 bytes on in A, 2 KiB in B
-                            tc::mma_f16_ss_pair(d, tc::desc64(a_lo + kA[s] * (kPartBytes >> 4) + 2 * kk, hi),
-                                                tc::desc64(b_lo + kB[s] * (kPartBytes >> 5) + 128 * kk, hi), idesc, (s | kk) ? 1u : 0u);
+                        for (int s = 0; s < 6; ++s)
+#pragma unroll
+                            for (int kk = 0; kk < kBlockK / 16; ++kk) product(s, kk);
+                    } else {
+#pragma unroll
+                        for (int s = 0; s < 6; ++s)
+                            for (int kk = 0; kk < steps; ++kk) product(s, kk);
+                    }
                     tc::mma_commit_pair_both(bar_done + 8 * slot);
                 }
             }
         }
     } else {
-        // epilogue warp (quarter, half): rows 32 quarter .. + 31 of the CTA's 128, half_cols columns from half_cols half
+        // epilogue warp (quarter, half): rows 32 quarter .. + 31 of the CTA's 128, kHalfCols columns from kHalfCols half
         const int quarter = warp & 3, half = warp >> 2;
         uint8_t *stg = sm + Smem::kStaging + warp * kBoxBytes;
         const uint32_t stg_u32 = base + Smem::kStaging + warp * kBoxBytes;
-        const uint32_t lane_taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * half_cols);
-        const uint32_t empty_first = tc::map_to_cta(bar_empty, 0);
+        const uint32_t lane_taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * kHalfCols);
+        const uint32_t empty_first = tc::map_to_cta(bar_acc_empty, 0);
         tc::tc_fence_before_sync();
-        for (int s = 0; s < kStages; ++s) tc::mbar_arrive_remote(empty_first + 8 * s);   // both buffers start out free
+        if (lane == 0)
+            for (int s = 0; s < 2; ++s) tc::mbar_arrive_remote(empty_first + 8 * s);   // both buffers start out free
         Walk walk;
         walk.init(pair, pairs, 0u, my_items, m_tiles, n_tiles, 1);
         bool ok_run = true, bad = false;
         uint32_t g = 0;
         for (uint32_t i = 0; i < my_items && ok_run; ++i, walk.advance(1)) {
-            float acc[128];
+            float acc[kHalfCols];
 #pragma unroll
-            for (int e = 0; e < 128; ++e) acc[e] = 0.f;
+            for (int e = 0; e < kHalfCols; ++e) acc[e] = 0.f;
             for (int kb = 0; kb < k_blocks; ++kb, ++g) {
-                const uint32_t slot = g % kStages;
+                const uint32_t buf = g & 1u, slot = g % kStages;
                 ok_run = __all_sync(0xffffffffu, wait_or_abort<0>(bar_done + 8 * slot, (g / kStages) & 1u, abort_flag, abort_addr, peer));
                 if (!ok_run) break;
                 tc::tc_fence_after_sync();
 #pragma unroll
-                for (int c = 0; c < 128; c += 16) {
-                    if (c >= half_cols) break;
+                for (int c = 0; c < kHalfCols; c += 16) {
                     uint32_t r[16];
-                    tc::tmem_ld_x16(lane_taddr + slot * kMaxTileN + (uint32_t)c, r);
+                    tc::tmem_ld_x16(lane_taddr + buf * kMaxTileN + (uint32_t)c, r);
 #pragma unroll
                     for (int e = 0; e < 16; ++e) acc[c + e] += __uint_as_float(r[e]);
                 }
                 tc::tc_fence_before_sync();
-                tc::mbar_arrive_remote(empty_first + 8 * slot);
+                __syncwarp();
+                if (lane == 0) tc::mbar_arrive_remote(empty_first + 8 * buf);   // one per warp: 512 a stage were slower than its products
             }
             if (!ok_run) break;
-            const int row0 = walk.mt * kTileM + (int)rank * kCtaRows + quarter * 32, col0 = walk.nt * tn + half * half_cols;
+            const int row0 = walk.mt * kTileM + (int)rank * kCtaRows + quarter * 32, col0 = walk.nt * kTn + half * kHalfCols;
             if (row0 < m_rows) {   // warp-uniform
 #pragma unroll
-                for (int c = 0; c < 128; c += kStoreCols) {
-                    if (c < half_cols && col0 + c < p.N) {
+                for (int c = 0; c < kHalfCols; c += kStoreCols) {
+                    if (col0 + c < p.N) {
                         if (row0 + lane < m_rows) {
 #pragma unroll
-                            for (int e = 0; e < 32; ++e) {   // columns past the matrix hold zeros
+                            for (int e = 0; e < kStoreCols; ++e) {   // columns past the matrix hold zeros
                                 const uint32_t bits = __float_as_uint(acc[c + e]) & 0x7fffffffu;
                                 bad |= bits >= 0x7f800000u || bits - 1u < kTinyResult - 1u;
                             }
                         }
                         if (lane == 0) tc::bulk_wait_group_read<0>();
                         __syncwarp();
-#pragma unroll
-                        for (int u = 0; u < 8; ++u)
-                            *reinterpret_cast<float4 *>(stg + lane * 128 + ((u ^ (lane & 7)) << 4)) =
-                                make_float4(acc[c + 4 * u], acc[c + 4 * u + 1], acc[c + 4 * u + 2], acc[c + 4 * u + 3]);
+                        float4 *row = reinterpret_cast<float4 *>(stg + lane * (kStoreCols * 4));
+                        row[0] = make_float4(acc[c], acc[c + 1], acc[c + 2], acc[c + 3]);
+                        row[1] = make_float4(acc[c + 4], acc[c + 5], acc[c + 6], acc[c + 7]);
                         tc::fence_proxy_async();
                         __syncwarp();
                         if (lane == 0) {

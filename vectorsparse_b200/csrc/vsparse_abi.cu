@@ -34,6 +34,7 @@
 #include "spmm_direct.cuh"
 #include "sddmm_pair.cuh"
 #include "spmm_pair.cuh"
+#include "densify.cuh"
 #include "spmm_split.cuh"
 #include "spmm_t.cuh"
 #include "sddmm_tc.cuh"
@@ -968,8 +969,8 @@ template <int V> int launch_spmm_split(const SpmmParams &p, int64_t vectors, cud
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return VS_OK;
     if (resident[dev] == 0) {
-        const int n = set_smem(splitspmm::spmm_split_kernel, splitspmm::kSmemBytes) == VS_OK
-                          ? max_resident_pairs(splitspmm::spmm_split_kernel, splitspmm::kThreads, splitspmm::kSmemBytes, d) : 0;
+        const bool fits = set_smem(splitspmm::spmm_split_kernel<256>, splitspmm::kSmemBytes) == VS_OK && set_smem(splitspmm::spmm_split_kernel<128>, splitspmm::kSmemBytes) == VS_OK;
+        const int n = fits ? max_resident_pairs(splitspmm::spmm_split_kernel<256>, splitspmm::kThreads, splitspmm::kSmemBytes, d) : 0;
         resident[dev] = n > 0 ? n : -1;
     }
     if (resident[dev] < 0) return VS_OK;
@@ -982,7 +983,7 @@ template <int V> int launch_spmm_split(const SpmmParams &p, int64_t vectors, cud
     const int k_blocks = q.Kp / 64, m_tiles = (int)((M + splitspmm::kTileM - 1) / splitspmm::kTileM);
     const int64_t row_items = (int64_t)p.batch * m_tiles, wide = (p.N + 255) / 256, narrow = (p.N + 127) / 128;
     auto waves = [&](int64_t items) { return (double)((items + resident[dev] - 1) / resident[dev]); };
-    const double t_wide = 2.2 * waves(row_items * wide), t_narrow = 1.2 * waves(row_items * narrow);
+    const double t_wide = 2.1 * waves(row_items * wide), t_narrow = 1.1 * waves(row_items * narrow);
     const int tn = t_narrow < t_wide ? 128 : 256, n_tiles = (int)(tn == 256 ? wide : narrow);
     const int row_tiles = (int)((M + 127) / 128), slabs = q.Np / 64;
     const int64_t a_elems = (int64_t)q.batch_a * row_tiles * 128 * q.Kp, b_elems = (int64_t)q.batch_b * q.Kp * q.Np;
@@ -996,13 +997,13 @@ template <int V> int launch_spmm_split(const SpmmParams &p, int64_t vectors, cud
     const int64_t header = ((4 + checks) * 4 + 255) / 256 * 256, a_bytes = (a_elems * 6 + 255) / 256 * 256, bytes = header + a_bytes + b_elems * 6;
     if (bytes > kMaxPlanBytes || row_items * n_tiles * k_blocks > 0x7fffffffll) return VS_OK;
     CUtensorMap map_out;
-    if (make_tile_map(&map_out, p.out, true, (uint64_t)M, (uint64_t)p.N, (uint64_t)p.batch, (uint64_t)p.stride_out, splitspmm::kStoreCols, 32) != VS_OK) return VS_OK;
+    if (make_tile_map(&map_out, p.out, true, (uint64_t)M, (uint64_t)p.N, (uint64_t)p.batch, (uint64_t)p.stride_out, splitspmm::kStoreCols, 32, false) != VS_OK) return VS_OK;
     uint8_t *mem = nullptr;
     PlanScratch scratch;
     if (scratch.take(d, s, (size_t)bytes, reinterpret_cast<void **>(&mem)) != VS_OK) return VS_OK;
     q.verdict = reinterpret_cast<int32_t *>(mem);
-    q.a = reinterpret_cast<__nv_bfloat16 *>(mem + header);
-    q.b = reinterpret_cast<__nv_bfloat16 *>(mem + header + a_bytes);
+    q.a = reinterpret_cast<uint16_t *>(mem + header);
+    q.b = reinterpret_cast<uint16_t *>(mem + header + a_bytes);
     CUtensorMap map_a, map_b;
     if (make_packed_map(&map_a, q.a, 64, 128, 3, (uint64_t)q.batch_a * row_tiles * k_blocks, 1) != VS_OK ||
         make_packed_map(&map_b, q.b, 64, 64, 3, (uint64_t)q.batch_b * k_blocks * slabs, (uint32_t)(tn / 128)) != VS_OK)
@@ -1011,8 +1012,8 @@ template <int V> int launch_spmm_split(const SpmmParams &p, int64_t vectors, cud
     int rc = (int)launch_overlapped(splitspmm::spmm_split_prepare<V>, (unsigned)checks, splitspmm::kPrepThreads, 0, s, p, q);
     if (rc != VS_OK) return rc;
     const int64_t items = row_items * n_tiles;
-    rc = (int)launch_pairs(splitspmm::spmm_split_kernel, (unsigned)std::min<int64_t>(items, resident[dev]), splitspmm::kThreads, (size_t)splitspmm::kSmemBytes, s, true,
-                           p, V, map_a, map_b, map_out, tn, q.batch_a, q.batch_b, m_tiles, n_tiles, k_blocks, row_tiles, slabs, d->status, q.verdict, checks);
+    rc = (int)launch_pairs(tn == 256 ? splitspmm::spmm_split_kernel<256> : splitspmm::spmm_split_kernel<128>, (unsigned)std::min<int64_t>(items, resident[dev]), splitspmm::kThreads, (size_t)splitspmm::kSmemBytes, s, true,
+                           p, V, map_a, map_b, map_out, q.batch_a, q.batch_b, m_tiles, n_tiles, k_blocks, row_tiles, slabs, d->status, q.verdict, checks);
     if (rc != VS_OK) return rc;
     const int chunks = spmm_cc_chunks(4 * V, 4, p.N);
     if constexpr (V <= 4) {
