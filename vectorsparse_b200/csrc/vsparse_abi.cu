@@ -1488,7 +1488,10 @@ SpmmTMode spmm_t_mode() {   // read at every call, so that a test can switch ker
 // plan kernel's units (SM-cycles per 128 columns): the CUDA-core kernel ~5 per value (0.92 ms for 256 products of
 // 2048 x 512, 90 % sparse, V = 8), the dense kernel ~1100 per stage plus ~1.5 per vector of fill work (0.170 ms on
 // the same problem against 0.137 for the forward product with the same tiles).
-template <typename TOut, int V> int launch_spmm_t(const spmmt::Params &p, int m_vec, cudaStream_t s) {
+// `count` products (at most kMaxTogether) with the same structure, sizes and strides: one plan serves them.
+constexpr int kMaxTogether = 2;
+template <typename TOut, int V> int launch_spmm_t(const spmmt::Params *list, int count, int m_vec, cudaStream_t s) {
+    const spmmt::Params &p = list[0];
     DeviceInfo *d;
     int rc = device_info(&d);
     if (rc != VS_OK) return rc;
@@ -1511,20 +1514,31 @@ template <typename TOut, int V> int launch_spmm_t(const spmmt::Params &p, int m_
     const int checks = spmm_plan_checks(q.m_vec);
     const size_t plan_words = (size_t)(2 * plan_blocks + rows_per_group + 1), check_words = (size_t)densespmm::kPlanWarps * plan_blocks;
     const size_t plan_smem = (plan_words > check_words ? plan_words : check_words) * 4;
+    auto by_cores = [&]() {
+        for (int i = 0; i < count; ++i) {
+            const int rc = launch_spmm_t_cc<TOut, V>(list[i], s, d, nullptr, 0);
+            if (rc != VS_OK) return rc;
+        }
+        return (int)VS_OK;
+    };
     const bool dense_ok = !t_no_scratch && mode != SpmmTMode::kGather && q.K > 0 && q.m_vec > 0 && plan_bytes <= kMaxPlanBytes &&
                           plan_smem <= 40 * 1024 && (q.batch == 1 || (q.stride_rhs * 2) % 16 == 0) &&
                           (q.batch == 1 || (q.stride_out * sizeof(TOut)) % 16 == 0);
-    if (!dense_ok) return launch_spmm_t_cc<TOut, V>(p, s, d, nullptr, 0);
+    if (!dense_ok) return by_cores();
 
     constexpr bool kOutF32 = sizeof(TOut) == 4;
-    CUtensorMap map, map_out;
-    if (make_tile_map(&map, q.rhs, false, (uint64_t)q.K, (uint64_t)q.N, (uint64_t)q.batch, (uint64_t)q.stride_rhs, 64, 64) != VS_OK ||
-        make_tile_map(&map_out, q.out, kOutF32, (uint64_t)q.m_vec, (uint64_t)q.N, (uint64_t)q.batch, (uint64_t)q.stride_out,
-                      densespmm::kStoreCols, 32) != VS_OK)
-        return launch_spmm_t_cc<TOut, V>(p, s, d, nullptr, 0);
-    CUtensorMap map_b4 = map;
-    const int use_b4 = (q.N % 64 == 0 && make_blocked_map(&map_b4, q.rhs, (uint64_t)q.K, (uint64_t)q.N, (uint64_t)q.batch,
-                                                          (uint64_t)q.stride_rhs, densespmm::kTileN / 64) == VS_OK) ? 1 : 0;
+    CUtensorMap map[kMaxTogether], map_out[kMaxTogether], map_b4[kMaxTogether];
+    int use_b4 = q.N % 64 == 0 ? 1 : 0;
+    for (int i = 0; i < count; ++i) {
+        if (make_tile_map(&map[i], list[i].rhs, false, (uint64_t)q.K, (uint64_t)q.N, (uint64_t)q.batch, (uint64_t)q.stride_rhs, 64, 64) != VS_OK ||
+            make_tile_map(&map_out[i], list[i].out, kOutF32, (uint64_t)q.m_vec, (uint64_t)q.N, (uint64_t)q.batch, (uint64_t)q.stride_out,
+                          densespmm::kStoreCols, 32) != VS_OK)
+            return by_cores();
+        map_b4[i] = map[i];
+        if (use_b4 && make_blocked_map(&map_b4[i], list[i].rhs, (uint64_t)q.K, (uint64_t)q.N, (uint64_t)q.batch, (uint64_t)q.stride_rhs,
+                                       densespmm::kTileN / 64) != VS_OK)
+            use_b4 = 0;
+    }
     auto kernel = densespmm::spmm_dense_kernel<TOut, V, true>;
     static DeviceBits smem_set;
     rc = set_smem_once(kernel, densespmm::kSmemBytes, smem_set);
@@ -1532,7 +1546,7 @@ template <typename TOut, int V> int launch_spmm_t(const spmmt::Params &p, int m_
     uint8_t *plan = nullptr;
     PlanScratch scratch;
     if (scratch.take(d, s, (size_t)plan_bytes, reinterpret_cast<void **>(&plan)) != VS_OK)
-        return launch_spmm_t_cc<TOut, V>(p, s, d, nullptr, 0);
+        return by_cores();
     int32_t *flag = reinterpret_cast<int32_t *>(plan);
     const int64_t header_bytes = spmm_plan_header_bytes(checks);
     int32_t *blk_offsets = reinterpret_cast<int32_t *>(plan + header_bytes);
@@ -1542,26 +1556,53 @@ template <typename TOut, int V> int launch_spmm_t(const spmmt::Params &p, int m_
                                 blk_entries, capacity, mode == SpmmTMode::kDense ? 1 : 0, 1100.0f, 0.0f, 5.0f * V, 1.5f, flag);
     const int64_t items = (int64_t)q.batch * n_tiles * m_tiles;
     const unsigned grid = (unsigned)(items < d->sm_count ? items : d->sm_count);   // one persistent CTA per SM
-    if (rc == VS_OK) {
+    for (int i = 0; i < count && rc == VS_OK; ++i) {
+        q.values = list[i].values; q.rhs = list[i].rhs; q.out = list[i].out;
         int rc_pair = VS_OK;
         if (use_b4 && spmm_pair_takes(q.N, (int64_t)q.batch * m_tiles, d) &&
-            launch_spmm_pair<TOut, V, true>(q, s, d, map, map_out, map_b4, blk_offsets, blk_entries, m_tiles, k_blocks, flag, checks, &rc_pair))
+            launch_spmm_pair<TOut, V, true>(q, s, d, map[i], map_out[i], map_b4[i], blk_offsets, blk_entries, m_tiles, k_blocks, flag, checks, &rc_pair))
             rc = rc_pair;
         else
-            rc = (int)launch_overlapped(kernel, grid, densespmm::kThreads, densespmm::kSmemBytes, s, q, map, map_out, map_b4, use_b4,
+            rc = (int)launch_overlapped(kernel, grid, densespmm::kThreads, densespmm::kSmemBytes, s, q, map[i], map_out[i], map_b4[i], use_b4,
                                         blk_offsets, blk_entries, m_tiles, n_tiles, k_blocks, d->status, flag, checks);
+        if (rc == VS_OK) rc = launch_spmm_t_cc<TOut, V>(list[i], s, d, flag, checks);
     }
-    if (rc == VS_OK) rc = launch_spmm_t_cc<TOut, V>(p, s, d, flag, checks);
     return rc;
 }
-template <typename TOut> int spmm_t_by_v(int V, const spmmt::Params &p, int m_vec, cudaStream_t s) {
+template <typename TOut> int spmm_t_by_v(int V, const spmmt::Params *p, int count, int m_vec, cudaStream_t s) {
     switch (V) {
-        case 1: return launch_spmm_t<TOut, 1>(p, m_vec, s);
-        case 2: return launch_spmm_t<TOut, 2>(p, m_vec, s);
-        case 4: return launch_spmm_t<TOut, 4>(p, m_vec, s);
-        case 8: return launch_spmm_t<TOut, 8>(p, m_vec, s);
+        case 1: return launch_spmm_t<TOut, 1>(p, count, m_vec, s);
+        case 2: return launch_spmm_t<TOut, 2>(p, count, m_vec, s);
+        case 4: return launch_spmm_t<TOut, 4>(p, count, m_vec, s);
+        case 8: return launch_spmm_t<TOut, 8>(p, count, m_vec, s);
     }
     return VS_ERR_VEC_LENGTH;
+}
+}  // namespace
+
+namespace {
+// Checks one batched product with the transposed matrix and fills in its parameters; *empty where there is nothing to compute.
+int spmm_t_params(int in_dtype, int out_dtype, int m_vec, int vec_length, int k, int n, const int32_t *t_offsets, const int32_t *t_rows,
+                  const int32_t *t_src, const void *values, const void *rhs_matrix, void *output_matrix, int batch, int64_t stride_values,
+                  int64_t stride_rhs, int64_t stride_out, spmmt::Params &p, bool &empty) {
+    empty = false;
+    if (!valid_v(vec_length)) return VS_ERR_VEC_LENGTH;
+    if (!(in_dtype == VS_F16 && (out_dtype == VS_F16 || out_dtype == VS_F32))) return VS_ERR_DTYPE;
+    if (m_vec < 0 || k < 0 || n < 0 || k % 8 != 0) return VS_ERR_SHAPE;
+    if ((int64_t)m_vec * vec_length > 0x7fffffffll) return VS_ERR_SHAPE;
+    if (batch < 1 || batch > kMaxBatch) return VS_ERR_ARG;
+    empty = n == 0 || k == 0;
+    if (empty) return VS_OK;
+    if (!t_offsets || !t_rows || !t_src || !values || !rhs_matrix || !output_matrix) return VS_ERR_NULL;
+    if (!aligned16(values) || !aligned16(rhs_matrix) || !aligned16(output_matrix)) return VS_ERR_ALIGN;
+    if (!stride_ok(stride_values, in_dtype) || !stride_ok(stride_rhs, in_dtype) || !stride_ok(stride_out, out_dtype))
+        return VS_ERR_ALIGN;
+    if (batch > 1 && stride_out == 0) return VS_ERR_ARG;
+    p.n = n; p.N = k; p.batch = batch;
+    p.t_offsets = t_offsets; p.t_rows = t_rows; p.t_src = t_src;
+    p.values = static_cast<const __half *>(values); p.rhs = static_cast<const __half *>(rhs_matrix); p.out = output_matrix;
+    p.stride_values = stride_values; p.stride_rhs = stride_rhs; p.stride_out = stride_out;
+    return VS_OK;
 }
 }  // namespace
 
@@ -1569,24 +1610,13 @@ VS_EXPORT int vs_spmm_t_batched(int in_dtype, int out_dtype, int m_vec, int vec_
                                 const int32_t *t_offsets, const int32_t *t_rows, const int32_t *t_src,
                                 const void *values, const void *rhs_matrix, void *output_matrix, int batch,
                                 int64_t stride_values, int64_t stride_rhs, int64_t stride_out, void *stream) {
-    if (!valid_v(vec_length)) return VS_ERR_VEC_LENGTH;
-    if (!(in_dtype == VS_F16 && (out_dtype == VS_F16 || out_dtype == VS_F32))) return VS_ERR_DTYPE;
-    if (m_vec < 0 || k < 0 || n < 0 || k % 8 != 0) return VS_ERR_SHAPE;
-    if ((int64_t)m_vec * vec_length > 0x7fffffffll) return VS_ERR_SHAPE;
-    if (batch < 1 || batch > kMaxBatch) return VS_ERR_ARG;
-    if (n == 0 || k == 0) return VS_OK;
-    if (!t_offsets || !t_rows || !t_src || !values || !rhs_matrix || !output_matrix) return VS_ERR_NULL;
-    if (!aligned16(values) || !aligned16(rhs_matrix) || !aligned16(output_matrix)) return VS_ERR_ALIGN;
-    if (!stride_ok(stride_values, in_dtype) || !stride_ok(stride_rhs, in_dtype) || !stride_ok(stride_out, out_dtype))
-        return VS_ERR_ALIGN;
-    if (batch > 1 && stride_out == 0) return VS_ERR_ARG;
     spmmt::Params p;
-    p.n = n; p.N = k; p.batch = batch;
-    p.t_offsets = t_offsets; p.t_rows = t_rows; p.t_src = t_src;
-    p.values = static_cast<const __half *>(values); p.rhs = static_cast<const __half *>(rhs_matrix); p.out = output_matrix;
-    p.stride_values = stride_values; p.stride_rhs = stride_rhs; p.stride_out = stride_out;
+    bool empty;
+    const int rc = spmm_t_params(in_dtype, out_dtype, m_vec, vec_length, k, n, t_offsets, t_rows, t_src, values, rhs_matrix, output_matrix, batch,
+                                 stride_values, stride_rhs, stride_out, p, empty);
+    if (rc != VS_OK || empty) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    return out_dtype == VS_F16 ? spmm_t_by_v<__half>(vec_length, p, m_vec, s) : spmm_t_by_v<float>(vec_length, p, m_vec, s);
+    return out_dtype == VS_F16 ? spmm_t_by_v<__half>(vec_length, &p, 1, m_vec, s) : spmm_t_by_v<float>(vec_length, &p, 1, m_vec, s);
 }
 
 VS_EXPORT int vs_spmm_t(int in_dtype, int out_dtype, int m_vec, int vec_length, int k, int n, const int32_t *t_offsets,
@@ -1773,12 +1803,14 @@ VS_EXPORT int vs_attention_cvse_backward(int path, int m_vec, int vec_length, in
         cudaStream_t st = static_cast<cudaStream_t>(stream);
         rc = d == 64 ? launch_attention_rows<64, true>(p, batch, info, st) : launch_attention_rows<128, true>(p, batch, info, st);
         if (rc != VS_OK) return rc;
-        // dV = P^T dO,  dK = dS^T Q
-        rc = vs_spmm_t_batched(VS_F16, VS_F16, m_vec, vec_length, d, n, t_offsets, t_rows, t_src, probs_workspace, grad_out, grad_v,
-                               batch, s_ws, s_q, s_k, stream);
-        if (rc != VS_OK) return rc;
-        return vs_spmm_t_batched(VS_F16, VS_F16, m_vec, vec_length, d, n, t_offsets, t_rows, t_src, grad_workspace, q, grad_k, batch,
-                                 s_ws, s_q, s_k, stream);
+        // dV = P^T dO and dK = dS^T Q from one plan
+        spmmt::Params both[2];
+        bool empty;
+        rc = spmm_t_params(VS_F16, VS_F16, m_vec, vec_length, d, n, t_offsets, t_rows, t_src, probs_workspace, grad_out, grad_v, batch, s_ws, s_q, s_k, both[0], empty);
+        if (rc == VS_OK && !empty)
+            rc = spmm_t_params(VS_F16, VS_F16, m_vec, vec_length, d, n, t_offsets, t_rows, t_src, grad_workspace, q, grad_k, batch, s_ws, s_q, s_k, both[1], empty);
+        if (rc != VS_OK || empty) return rc;
+        return spmm_t_by_v<__half>(vec_length, both, 2, m_vec, st);
     }
     // P = softmax(scale * Q K^T) at the mask, recomputed rather than kept from the forward pass
     int rc = vs_sddmm_batched(path, VS_F16, VS_F16, m_vec, d, n, nonzeros_vec, row_indices, row_offsets, col_indices, q, kmat,
