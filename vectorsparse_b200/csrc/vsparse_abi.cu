@@ -987,9 +987,12 @@ template <int V> int launch_spmm_split(const SpmmParams &p, int64_t vectors, cud
     const int tn = t_narrow < t_wide ? 128 : 256, n_tiles = (int)(tn == 256 ? wide : narrow);
     const int row_tiles = (int)((M + 127) / 128), slabs = q.Np / 64;
     const int64_t a_elems = (int64_t)q.batch_a * row_tiles * 128 * q.Kp, b_elems = (int64_t)q.batch_b * q.Kp * q.Np;
-    // us: 64 columns of an item by a pair, the preparation at 4 TB/s, launches; against the CUDA-core kernel per vector and column
+    // us: 64 columns of an item by a pair, the preparation at 4 TB/s, launches (180 estimated, 165 to 180 measured at 4096 x 4096 x 1024; 94
+    // and 92 to 100 at 2048 cubed; 136 and 142 at 8 x (2000 x 1000 x 640)); against the CUDA-core kernel's time per vector and column (611 us
+    // at V = 1, 305 at V = 2, 301 at V = 4, 258 at V = 8 for 4096 x 4096 x 1024, 80 % sparse).  Below kMinDensity that kernel keeps every
+    // dense width, so that column shards of usual matrices (90 %, at V = 4 80 % sparse) have the bits of the whole product.
     const double split_us = k_blocks * std::min(t_wide, t_narrow) + (double)(6 * a_elems + 10 * b_elems) / 4e6 + 10.0;
-    constexpr double kCoresPs = V == 1 ? 0.195 : V == 2 ? 0.23 : V == 4 ? 0.29 : 0.45, kMinDensity = V == 1 ? 0.102 : V == 2 ? 0.11 : V == 4 ? 0.205 : 0.13;
+    constexpr double kCoresPs = V <= 2 ? 0.18 : V == 4 ? 0.35 : 0.6, kMinDensity = V == 1 ? 0.102 : V == 2 ? 0.11 : V == 4 ? 0.205 : 0.13;
     q.min_vectors = forced ? 0 : (int64_t)std::max(1.1 * split_us / (kCoresPs * 1e-6 * p.N * p.batch), kMinDensity * p.m_vec * (double)p.K);
     if (!forced && (vectors < q.min_vectors || p.N < 256)) return VS_OK;
     const int64_t units = (int64_t)q.batch_a * p.m_vec + b_elems / (8 * splitspmm::kPrepThreads) + 1;
