@@ -147,3 +147,53 @@ def test_kernel_timing_brackets_the_multiplying_kernel(monkeypatch):
     assert all(np.array_equal(t, plain) for t in timed)
     run(a, 256, vals, B, torch.float16, True, monkeypatch)
     assert ops.kernel_timing(False) == (0.0, 0)
+
+
+# rows around a CTA's 128 and the pair's 256, columns around a stage's 64 and the 8192 / V that are laid out at a time, several and single
+# vector-rows at a time
+@pytest.mark.parametrize("V,m_vec,K,N", [(1, 1, 1, 128), (1, 257, 63, 192), (1, 130, 8250, 256), (2, 65, 129, 320), (2, 300, 64, 1024), (2, 129, 4160, 448)])
+@pytest.mark.parametrize("what", ["plain", "repeated", "non-finite"])
+def test_a_laid_out_beforehand(V, m_vec, K, N, what, monkeypatch):
+    """The same bits as with A filled in from a plan (which at K = 8250 is too large, so that call goes to the CUDA cores); a column named twice
+    and an Inf that some vector-rows name go to the kernel behind."""
+    monkeypatch.setenv("VSPARSE_B200_SPMM", "dense")
+    monkeypatch.setenv("VSPARSE_B200_SPMM_PAIR", "1")
+    a = problem(cvse.GEN_UNIFORM, 3, m_vec, K, V, 0.0 if K == 1 else 0.7)
+    vals = cvse.fill_random((a.nnz_vec * V,), np.float16, cvse.DIST_NORMAL, 1, 0.25)
+    B = cvse.fill_random((K, N), np.float16, cvse.DIST_NORMAL, 2, 0.5)
+    if what == "repeated":
+        i = int(np.argmax(np.diff(a.row_offsets)))
+        if np.diff(a.row_offsets)[i] > 1:
+            a.col_indices[a.row_offsets[i] + 1] = a.col_indices[a.row_offsets[i]]
+    elif what == "non-finite":
+        B[a.col_indices[0], 5] = np.inf
+    got = {}
+    for how in ("plan", "laid-out"):
+        monkeypatch.setenv("VSPARSE_B200_SPMM_A", how)
+        out = torch.full((a.m * N + 64,), float("nan"), dtype=torch.float16, device=DEV)
+        (ops.spmm.cudaSpmm if V == 1 else ops.spmm.wmmaSpmm)(m_vec, V, N, K, *structure(a), dev(vals), dev(B), out)
+        torch.cuda.synchronize()
+        assert ops.device_status() == 0
+        assert bool(torch.isnan(out[a.m * N:]).all()), "wrote past the end"
+        got[how] = out[:a.m * N].view(a.m, N).float().cpu().numpy()
+    assert K > 5000 or np.array_equal(got["plan"], got["laid-out"], equal_nan=True)
+    want = spmm_oracle(a, N, vals, B).reshape(a.m, N)
+    finite = np.isfinite(want)
+    assert_close(np.where(finite, got["laid-out"], 0), np.where(finite, want, 0), f"{V} {what}")
+
+
+def test_batches_of_matrices_laid_out_beforehand(monkeypatch):
+    monkeypatch.setenv("VSPARSE_B200_SPMM", "dense")
+    monkeypatch.setenv("VSPARSE_B200_SPMM_A", "laid-out")
+    V, N, K, batch = 2, 192, 200, 5
+    a = problem(cvse.GEN_BETA, 4, 150, K, V, 0.8)
+    row = (a.nnz_vec * V + 7) // 8 * 8
+    vals = cvse.fill_random((batch, row), np.float16, cvse.DIST_NORMAL, 1, 0.5)
+    B = cvse.fill_random((batch, K, N), np.float16, cvse.DIST_NORMAL, 2, 1.0)
+    for shared in (False, True):
+        out = torch.full((batch, a.m, N), float("nan"), dtype=torch.float32, device=DEV)
+        ops.spmm_batched(VS_PATH_TENSOR, a.m_vec, V, N, K, *structure(a), dev(vals[0] if shared else vals), dev(B), out)
+        torch.cuda.synchronize()
+        assert ops.device_status() == 0
+        for i in range(batch):
+            assert_close(out[i].cpu().numpy(), spmm_oracle(a, N, vals[0 if shared else i][:a.nnz_vec * V], B[i]), f"problem {i}")

@@ -68,6 +68,7 @@ constexpr int kOverflowBatches = 4;
 constexpr int kLoadWarp = kFillWarp0 + kFillWarps;        // 20
 constexpr int kMmaWarp = kLoadWarp + 1;
 constexpr int kThreads = (kMmaWarp + 1) * 32;
+constexpr int kPreparedThreads = (kEpiWarps + 2) * 32;    // with A laid out beforehand: no fill warps
 static_assert(kThreads <= 1024, "too many fill warps for one CTA");
 constexpr int kAStageBytes = kCtaRows * kBlockK * 2;      // 16 KiB
 constexpr int kBSlabBytes = kBlockK * 64 * 2;             // 8 KiB: 64 rows of B x 64 columns
@@ -152,9 +153,11 @@ struct Walk {
 // box {64, 64, 2, 1} (both 64-column slabs of a CTA's half of a 256-column tile in one copy); map_out: the output
 // as {N, rows, batch}, box {32, 32, 1}.  All with zero fill / clipping outside the matrix; no multicast anywhere.
 // tn: columns per work item (256 or 128), N % 64 == 0; the last tile of a row may be wider than what is left of the matrix.
-template <typename TOut, int V, bool kTransposed>
-__global__ void __launch_bounds__(kThreads, 1)
-spmm_pair_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_out,
+// kPrepared: the tiles of A have been laid out in memory, 128 rows by 64 columns with the columns contiguous (densify_kernel), and come
+// through map_a, {64, 128, 1, tiles}, box {64, 128, 1, 1}, beside those of B; batch_a == 1: one matrix for the whole batch; no fill warps.
+template <typename TOut, int V, bool kTransposed, bool kPrepared = false>
+__global__ void __launch_bounds__(kPrepared ? kPreparedThreads : kThreads, 1)
+spmm_pair_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_a, int batch_a, int row_tiles, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_out,
                  const __grid_constant__ CUtensorMap map_b2, int tn, const int32_t *__restrict__ blk_offsets,
                  const uint2 *__restrict__ blk_entries, int m_tiles, int n_tiles, int k_blocks, uint32_t *status, int32_t *use_dense,
                  int plan_checks) {
@@ -167,7 +170,7 @@ spmm_pair_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b, 
     uint8_t *sm = smem_raw + (base - raw);
 
     const int t = threadIdx.x;
-    const int warp = t >> 5;
+    const int warp = kPrepared && t >= kEpiWarps * 32 ? (t >> 5) + kFillWarps : t >> 5;   // the number of the role
     const int lane = t & 31;
     const uint32_t rank = tc::cluster_ctarank();   // 0: the CTA that issues the MMAs
     const uint32_t peer = rank ^ 1u;
@@ -179,12 +182,13 @@ spmm_pair_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b, 
     const uint32_t bar_acc_full = base + Smem::kBarAccFull;
     const uint32_t bar_acc_empty = base + Smem::kBarAccEmpty;
 
+    if constexpr (!kPrepared)
     for (int i = t; i < kAStages * kAStageBytes / 16; i += kThreads)   // the A slots start out as zeros
         reinterpret_cast<uint4 *>(sm + Smem::kA)[i] = make_uint4(0, 0, 0, 0);
     if (t == 0) {
         for (int s = 0; s < kBarStages; ++s) {
             // first CTA only: the fill warps of both CTAs, its loader's arrival + the bytes of BOTH CTAs' B tiles
-            tc::mbar_init(bar_full + 8 * s, 2 * kFillPerSlot + 1);
+            tc::mbar_init(bar_full + 8 * s, kPrepared ? 1 : 2 * kFillPerSlot + 1);
             tc::mbar_init(bar_done + 8 * s, 1);   // a commit of the MMA-issuing thread, which arrives in both CTAs
         }
         for (int s = 0; s < 2; ++s) {
@@ -215,6 +219,7 @@ spmm_pair_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b, 
     // g % kBStages and barrier set g % kBarStages.  done[g % kBarStages] completing phase g / kBarStages says "stage g
     // has been multiplied": the fill warps of stage g + kAStages and the loader of stage g + kBStages wait for it.
     if (warp >= kFillWarp0 && warp < kLoadWarp) {
+        if constexpr (!kPrepared) {
         // =========================== fill ================================================================
         // Warp (a_slot, quarter) drops the entries of one plan bucket (this CTA's 128 rows x columns 16 quarter .. + 15
         // of the stage) into the A slot, after taking out what it dropped there for the stage kAStages earlier: a
@@ -342,6 +347,7 @@ spmm_pair_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b, 
             }
             { const Pos q = locate(); bounds(q, f_e0, f_e1); f_b = q.b; }
         }
+        }
     } else if (warp == kLoadWarp) {
         // =========================== B loader ============================================================
         // This CTA's half of every B tile, up to kBStages stages ahead, into its own shared memory, completing on its
@@ -363,7 +369,10 @@ spmm_pair_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b, 
                 // CTA's loader arms with the bytes of both halves
                 const uint32_t bar = full_first + 8 * (g % kBarStages);
                 const int n0 = walk.nt * tn + (int)rank * half_cols;   // first column of this CTA's half
-                if (rank == 0) tc::mbar_expect_tx(bar_full + 8 * (g % kBarStages), 2u * (uint32_t)slabs * kBSlabBytes);
+                if (rank == 0) tc::mbar_expect_tx(bar_full + 8 * (g % kBarStages), 2u * ((uint32_t)slabs * kBSlabBytes + (kPrepared ? kAStageBytes : 0)));
+                if constexpr (kPrepared)
+                    tc::tma_load_4d_pair(base + Smem::kA + slot * kAStageBytes, &map_a, bar, 0, 0, 0,
+                                         ((batch_a == 1 ? 0 : walk.b) * row_tiles + 2 * walk.mt + (int)rank) * k_blocks + walk.kb);
                 if (slabs == 2) {
                     tc::tma_load_4d_pair(base + Smem::kB + slot * kBStageBytes, &map_b2, bar, 0, walk.kb * kBlockK, n0 >> 6, walk.b);
                 } else {
@@ -377,11 +386,12 @@ spmm_pair_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b, 
     } else if (warp == kMmaWarp) {
         if (lane == 0 && rank == 0) {
             // =========================== MMA issuer of the pair ==========================================
-            const uint32_t a_lo0 = tc::smem_desc_lo(base + Smem::kA, 8192);   // 64-row atoms 8 KiB apart
+            const uint32_t a_lo0 = tc::smem_desc_lo(base + Smem::kA, kPrepared ? 16 : 8192);   // 64-row atoms 8 KiB apart; K-major: 8-row groups 1 KiB apart
+            constexpr uint32_t kStepA = kPrepared ? 2 : 128;   // 16 columns of A: 32 bytes on in a row, or 2 KiB
             const uint32_t a_hi = tc::smem_desc_hi(1024, (uint32_t)tc::kSwizzle128B);
             const uint32_t b_lo0 = tc::smem_desc_lo(base + Smem::kB, kBSlabBytes);   // 64-column slabs 8 KiB apart
             const uint32_t b_hi = tc::smem_desc_hi(1024, (uint32_t)tc::kSwizzle128B);
-            const uint32_t idesc = tc::make_idesc_f16(256, tn, 1, 1);   // both operands MN-major
+            const uint32_t idesc = tc::make_idesc_f16(256, tn, kPrepared ? 0 : 1, 1);   // MN-major, a prepared A K-major
             // Per stage: one barrier poll, four MMAs, one commit.  No tensor-core fence per stage: the operands were
             // written by TMA, or by stores that their writers fenced for the async proxy before arriving.
             uint32_t a_slot = 0, b_slot = 0, bar = 0, parity = 0;
@@ -397,15 +407,15 @@ spmm_pair_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b, 
                     ok_run = wait_or_abort<kSleepMma>(bar_full + 8 * bar, parity, abort_flag, abort_addr, peer);
                     if (!ok_run) break;
                     const uint32_t a_lo = a_lo0 + a_slot * (kAStageBytes >> 4), b_lo = b_lo0 + b_slot * (kBStageBytes >> 4);
-                    // 16 columns of A = 16 rows of B = 2 KiB further on in either operand
+                    // 16 rows of B are 2 KiB further on
                     if (kb + 1 < k_blocks || steps_last == kBlockK / 16) {
                         tc::mma_f16_ss_pair(d, tc::desc64(a_lo, a_hi), tc::desc64(b_lo, b_hi), idesc, kb > 0 ? 1u : 0u);
-                        tc::mma_f16_ss_pair(d, tc::desc64(a_lo + 128, a_hi), tc::desc64(b_lo + 128, b_hi), idesc, 1u);
-                        tc::mma_f16_ss_pair(d, tc::desc64(a_lo + 256, a_hi), tc::desc64(b_lo + 256, b_hi), idesc, 1u);
-                        tc::mma_f16_ss_pair(d, tc::desc64(a_lo + 384, a_hi), tc::desc64(b_lo + 384, b_hi), idesc, 1u);
+                        tc::mma_f16_ss_pair(d, tc::desc64(a_lo + 1 * kStepA, a_hi), tc::desc64(b_lo + 128, b_hi), idesc, 1u);
+                        tc::mma_f16_ss_pair(d, tc::desc64(a_lo + 2 * kStepA, a_hi), tc::desc64(b_lo + 256, b_hi), idesc, 1u);
+                        tc::mma_f16_ss_pair(d, tc::desc64(a_lo + 3 * kStepA, a_hi), tc::desc64(b_lo + 384, b_hi), idesc, 1u);
                     } else {
                         for (int kk = 0; kk < steps_last; ++kk)
-                            tc::mma_f16_ss_pair(d, tc::desc64(a_lo + 128 * kk, a_hi), tc::desc64(b_lo + 128 * kk, b_hi), idesc,
+                            tc::mma_f16_ss_pair(d, tc::desc64(a_lo + kk * kStepA, a_hi), tc::desc64(b_lo + 128 * kk, b_hi), idesc,
                                                 (kb > 0 || kk > 0) ? 1u : 0u);
                     }
                     tc::mma_commit_pair_both(bar_done + 8 * bar);   // "stage multiplied", in both CTAs at once

@@ -740,30 +740,31 @@ int spmm_pair_width(int N, int64_t row_items, int pairs) {
     const int64_t wide = row_items * ((N + 255) / 256), narrow = row_items * ((N + 127) / 128);
     return 9 * ((narrow + pairs - 1) / pairs) < 10 * ((wide + pairs - 1) / pairs) ? 128 : 256;
 }
+// How many pairs of `kernel` this device holds; -1 where it cannot run it.
+template <typename K> int pair_capacity(K kernel, int threads, int (&resident)[kMaxDevices], DeviceInfo *d) {
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return -1;
+    if (resident[dev] == 0) {   // not asked yet
+        const int n = set_smem(kernel, pairspmm::kSmemBytes) == VS_OK ? max_resident_pairs(kernel, threads, pairspmm::kSmemBytes, d) : 0;
+        resident[dev] = n > 0 ? n : -1;
+    }
+    return resident[dev];
+}
 // Enqueues the pair kernel for a call whose plan kernel has been enqueued; false if this device cannot hold it.
 template <typename TOut, int V, bool kTransposed>
 bool launch_spmm_pair(const SpmmParams &q, cudaStream_t s, DeviceInfo *d, const CUtensorMap &map, const CUtensorMap &map_out,
                       const CUtensorMap &map_b2, const int32_t *blk_offsets, const uint2 *blk_entries, int m_tiles, int k_blocks,
                       int32_t *flag, int checks, int *rc_out) {
-    static int resident[kMaxDevices];   // 0 = not asked yet, -1 = the kernel cannot run here
+    static int resident[kMaxDevices];
     auto kernel = pairspmm::spmm_pair_kernel<TOut, V, kTransposed>;
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return false;
-    if (resident[dev] == 0) {
-        if (set_smem(kernel, pairspmm::kSmemBytes) != VS_OK) {
-            resident[dev] = -1;
-        } else {
-            const int n = max_resident_pairs(kernel, pairspmm::kThreads, pairspmm::kSmemBytes, d);
-            resident[dev] = n > 0 ? n : -1;
-        }
-    }
-    if (resident[dev] < 0) return false;
-    const int tn = spmm_pair_width(q.N, (int64_t)q.batch * m_tiles, resident[dev]);
+    const int capacity = pair_capacity(kernel, pairspmm::kThreads, resident, d);
+    if (capacity < 0) return false;
+    const int tn = spmm_pair_width(q.N, (int64_t)q.batch * m_tiles, capacity);
     const int n_tiles = (q.N + tn - 1) / tn;
     const int64_t items = (int64_t)q.batch * n_tiles * m_tiles;
-    const unsigned pairs = (unsigned)(items < resident[dev] ? items : resident[dev]);
+    const unsigned pairs = (unsigned)(items < capacity ? items : capacity);
     TimedLaunch timed(s);
-    *rc_out = (int)launch_pairs(kernel, pairs, pairspmm::kThreads, (size_t)pairspmm::kSmemBytes, s, true, q, map, map_out, map_b2, tn,
+    *rc_out = (int)launch_pairs(kernel, pairs, pairspmm::kThreads, (size_t)pairspmm::kSmemBytes, s, true, q, map, 1, 0, map, map_out, map_b2, tn,
                                 blk_offsets, blk_entries, m_tiles, n_tiles, k_blocks, d->status, flag, checks);
     return true;
 }
@@ -857,6 +858,61 @@ bool spmm_direct_wanted(const SpmmParams &p, int V, bool cores, const DeviceInfo
     return tiles <= 4 * d->sm_count && chunks <= (V >= 4 ? 4 : 1);
 }
 
+// The same product with A laid out densely in memory first (densify.cuh), at V <= 2, where filling the tiles from a plan is what the pair
+// kernel spends its time on: a stage takes it 1 to 3 us at V = 1 (95 to 80 % sparse) and 0.8 to 1.2 at V = 2, with A laid out 0.5.  Laying it out
+// takes 0.67 us per MB, once instead of for every 256 columns of B.  us, plan / laid out: V = 1, 4096 x 4096 x 1024, 80 / 95 %: 190 / 52 and
+// 69 / 44, 8 x (1000 x 1000 x 640), 70 %: 79 / 39; V = 2, 4096 x 4096 x 1984, 70 %: 156 / 73, 4096 x 4096 x 256, 90 %: 50 / 41; but
+// 64 x (1024 x 256 x 256), V = 1, 80 %: 34 / 41, 64 x (2048 x 512 x 256), V = 2, 90 %: 41 / 97.
+// Enqueues everything and returns true, or leaves the call alone.  VSPARSE_B200_SPMM_A=plan|laid-out.
+template <typename TOut, int V, bool kCores> bool launch_spmm_laid_out(const SpmmParams &p, cudaStream_t s, DeviceInfo *d, bool forced, int *rc_out) {
+    const char *e = std::getenv("VSPARSE_B200_SPMM_A");
+    if (e && !std::strcmp(e, "plan")) return false;
+    static int resident[kMaxDevices];
+    auto kernel = pairspmm::spmm_pair_kernel<TOut, 1, false, true>;   // V is the layout's business
+    const int capacity = pair_capacity(kernel, pairspmm::kPreparedThreads, resident, d);
+    const int64_t M = (int64_t)p.m_vec * V;
+    const int m_tiles = (int)((M + pairspmm::kTileM - 1) / pairspmm::kTileM), row_tiles = (int)((M + 127) / 128);
+    const int Kp = (p.K + 63) / 64 * 64, k_blocks = Kp / 64, batch_a = p.batch > 1 && p.stride_values ? p.batch : 1;
+    const int64_t row_items = (int64_t)p.batch * m_tiles, a_bytes = (int64_t)batch_a * row_tiles * 128 * Kp * 2;
+    if (capacity < 0 || !spmm_pair_takes(p.N, row_items, d) || a_bytes > (128ll << 20)) return false;
+    const int tn = spmm_pair_width(p.N, row_items, capacity), n_tiles = (p.N + tn - 1) / tn;
+    const int64_t items = row_items * n_tiles;
+    if (items * k_blocks > 0x7fffffffll) return false;
+    if (!e) {
+        const double waves = (double)((items + capacity - 1) / capacity);
+        if (waves * k_blocks * (V == 1 ? 1.1 : 0.4) < 0.67e-6 * (double)a_bytes + 3.0) return false;
+    }
+    SpmmCosts c = kGatherCosts;
+    if constexpr (kCores) c = cores_costs_of(p, V, items, d->sm_count / 2, d);
+    const double stages = (double)m_tiles * k_blocks;
+    const int64_t min_vectors = forced ? 0 : (int64_t)std::max(0.0, std::ceil((stages * c.dense_per_stage - (double)p.m_vec * c.gather_per_row) / (c.gather_per_entry - c.dense_per_entry)));
+    const int checks = (int)std::min<int64_t>((int64_t)batch_a * p.m_vec, 8 * d->sm_count);
+    const int64_t header = ((4 + checks) * 4 + 255) / 256 * 256;
+    CUtensorMap map_a, map_b, map_b2, map_out;
+    if (make_tile_map(&map_b, p.rhs, false, (uint64_t)p.K, (uint64_t)p.N, (uint64_t)p.batch, (uint64_t)p.stride_rhs, 64, 64) != VS_OK ||
+        make_blocked_map(&map_b2, p.rhs, (uint64_t)p.K, (uint64_t)p.N, (uint64_t)p.batch, (uint64_t)p.stride_rhs, 2) != VS_OK ||
+        make_tile_map(&map_out, p.out, sizeof(TOut) == 4, (uint64_t)M, (uint64_t)p.N, (uint64_t)p.batch, (uint64_t)p.stride_out, pairspmm::kStoreCols, 32) != VS_OK)
+        return false;
+    uint8_t *mem = nullptr;
+    PlanScratch scratch;
+    if (scratch.take(d, s, (size_t)(header + a_bytes), reinterpret_cast<void **>(&mem)) != VS_OK) return false;
+    if (make_packed_map(&map_a, mem + header, 64, 128, 1, (uint64_t)batch_a * row_tiles * k_blocks, 1) != VS_OK) return false;
+    int32_t *verdict = reinterpret_cast<int32_t *>(mem);
+    int rc = (int)launch_overlapped(densify::densify_kernel<V>, (unsigned)checks, densify::kPrepThreads, 0, s, p, batch_a, Kp, min_vectors,
+                                    reinterpret_cast<uint16_t *>(mem + header), verdict);
+    if (rc == VS_OK) {
+        TimedLaunch timed(s);
+        SpmmParams q = p;
+        q.m_vec = (int)M;
+        rc = (int)launch_pairs(kernel, (unsigned)std::min<int64_t>(items, capacity), pairspmm::kPreparedThreads, (size_t)pairspmm::kSmemBytes, s, true, q, map_a,
+                               batch_a, row_tiles, map_b, map_out, map_b2, tn, (const int32_t *)nullptr, (const uint2 *)nullptr, m_tiles, n_tiles,
+                               k_blocks, d->status, verdict, checks);
+    }
+    if (rc == VS_OK) rc = launch_spmm_other<TOut, V, kCores>(p, s, d, verdict, checks);
+    *rc_out = rc;
+    return true;
+}
+
 template <typename TOut, int V, bool kCores> int launch_spmm_tc(const SpmmParams &p, cudaStream_t s) {
     DeviceInfo *d;
     int rc = device_info(&d);
@@ -866,6 +922,11 @@ template <typename TOut, int V, bool kCores> int launch_spmm_tc(const SpmmParams
     if ((mode == SpmmMode::kDirect || (mode == SpmmMode::kAuto && spmm_direct_wanted(p, V, kCores, d))) &&
         launch_spmm_direct<TOut, V, kCores>(p, s, d, cost, mode == SpmmMode::kDirect, &rc))
         return rc;
+    if constexpr (V <= 2) {
+        if (!t_no_scratch && mode != SpmmMode::kGather && p.K > 0 && (p.batch == 1 || (p.stride_rhs * 2) % 16 == 0) &&
+            (p.batch == 1 || (p.stride_out * sizeof(TOut)) % 16 == 0) && launch_spmm_laid_out<TOut, V, kCores>(p, s, d, mode == SpmmMode::kDense, &rc))
+            return rc;
+    }
     const int k_blocks = (p.K + densespmm::kBlockK - 1) / densespmm::kBlockK;
     const int m_tiles = (p.m_vec * V + densespmm::kTileM - 1) / densespmm::kTileM;
     const int n_tiles = (p.N + densespmm::kTileN - 1) / densespmm::kTileN;
