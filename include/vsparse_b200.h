@@ -4,7 +4,7 @@
  * Every entry point takes plain pointers and sizes.  Unless a function says "host", pointers are DEVICE
  * pointers owned by the caller; the library enqueues its kernels on `stream` (a cudaStream_t passed as void*)
  * and returns without synchronising.  One piece of device memory is the library's own: the operators that
- * multiply on the tensor cores (wmma*, and cuda* with fp16 results) keep a plan scratch per calling stream (cudaMallocAsync at the
+ * multiply on the tensor cores (wmma*, and cuda* products large enough for it) keep a plan scratch per calling stream (cudaMallocAsync at the
  * first call on a stream that needs one, and again when a larger matrix needs more; vs_release_scratch frees it; under capture, see vs_spmm).
  * A caller that hands over a buffer with vs_set_workspace gets a library that never allocates.
  *
@@ -79,10 +79,15 @@ const char *vs_version(void);
  * way, include/bm_test_utils.h:110-124, and its kernels add both values) is recognised on the device and goes
  * to the gather kernel, which adds them too.
  * Products of up to about one wave of tiles do the same in one kernel without a plan.  fp16 results with VS_PATH_CUDA_CORE take
- * the same formulations, with the CUDA-core kernel in the place of the gather kernels; fp32 results there stay on the CUDA cores.
+ * the same formulations, with the CUDA-core kernel in the place of the gather kernels; fp16 operands with fp32 results there stay on the
+ * CUDA cores.  fp32 products of 256 and more dense columns that are not too sparse are multiplied on the tensor cores from three bf16
+ * parts of each operand, with sums in fp32 registers: no further from the exact result than the CUDA-core kernel's, which takes the
+ * rest (sparser matrices, repeated columns, non-finite results, operands below 2^-100 or results below 2^-96 in magnitude).
+ * Environment variable VSPARSE_B200_SPMM_F32 = "cores" | "split" forces one of the two.
  * Environment variable VSPARSE_B200_SPMM = "dense" | "gather" | "direct" (one kernel) forces one formulation.  The first call with a plan on a
  * stream allocates a scratch buffer with cudaMallocAsync on that stream (8 bytes per possible nonzero vector, m_vec * n
- * of them, at most 512 MB; reused and grown by later calls on the stream, freed by vs_release_scratch).  Under stream
+ * of them; up to 128 MB for a matrix with vectors of 1 or 2 that is laid out densely; 6 bytes per element of a dense A and of B for fp32
+ * products; at most 512 MB; reused and grown by later calls on the stream, freed by vs_release_scratch).  Under stream
  * capture a call's scratch belongs to the graph: it is allocated with cudaMalloc while the call is captured, shared by the
  * calls of one capture on one stream, and given back to the library when the graph and all that was instantiated from
  * it are gone.  Two executable graphs of one captured graph share it and must not run at the same time.  Everything else about
@@ -94,7 +99,8 @@ int vs_spmm(int path, int in_dtype, int out_dtype, int m_vec, int vec_length, in
 
 /* `batch` independent products that share one CVSE structure (row_indices/row_offsets/col_indices) and differ
  * in values, rhs and output, found at element strides stride_values / stride_rhs / stride_out from the first
- * (a stride of 0 shares that operand; stride_out must not be 0).  Strides must keep 16-byte alignment.
+ * (a stride of 0 shares that operand; stride_out must not be 0).  Strides must keep 16-byte alignment.  With batch 1 stride_values may
+ * say how many values there are, or an upper bound: calls too sparse for the tensor-core form of fp32 products then skip its kernels.
  * One launch covers the whole batch.  The reference has no batched call; this is the batch x head form of its
  * SpMM for fixed-mask sparse attention. */
 int vs_spmm_batched(int path, int in_dtype, int out_dtype, int m_vec, int vec_length, int k, int n,
@@ -181,8 +187,9 @@ int vs_softmax_cvse(int dtype, int m_vec, int vec_length, const int32_t *row_ind
  *   O_b = softmax(scale * SDDMM(Q_b, K_b)) . V_b, fp16 in and out, head dimension d (d % 64 == 0).
  * q [batch][m][d], kmat / vmat [batch][n][d], out [batch][m][d], all contiguous.
  * `workspace` must hold batch * nonzeros_vec * V fp16 values (the probabilities); the caller owns it.
- * One call for the whole batch (the batched form of the pipeline): it enqueues the SDDMM, the masked softmax and
- * the SpMM on `stream` (up to five kernels with their plan and fallback kernels); they are not fused into one. */
+ * One kernel for the whole batch on VS_PATH_TENSOR with d 64 or 128, vec_length 2, 4 or 8 and q, kmat, vmat on 32-byte boundaries (but
+ * not for d = 128, vec_length < 8 and more than a million keys); else the SDDMM, the masked softmax and the SpMM one after the other
+ * (up to five kernels with their plan and fallback kernels).  Environment variable VSPARSE_B200_ATTENTION = "fused" | "steps". */
 int vs_attention_cvse(int path, int m_vec, int vec_length, int n, int d, int nonzeros_vec,
                       const int32_t *row_indices, const int32_t *row_offsets, const int32_t *col_indices,
                       const void *q, const void *kmat, const void *vmat, void *out, void *workspace,
@@ -199,7 +206,8 @@ int vs_softmax_cvse_backward(int dtype, int m_vec, int vec_length, const int32_t
 /* Backward of vs_attention_cvse for fp16 q [m x d], kmat, vmat [n x d] per batch entry and one shared mask:
  * given grad_out [m x d] it writes grad_q [m x d], grad_k and grad_v [n x d] (fp16).  The probabilities are
  * recomputed (SDDMM + softmax into probs_workspace), then dV = P^T dO (vs_spmm_t), dP = dO V^T at the mask
- * (SDDMM), dS = softmax backward (in grad_workspace), dQ = dS K (SpMM), dK = dS^T Q (vs_spmm_t): seven calls of
+ * (SDDMM), dS = softmax backward (in grad_workspace), dQ = dS K (SpMM), dK = dS^T Q (vs_spmm_t).  Where vs_attention_cvse is one
+ * kernel (here with grad_out too), one kernel writes P, dS and dQ and the two transposed products share a plan; else seven calls of
  * the operators above on `stream`.  t_offsets / t_rows / t_src: the mask's transposed structure from
  * vs_cvse_transpose.  Both workspaces hold batch * nonzeros_vec * vec_length fp16 values and must differ.
  * No counterpart in the reference. */
