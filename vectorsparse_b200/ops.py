@@ -163,7 +163,7 @@ def _wmmaSpmm(m_vec, vec_length, k, n, row_indices, row_offsets, column_indices,
 def _cudaSpmm(m_vec, vec_length, k, n, row_indices, row_offsets, column_indices, values, rhs_matrix, output_matrix,
               nonzeros_vec=None):
     """SpMM for V in {1,2,4,8}; fp16 or fp32 (src/cuda_spmm.cu:304-338; fp32 is a stub there), on CUDA cores except for
-    fp16 results of fp16 operands, which come from the tensor cores where that is quicker.  nonzeros_vec: as for
+    fp16 results of fp16 operands and large fp32 products that are not too sparse, which come from the tensor cores where that is quicker.  nonzeros_vec: as for
     wmmaSpmm."""
     return _spmm(VS_PATH_CUDA_CORE, m_vec, vec_length, k, n, row_indices, row_offsets, column_indices, values,
                  rhs_matrix, output_matrix, nonzeros_vec=nonzeros_vec)
