@@ -1055,7 +1055,8 @@ template <int V> int launch_spmm_split(const SpmmParams &p, int64_t vectors, cud
     const double split_us = k_blocks * std::min(t_wide, t_narrow) + (double)(6 * a_elems + 10 * b_elems) / 4e6 + 10.0;
     constexpr double kCoresPs = V <= 2 ? 0.18 : V == 4 ? 0.35 : 0.6, kMinDensity = V == 1 ? 0.102 : V == 2 ? 0.11 : V == 4 ? 0.205 : 0.13;
     q.min_vectors = forced ? 0 : (int64_t)std::max(1.1 * split_us / (kCoresPs * 1e-6 * p.N * p.batch), kMinDensity * p.m_vec * (double)p.K);
-    if (!forced && (vectors < q.min_vectors || p.N < 256)) return VS_OK;
+    // A caller that does not say how many values there are: large products only, where two kernels that may return at once cost little.
+    if (!forced && (vectors < q.min_vectors || p.N < 256 || (p.stride_values == 0 && split_us < 100.0))) return VS_OK;
     const int64_t units = (int64_t)q.batch_a * p.m_vec + b_elems / (8 * splitspmm::kPrepThreads) + 1;
     const int checks = (int)std::min<int64_t>(units, 8 * d->sm_count);
     const int64_t header = ((4 + checks) * 4 + 255) / 256 * 256, a_bytes = (a_elems * 6 + 255) / 256 * 256, bytes = header + a_bytes + b_elems * 6;
