@@ -13,7 +13,8 @@
 //
 // The tensor cores that tcgen05 reaches need 128 rows that share their columns; here 8 do.  Reading 32 bytes per lane matters:
 // with 16, eight rows at a time hit the same half of the L1 banks, and reading V^T directly (four rows a lane at one 16-byte
-// position) hit a quarter of them: 103 L1 wavefronts per 16 keys, now about 60.
+// position) hit a quarter of them: 103 L1 wavefronts per 16 keys, now 80, a quarter of which transpose registers.  Those are what bounds
+// it: 70 % of their peak rate, at 54 % of the issue slots (32 heads, sequence 4096, 410 keys: 171 us).
 #pragma once
 #include "common.cuh"
 

@@ -12,8 +12,8 @@
 //
 // B200, us, spmm_cc_kernel -> this one, 50 / 90 / 98 % sparse: 512 x 512 x 512 at V = 1 53 -> 17 / 20 -> 8.4 / 8.4 -> 6.3, at V = 8
 // 70 -> 33 / 21 -> 12.5 / 8.4 -> 6.8; 1024 x 1024 x 1024 at V = 4 142 -> 41 / 38 -> 15 / 13.5 -> 8.4.  More vector-rows per warp, for
-// larger products, measured 15 % faster at 90 % sparsity and twice as slow at 98 % (4096 x 4096 x 1024, V = 4); the
-// host does not know the sparsity, so spmm_cc_kernel keeps those.
+// larger products, 4096 x 4096 x 1024 at V = 4, 80 / 90 / 95 % sparse: 248 / 161 / 124 us with two of them, 325 / 230 / 189 with four,
+// against 297 / 161 / 90, so spmm_cc_kernel keeps those (and spmm_split.cuh the denser ones).
 //
 // Entries are taken in the order of col_indices, so every sum is formed in the order, and with the roundings, of
 // spmm_cc_kernel.  Entries whose tile has gone by (columns that are not ascending) are gathered from global memory when
