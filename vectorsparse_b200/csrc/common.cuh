@@ -30,14 +30,35 @@ __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepc
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // Header of the plan scratch of the densifying SpMM, read by the kernels enqueued behind the plan kernel:
-// word 0 = the plan kernel chose the dense kernel; words 4 .. 4 + checks = one verdict per duplicate-checking CTA
+// word 0 = the plan kernel chose the dense kernel; words 1, 2 = the multiplying kernel of the plan's first (second) product met
+// sums that it hands on to the kernel behind it ("redo"); words 4 .. 4 + checks = one verdict per duplicate-checking CTA
 // of the plan kernel, set when it met the same column twice in one vector-row (the dense tile would keep one of
-// the two values, the reference adds them: such matrices go to the gather kernel).  Block-uniform result; every
-// thread of the block must call it.  The early way out ahead of the barrier is deliberate (word 0 is the same for
-// every thread): with the barrier reached on every path the multiplying kernel came out 14 % slower at 50 %
+// the two values, the reference adds them: such matrices go to the gather kernel).  A word is never written by a grid that
+// reads it: the plan kernel writes word 0 and the verdicts and clears the redo words, the multiplying kernels read the
+// former and set the latter, the kernels behind them read all.  CTAs of one multiplying grid may start while others end, and
+// with a word that the grid changes the CTAs of a pair, or the warps of a CTA, could disagree on whether there is work.
+//
+// Block-uniform result; every thread of the block must call it.  The early way out ahead of the barrier is deliberate (word 0 is
+// the same for every thread): with the barrier reached on every path the multiplying kernel came out 14 % slower at 50 %
 // sparsity, for the same instructions.
-__device__ __forceinline__ bool plan_dense_chosen(const int32_t *hdr, int checks) {
+constexpr int kPlanRedo = 1, kPlanProducts = 2;   // first redo word; products that may share a plan
+__device__ __forceinline__ void plan_publish(int32_t *hdr, bool dense) {   // one thread of the plan kernel
+    hdr[0] = dense ? 1 : 0;
+#pragma unroll
+    for (int i = 0; i < kPlanProducts; ++i) hdr[kPlanRedo + i] = 0;
+}
+__device__ __forceinline__ bool plan_dense_chosen(const int32_t *hdr, int checks) {   // in a multiplying kernel
     if (*reinterpret_cast<const volatile int32_t *>(hdr) == 0) return false;
+    int dup = 0;
+    for (int i = threadIdx.x; i < checks; i += blockDim.x) dup |= hdr[4 + i];
+    return __syncthreads_or(dup) == 0;
+}
+// In a kernel behind the multiplying one: whether that one's results stand.  One load for the header's words (the header is 16-byte
+// aligned): small calls wait for every trip to L2 here.
+__device__ __forceinline__ bool plan_dense_stands(const int32_t *hdr, int checks, int redo = kPlanRedo) {
+    static_assert(kPlanRedo == 1 && kPlanProducts == 2, "words of the header");
+    const int4 w = __ldcg(reinterpret_cast<const int4 *>(hdr));
+    if (w.x == 0 || (redo == kPlanRedo ? w.y : w.z) != 0) return false;
     int dup = 0;
     for (int i = threadIdx.x; i < checks; i += blockDim.x) dup |= hdr[4 + i];
     return __syncthreads_or(dup) == 0;

@@ -105,7 +105,7 @@ template <typename TIn, typename TOut, int V, int kChunks = 1>
 __global__ void __launch_bounds__(kCcThreads) spmm_cc_standby_kernel(const SpmmParams p, const int32_t *plan_hdr, int plan_checks) {
     pdl_launch_dependents();
     pdl_wait();
-    if (plan_dense_chosen(plan_hdr, plan_checks)) return;
+    if (plan_dense_stands(plan_hdr, plan_checks)) return;
     const int64_t per = (int64_t)p.m_vec * (p.N / (Chunk<TIn>::kElems * kChunks)), total = per * p.batch;
     for (int64_t i = (int64_t)blockIdx.x * kCcThreads + threadIdx.x; i < total; i += (int64_t)gridDim.x * kCcThreads)
         spmm_cc_item<TIn, TOut, V, kChunks>(p, (int)(i / per), i % per);

@@ -108,7 +108,7 @@ __device__ __forceinline__ bool lay_out_rows(const SpmmParams &p, int batch_a, i
     return bad;
 }
 
-// verdict: the plan header of spmm_dense.cuh: word 0 = from min_vectors nonzero vectors on the dense product is the quicker one, words
+// verdict: the plan header (common.cuh): word 0 = from min_vectors nonzero vectors on the dense product is the quicker one, words
 // 4 ..: one per CTA, nonzero if it met a column twice.
 template <int V>
 __global__ void __launch_bounds__(kPrepThreads) densify_kernel(const SpmmParams p, int batch_a, int Kp, int64_t min_vectors, uint16_t *dst, int32_t *verdict) {
@@ -116,7 +116,7 @@ __global__ void __launch_bounds__(kPrepThreads) densify_kernel(const SpmmParams 
     pdl_wait();
     __shared__ __align__(16) Shared<__half> sh;
     const bool taken = (int64_t)__ldg(p.row_offsets + p.m_vec) - __ldg(p.row_offsets) >= min_vectors;
-    if (blockIdx.x == 0 && threadIdx.x == 0) verdict[0] = taken ? 1 : 0;
+    if (blockIdx.x == 0 && threadIdx.x == 0) plan_publish(verdict, taken);
     if (!taken) return;
     const int any = __syncthreads_or(lay_out_rows<__half, V, 1>(p, batch_a, Kp, dst, sh));
     if (threadIdx.x == 0) verdict[4 + blockIdx.x] = any;

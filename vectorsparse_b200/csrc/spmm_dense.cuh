@@ -139,7 +139,7 @@ dense_plan_kernel(const int32_t *__restrict__ row_offsets, const int32_t *__rest
         const float dense_cost = stages * dense_per_stage + dense_per_entry * (float)nnz;
         const float gather_cost = (float)m_vec * gather_per_row + gather_per_entry * (float)nnz;
         const bool dense = nnz <= entry_capacity && (force_dense || dense_cost < gather_cost);
-        if (blockIdx.x == 0 && threadIdx.x == 0) *use_dense = dense ? 1 : 0;
+        if (blockIdx.x == 0 && threadIdx.x == 0) plan_publish(use_dense, dense);
         if (!dense) return;
     }
     if ((int)blockIdx.x >= groups) {
@@ -358,7 +358,7 @@ spmm_dense_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b,
                   const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_b4, int use_b4,
                   const int32_t *__restrict__ blk_offsets,
                   const uint2 *__restrict__ blk_entries, int m_tiles, int n_tiles, int k_blocks, uint32_t *status,
-                  int32_t *use_dense, int plan_checks) {
+                  const int32_t *use_dense, int plan_checks, int32_t *redo) {
     pdl_launch_dependents();   // the gather kernel behind this one may queue up
     pdl_wait();                // launched while the plan kernel may still be at work: nothing it writes is read before here
     // Not chosen (the gather kernel behind this one takes the call): the CTA still sets itself up and tears itself
@@ -731,7 +731,7 @@ spmm_dense_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b,
         // kernel enqueued behind this one, which then overwrites the output.
         if (lane == 0) tc::bulk_wait_group<0>();   // every store of this warp has reached global memory
         const float probe = (finite_probe[0] + finite_probe[1]) + (finite_probe[2] + finite_probe[3]);
-        if (__any_sync(0xffffffffu, probe != 0.0f) && lane == 0) atomicExch(use_dense, 0);
+        if (__any_sync(0xffffffffu, probe != 0.0f) && lane == 0) atomicExch(redo, 1);
     }
 
     // ---- teardown ---------------------------------------------------------------------------------------

@@ -210,7 +210,7 @@ spmm_direct_kernel(const __grid_constant__ SpmmParams p, const __grid_constant__
     if (verdict) {
         const float nnz = (float)__ldg(p.row_offsets + p.m_vec);
         mine = dense_cost + dense_per_entry * nnz < (float)p.m_vec * gather_per_row + gather_per_entry * nnz;
-        if (blockIdx.x == 0 && t == 0) *verdict = mine ? 1 : 0;
+        if (blockIdx.x == 0 && t == 0) plan_publish(verdict, mine);
     }
     const int mt = (int)(blockIdx.x % (unsigned)m_tiles);
     const unsigned rest = blockIdx.x / (unsigned)m_tiles;

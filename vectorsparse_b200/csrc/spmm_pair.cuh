@@ -159,8 +159,8 @@ template <typename TOut, int V, bool kTransposed, bool kPrepared = false>
 __global__ void __launch_bounds__(kPrepared ? kPreparedThreads : kThreads, 1)
 spmm_pair_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_a, int batch_a, int row_tiles, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ CUtensorMap map_out,
                  const __grid_constant__ CUtensorMap map_b2, int tn, const int32_t *__restrict__ blk_offsets,
-                 const uint2 *__restrict__ blk_entries, int m_tiles, int n_tiles, int k_blocks, uint32_t *status, int32_t *use_dense,
-                 int plan_checks) {
+                 const uint2 *__restrict__ blk_entries, int m_tiles, int n_tiles, int k_blocks, uint32_t *status, const int32_t *use_dense,
+                 int plan_checks, int32_t *redo) {
     pdl_launch_dependents();
     pdl_wait();
     const bool chosen = plan_dense_chosen(use_dense, plan_checks);
@@ -529,7 +529,7 @@ spmm_pair_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_a, 
         }
         if (lane == 0) tc::bulk_wait_group<0>();
         const float probe = (finite_probe[0] + finite_probe[1]) + (finite_probe[2] + finite_probe[3]);
-        if (__any_sync(0xffffffffu, probe != 0.0f) && lane == 0) atomicExch(use_dense, 0);
+        if (__any_sync(0xffffffffu, probe != 0.0f) && lane == 0) atomicExch(redo, 1);
     }
 
     // ---- teardown ---------------------------------------------------------------------------------------

@@ -66,7 +66,7 @@ struct PrepParams {
     int64_t min_vectors;        // nonzero vectors from which the split product is the quicker one
     uint16_t *a;                // bf16 [batch][M / 128, rounded up][Kp / 64][part][128 rows][64 columns]
     uint16_t *b;                // bf16 [batch][Kp / 64][Np / 64][part][64 rows][64 columns]
-    int32_t *verdict;           // word 0: taken; words 4 ..: one per CTA of this kernel, nonzero if it met what the product cannot do
+    int32_t *verdict;           // plan header (common.cuh); words 4 ..: one per CTA of this kernel, nonzero if it met what the product cannot do
 };
 
 template <int V> __global__ void __launch_bounds__(kPrepThreads) spmm_split_prepare(const SpmmParams p, const PrepParams q) {
@@ -76,7 +76,7 @@ template <int V> __global__ void __launch_bounds__(kPrepThreads) spmm_split_prep
     const int t = threadIdx.x;
     const int64_t vectors = (int64_t)__ldg(p.row_offsets + p.m_vec) - __ldg(p.row_offsets);
     const bool taken = vectors >= q.min_vectors;
-    if (blockIdx.x == 0 && t == 0) q.verdict[0] = taken ? 1 : 0;
+    if (blockIdx.x == 0 && t == 0) plan_publish(q.verdict, taken);
     if (!taken) return;
     bool bad = densify::lay_out_rows<float, V, kParts>(p, q.batch_a, q.Kp, q.a, sh);
     const int k_blocks = q.Kp / kBlockK;
@@ -112,7 +112,7 @@ template <int kTn>
 __global__ void __launch_bounds__(kThreads, 1)
 spmm_split_kernel(const SpmmParams p, int V, const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                   const __grid_constant__ CUtensorMap map_out, int batch_a, int batch_b, int m_tiles, int n_tiles, int k_blocks, int row_tiles, int slabs,
-                  uint32_t *status, int32_t *verdict, int checks) {
+                  uint32_t *status, const int32_t *verdict, int checks, int32_t *redo) {
     pdl_launch_dependents();
     pdl_wait();
     const bool chosen = plan_dense_chosen(verdict, checks);
@@ -279,7 +279,7 @@ spmm_split_kernel(const SpmmParams p, int V, const __grid_constant__ CUtensorMap
             }
         }
         if (lane == 0) tc::bulk_wait_group<0>();
-        if (__any_sync(0xffffffffu, bad) && lane == 0) atomicExch(verdict, 0);
+        if (__any_sync(0xffffffffu, bad) && lane == 0) atomicExch(redo, 1);
     }
 
     tc::tc_fence_before_sync();

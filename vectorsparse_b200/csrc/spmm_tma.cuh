@@ -150,7 +150,7 @@ spmm_tma_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map, int
                 uint32_t *status, const int32_t *plan_hdr, int plan_checks) {
     pdl_launch_dependents();   // the next call's plan kernel may queue up behind this one
     pdl_wait();   // launched behind the dense kernel without waiting for its end: wait here, before its verdict is read
-    if (plan_hdr && plan_dense_chosen(plan_hdr, plan_checks)) return;   // the dense kernel has taken this call (decided on the device)
+    if (plan_hdr && plan_dense_stands(plan_hdr, plan_checks)) return;   // the dense kernel has taken this call (decided on the device)
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = tc::smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;

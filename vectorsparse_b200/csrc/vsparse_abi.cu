@@ -648,7 +648,7 @@ int launch_spmm_gather(const SpmmParams &p, cudaStream_t s, DeviceInfo *d, const
 // proportional to the nonzeros.  The number of nonzeros is only known on the device (the reference signature
 // does not pass it), so the choice is made there: the plan kernel compares the two costs (see there) and
 // leaves a flag that one of the two kernels, both enqueued, finds set against it and returns at once.  The
-// densifying kernel clears the flag again if it produced a non-finite sum, so that the gather kernel redoes the
+// densifying kernel sets the plan's redo word if it produced a non-finite sum, so that the gather kernel redoes the
 // call with the reference's semantics for Inf / NaN in rows of B that no nonzero names.
 enum class SpmmMode { kAuto, kDense, kGather, kDirect };
 SpmmMode spmm_mode() {   // read at every call, so that a test can switch kernels inside one process
@@ -754,7 +754,7 @@ template <typename K> int pair_capacity(K kernel, int threads, int (&resident)[k
 template <typename TOut, int V, bool kTransposed>
 bool launch_spmm_pair(const SpmmParams &q, cudaStream_t s, DeviceInfo *d, const CUtensorMap &map, const CUtensorMap &map_out,
                       const CUtensorMap &map_b2, const int32_t *blk_offsets, const uint2 *blk_entries, int m_tiles, int k_blocks,
-                      int32_t *flag, int checks, int *rc_out) {
+                      int32_t *flag, int checks, int32_t *redo, int *rc_out) {
     static int resident[kMaxDevices];
     auto kernel = pairspmm::spmm_pair_kernel<TOut, V, kTransposed>;
     const int capacity = pair_capacity(kernel, pairspmm::kThreads, resident, d);
@@ -765,7 +765,7 @@ bool launch_spmm_pair(const SpmmParams &q, cudaStream_t s, DeviceInfo *d, const 
     const unsigned pairs = (unsigned)(items < capacity ? items : capacity);
     TimedLaunch timed(s);
     *rc_out = (int)launch_pairs(kernel, pairs, pairspmm::kThreads, (size_t)pairspmm::kSmemBytes, s, true, q, map, 1, 0, map, map_out, map_b2, tn,
-                                blk_offsets, blk_entries, m_tiles, n_tiles, k_blocks, d->status, flag, checks);
+                                blk_offsets, blk_entries, m_tiles, n_tiles, k_blocks, d->status, flag, checks, redo);
     return true;
 }
 
@@ -906,7 +906,7 @@ template <typename TOut, int V, bool kCores> bool launch_spmm_laid_out(const Spm
         q.m_vec = (int)M;
         rc = (int)launch_pairs(kernel, (unsigned)std::min<int64_t>(items, capacity), pairspmm::kPreparedThreads, (size_t)pairspmm::kSmemBytes, s, true, q, map_a,
                                batch_a, row_tiles, map_b, map_out, map_b2, tn, (const int32_t *)nullptr, (const uint2 *)nullptr, m_tiles, n_tiles,
-                               k_blocks, d->status, verdict, checks);
+                               k_blocks, d->status, verdict, checks, verdict + kPlanRedo);
     }
     if (rc == VS_OK) rc = launch_spmm_other<TOut, V, kCores>(p, s, d, verdict, checks);
     *rc_out = rc;
@@ -984,11 +984,11 @@ template <typename TOut, int V, bool kCores> int launch_spmm_tc(const SpmmParams
     if (rc == VS_OK) {
         int rc_pair = VS_OK;
         if (use_b4 && spmm_pair_takes(p.N, (int64_t)p.batch * m_tiles, d) &&
-            launch_spmm_pair<TOut, V, false>(p, s, d, map, map_out, map_b4, blk_offsets, blk_entries, m_tiles, k_blocks, flag, checks, &rc_pair))
+            launch_spmm_pair<TOut, V, false>(p, s, d, map, map_out, map_b4, blk_offsets, blk_entries, m_tiles, k_blocks, flag, checks, flag + kPlanRedo, &rc_pair))
             rc = rc_pair;
         else
             rc = (int)launch_overlapped(kernel, grid, densespmm::kThreads, densespmm::kSmemBytes, s, p, map, map_out, map_b4, use_b4,
-                                        blk_offsets, blk_entries, m_tiles, n_tiles, k_blocks, d->status, flag, checks);
+                                        blk_offsets, blk_entries, m_tiles, n_tiles, k_blocks, d->status, flag, checks, flag + kPlanRedo);
     }
     if (rc == VS_OK) rc = launch_spmm_other<TOut, V, kCores>(p, s, d, flag, checks);
     return rc;
@@ -1078,7 +1078,7 @@ template <int V> int launch_spmm_split(const SpmmParams &p, int64_t vectors, cud
     if (rc != VS_OK) return rc;
     const int64_t items = row_items * n_tiles;
     rc = (int)launch_pairs(tn == 256 ? splitspmm::spmm_split_kernel<256> : splitspmm::spmm_split_kernel<128>, (unsigned)std::min<int64_t>(items, resident[dev]), splitspmm::kThreads, (size_t)splitspmm::kSmemBytes, s, true,
-                           p, V, map_a, map_b, map_out, q.batch_a, q.batch_b, m_tiles, n_tiles, k_blocks, row_tiles, slabs, d->status, q.verdict, checks);
+                           p, V, map_a, map_b, map_out, q.batch_a, q.batch_b, m_tiles, n_tiles, k_blocks, row_tiles, slabs, d->status, q.verdict, checks, q.verdict + kPlanRedo);
     if (rc != VS_OK) return rc;
     const int chunks = spmm_cc_chunks(4 * V, 4, p.N);
     if constexpr (V <= 4) {
@@ -1525,7 +1525,7 @@ namespace {
 // CUDA-core kernel.  With `plan_hdr` it is enqueued behind the dense kernel and returns at once unless that kernel
 // left the call to it.
 template <typename TOut, int V>
-int launch_spmm_t_cc(const spmmt::Params &p, cudaStream_t s, DeviceInfo *d, const int32_t *plan_hdr, int plan_checks) {
+int launch_spmm_t_cc(const spmmt::Params &p, cudaStream_t s, DeviceInfo *d, const int32_t *plan_hdr, int plan_checks, int redo = kPlanRedo) {
     const int row_groups = (p.n + spmmt::kWarps - 1) / spmmt::kWarps;
     const int chunks = (p.N + spmmt::kChunk - 1) / spmmt::kChunk;
     const int64_t items = (int64_t)p.batch * chunks * row_groups;
@@ -1534,8 +1534,8 @@ int launch_spmm_t_cc(const spmmt::Params &p, cudaStream_t s, DeviceInfo *d, cons
                                                       // took 14 us to do so, a quarter of them a quarter of that)
     const unsigned grid = (unsigned)(items < cap ? items : cap);
     auto kernel = spmmt::spmm_t_kernel<TOut, V>;
-    if (plan_hdr) return (int)launch_overlapped(kernel, grid, spmmt::kThreads, 0, s, p, items, row_groups, chunks, plan_hdr, plan_checks);
-    kernel<<<grid, spmmt::kThreads, 0, s>>>(p, items, row_groups, chunks, plan_hdr, plan_checks);
+    if (plan_hdr) return (int)launch_overlapped(kernel, grid, spmmt::kThreads, 0, s, p, items, row_groups, chunks, plan_hdr, plan_checks, redo);
+    kernel<<<grid, spmmt::kThreads, 0, s>>>(p, items, row_groups, chunks, plan_hdr, plan_checks, redo);
     return (int)cudaGetLastError();
 }
 
@@ -1553,8 +1553,7 @@ SpmmTMode spmm_t_mode() {   // read at every call, so that a test can switch ker
 // plan kernel's units (SM-cycles per 128 columns): the CUDA-core kernel ~5 per value (0.92 ms for 256 products of
 // 2048 x 512, 90 % sparse, V = 8), the dense kernel ~1100 per stage plus ~1.5 per vector of fill work (0.170 ms on
 // the same problem against 0.137 for the forward product with the same tiles).
-// `count` products (at most kMaxTogether) with the same structure, sizes and strides: one plan serves them.
-constexpr int kMaxTogether = 2;
+// `count` products (at most kPlanProducts) with the same structure, sizes and strides: one plan serves them.
 template <typename TOut, int V> int launch_spmm_t(const spmmt::Params *list, int count, int m_vec, cudaStream_t s) {
     const spmmt::Params &p = list[0];
     DeviceInfo *d;
@@ -1592,7 +1591,7 @@ template <typename TOut, int V> int launch_spmm_t(const spmmt::Params *list, int
     if (!dense_ok) return by_cores();
 
     constexpr bool kOutF32 = sizeof(TOut) == 4;
-    CUtensorMap map[kMaxTogether], map_out[kMaxTogether], map_b4[kMaxTogether];
+    CUtensorMap map[kPlanProducts], map_out[kPlanProducts], map_b4[kPlanProducts];
     int use_b4 = q.N % 64 == 0 ? 1 : 0;
     for (int i = 0; i < count; ++i) {
         if (make_tile_map(&map[i], list[i].rhs, false, (uint64_t)q.K, (uint64_t)q.N, (uint64_t)q.batch, (uint64_t)q.stride_rhs, 64, 64) != VS_OK ||
@@ -1625,12 +1624,12 @@ template <typename TOut, int V> int launch_spmm_t(const spmmt::Params *list, int
         q.values = list[i].values; q.rhs = list[i].rhs; q.out = list[i].out;
         int rc_pair = VS_OK;
         if (use_b4 && spmm_pair_takes(q.N, (int64_t)q.batch * m_tiles, d) &&
-            launch_spmm_pair<TOut, V, true>(q, s, d, map[i], map_out[i], map_b4[i], blk_offsets, blk_entries, m_tiles, k_blocks, flag, checks, &rc_pair))
+            launch_spmm_pair<TOut, V, true>(q, s, d, map[i], map_out[i], map_b4[i], blk_offsets, blk_entries, m_tiles, k_blocks, flag, checks, flag + kPlanRedo + i, &rc_pair))
             rc = rc_pair;
         else
             rc = (int)launch_overlapped(kernel, grid, densespmm::kThreads, densespmm::kSmemBytes, s, q, map[i], map_out[i], map_b4[i], use_b4,
-                                        blk_offsets, blk_entries, m_tiles, n_tiles, k_blocks, d->status, flag, checks);
-        if (rc == VS_OK) rc = launch_spmm_t_cc<TOut, V>(list[i], s, d, flag, checks);
+                                        blk_offsets, blk_entries, m_tiles, n_tiles, k_blocks, d->status, flag, checks, flag + kPlanRedo + i);
+        if (rc == VS_OK) rc = launch_spmm_t_cc<TOut, V>(list[i], s, d, flag, checks, kPlanRedo + i);
     }
     return rc;
 }
