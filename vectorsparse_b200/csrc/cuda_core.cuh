@@ -18,18 +18,23 @@ constexpr int kCcThreads = 128;
 // per 16 bytes) and walks the row's nonzero vectors four at a time so that four independent gathers of B are in
 // flight.  With two or four chunks per thread the warp-uniform loads of an entry (column index, value vector) feed
 // that many times the FMAs; it needs the dense width to be a multiple of 32 kChunks chunks.
-template <typename TIn, typename TOut, int V, int kChunks>
+//
+// kSlabs: wide fp32 products go slab by slab: the warps of an SM take the same columns, so that a row of B serves several of them from L1.  A kernel of
+// its own: the choice inside this one cost the narrow products up to 8 % (fp16 operands, V = 1, 3 x (452 x 4237 x 72), 94.5 %: 51.9 -> 55.4 us).
+constexpr int kSlabColumns = 4096;
+template <typename TIn, typename TOut, int V, int kChunks, bool kSlabs>
 __device__ __forceinline__ void spmm_cc_item(const SpmmParams &p, int b, int64_t item) {
     constexpr int E = Chunk<TIn>::kElems;
     constexpr int U = kChunks == 1 ? 4 : (kChunks == 2 ? 2 : 1);
     const int chunks = p.N / (E * kChunks);            // items per vector-row
-    int order = (int)(item / chunks), piece = (int)(item - (int64_t)order * chunks);
-    // Wide products slab by slab: the warps of an SM take the same columns, so that a row of B serves several of them from L1 (fp32,
-    // 4096 x 4096 x 8192: 1377 -> 1206 us at V = 1, 95 % sparse, 1010 -> 986 at V = 4, 90 %; with 1024 columns nothing, or 3 % lost).
-    if (chunks % 32 == 0 && chunks >= 256) {
+    int order, piece;
+    if constexpr (kSlabs) {   // chunks is a multiple of 32
         const int64_t w = item / 32;
         order = (int)(w % p.m_vec);
         piece = (int)(w / p.m_vec) * 32 + (int)(item % 32);
+    } else {
+        order = (int)(item / chunks);
+        piece = (int)(item - (int64_t)order * chunks);
     }
     // kChunks > 1: warp-sized groups of items take chunks 32 kChunks g + lane, + 32 + lane, ...
     const int chunk = kChunks == 1 ? piece : (piece / 32) * (32 * kChunks) + (piece % 32);
@@ -92,23 +97,23 @@ __device__ __forceinline__ void spmm_cc_item(const SpmmParams &p, int b, int64_t
         for (int v = 0; v < V; ++v) store_chunk(out + ((int64_t)row * V + v) * p.N + q * 32 * E, acc[q][v]);
 }
 
-template <typename TIn, typename TOut, int V, int kChunks>
+template <typename TIn, typename TOut, int V, int kChunks, bool kSlabs = false>
 __global__ void __launch_bounds__(kCcThreads) spmm_cc_kernel(const SpmmParams p) {
     const int64_t item = (int64_t)blockIdx.x * kCcThreads + threadIdx.x;
-    if (item < (int64_t)p.m_vec * (p.N / (Chunk<TIn>::kElems * kChunks))) spmm_cc_item<TIn, TOut, V, kChunks>(p, blockIdx.y, item);
+    if (item < (int64_t)p.m_vec * (p.N / (Chunk<TIn>::kElems * kChunks))) spmm_cc_item<TIn, TOut, V, kChunks, kSlabs>(p, blockIdx.y, item);
 }
 
 // The same work enqueued behind a densifying kernel that usually has taken the call: returns at once unless the plan
 // header says otherwise, and walks its items in strides, because a grid of one thread per item takes longer to start and
 // return than the rest of a small call.
-template <typename TIn, typename TOut, int V, int kChunks = 1>
+template <typename TIn, typename TOut, int V, int kChunks = 1, bool kSlabs = false>
 __global__ void __launch_bounds__(kCcThreads) spmm_cc_standby_kernel(const SpmmParams p, const int32_t *plan_hdr, int plan_checks) {
     pdl_launch_dependents();
     pdl_wait();
     if (plan_dense_stands(plan_hdr, plan_checks)) return;
     const int64_t per = (int64_t)p.m_vec * (p.N / (Chunk<TIn>::kElems * kChunks)), total = per * p.batch;
     for (int64_t i = (int64_t)blockIdx.x * kCcThreads + threadIdx.x; i < total; i += (int64_t)gridDim.x * kCcThreads)
-        spmm_cc_item<TIn, TOut, V, kChunks>(p, (int)(i / per), i % per);
+        spmm_cc_item<TIn, TOut, V, kChunks, kSlabs>(p, (int)(i / per), i % per);
 }
 
 // ---- SDDMM --------------------------------------------------------------------------------------------------

@@ -542,6 +542,25 @@ int spmm_cc_tile(int V, const SpmmParams &p, cudaStream_t s, bool *taken) {
     return VS_OK;
 }
 
+// Slab by slab (cuda_core.cuh) where the pieces of a row, of `want` chunks each, come in warps, and there are enough of those that the ones at work
+// together share columns; half as many will do where B does not stay in L2.  us, row by row / slab by slab, 90 % sparse, thousands of warps: 4096 x 4096 x 8192
+// V = 1 (64) 2628 / 2377, V = 2 (32) 1379 / 1248, V = 8 (16) 1033 / 924; 4096 x 1024 x 8192 V = 1 (64) 641 / 528, V = 4 (16) 263 / 255; 2048 x 2048 x 4096 V = 1 (16)
+// 322 / 306, V = 2 (8) 169 / 180, V = 8 (4) 135 / 142; 1024 x 1024 x 8192 V = 1 (16) 167 / 157, V = 2 (8) 91 / 97; 2048 x 2048 x 8192, 67 MB of B, V = 8 (8) 297 / 268;
+// 512 x 4096 x 8192 V = 2 (4) 186 / 191.  With 1024 columns nothing, or 3 % lost.
+bool spmm_cc_slabs(const SpmmParams &p, int want) {
+    if (p.N < kSlabColumns || p.N % (128 * want) != 0) return false;
+    const int64_t warps = (int64_t)p.m_vec * (p.N / (128 * want));
+    return warps >= 16384 || (warps >= 8192 && (int64_t)p.K * p.N * 4 >= 64 << 20);
+}
+template <typename TIn, typename TOut, int V, int kChunks> void launch_spmm_cc_as(const SpmmParams &p, dim3 grid, cudaStream_t s) {
+    if constexpr (sizeof(TIn) == 4) {
+        if (spmm_cc_slabs(p, kChunks)) {
+            spmm_cc_kernel<TIn, TOut, V, kChunks, true><<<grid, kCcThreads, 0, s>>>(p);
+            return;
+        }
+    }
+    spmm_cc_kernel<TIn, TOut, V, kChunks><<<grid, kCcThreads, 0, s>>>(p);
+}
 template <typename TIn, typename TOut, int V> int launch_spmm_cc(const SpmmParams &p, cudaStream_t s) {
     constexpr int E = Chunk<TIn>::kElems;
     const int want = spmm_cc_chunks(V * E, E, p.N);
@@ -551,17 +570,17 @@ template <typename TIn, typename TOut, int V> int launch_spmm_cc(const SpmmParam
     dim3 grid((unsigned)blocks, (unsigned)p.batch, 1);
     if constexpr (V * E <= 16) {
         if (want == 4) {
-            spmm_cc_kernel<TIn, TOut, V, 4><<<grid, kCcThreads, 0, s>>>(p);
+            launch_spmm_cc_as<TIn, TOut, V, 4>(p, grid, s);
             return (int)cudaGetLastError();
         }
     }
     if constexpr (V * E <= 32) {
         if (want == 2) {
-            spmm_cc_kernel<TIn, TOut, V, 2><<<grid, kCcThreads, 0, s>>>(p);
+            launch_spmm_cc_as<TIn, TOut, V, 2>(p, grid, s);
             return (int)cudaGetLastError();
         }
     }
-    spmm_cc_kernel<TIn, TOut, V, 1><<<grid, kCcThreads, 0, s>>>(p);
+    launch_spmm_cc_as<TIn, TOut, V, 1>(p, grid, s);
     return (int)cudaGetLastError();
 }
 
@@ -1022,7 +1041,8 @@ int spmm_cores_by_v(int V, const SpmmParams &p, cudaStream_t s) {
 // ---- fp32 SpMM from bf16 parts ------------------------------------------------------------------------------
 template <int V, int kChunks> int launch_spmm_f32_standby(const SpmmParams &p, cudaStream_t s, DeviceInfo *d, const int32_t *verdict, int checks) {
     const int64_t blocks = ((int64_t)p.m_vec * (p.N / (4 * kChunks)) * p.batch + kCcThreads - 1) / kCcThreads, cap = (int64_t)d->sm_count * 8;
-    return (int)launch_overlapped(spmm_cc_standby_kernel<float, float, V, kChunks>, (unsigned)(blocks < cap ? blocks : cap), kCcThreads, 0, s, p, verdict, checks);
+    auto kernel = spmm_cc_slabs(p, kChunks) ? spmm_cc_standby_kernel<float, float, V, kChunks, true> : spmm_cc_standby_kernel<float, float, V, kChunks>;
+    return (int)launch_overlapped(kernel, (unsigned)(blocks < cap ? blocks : cap), kCcThreads, 0, s, p, verdict, checks);
 }
 // Leaves *taken false where the call is not one for it.
 template <int V> int launch_spmm_split(const SpmmParams &p, int64_t vectors, cudaStream_t s, bool forced, DeviceInfo *d, bool *taken) {
