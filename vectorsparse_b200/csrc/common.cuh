@@ -32,8 +32,8 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // Header of the plan scratch of the densifying SpMM, read by the kernels enqueued behind the plan kernel:
 // word 0 = the plan kernel chose the dense kernel; words 1, 2 = the multiplying kernel of the plan's first (second) product met
 // sums that it hands on to the kernel behind it ("redo"); words 4 .. 4 + checks = one verdict per duplicate-checking CTA
-// of the plan kernel, set when it met the same column twice in one vector-row (the dense tile would keep one of
-// the two values, the reference adds them: such matrices go to the gather kernel).  A word is never written by a grid that
+// of the plan kernel, bit 0 set when it met the same column twice in one vector-row (the dense tile would keep one of
+// the two values, the reference adds them: such matrices go to the gather kernel); bit 1 see spmm_split.cuh.  A word is never written by a grid that
 // reads it: the plan kernel writes word 0 and the verdicts and clears the redo words, the multiplying kernels read the
 // former and set the latter, the kernels behind them read all.  CTAs of one multiplying grid may start while others end, and
 // with a word that the grid changes the CTAs of a pair, or the warps of a CTA, could disagree on whether there is work.
@@ -42,6 +42,7 @@ __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;"
 // the same for every thread): with the barrier reached on every path the multiplying kernel came out 14 % slower at 50 %
 // sparsity, for the same instructions.
 constexpr int kPlanRedo = 1, kPlanProducts = 2;   // first redo word; products that may share a plan
+constexpr int kPlanLeft = 1, kPlanFew = 2;        // bits of the verdicts: the call is left to the kernel behind; some of its rows are
 __device__ __forceinline__ void plan_publish(int32_t *hdr, bool dense) {   // one thread of the plan kernel
     hdr[0] = dense ? 1 : 0;
 #pragma unroll
@@ -62,6 +63,21 @@ __device__ __forceinline__ bool plan_dense_stands(const int32_t *hdr, int checks
     int dup = 0;
     for (int i = threadIdx.x; i < checks; i += blockDim.x) dup |= hdr[4 + i];
     return __syncthreads_or(dup) == 0;
+}
+// The two for the split product, whose verdicts have both bits.
+__device__ __forceinline__ bool plan_split_chosen(const int32_t *hdr, int checks) {
+    if (*reinterpret_cast<const volatile int32_t *>(hdr) == 0) return false;
+    int dup = 0;
+    for (int i = threadIdx.x; i < checks; i += blockDim.x) dup |= hdr[4 + i] & kPlanLeft;
+    return __syncthreads_or(dup) == 0;
+}
+__device__ __forceinline__ bool plan_split_stands(const int32_t *hdr, int checks, bool &few) {
+    const int4 w = __ldcg(reinterpret_cast<const int4 *>(hdr));
+    if (w.x == 0 || w.y != 0) return false;
+    int v = 0;
+    for (int i = threadIdx.x; i < checks; i += blockDim.x) v |= hdr[4 + i];
+    few = __syncthreads_or(v & kPlanFew) != 0;
+    return __syncthreads_or(v & kPlanLeft) == 0;
 }
 
 struct SddmmParams {

@@ -23,7 +23,7 @@ constexpr int kCcThreads = 128;
 // its own: the choice inside this one cost the narrow products up to 8 % (fp16 operands, V = 1, 3 x (452 x 4237 x 72), 94.5 %: 51.9 -> 55.4 us).
 constexpr int kSlabColumns = 4096;
 template <typename TIn, typename TOut, int V, int kChunks, bool kSlabs>
-__device__ __forceinline__ void spmm_cc_item(const SpmmParams &p, int b, int64_t item) {
+__device__ __forceinline__ void spmm_cc_item(const SpmmParams &p, int b, int64_t item, int few = 0) {   // few > 0: only rows of 1 .. few - 1 entries
     constexpr int E = Chunk<TIn>::kElems;
     constexpr int U = kChunks == 1 ? 4 : (kChunks == 2 ? 2 : 1);
     const int chunks = p.N / (E * kChunks);            // items per vector-row
@@ -54,6 +54,7 @@ __device__ __forceinline__ void spmm_cc_item(const SpmmParams &p, int b, int64_t
 
     int j = __ldg(p.row_offsets + row);
     const int end = __ldg(p.row_offsets + row + 1);
+    if (few > 0 && (end <= j || end - j >= few)) return;
 
     for (; j + U <= end; j += U) {
         int col[U];
@@ -105,15 +106,18 @@ __global__ void __launch_bounds__(kCcThreads) spmm_cc_kernel(const SpmmParams p)
 
 // The same work enqueued behind a densifying kernel that usually has taken the call: returns at once unless the plan
 // header says otherwise, and walks its items in strides, because a grid of one thread per item takes longer to start and
-// return than the rest of a small call.
+// return than the rest of a small call.  fp32: rows of fewer than `few` entries it computes even then.
 template <typename TIn, typename TOut, int V, int kChunks = 1, bool kSlabs = false>
-__global__ void __launch_bounds__(kCcThreads) spmm_cc_standby_kernel(const SpmmParams p, const int32_t *plan_hdr, int plan_checks) {
+__global__ void __launch_bounds__(kCcThreads) spmm_cc_standby_kernel(const SpmmParams p, const int32_t *plan_hdr, int plan_checks, int few) {
     pdl_launch_dependents();
     pdl_wait();
-    if (plan_dense_stands(plan_hdr, plan_checks)) return;
+    bool stands, some = false;
+    if constexpr (sizeof(TIn) == 4) stands = plan_split_stands(plan_hdr, plan_checks, some);
+    else stands = plan_dense_stands(plan_hdr, plan_checks);
+    if (stands && !some) return;
     const int64_t per = (int64_t)p.m_vec * (p.N / (Chunk<TIn>::kElems * kChunks)), total = per * p.batch;
     for (int64_t i = (int64_t)blockIdx.x * kCcThreads + threadIdx.x; i < total; i += (int64_t)gridDim.x * kCcThreads)
-        spmm_cc_item<TIn, TOut, V, kChunks, kSlabs>(p, (int)(i / per), i % per);
+        spmm_cc_item<TIn, TOut, V, kChunks, kSlabs>(p, (int)(i / per), i % per, sizeof(TIn) == 4 && stands ? few : 0);
 }
 
 // ---- SDDMM --------------------------------------------------------------------------------------------------

@@ -45,9 +45,10 @@ template <typename T> struct Shared {
 
 // This CTA's share of the vector-rows, several short ones or a piece of a long one at a time; the entries of such a group lie side by
 // side, so the threads walk them together, four loads in flight each, and look up their rows.  Returns whether the thread met a column named
-// twice in a vector-row or a value that cannot be split; columns outside the matrix are left out.
+// twice in a vector-row or a value that cannot be split; columns outside the matrix are left out.  `found` is set where the thread
+// met a vector-row of 1 .. few - 1 entries.
 template <typename T, int V, int kParts>
-__device__ __forceinline__ bool lay_out_rows(const SpmmParams &p, int batch_a, int Kp, uint16_t *dst, Shared<T> &sh) {
+__device__ __forceinline__ bool lay_out_rows(const SpmmParams &p, int batch_a, int Kp, uint16_t *dst, Shared<T> &sh, int few, bool &found) {
     constexpr int kCols = kPrepValues / V, kChunk = 16 / (int)sizeof(T);
     const int t = threadIdx.x, pieces = (Kp + kCols - 1) / kCols;
     const int group = max(min(kCols / Kp, (int)min((int64_t)kMaxGroup, (int64_t)batch_a * p.m_vec / gridDim.x)), 1), groups = (p.m_vec + group - 1) / group;
@@ -62,6 +63,7 @@ __device__ __forceinline__ bool lay_out_rows(const SpmmParams &p, int batch_a, i
         for (int i = t; i < count * cols / 32; i += kPrepThreads) sh.named[i] = 0u;
         if (t <= count) sh.offsets[t] = __ldg(p.row_offsets + row0 + t);
         __syncthreads();
+        if (t < count && sh.offsets[t + 1] > sh.offsets[t] && sh.offsets[t + 1] - sh.offsets[t] < few) found = true;
         const T *values = static_cast<const T *>(p.values) + (int64_t)b * p.stride_values;
         const int end = sh.offsets[count];
         constexpr int U = 4;
@@ -118,7 +120,8 @@ __global__ void __launch_bounds__(kPrepThreads) densify_kernel(const SpmmParams 
     const bool taken = (int64_t)__ldg(p.row_offsets + p.m_vec) - __ldg(p.row_offsets) >= min_vectors;
     if (blockIdx.x == 0 && threadIdx.x == 0) plan_publish(verdict, taken);
     if (!taken) return;
-    const int any = __syncthreads_or(lay_out_rows<__half, V, 1>(p, batch_a, Kp, dst, sh));
+    bool found = false;
+    const int any = __syncthreads_or(lay_out_rows<__half, V, 1>(p, batch_a, Kp, dst, sh, 0, found));
     if (threadIdx.x == 0) verdict[4 + blockIdx.x] = any;
 }
 

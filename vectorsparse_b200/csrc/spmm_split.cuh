@@ -1,20 +1,27 @@
 // fp32 SpMM on the tensor cores: the `cudaSpmm` float entry point (a stub in the reference, src/cuda_spmm.cu:328-338) for large
 // products that are not too sparse.
 //
-// An fp32 number is the exact sum of three bf16 numbers (8 + 8 + 8 significant bits): x = x1 + x2 + x3.  Of the nine products of
+// An fp32 number is the exact sum of three bf16 numbers (8 + 8 + 8 significant bits): x = x1 + x2 + x3 (the decomposition of Henry, Tang and
+// Heinecke, "Leveraging the bfloat16 Artificial Intelligence Datatype For Higher-Precision Computations", 2019).  Of the nine products of
 // two such sums the six largest are kept,
-//     a b = a1 b1 + (a1 b2 + a2 b1) + (a1 b3 + a2 b2 + a3 b1) + dropped,   |dropped| < 2^-25 |a b|,
-// each exact in the tensor core's fp32.  Its sums are where precision could go: it truncates at every addition.  So the small
-// products of a block of 64 columns are added first and the large ones last, and the block's sum is then taken out of tensor memory
-// and added, rounded to nearest, to sums in registers: an output sees four truncations per 64 columns, of a partial sum that is
-// small against the result, and no more roundings than the CUDA-core kernel's chain of one per nonzero.
+//     a b = a1 b1 + (a1 b2 + a2 b1) + (a1 b3 + a2 b2 + a3 b1) + dropped,
+// each exact in the tensor core's fp32.  |x2| <= 2^-8 |x| and |x3| <= 2^-17 |x|, so |dropped| = |a2 b3 + a3 b2 + a3 b3| is at most a little above
+// 2^-24 |a b|, half an ulp of the product.  The sums lose as much: the tensor core truncates at every addition.  So the small products of a block
+// of 64 columns are added first and the large ones last, and the block's sum is then taken out of tensor memory and added, rounded to nearest, to sums in
+// registers: an output sees four truncations per 64 columns, each of that block's partial sum.
+//
+// Against the CUDA-core kernel's chain of one rounding per entry that is the nearer one where many entries share a block and the farther one where few
+// do.  Error of a row of L entries against 64 bits (2-norm over 256 columns, operands U(-1,1), CUDA cores / this one, times 1e-8): K = 64: L = 4 4.0 / 5.2, 8 5.4 / 5.4,
+// 24 8.9 / 5.9; K = 512: L = 8 5.4 / 6.7, 16 7.4 / 7.3, 64 14 / 7.9, 512 41 / 9.1; K = 4096: L = 16 7.4 / 8.6, 32 10.4 / 10.7, 48 12.5 / 11.9, 512 41 / 16.
+// All operands positive, or all near 1, it takes up to 24 resp. 48 entries to draw level.  So rows of fewer than few_entries(K) entries are computed
+// anew by the CUDA-core kernel behind the product, and matrices whose rows are that short on average do not come here.
 //
 // spmm_split_prepare writes A, zeros included, and B as three bf16 matrices each (scratch of 6 bytes per element), in the order in which
 // the tiles are read: a tile of a row-major matrix is 128-byte pieces kilobytes apart, and waiting for those took longer than multiplying
 // (4096 x 4096 x 256: 114 us of the product's 70).  The product is
 // a dense one in pairs of CTAs (tcgen05 cta_group::2) with the tiles and the protocol of spmm_pair.cuh: per stage of 64 columns six
 // times four 256 x 256 x 16 MMAs.  What it cannot do as well as the CUDA-core kernel, that kernel does behind it, from a
-// verdict: matrices too sparse, a column named twice in a vector-row, and numbers whose parts or products would leave the range of
+// verdict: rows with few entries, and all of matrices too sparse, a column named twice in a vector-row, and numbers whose parts or products would leave the range of
 // normal fp32: non-finite results, inputs below 2^-100, results below 2^-96.
 //
 // Bound by the tensor pipe: 6 x the dense flops.
@@ -42,6 +49,8 @@ constexpr int kMaxStages = 3, kOperandBytes = 3 * Stage<128>::kBytes;
 static_assert(2 * Stage<256>::kBytes <= kOperandBytes, "operand slots");
 constexpr int kEpiWarps = 8, kLoadWarp = 8, kMmaWarp = 9, kThreads = 320;
 constexpr int kStoreCols = 8, kBoxBytes = 32 * kStoreCols * 4;   // 1 KiB of staging per epilogue warp: once per item, and the operands need the room
+// One entry per block of 64 columns and some, at least 24: 1.2 to 2 times those where the two draw level.
+inline int few_entries(int K) { return K / kBlockK + 16 > 24 ? K / kBlockK + 16 : 24; }
 constexpr uint32_t kTinyResult = (127u - 96u) << 23;
 
 struct Smem {
@@ -66,7 +75,9 @@ struct PrepParams {
     int64_t min_vectors;        // nonzero vectors from which the split product is the quicker one
     uint16_t *a;                // bf16 [batch][M / 128, rounded up][Kp / 64][part][128 rows][64 columns]
     uint16_t *b;                // bf16 [batch][Kp / 64][Np / 64][part][64 rows][64 columns]
-    int32_t *verdict;           // plan header (common.cuh); words 4 ..: one per CTA of this kernel, nonzero if it met what the product cannot do
+    int few;                    // vector-rows of 1 .. few - 1 entries are the CUDA-core kernel's; 0: none are
+    int32_t *verdict;           // plan header (common.cuh); words 4 ..: one per CTA of this kernel, kPlanLeft if it met what the product cannot do,
+                                // kPlanFew if it met a vector-row with few entries
 };
 
 template <int V> __global__ void __launch_bounds__(kPrepThreads) spmm_split_prepare(const SpmmParams p, const PrepParams q) {
@@ -78,7 +89,8 @@ template <int V> __global__ void __launch_bounds__(kPrepThreads) spmm_split_prep
     const bool taken = vectors >= q.min_vectors;
     if (blockIdx.x == 0 && t == 0) plan_publish(q.verdict, taken);
     if (!taken) return;
-    bool bad = densify::lay_out_rows<float, V, kParts>(p, q.batch_a, q.Kp, q.a, sh);
+    bool found = false;
+    bool bad = densify::lay_out_rows<float, V, kParts>(p, q.batch_a, q.Kp, q.a, sh, q.few, found);
     const int k_blocks = q.Kp / kBlockK;
     const int chunks = q.Np / 8;
     const int64_t total = (int64_t)q.batch_b * q.Kp * chunks;
@@ -99,8 +111,8 @@ template <int V> __global__ void __launch_bounds__(kPrepThreads) spmm_split_prep
             *reinterpret_cast<uint4 *>(q.b + tile * (kBlockK * 64) + (k % kBlockK) * 64 + c % 64) = part[s];
         }
     }
-    const int any = __syncthreads_or(bad);
-    if (t == 0) q.verdict[4 + blockIdx.x] = any;
+    const int any = __syncthreads_or(bad), some = __syncthreads_or(found);
+    if (t == 0) q.verdict[4 + blockIdx.x] = (any ? kPlanLeft : 0) | (some ? kPlanFew : 0);
 }
 
 // ---- product ----------------------------------------------------------------------------------------------
@@ -115,7 +127,7 @@ spmm_split_kernel(const SpmmParams p, int V, const __grid_constant__ CUtensorMap
                   uint32_t *status, const int32_t *verdict, int checks, int32_t *redo) {
     pdl_launch_dependents();
     pdl_wait();
-    const bool chosen = plan_dense_chosen(verdict, checks);
+    const bool chosen = plan_split_chosen(verdict, checks);
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = tc::smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;   // the same offset in both CTAs

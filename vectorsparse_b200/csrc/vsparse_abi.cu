@@ -607,10 +607,10 @@ template <typename TOut, int V> int launch_spmm_cc_standby(const SpmmParams &p, 
     const int64_t cap = (int64_t)d->sm_count * 8;
     const unsigned grid = (unsigned)(blocks < cap ? blocks : cap);
     if (!overlapped) {
-        spmm_cc_standby_kernel<__half, TOut, V><<<grid, kCcThreads, 0, s>>>(p, plan_hdr, plan_checks);
+        spmm_cc_standby_kernel<__half, TOut, V><<<grid, kCcThreads, 0, s>>>(p, plan_hdr, plan_checks, 0);
         return (int)cudaGetLastError();
     }
-    return (int)launch_overlapped(spmm_cc_standby_kernel<__half, TOut, V>, grid, kCcThreads, 0, s, p, plan_hdr, plan_checks);
+    return (int)launch_overlapped(spmm_cc_standby_kernel<__half, TOut, V>, grid, kCcThreads, 0, s, p, plan_hdr, plan_checks, 0);
 }
 
 // Software (cp.async) gather: works for any batch stride.
@@ -1039,10 +1039,10 @@ int spmm_cores_by_v(int V, const SpmmParams &p, cudaStream_t s) {
 }
 
 // ---- fp32 SpMM from bf16 parts ------------------------------------------------------------------------------
-template <int V, int kChunks> int launch_spmm_f32_standby(const SpmmParams &p, cudaStream_t s, DeviceInfo *d, const int32_t *verdict, int checks) {
+template <int V, int kChunks> int launch_spmm_f32_standby(const SpmmParams &p, cudaStream_t s, DeviceInfo *d, const int32_t *verdict, int checks, int few) {
     const int64_t blocks = ((int64_t)p.m_vec * (p.N / (4 * kChunks)) * p.batch + kCcThreads - 1) / kCcThreads, cap = (int64_t)d->sm_count * 8;
     auto kernel = spmm_cc_slabs(p, kChunks) ? spmm_cc_standby_kernel<float, float, V, kChunks, true> : spmm_cc_standby_kernel<float, float, V, kChunks>;
-    return (int)launch_overlapped(kernel, (unsigned)(blocks < cap ? blocks : cap), kCcThreads, 0, s, p, verdict, checks);
+    return (int)launch_overlapped(kernel, (unsigned)(blocks < cap ? blocks : cap), kCcThreads, 0, s, p, verdict, checks, few);
 }
 // Leaves *taken false where the call is not one for it.
 template <int V> int launch_spmm_split(const SpmmParams &p, int64_t vectors, cudaStream_t s, bool forced, DeviceInfo *d, bool *taken) {
@@ -1074,7 +1074,9 @@ template <int V> int launch_spmm_split(const SpmmParams &p, int64_t vectors, cud
     // dense width, so that column shards of usual matrices (90 %, at V = 4 80 % sparse) have the bits of the whole product.
     const double split_us = k_blocks * std::min(t_wide, t_narrow) + (double)(6 * a_elems + 10 * b_elems) / 4e6 + 10.0;
     constexpr double kCoresPs = V <= 2 ? 0.18 : V == 4 ? 0.35 : 0.6, kMinDensity = V == 1 ? 0.102 : V == 2 ? 0.11 : V == 4 ? 0.205 : 0.13;
-    q.min_vectors = forced ? 0 : (int64_t)std::max(1.1 * split_us / (kCoresPs * 1e-6 * p.N * p.batch), kMinDensity * p.m_vec * (double)p.K);
+    // Nor does it take a matrix whose rows are about as short on average as those that the CUDA-core kernel computes behind it.
+    q.few = forced ? 0 : splitspmm::few_entries(p.K);
+    q.min_vectors = forced ? 0 : (int64_t)std::max({1.1 * split_us / (kCoresPs * 1e-6 * p.N * p.batch), kMinDensity * p.m_vec * (double)p.K, 1.125 * q.few * p.m_vec});
     // A caller that does not say how many values there are: large products only, where two kernels that may return at once cost little.
     if (!forced && (vectors < q.min_vectors || p.N < 256 || (p.stride_values == 0 && split_us < 100.0))) return VS_OK;
     const int64_t units = (int64_t)q.batch_a * p.m_vec + b_elems / (8 * splitspmm::kPrepThreads) + 1;
@@ -1102,12 +1104,12 @@ template <int V> int launch_spmm_split(const SpmmParams &p, int64_t vectors, cud
     if (rc != VS_OK) return rc;
     const int chunks = spmm_cc_chunks(4 * V, 4, p.N);
     if constexpr (V <= 4) {
-        if (chunks == 4) return launch_spmm_f32_standby<V, 4>(p, s, d, q.verdict, checks);
+        if (chunks == 4) return launch_spmm_f32_standby<V, 4>(p, s, d, q.verdict, checks, q.few);
     }
-    if (chunks == 2) return launch_spmm_f32_standby<V, 2>(p, s, d, q.verdict, checks);
-    return launch_spmm_f32_standby<V, 1>(p, s, d, q.verdict, checks);
+    if (chunks == 2) return launch_spmm_f32_standby<V, 2>(p, s, d, q.verdict, checks, q.few);
+    return launch_spmm_f32_standby<V, 1>(p, s, d, q.verdict, checks, q.few);
 }
-// VSPARSE_B200_SPMM_F32=cores|split chooses one.
+// VSPARSE_B200_SPMM_F32=cores|split chooses one, for all rows.
 int spmm_split(int V, const SpmmParams &p, cudaStream_t s, bool *taken) {
     const char *e = std::getenv("VSPARSE_B200_SPMM_F32");
     const bool forced = e && !std::strcmp(e, "split");
