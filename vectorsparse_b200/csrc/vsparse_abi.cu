@@ -1831,10 +1831,15 @@ template <int D, bool kBackward> int launch_attention_rows(const attention::Para
     if (warps == 2) return launch_attention<D, 2, kBackward>(p, batch, s);
     return launch_attention<D, 4, kBackward>(p, batch, s);
 }
-// Whether the one-kernel form takes a call; what it does not take, and every refusal, is the operators' own.
+struct Span {
+    const void *at;
+    int64_t elems;   // fp16
+};
+// Whether the one-kernel form takes a call; what it does not take, and every refusal, is the operators' own.  Their steps read an operand for the
+// last time before a later step writes (grad_q in the place of grad_out, out in the place of kmat): where a result lies on an operand, they stay.
 // VSPARSE_B200_ATTENTION=steps|fused.
 bool attention_fused(int path, int m_vec, int V, int n, int d, int nnz_vec, int batch, std::initializer_list<const void *> indices,
-                     std::initializer_list<const void *> sources, std::initializer_list<const void *> results) {
+                     std::initializer_list<Span> sources, std::initializer_list<Span> results) {
     const char *e = std::getenv("VSPARSE_B200_ATTENTION");
     if (e && !std::strcmp(e, "steps")) return false;
     if (path != VS_PATH_TENSOR || !(V == 2 || V == 4 || V == 8) || (d != 64 && d != 128)) return false;
@@ -1844,10 +1849,14 @@ bool attention_fused(int path, int m_vec, int V, int n, int d, int nnz_vec, int 
     if (d == 128 && V < 8 && (int64_t)nnz_vec * batch > 1000000 && !(e && !std::strcmp(e, "fused"))) return false;
     for (const void *x : indices)
         if (!x) return false;
-    for (const void *x : sources)   // read 32 bytes at a time
-        if (!x || reinterpret_cast<uintptr_t>(x) % 32 != 0) return false;
-    for (const void *x : results)
-        if (!x || !aligned16(x)) return false;
+    for (const Span &x : sources)   // read 32 bytes at a time
+        if (!x.at || reinterpret_cast<uintptr_t>(x.at) % 32 != 0) return false;
+    for (const Span &x : results) {
+        if (!x.at || !aligned16(x.at)) return false;
+        const uintptr_t first = reinterpret_cast<uintptr_t>(x.at), end = first + 2 * (uintptr_t)x.elems * batch;
+        for (const Span &y : sources)
+            if (first < reinterpret_cast<uintptr_t>(y.at) + 2 * (uintptr_t)y.elems * batch && reinterpret_cast<uintptr_t>(y.at) < end) return false;
+    }
     return (int64_t)nnz_vec * V % 8 == 0;
 }
 }  // namespace
@@ -1875,7 +1884,8 @@ VS_EXPORT int vs_attention_cvse_backward(int path, int m_vec, int vec_length, in
         return VS_OK;
     }
     if (attention_fused(path, m_vec, vec_length, n, d, nonzeros_vec, batch, {row_indices, row_offsets, col_indices, t_offsets, t_rows, t_src},
-                        {q, kmat, vmat, grad_out}, {grad_q, grad_k, grad_v, probs_workspace, grad_workspace})) {
+                        {{q, s_q}, {kmat, s_k}, {vmat, s_k}, {grad_out, s_q}},
+                        {{grad_q, s_q}, {grad_k, s_k}, {grad_v, s_k}, {probs_workspace, s_ws}, {grad_workspace, s_ws}})) {
         DeviceInfo *info = nullptr;
         int rc = device_info(&info);
         if (rc != VS_OK) return rc;
@@ -1938,7 +1948,8 @@ VS_EXPORT int vs_attention_cvse(int path, int m_vec, int vec_length, int n, int 
         if (!out) return VS_ERR_NULL;
         return (int)cudaMemsetAsync(out, 0, (size_t)batch * m * d * 2, static_cast<cudaStream_t>(stream));
     }
-    if (attention_fused(path, m_vec, vec_length, n, d, nonzeros_vec, batch, {row_indices, row_offsets, col_indices}, {q, kmat, vmat}, {out, workspace})) {
+    if (attention_fused(path, m_vec, vec_length, n, d, nonzeros_vec, batch, {row_indices, row_offsets, col_indices},
+                        {{q, m * d}, {kmat, (int64_t)n * d}, {vmat, (int64_t)n * d}}, {{out, m * d}, {workspace, s_ws}})) {
         DeviceInfo *info = nullptr;
         const int rc = device_info(&info);
         if (rc != VS_OK) return rc;
