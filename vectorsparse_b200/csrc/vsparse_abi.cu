@@ -496,6 +496,9 @@ int spmm_cc_chunks(int VE, int E, int N) {
     const int cap = e ? std::atoi(e) : 4;
     return (VE <= 16 && cap >= 4 && N % (128 * E) == 0) ? 4 : (VE <= 32 && cap >= 2 && N % (64 * E) == 0) ? 2 : 1;
 }
+int64_t spmm_cc_tile_ctas(const SpmmParams &p) {
+    return (((int64_t)p.m_vec + cctile::kWarps - 1) / cctile::kWarps) * (((int64_t)p.N + cctile::kCols - 1) / cctile::kCols) * p.batch;
+}
 // Whether the fp32 product goes to the kernel that stages tiles of B.  Its CTAs take an SM each: where one wave of them
 // holds the product it won or drew at every V, size and sparsity measured from 128 columns up (up to 4x; with 64 columns
 // and a few entries per vector-row it lost, 5.5 against 4.3 us).  With two waves it still wins where the other kernel is
@@ -504,7 +507,7 @@ int spmm_cc_chunks(int VE, int E, int N) {
 // VSPARSE_B200_SPMM_CC=rows|tiles chooses one.
 bool spmm_cc_tiles_chosen(int V, const SpmmParams &p, const DeviceInfo *d) {
     if (p.K < 1 || p.K > 1 << 30) return false;   // tile coordinates and column sums in 32 bits
-    const int64_t ctas = (((int64_t)p.m_vec + cctile::kWarps - 1) / cctile::kWarps) * (((int64_t)p.N + cctile::kCols - 1) / cctile::kCols) * p.batch;
+    const int64_t ctas = spmm_cc_tile_ctas(p);
     if (ctas > 0x7fffffffll) return false;
     const char *e = std::getenv("VSPARSE_B200_SPMM_CC");
     if (e && !std::strcmp(e, "rows")) return false;
@@ -1068,15 +1071,20 @@ template <int V> int launch_spmm_split(const SpmmParams &p, int64_t vectors, cud
     const int tn = t_narrow < t_wide ? 128 : 256, n_tiles = (int)(tn == 256 ? wide : narrow);
     const int row_tiles = (int)((M + 127) / 128), slabs = q.Np / 64;
     const int64_t a_elems = (int64_t)q.batch_a * row_tiles * 128 * q.Kp, b_elems = (int64_t)q.batch_b * q.Kp * q.Np;
-    // us: 64 columns of an item by a pair, the preparation at 4 TB/s, launches (180 estimated, 165 to 180 measured at 4096 x 4096 x 1024; 94
-    // and 92 to 100 at 2048 cubed; 136 and 142 at 8 x (2000 x 1000 x 640)); against the CUDA-core kernel's time per vector and column (611 us
-    // at V = 1, 305 at V = 2, 301 at V = 4, 258 at V = 8 for 4096 x 4096 x 1024, 80 % sparse).  Below kMinDensity that kernel keeps every
+    // us: 64 columns of an item by a pair, the preparation at 4.6 TB/s, launches (180 estimated, 165 to 180 measured at 4096 x 4096 x 1024; 36
+    // and 36 at 1024 cubed; 25 and 25 at 512 cubed); against the CUDA-core kernel's time per vector and column (611 us
+    // at V = 1, 305 at V = 2, 301 at V = 4, 258 at V = 8 for 4096 x 4096 x 1024, 80 % sparse), or, where it takes the call otherwise, against that of the
+    // kernel that stages tiles of B: per wave a start, the tiles, the entries of a vector-row (V = 8, 2048 x 4096 x 1024, 50 / 65 / 80 %
+    // sparse: that kernel 228 / 165 / 103, this one 114 / 111 / 106; V = 1, 1024 x 1024 x 512: 54 / 41 / 29 and 38 / 37 / 36).  Below kMinDensity that kernel keeps every
     // dense width, so that column shards of usual matrices (90 %, at V = 4 80 % sparse) have the bits of the whole product.
-    const double split_us = k_blocks * std::min(t_wide, t_narrow) + (double)(6 * a_elems + 10 * b_elems) / 4e6 + 10.0;
-    constexpr double kCoresPs = V <= 2 ? 0.18 : V == 4 ? 0.35 : 0.6, kMinDensity = V == 1 ? 0.102 : V == 2 ? 0.11 : V == 4 ? 0.205 : 0.13;
+    const double split_us = k_blocks * std::min(t_wide, t_narrow) + (double)(6 * a_elems + 10 * b_elems) / 4.6e6 + 15.0;
+    constexpr double kCoresPs = V <= 2 ? 0.18 : V == 4 ? 0.35 : 0.6, kTileEntryUs = V == 1 ? 0.043 : V == 2 ? 0.047 : V == 4 ? 0.061 : 0.102, kMinDensity = V == 1 ? 0.102 : V == 2 ? 0.11 : V == 4 ? 0.205 : 0.13;
     // Nor does it take a matrix whose rows are about as short on average as those that the CUDA-core kernel computes behind it.
     q.few = forced ? 0 : splitspmm::few_entries(p.K);
-    q.min_vectors = forced ? 0 : (int64_t)std::max({1.1 * split_us / (kCoresPs * 1e-6 * p.N * p.batch), kMinDensity * p.m_vec * (double)p.K, 1.125 * q.few * p.m_vec});
+    double line = 1.1 * split_us / (kCoresPs * 1e-6 * p.N * p.batch);
+    if (spmm_cc_tiles_chosen(V, p, d))
+        line = p.m_vec * (1.1 * split_us / (double)((spmm_cc_tile_ctas(p) + d->sm_count - 1) / d->sm_count) - 6.0 - 0.002 * p.K) / kTileEntryUs;
+    q.min_vectors = forced ? 0 : (int64_t)std::max({line, kMinDensity * p.m_vec * (double)p.K, 1.125 * q.few * p.m_vec});
     // A caller that does not say how many values there are: large products only, where two kernels that may return at once cost little.
     if (!forced && (vectors < q.min_vectors || p.N < 256 || (p.stride_values == 0 && split_us < 100.0))) return VS_OK;
     const int64_t units = (int64_t)q.batch_a * p.m_vec + b_elems / (8 * splitspmm::kPrepThreads) + 1;
@@ -1109,11 +1117,11 @@ template <int V> int launch_spmm_split(const SpmmParams &p, int64_t vectors, cud
     if (chunks == 2) return launch_spmm_f32_standby<V, 2>(p, s, d, q.verdict, checks, q.few);
     return launch_spmm_f32_standby<V, 1>(p, s, d, q.verdict, checks, q.few);
 }
-// VSPARSE_B200_SPMM_F32=cores|split chooses one, for all rows.
+// VSPARSE_B200_SPMM_F32=cores|split chooses one, for all rows; VSPARSE_B200_SPMM_CC, a choice among the CUDA-core kernels, chooses those.
 int spmm_split(int V, const SpmmParams &p, cudaStream_t s, bool *taken) {
     const char *e = std::getenv("VSPARSE_B200_SPMM_F32");
     const bool forced = e && !std::strcmp(e, "split");
-    if ((e && !std::strcmp(e, "cores")) || t_no_scratch || t_ws_set || p.K < 1) return VS_OK;
+    if ((e && !std::strcmp(e, "cores")) || (!forced && std::getenv("VSPARSE_B200_SPMM_CC")) || t_no_scratch || t_ws_set || p.K < 1) return VS_OK;
     DeviceInfo *d = nullptr;
     const int rc = device_info(&d);
     if (rc != VS_OK) return rc;
