@@ -188,7 +188,7 @@ int vs_softmax_cvse(int dtype, int m_vec, int vec_length, const int32_t *row_ind
  * q [batch][m][d], kmat / vmat [batch][n][d], out [batch][m][d], all contiguous.
  * `workspace` must hold batch * nonzeros_vec * V fp16 values (the probabilities); the caller owns it.
  * One kernel for the whole batch on VS_PATH_TENSOR with d 64 or 128, vec_length 2, 4 or 8 and q, kmat, vmat on 32-byte boundaries (but
- * not for d = 128, vec_length < 8 and more than a million keys, nor where out or workspace overlaps an operand); else the SDDMM, the masked softmax and the SpMM one after the other
+ * not for millions of keys in dense masks of short vectors or at d = 128, nor where out or workspace overlaps an operand); else the SDDMM, the masked softmax and the SpMM one after the other
  * (up to five kernels with their plan and fallback kernels).  Environment variable VSPARSE_B200_ATTENTION = "fused" | "steps". */
 int vs_attention_cvse(int path, int m_vec, int vec_length, int n, int d, int nonzeros_vec,
                       const int32_t *row_indices, const int32_t *row_offsets, const int32_t *col_indices,

@@ -1852,9 +1852,13 @@ bool attention_fused(int path, int m_vec, int V, int n, int d, int nnz_vec, int 
     if (e && !std::strcmp(e, "steps")) return false;
     if (path != VS_PATH_TENSOR || !(V == 2 || V == 4 || V == 8) || (d != 64 && d != 128)) return false;
     if (m_vec < 1 || n < 1 || nnz_vec < 1 || batch < 1 || batch > kMaxBatch || (int64_t)m_vec * V > 0x7fffffffll || (int64_t)nnz_vec * V > 0x7fffffffll) return false;
-    // Gathering costs the same for 2 queries as for 8, the operators' dense tiles do not: at d = 128 and V < 8 they win once there is
-    // enough work (32 heads, sequence 2048, V = 4, 205 keys: 142 against 171 us; one million keys break even).
-    if (d == 128 && V < 8 && (int64_t)nnz_vec * batch > 1000000 && !(e && !std::strcmp(e, "fused"))) return false;
+    // Gathering costs what the mask names, the operators' dense tiles cost the whole matrix, and the same for 2 queries as for 8: dense masks of short
+    // vectors are theirs once there is enough work to fill the GPU, at 2048 columns more than at 4096.  us, operators / this, forward (backward alike): 32 heads,
+    // sequence 2048, 20 % of the keys, d = 64: V = 2 257 / 344, V = 4 155 / 186, V = 8 137 / 99; d = 128: 266 / 652, 164 / 336, 147 / 178; 15 %: 235 / 255,
+    // 141 / 139, 122 / 81; 244 / 488, 150 / 254, 129 / 148; 8 heads, 4096, 15 %: 319 / 267, 198 / 149, 196 / 74; 323 / 477, 231 / 537, 228 / 127; 128 heads, 1024,
+    // 5 %, d = 128: 168 / 219, 136 / 114, 119 / 64; 4 heads, 2048, 20 %, d = 64: 80 / 61, 62 / 36, 54 / 20.
+    const double named = (double)nnz_vec / ((double)m_vec * n), line = d == 64 ? (V == 2 ? 0.125 : V == 4 ? 0.145 : 1.0) : (V == 2 ? 0.04 : V == 4 ? 0.065 : 0.14);
+    if (named > line * std::sqrt(std::max(1.0, n / 2048.0)) && (int64_t)nnz_vec * batch * (d / 64) > 3000000 && !(e && !std::strcmp(e, "fused"))) return false;
     for (const void *x : indices)
         if (!x) return false;
     for (const Span &x : sources)   // read 32 bytes at a time
