@@ -187,7 +187,7 @@ int vs_softmax_cvse(int dtype, int m_vec, int vec_length, const int32_t *row_ind
  *   O_b = softmax(scale * SDDMM(Q_b, K_b)) . V_b, fp16 in and out, head dimension d (d % 64 == 0).
  * q [batch][m][d], kmat / vmat [batch][n][d], out [batch][m][d], all contiguous.
  * `workspace` must hold batch * nonzeros_vec * V fp16 values (the probabilities); the caller owns it.
- * One kernel for the whole batch on VS_PATH_TENSOR with d 64 or 128, vec_length 2, 4 or 8 and q, kmat, vmat on 32-byte boundaries (but
+ * One kernel for the whole batch on VS_PATH_TENSOR with d 64 or 128, vec_length 2, 4 or 8, scale > 0 and q, kmat, vmat on 32-byte boundaries (but
  * not for millions of keys in dense masks of short vectors or at d = 128, nor where out or workspace overlaps an operand); else the SDDMM, the masked softmax and the SpMM one after the other
  * (up to five kernels with their plan and fallback kernels).  Environment variable VSPARSE_B200_ATTENTION = "fused" | "steps". */
 int vs_attention_cvse(int path, int m_vec, int vec_length, int n, int d, int nonzeros_vec,

@@ -6,7 +6,7 @@
 //                fragment (a lane reads 32 contiguous bytes of row lane/4; the contraction index is permuted alike in Q).  The
 //                scores go to the caller's workspace in fp16, each to the place that the same lane reads again; a lane keeps a
 //                running maximum and sum for its two queries.
-//   second pass  P = exp(S - log sum), to the workspace in place of S; O^T[d, query] += V^T[d, key] . P^T[key, query], where P and
+//   second pass  P = exp(S - maximum) / sum, to the workspace in place of S; O^T[d, query] += V^T[d, key] . P^T[key, query], where P and
 //                the rows of V, read as those of K, are transposed in registers (movmatrix).
 // No shared memory holds an operand: it is left to L1, which serves the keys that neighbouring vector-rows share (the band of a
 // local mask); a CTA therefore holds consecutive vector-rows.
@@ -16,6 +16,8 @@
 // position) hit a quarter of them: 103 L1 wavefronts per 16 keys, now 80, a quarter of which transpose registers.  Those are what bounds
 // it: 70 % of their peak rate, at 54 % of the issue slots (32 heads, sequence 4096, 410 keys: 171 us).
 #pragma once
+#include <type_traits>
+
 #include "common.cuh"
 
 namespace attention {
@@ -36,8 +38,9 @@ struct Params {
     __half *probs;            // [batch][nnz_vec * V]: the probabilities
     const __half *grad_out;   // backward only; `out` is then dQ
     __half *grad_scores;      // backward only: [batch][nnz_vec * V], the gradient of the scores
-    float scale;
+    float scale;              // positive
 };
+constexpr float kLargeScore = 64.f;   // of a score times scale and log2(e)
 
 __device__ __forceinline__ void mma16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
@@ -72,13 +75,15 @@ __device__ __forceinline__ void load32(const __half *src, uint32_t (&r)[8]) {
 // The lane's pieces of 16 gathered rows: row lane/4 and row lane/4 + 8.
 template <int D> struct Rows {
     uint32_t r[2][D / 64][8];
-    // base: the matrix at the lane's first piece; col: the columns of a chunk, one per lane; s: which half of the chunk
+    // base: the matrix, the same for the whole CTA, so that a lane holds a 32-bit offset and no address (fewer than 2^32 elements); col: the columns of a
+    // chunk, one per lane; s: which half of the chunk
     __device__ __forceinline__ void fetch(const __half *base, int col, int s, int g) {
+        const uint32_t at = (threadIdx.x & 3) * 16;
         const int c0 = __shfl_sync(0xffffffffu, col, 16 * s + g), c1 = __shfl_sync(0xffffffffu, col, 16 * s + 8 + g);
 #pragma unroll
         for (int h = 0; h < D / 64; ++h) {
-            load32(base + (int64_t)c0 * D + 64 * h, r[0][h]);
-            load32(base + (int64_t)c1 * D + 64 * h, r[1][h]);
+            load32(base + ((uint32_t)c0 * D + 64 * h + at), r[0][h]);
+            load32(base + ((uint32_t)c1 * D + 64 * h + at), r[1][h]);
         }
     }
     __device__ __forceinline__ void clear(bool first, bool second) {
@@ -143,7 +148,7 @@ __global__ void __launch_bounds__(kThreads, (kCtasPerSm<D, kBackward>)) attentio
     __shared__ __align__(16) float part[W > 1 ? kGroups : 1][W > 1 ? W : 1][W > 1 ? 8 : 1][W > 1 ? kPitch : 4];
     const int group = threadIdx.x / (32 * W), w = (threadIdx.x >> 5) % W, lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int64_t b = blockIdx.y;
-    const __half *kmat = p.k + b * p.n * D + 16 * t, *vmat = p.v + b * p.n * D + 16 * t;
+    const __half *kmat = p.k + b * p.n * D, *vmat = p.v + b * p.n * D;
     const __half *q = p.q + b * p.m_vec * V * D + 16 * t;
     const __half *go = kBackward ? p.grad_out + b * p.m_vec * V * D + 16 * t : nullptr;
     __half *out = p.out + b * p.m_vec * V * D;
@@ -182,8 +187,8 @@ __global__ void __launch_bounds__(kThreads, (kCtasPerSm<D, kBackward>)) attentio
                     const bool here = key + 8 * i + g < end;
                     if (here && stores) *reinterpret_cast<uint32_t *>(to + 8 * i * V) = raw;
                     const float2 r = unpack2(raw);
-                    x[i >> 1][2 * (i & 1)] = here ? r.x * sl2 : -INFINITY;
-                    x[i >> 1][2 * (i & 1) + 1] = here ? r.y * sl2 : -INFINITY;
+                    x[i >> 1][2 * (i & 1)] = here ? r.x : -INFINITY;
+                    x[i >> 1][2 * (i & 1) + 1] = here ? r.y : -INFINITY;
                     if constexpr (kBackward) {
                         const uint32_t grad = here ? pack2(dp[i >> 1][2 * (i & 1)], dp[i >> 1][2 * (i & 1) + 1]) : 0u;
                         if (here && stores) *reinterpret_cast<uint32_t *>(tg + 8 * i * V) = grad;
@@ -194,13 +199,13 @@ __global__ void __launch_bounds__(kThreads, (kCtasPerSm<D, kBackward>)) attentio
                 }
 #pragma unroll
                 for (int i = 0; i < 2; ++i) {
-                    const float top = fmaxf(mx[i], fmaxf(fmaxf(x[0][i], x[0][i + 2]), fmaxf(x[1][i], x[1][i + 2])));
+                    const float top = fmaxf(mx[i], sl2 * fmaxf(fmaxf(x[0][i], x[0][i + 2]), fmaxf(x[1][i], x[1][i + 2])));
                     const float base = top == -INFINITY ? 0.f : top, keep = exp2_fast(mx[i] - base);
                     sum[i] *= keep;
                     if constexpr (kBackward) dot[i] *= keep;
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
-                        const float e = exp2_fast(x[j >> 1][i + 2 * (j & 1)] - base);
+                        const float e = exp2_fast(fmaf(x[j >> 1][i + 2 * (j & 1)], sl2, -base));   // the product unrounded, as in the second pass
                         sum[i] += e;
                         if constexpr (kBackward) dot[i] = fmaf(e, dp[j >> 1][i + 2 * (j & 1)], dot[i]);
                     }
@@ -209,7 +214,7 @@ __global__ void __launch_bounds__(kThreads, (kCtasPerSm<D, kBackward>)) attentio
             }
         }
         // over the lanes that share a query, then over the warps that share the row
-        float lse[2];
+        float inv[2];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             float top = mx[i];
@@ -252,8 +257,8 @@ __global__ void __launch_bounds__(kThreads, (kCtasPerSm<D, kBackward>)) attentio
         }
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            lse[i] = mx[i] + __log2f(sum[i]);   // NaN where no score is finite
-            if constexpr (kBackward) dot[i] /= sum[i];
+            inv[i] = 1.0f / sum[i];
+            if constexpr (kBackward) dot[i] *= inv[i];
         }
 
         // second pass: probabilities (and score gradients) in the place of the scores, and their product with the rows of V (of K)
@@ -264,7 +269,7 @@ __global__ void __launch_bounds__(kThreads, (kCtasPerSm<D, kBackward>)) attentio
             for (int j = 0; j < 4; ++j)
 #pragma unroll
                 for (int i = 0; i < 4; ++i) acc[h][j][i] = 0.f;
-        {
+        auto second_pass = [&](auto inside) {   // 1 / sum inside the exponent
             int next = chunk_column(p, beg + 32 * w + lane, end);
 #pragma unroll 1
             for (int key = beg + 32 * w; key < end; key += 32 * W) {
@@ -279,7 +284,11 @@ __global__ void __launch_bounds__(kThreads, (kCtasPerSm<D, kBackward>)) attentio
                     wt[i] = 0u;
                     if (here && stores) {
                         const float2 r = unpack2(*reinterpret_cast<const uint32_t *>(to + 8 * i * V));
-                        const float p0 = exp2_fast(fmaf(r.x, sl2, -lse[0])), p1 = exp2_fast(fmaf(r.y, sl2, -lse[1]));
+                        float p0 = exp2_fast(fmaf(r.x, sl2, -mx[0])), p1 = exp2_fast(fmaf(r.y, sl2, -mx[1]));   // NaN where no score is finite
+                        if constexpr (!decltype(inside)::value) {
+                            p0 *= inv[0];
+                            p1 *= inv[1];
+                        }
                         wt[i] = pack2(p0, p1);
                         *reinterpret_cast<uint32_t *>(to + 8 * i * V) = wt[i];
                         if constexpr (kBackward) {
@@ -298,7 +307,22 @@ __global__ void __launch_bounds__(kThreads, (kCtasPerSm<D, kBackward>)) attentio
                     r.weighted(transpose8(wt[2 * s]), transpose8(wt[2 * s + 1]), acc);
                 }
             }
+        };
+        // Next to scores of thousands an exponent has no room for the logarithm of the sum: up to 2^-9 of it, the same for all keys of a query, would be
+        // lost.  Outside, 1 / sum costs registers that are spent: 128 heads, sequence 4096, 583 -> 591 us, 29 heads, 688, V = 2, two warps to a row, 26.9 -> 28.7.  So
+        // forward with several warps to a row it is inside where scores are small enough for an error of 2^-19; with one warp a second body of the loop
+        // costs more (600), backward too (142 -> 148 at 110 heads, 424, V = 2).
+        bool small = false;
+        if constexpr (W > 1 && !kBackward) {
+            const float l0 = mx[0] - __log2f(inv[0]), l1 = mx[1] - __log2f(inv[1]);
+            small = __all_sync(0xffffffffu, fabsf(l0) < kLargeScore && fabsf(l1) < kLargeScore);
+            if (small) {
+                mx[0] = l0;
+                mx[1] = l1;
+                second_pass(std::true_type{});
+            }
         }
+        if (!small) second_pass(std::false_type{});
 
         // a lane holds queries 2t, 2t+1 of columns 64 h + 16 (g / 2) + (g & 1) + 2 x (0 .. 7); lane g ^ 1 has those between.  Of the
         // sixteen the even one takes the first eight, the odd one the others

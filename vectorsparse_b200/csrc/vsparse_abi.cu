@@ -1846,11 +1846,13 @@ struct Span {
 // Whether the one-kernel form takes a call; what it does not take, and every refusal, is the operators' own.  Their steps read an operand for the
 // last time before a later step writes (grad_q in the place of grad_out, out in the place of kmat): where a result lies on an operand, they stay.
 // VSPARSE_B200_ATTENTION=steps|fused.
-bool attention_fused(int path, int m_vec, int V, int n, int d, int nnz_vec, int batch, std::initializer_list<const void *> indices,
+bool attention_fused(int path, int m_vec, int V, int n, int d, int nnz_vec, int batch, float scale, std::initializer_list<const void *> indices,
                      std::initializer_list<Span> sources, std::initializer_list<Span> results) {
     const char *e = std::getenv("VSPARSE_B200_ATTENTION");
     if (e && !std::strcmp(e, "steps")) return false;
     if (path != VS_PATH_TENSOR || !(V == 2 || V == 4 || V == 8) || (d != 64 && d != 128)) return false;
+    if (!(scale > 0.f)) return false;   // it takes the maximum of scores ahead of the scale
+    if ((int64_t)n * d > 0xffffffffll) return false;   // 32-bit offsets
     if (m_vec < 1 || n < 1 || nnz_vec < 1 || batch < 1 || batch > kMaxBatch || (int64_t)m_vec * V > 0x7fffffffll || (int64_t)nnz_vec * V > 0x7fffffffll) return false;
     // Gathering costs what the mask names, the operators' dense tiles cost the whole matrix, and the same for 2 queries as for 8: dense masks of short
     // vectors are theirs once there is enough work to fill the GPU, at 2048 columns more than at 4096.  us, operators / this, forward (backward alike): 32 heads,
@@ -1895,7 +1897,7 @@ VS_EXPORT int vs_attention_cvse_backward(int path, int m_vec, int vec_length, in
         if (s_k > 0) VS_CUDA_TRY(cudaMemsetAsync(grad_v, 0, (size_t)batch * s_k * 2, st));
         return VS_OK;
     }
-    if (attention_fused(path, m_vec, vec_length, n, d, nonzeros_vec, batch, {row_indices, row_offsets, col_indices, t_offsets, t_rows, t_src},
+    if (attention_fused(path, m_vec, vec_length, n, d, nonzeros_vec, batch, scale, {row_indices, row_offsets, col_indices, t_offsets, t_rows, t_src},
                         {{q, s_q}, {kmat, s_k}, {vmat, s_k}, {grad_out, s_q}},
                         {{grad_q, s_q}, {grad_k, s_k}, {grad_v, s_k}, {probs_workspace, s_ws}, {grad_workspace, s_ws}})) {
         DeviceInfo *info = nullptr;
@@ -1960,7 +1962,7 @@ VS_EXPORT int vs_attention_cvse(int path, int m_vec, int vec_length, int n, int 
         if (!out) return VS_ERR_NULL;
         return (int)cudaMemsetAsync(out, 0, (size_t)batch * m * d * 2, static_cast<cudaStream_t>(stream));
     }
-    if (attention_fused(path, m_vec, vec_length, n, d, nonzeros_vec, batch, {row_indices, row_offsets, col_indices},
+    if (attention_fused(path, m_vec, vec_length, n, d, nonzeros_vec, batch, scale, {row_indices, row_offsets, col_indices},
                         {{q, m * d}, {kmat, (int64_t)n * d}, {vmat, (int64_t)n * d}}, {{out, m * d}, {workspace, s_ws}})) {
         DeviceInfo *info = nullptr;
         const int rc = device_info(&info);
