@@ -55,6 +55,7 @@ SIGNATURES = {
     "vs_sddmm_workspace_bytes": (_i64, [_i, _i, _i]),
     "vs_spmm_t_workspace_bytes": (_i64, [_i, _i, _i, _i, _i64]),
     "vs_set_workspace": (_i, [_vp, _i64]),
+    "vs_set_part_of": (_i, [_i, _i]),
     "vs_release_scratch": (_i, [_vp, _i]),
     "vs_selftest_mma": (_i, [_vp, _i, _vp, _i, C.c_uint32, _i, _f, _vp, _vp]),
     "vs_selftest_mma_pair": (_i, [_vp, _vp, _i, _vp, _i, C.c_uint32, _i, _f, _vp, _vp]),

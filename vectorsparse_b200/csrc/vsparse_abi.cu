@@ -143,6 +143,10 @@ thread_local bool t_ws_set = false;
 thread_local void *t_ws_ptr = nullptr;
 thread_local int64_t t_ws_bytes = 0;
 
+// What the calls of this host thread are parts of (vs_set_part_of; 0: nothing): choices that decide in which order sums are formed are made as
+// for the whole call.
+thread_local int t_whole_columns = 0, t_whole_batch = 0;
+
 // Scratch for captured work belongs to the graph: a buffer that the library keeps for a stream is replaced by a later, larger
 // call and used by other calls beside a replay.  The graph and whatever is instantiated from it hold a reference (a CUDA user
 // object); when the last one goes, the buffer comes back to this list and serves another capture, or is freed: by
@@ -1047,6 +1051,34 @@ template <int V, int kChunks> int launch_spmm_f32_standby(const SpmmParams &p, c
     auto kernel = spmm_cc_slabs(p, kChunks) ? spmm_cc_standby_kernel<float, float, V, kChunks, true> : spmm_cc_standby_kernel<float, float, V, kChunks>;
     return (int)launch_overlapped(kernel, (unsigned)(blocks < cap ? blocks : cap), kCcThreads, 0, s, p, verdict, checks, few);
 }
+// Tiles, scratch and estimated time of the split product of p's matrix with N columns in `batch` problems.
+struct SplitSizes {
+    int batch_a, batch_b, Kp, Np, k_blocks, m_tiles, tn, n_tiles, row_tiles, slabs;
+    int64_t row_items, a_elems, b_elems;
+    double us;
+};
+SplitSizes split_sizes(const SpmmParams &p, int V, int N, int batch, int resident) {
+    SplitSizes z;
+    const int64_t M = (int64_t)p.m_vec * V;
+    z.batch_a = batch > 1 && (p.stride_values || p.batch == 1) ? batch : 1;
+    z.batch_b = batch > 1 && (p.stride_rhs || p.batch == 1) ? batch : 1;
+    z.Kp = (p.K + 63) / 64 * 64;
+    z.Np = (N + 63) / 64 * 64;
+    z.k_blocks = z.Kp / 64;
+    z.m_tiles = (int)((M + splitspmm::kTileM - 1) / splitspmm::kTileM);
+    z.row_items = (int64_t)batch * z.m_tiles;
+    const int64_t wide = (N + 255) / 256, narrow = (N + 127) / 128;
+    auto waves = [&](int64_t items) { return (double)((items + resident - 1) / resident); };
+    const double t_wide = 2.1 * waves(z.row_items * wide), t_narrow = 1.1 * waves(z.row_items * narrow);
+    z.tn = t_narrow < t_wide ? 128 : 256;
+    z.n_tiles = (int)(z.tn == 256 ? wide : narrow);
+    z.row_tiles = (int)((M + 127) / 128);
+    z.slabs = z.Np / 64;
+    z.a_elems = (int64_t)z.batch_a * z.row_tiles * 128 * z.Kp;
+    z.b_elems = (int64_t)z.batch_b * z.Kp * z.Np;
+    z.us = z.k_blocks * std::min(t_wide, t_narrow) + (double)(6 * z.a_elems + 10 * z.b_elems) / 4.6e6 + 15.0;
+    return z;
+}
 // Leaves *taken false where the call is not one for it.
 template <int V> int launch_spmm_split(const SpmmParams &p, int64_t vectors, cudaStream_t s, bool forced, DeviceInfo *d, bool *taken) {
     static int resident[kMaxDevices];   // 0 = not asked yet, -1 = the kernel cannot run here
@@ -1059,38 +1091,33 @@ template <int V> int launch_spmm_split(const SpmmParams &p, int64_t vectors, cud
     }
     if (resident[dev] < 0) return VS_OK;
     const int64_t M = (int64_t)p.m_vec * V;
+    SpmmParams whole = p;
+    whole.N = std::max(p.N, t_whole_columns);
+    whole.batch = std::max(p.batch, t_whole_batch);
+    const SplitSizes z = split_sizes(p, V, p.N, p.batch, resident[dev]), zw = split_sizes(p, V, whole.N, whole.batch, resident[dev]);
     splitspmm::PrepParams q;
-    q.batch_a = p.batch > 1 && p.stride_values ? p.batch : 1;
-    q.batch_b = p.batch > 1 && p.stride_rhs ? p.batch : 1;
-    q.Kp = (p.K + 63) / 64 * 64;
-    q.Np = (p.N + 63) / 64 * 64;
-    const int k_blocks = q.Kp / 64, m_tiles = (int)((M + splitspmm::kTileM - 1) / splitspmm::kTileM);
-    const int64_t row_items = (int64_t)p.batch * m_tiles, wide = (p.N + 255) / 256, narrow = (p.N + 127) / 128;
-    auto waves = [&](int64_t items) { return (double)((items + resident[dev] - 1) / resident[dev]); };
-    const double t_wide = 2.1 * waves(row_items * wide), t_narrow = 1.1 * waves(row_items * narrow);
-    const int tn = t_narrow < t_wide ? 128 : 256, n_tiles = (int)(tn == 256 ? wide : narrow);
-    const int row_tiles = (int)((M + 127) / 128), slabs = q.Np / 64;
-    const int64_t a_elems = (int64_t)q.batch_a * row_tiles * 128 * q.Kp, b_elems = (int64_t)q.batch_b * q.Kp * q.Np;
+    q.batch_a = z.batch_a; q.batch_b = z.batch_b; q.Kp = z.Kp; q.Np = z.Np;
+    const int k_blocks = z.k_blocks, m_tiles = z.m_tiles, tn = z.tn, n_tiles = z.n_tiles, row_tiles = z.row_tiles, slabs = z.slabs;
+    const int64_t row_items = z.row_items, a_elems = z.a_elems, b_elems = z.b_elems;
     // us: 64 columns of an item by a pair, the preparation at 4.6 TB/s, launches (180 estimated, 165 to 180 measured at 4096 x 4096 x 1024; 36
     // and 36 at 1024 cubed; 25 and 25 at 512 cubed); against the CUDA-core kernel's time per vector and column (611 us
     // at V = 1, 305 at V = 2, 301 at V = 4, 258 at V = 8 for 4096 x 4096 x 1024, 80 % sparse), or, where it takes the call otherwise, against that of the
     // kernel that stages tiles of B: per wave a start, the tiles, the entries of a vector-row (V = 8, 2048 x 4096 x 1024, 50 / 65 / 80 %
     // sparse: that kernel 228 / 165 / 103, this one 114 / 111 / 106; V = 1, 1024 x 1024 x 512: 54 / 41 / 29 and 38 / 37 / 36).  Below kMinDensity that kernel keeps every
     // dense width, so that column shards of usual matrices (90 %, at V = 4 80 % sparse) have the bits of the whole product.
-    const double split_us = k_blocks * std::min(t_wide, t_narrow) + (double)(6 * a_elems + 10 * b_elems) / 4.6e6 + 15.0;
     constexpr double kCoresPs = V <= 2 ? 0.18 : V == 4 ? 0.35 : 0.6, kTileEntryUs = V == 1 ? 0.043 : V == 2 ? 0.047 : V == 4 ? 0.061 : 0.102, kMinDensity = V == 1 ? 0.102 : V == 2 ? 0.11 : V == 4 ? 0.205 : 0.13;
     // Nor does it take a matrix whose rows are about as short on average as those that the CUDA-core kernel computes behind it.
     q.few = forced ? 0 : splitspmm::few_entries(p.K);
-    double line = 1.1 * split_us / (kCoresPs * 1e-6 * p.N * p.batch);
-    if (spmm_cc_tiles_chosen(V, p, d))
-        line = p.m_vec * (1.1 * split_us / (double)((spmm_cc_tile_ctas(p) + d->sm_count - 1) / d->sm_count) - 6.0 - 0.002 * p.K) / kTileEntryUs;
+    double line = 1.1 * zw.us / (kCoresPs * 1e-6 * whole.N * whole.batch);
+    if (spmm_cc_tiles_chosen(V, whole, d))
+        line = p.m_vec * (1.1 * zw.us / (double)((spmm_cc_tile_ctas(whole) + d->sm_count - 1) / d->sm_count) - 6.0 - 0.002 * p.K) / kTileEntryUs;
     q.min_vectors = forced ? 0 : (int64_t)std::max({line, kMinDensity * p.m_vec * (double)p.K, 1.125 * q.few * p.m_vec});
     // A caller that does not say how many values there are: large products only, where two kernels that may return at once cost little.
-    if (!forced && (vectors < q.min_vectors || p.N < 256 || (p.stride_values == 0 && split_us < 100.0))) return VS_OK;
+    if (!forced && (vectors < q.min_vectors || whole.N < 256 || (p.stride_values == 0 && zw.us < 100.0))) return VS_OK;
     const int64_t units = (int64_t)q.batch_a * p.m_vec + b_elems / (8 * splitspmm::kPrepThreads) + 1;
     const int checks = (int)std::min<int64_t>(units, 8 * d->sm_count);
     const int64_t header = ((4 + checks) * 4 + 255) / 256 * 256, a_bytes = (a_elems * 6 + 255) / 256 * 256, bytes = header + a_bytes + b_elems * 6;
-    if (bytes > kMaxPlanBytes || row_items * n_tiles * k_blocks > 0x7fffffffll) return VS_OK;
+    if (std::max(bytes, (zw.a_elems + zw.b_elems) * 6) > kMaxPlanBytes || zw.row_items * zw.n_tiles * k_blocks > 0x7fffffffll) return VS_OK;
     CUtensorMap map_out;
     if (make_tile_map(&map_out, p.out, true, (uint64_t)M, (uint64_t)p.N, (uint64_t)p.batch, (uint64_t)p.stride_out, splitspmm::kStoreCols, 32, false) != VS_OK) return VS_OK;
     uint8_t *mem = nullptr;
@@ -1831,7 +1858,7 @@ template <int D, int W, bool kBackward> int launch_attention(const attention::Pa
 // 4096: 588 / 670 / 793 us with 1 / 2 / 4 warps); more where the rows are few (2 heads, sequence 1024, 154 keys: 12.6 / 9.3 / 8.5 us) and long enough
 // for a chunk each.  VSPARSE_B200_ATTENTION_WARPS chooses.
 template <int D, bool kBackward> int launch_attention_rows(const attention::Params &p, int batch, DeviceInfo *d, cudaStream_t s) {
-    const int64_t rows = (int64_t)p.m_vec * batch, wave = (int64_t)d->sm_count * attention::kCtasPerSm<D, kBackward> * (attention::kThreads / 32);
+    const int64_t rows = (int64_t)p.m_vec * std::max(batch, t_whole_batch), wave = (int64_t)d->sm_count * attention::kCtasPerSm<D, kBackward> * (attention::kThreads / 32);
     const int keys = p.nnz_vec / p.m_vec;
     const char *e = std::getenv("VSPARSE_B200_ATTENTION_WARPS");
     const int warps = e ? std::atoi(e) : rows >= 3 * wave || keys <= 32 ? 1 : 2 * rows >= 3 * wave || keys <= 64 ? 2 : 4;
@@ -1860,7 +1887,7 @@ bool attention_fused(int path, int m_vec, int V, int n, int d, int nnz_vec, int 
     // 141 / 139, 122 / 81; 244 / 488, 150 / 254, 129 / 148; 8 heads, 4096, 15 %: 319 / 267, 198 / 149, 196 / 74; 323 / 477, 231 / 537, 228 / 127; 128 heads, 1024,
     // 5 %, d = 128: 168 / 219, 136 / 114, 119 / 64; 4 heads, 2048, 20 %, d = 64: 80 / 61, 62 / 36, 54 / 20.
     const double named = (double)nnz_vec / ((double)m_vec * n), line = d == 64 ? (V == 2 ? 0.125 : V == 4 ? 0.145 : 1.0) : (V == 2 ? 0.04 : V == 4 ? 0.065 : 0.14);
-    if (named > line * std::sqrt(std::max(1.0, n / 2048.0)) && (int64_t)nnz_vec * batch * (d / 64) > 3000000 && !(e && !std::strcmp(e, "fused"))) return false;
+    if (named > line * std::sqrt(std::max(1.0, n / 2048.0)) && (int64_t)nnz_vec * std::max(batch, t_whole_batch) * (d / 64) > 3000000 && !(e && !std::strcmp(e, "fused"))) return false;
     for (const void *x : indices)
         if (!x) return false;
     for (const Span &x : sources)   // read 32 bytes at a time
@@ -2156,6 +2183,13 @@ VS_EXPORT int vs_set_workspace(void *workspace, int64_t bytes) {
     t_ws_set = workspace != nullptr;
     t_ws_ptr = workspace;
     t_ws_bytes = bytes;
+    return VS_OK;
+}
+
+VS_EXPORT int vs_set_part_of(int columns, int batch) {
+    if (columns < 0 || batch < 0) return VS_ERR_ARG;
+    t_whole_columns = columns;
+    t_whole_batch = batch;
     return VS_OK;
 }
 

@@ -10,10 +10,31 @@ PyTorch is plumbing here (process group, device memory); the arithmetic is in li
 """
 from __future__ import annotations
 
+import contextlib
+import threading
 from typing import Callable, List, Tuple
 
 import torch
 import torch.distributed as dist
+
+
+_scope = threading.local()
+
+
+@contextlib.contextmanager
+def part_of(columns: int = 0, batch: int = 0):
+    """Calls of this host thread inside the block are parts of one call with that many dense columns or problems, and choose the order of their sums
+    as that call would (vs_set_part_of): fp32 SpMM between the CUDA cores and the tensor cores, attention between its forms and the warps that
+    share a row.  A part then has the bits of the whole, at the price of a kernel that may not be the quickest for the part alone."""
+    from . import _lib
+    outer = getattr(_scope, "value", (0, 0))
+    _scope.value = (columns, batch)
+    _lib.check(_lib.lib().vs_set_part_of(columns, batch), "vs_set_part_of")
+    try:
+        yield
+    finally:
+        _scope.value = outer
+        _lib.lib().vs_set_part_of(*outer)
 
 
 def column_shards(n_cols: int, world: int, multiple: int = 64) -> List[Tuple[int, int]]:
@@ -52,12 +73,13 @@ def take_columns(dense: torch.Tensor, rank: int, world: int, multiple: int = 64)
 def spmm_column_sharded(spmm_fn: Callable, m_vec: int, vec_length: int, n_cols: int, k_sparse: int, structure,
                         values: torch.Tensor, rhs_local: torch.Tensor, out_local: torch.Tensor) -> None:
     """Runs this rank's share: spmm_fn is ops.spmm.wmmaSpmm / ops.spmm.cudaSpmm (or any callable with that
-    signature); rhs_local / out_local are the rank's [K, w] / [M, w] blocks.  A rank whose width is 0 does nothing."""
+    signature); rhs_local / out_local are the rank's [K, w] / [M, w] blocks of the n_cols columns.  A rank whose width is 0 does nothing."""
     w = rhs_local.shape[-1]
     if w == 0:
         return
     ri, ro, ci = structure
-    spmm_fn(m_vec, vec_length, w, k_sparse, ri, ro, ci, values, rhs_local, out_local)
+    with part_of(columns=n_cols) if rhs_local.is_cuda else contextlib.nullcontext():
+        spmm_fn(m_vec, vec_length, w, k_sparse, ri, ro, ci, values, rhs_local, out_local)
 
 
 def gather_columns(out_local: torch.Tensor, n_cols: int, multiple: int = 64, group=None) -> torch.Tensor:
