@@ -143,6 +143,7 @@ template <int D, int W, bool kBackward>
 __global__ void __launch_bounds__(kThreads, (kCtasPerSm<D, kBackward>)) attention_kernel(const Params p) {
     constexpr int kGroups = kThreads / (32 * W);
     constexpr int kPitch = 64 + 4;
+    constexpr bool kTwoForms = W > 1 && !kBackward;   // of the second pass
     const int V = p.V;
     __shared__ float red[kGroups][W][8][3];
     __shared__ __align__(16) float part[W > 1 ? kGroups : 1][W > 1 ? W : 1][W > 1 ? 8 : 1][W > 1 ? kPitch : 4];
@@ -257,7 +258,7 @@ __global__ void __launch_bounds__(kThreads, (kCtasPerSm<D, kBackward>)) attentio
         }
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
-            inv[i] = 1.0f / sum[i];
+            if constexpr (!kTwoForms) inv[i] = 1.0f / sum[i];
             if constexpr (kBackward) dot[i] *= inv[i];
         }
 
@@ -312,17 +313,20 @@ __global__ void __launch_bounds__(kThreads, (kCtasPerSm<D, kBackward>)) attentio
         // lost.  Outside, 1 / sum costs registers that are spent: 128 heads, sequence 4096, 583 -> 591 us, 29 heads, 688, V = 2, two warps to a row, 26.9 -> 28.7.  So
         // forward with several warps to a row it is inside where scores are small enough for an error of 2^-19; with one warp a second body of the loop
         // costs more (600), backward too (142 -> 148 at 110 heads, 424, V = 2).
-        bool small = false;
-        if constexpr (W > 1 && !kBackward) {
-            const float l0 = mx[0] - __log2f(inv[0]), l1 = mx[1] - __log2f(inv[1]);
-            small = __all_sync(0xffffffffu, fabsf(l0) < kLargeScore && fabsf(l1) < kLargeScore);
-            if (small) {
+        if constexpr (kTwoForms) {
+            const float l0 = mx[0] + __log2f(sum[0]), l1 = mx[1] + __log2f(sum[1]);
+            if (__all_sync(0xffffffffu, fabsf(l0) < kLargeScore && fabsf(l1) < kLargeScore)) {
                 mx[0] = l0;
                 mx[1] = l1;
                 second_pass(std::true_type{});
+            } else {
+                inv[0] = 1.0f / sum[0];
+                inv[1] = 1.0f / sum[1];
+                second_pass(std::false_type{});
             }
+        } else {
+            second_pass(std::false_type{});
         }
-        if (!small) second_pass(std::false_type{});
 
         // a lane holds queries 2t, 2t+1 of columns 64 h + 16 (g / 2) + (g & 1) + 2 x (0 .. 7); lane g ^ 1 has those between.  Of the
         // sixteen the even one takes the first eight, the odd one the others
