@@ -33,6 +33,30 @@ def structure(a):
     return ri, ro, ci
 
 
+def captured_kernels(call):
+    """Names (mangled) of the kernels that a call enqueues, from its graph, which is then replayed once."""
+    from cuda.bindings import driver
+
+    def ok(result):
+        assert result[0] == driver.CUresult.CUDA_SUCCESS, result
+        return result[1] if len(result) == 2 else result[1:]
+
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        call()
+    raw = driver.CUgraph(graph.raw_cuda_graph())
+    nodes = ok(driver.cuGraphGetNodes(raw, ok(driver.cuGraphGetNodes(raw))[1]))[0]
+    names = []
+    for node in nodes:
+        if ok(driver.cuGraphNodeGetType(node)) == driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL:
+            params = ok(driver.cuGraphKernelNodeGetParams(node))
+            names.append(ok(driver.cuFuncGetName(params.func)) if int(params.func) else ok(driver.cuKernelGetName(params.kern)))
+    graph.replay()
+    torch.cuda.synchronize()
+    return " ".join(n.decode() for n in names)
+
+
 def spmm_inputs(a, N, dtype, seed, sigma=None):
     """values and B as numpy arrays of `dtype` (fp16 values are the rounded fp32 draws)."""
     if sigma is None:

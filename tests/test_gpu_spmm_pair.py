@@ -6,7 +6,7 @@ import pytest
 import torch
 
 from conftest import assert_close
-from gpu_util import DEV, custom, dev, problem, spmm_inputs, spmm_oracle, structure
+from gpu_util import captured_kernels, DEV, custom, dev, problem, spmm_inputs, spmm_oracle, structure
 from vectorsparse_b200 import VS_PATH_TENSOR, _lib, cvse, ops
 
 pytestmark = pytest.mark.gpu
@@ -171,8 +171,11 @@ def test_a_laid_out_beforehand(V, m_vec, K, N, what, monkeypatch):
     for how in ("plan", "laid-out"):
         monkeypatch.setenv("VSPARSE_B200_SPMM_A", how)
         out = torch.full((a.m * N + 64,), float("nan"), dtype=torch.float16, device=DEV)
-        (ops.spmm.cudaSpmm if V == 1 else ops.spmm.wmmaSpmm)(m_vec, V, N, K, *structure(a), dev(vals), dev(B), out)
+        args = (m_vec, V, N, K, *structure(a), dev(vals), dev(B), out)
+        (ops.spmm.cudaSpmm if V == 1 else ops.spmm.wmmaSpmm)(*args)
         torch.cuda.synchronize()
+        kernels = captured_kernels(lambda: (ops.spmm.cudaSpmm if V == 1 else ops.spmm.wmmaSpmm)(*args))
+        assert ("densify_kernel" in kernels) == (how == "laid-out") and ("dense_plan_kernel" in kernels) == (how == "plan" and K < 5000)
         assert ops.device_status() == 0
         assert bool(torch.isnan(out[a.m * N:]).all()), "wrote past the end"
         got[how] = out[:a.m * N].view(a.m, N).float().cpu().numpy()

@@ -14,10 +14,12 @@ def run(monkeypatch, a, N, vals, B, mode, batch=1):
     monkeypatch.setenv("VSPARSE_B200_SPMM_F32", mode)
     out = torch.full((batch * a.m * N + 64,), float("nan"), device=DEV)
     view = out[:batch * a.m * N].view(batch, a.m, N)
+    ops.kernel_timing(True)
     if batch > 1:
         ops.spmm_batched(VS_PATH_CUDA_CORE, a.m_vec, a.V, N, a.n, *structure(a), dev(vals), dev(B), view)
     else:
         ops.spmm.cudaSpmm(a.m_vec, a.V, N, a.n, *structure(a), dev(vals), dev(B), view)
+    assert ops.kernel_timing(False)[1] == (1 if mode == "split" else 0), "not the kernels this is about"
     torch.cuda.synchronize()
     assert ops.device_status() == 0
     assert bool(torch.isnan(out[batch * a.m * N:]).all()), "wrote past the end"

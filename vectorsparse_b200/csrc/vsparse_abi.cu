@@ -1134,8 +1134,11 @@ template <int V> int launch_spmm_split(const SpmmParams &p, int64_t vectors, cud
     int rc = (int)launch_overlapped(splitspmm::spmm_split_prepare<V>, (unsigned)checks, splitspmm::kPrepThreads, 0, s, p, q);
     if (rc != VS_OK) return rc;
     const int64_t items = row_items * n_tiles;
-    rc = (int)launch_pairs(tn == 256 ? splitspmm::spmm_split_kernel<256> : splitspmm::spmm_split_kernel<128>, (unsigned)std::min<int64_t>(items, resident[dev]), splitspmm::kThreads, (size_t)splitspmm::kSmemBytes, s, true,
-                           p, V, map_a, map_b, map_out, q.batch_a, q.batch_b, m_tiles, n_tiles, k_blocks, row_tiles, slabs, d->status, q.verdict, checks, q.verdict + kPlanRedo);
+    {
+        TimedLaunch timed(s);
+        rc = (int)launch_pairs(tn == 256 ? splitspmm::spmm_split_kernel<256> : splitspmm::spmm_split_kernel<128>, (unsigned)std::min<int64_t>(items, resident[dev]), splitspmm::kThreads, (size_t)splitspmm::kSmemBytes, s, true,
+                               p, V, map_a, map_b, map_out, q.batch_a, q.batch_b, m_tiles, n_tiles, k_blocks, row_tiles, slabs, d->status, q.verdict, checks, q.verdict + kPlanRedo);
+    }
     if (rc != VS_OK) return rc;
     const int chunks = spmm_cc_chunks(4 * V, 4, p.N);
     if constexpr (V <= 4) {
