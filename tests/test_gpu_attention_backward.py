@@ -50,10 +50,11 @@ def test_softmax_backward_batched():
         assert_close(out[b].float().cpu().numpy(), want, f"batch entry {b}")
 
 
-@pytest.mark.parametrize("path", [VS_PATH_TENSOR, VS_PATH_CUDA_CORE])
-def test_attention_backward_small(path):
-    """Seven operator calls (SDDMM, softmax, SpMM^T, SDDMM, softmax backward, SpMM, SpMM^T) on a band + strided mask,
-    two heads sharing it; intermediates are fp16 on the GPU and double in the oracle."""
+@pytest.mark.parametrize("path,form", [(VS_PATH_TENSOR, "steps"), (VS_PATH_TENSOR, "fused"), (VS_PATH_CUDA_CORE, "steps")])
+def test_attention_backward_small(path, form, monkeypatch):
+    """Seven operator calls (SDDMM, softmax, SpMM^T, SDDMM, softmax backward, SpMM, SpMM^T), or one kernel and two of them, on a band + strided
+    mask, two heads sharing it; intermediates are fp16 on the GPU and double in the oracle."""
+    monkeypatch.setenv("VSPARSE_B200_ATTENTION", form)
     V, d, n, heads = 8, 64, 512, 2
     a = problem(cvse.GEN_BAND, 6, n // V, n, V, 0.8, band=64)
     q, k, v, go = (cvse.fill_random((heads, n, d), np.float16, cvse.DIST_NORMAL, 10 + i, 1.0) for i in range(4))

@@ -46,9 +46,12 @@ def attention_pair(path, seed, heads, n, band, sparsity, check_oracle=False):
 
 
 @pytest.mark.parametrize("path", [VS_PATH_TENSOR, VS_PATH_CUDA_CORE])
-def test_two_calls_in_a_row_match_the_workspace_form(path, monkeypatch):
-    # The no-allocation form always runs the row-gather tensor kernels (the dense formulations keep plan scratch);
-    # the workspace form is pinned to the same ones here, so that the comparison can be bit for bit.
+@pytest.mark.parametrize("form", ["steps", "fused"])
+def test_two_calls_in_a_row_match_the_workspace_form(path, form, monkeypatch):
+    # Operator by operator the no-allocation form runs the row-gather tensor kernels (the dense formulations keep plan scratch);
+    # the workspace form is pinned to the same ones here, so that the comparison can be bit for bit.  The one-kernel form (tensor
+    # path) keeps nothing and is the same in both.
+    monkeypatch.setenv("VSPARSE_B200_ATTENTION", form)
     monkeypatch.setenv("VSPARSE_B200_SPMM", "gather")
     monkeypatch.setenv("VSPARSE_B200_SDDMM", "gather")
     want, got = attention_pair(path, seed=31, heads=3, n=512, band=64, sparsity=0.8, check_oracle=True)
@@ -61,7 +64,8 @@ def test_two_calls_in_a_row_match_the_workspace_form(path, monkeypatch):
 
 
 def test_matches_the_default_formulations_within_tolerance(monkeypatch):
-    """Left to choose, the workspace form may run the dense formulations: same values up to fp16 rounding."""
+    """Left to choose, the workspace form may run the dense formulations of the operators: same values up to fp16 rounding."""
+    monkeypatch.setenv("VSPARSE_B200_ATTENTION", "steps")
     monkeypatch.delenv("VSPARSE_B200_SPMM", raising=False)
     monkeypatch.delenv("VSPARSE_B200_SDDMM", raising=False)
     want, got = attention_pair(VS_PATH_TENSOR, seed=5, heads=2, n=512, band=64, sparsity=0.8)
@@ -82,6 +86,7 @@ def test_requests_beyond_the_built_in_scratch_are_refused():
 def test_a_request_of_exactly_the_built_in_size_runs_and_one_vector_more_is_refused(monkeypatch):
     """4 heads x 131072 vectors x 8 values x 2 bytes = 8 388 608 bytes: the whole array, accepted and correct; one
     vector more per head is refused on the host."""
+    monkeypatch.setenv("VSPARSE_B200_ATTENTION", "steps")
     monkeypatch.setenv("VSPARSE_B200_SPMM", "gather")
     monkeypatch.setenv("VSPARSE_B200_SDDMM", "gather")
     V, n, heads = 8, 2048, 4
