@@ -81,8 +81,11 @@ const char *vs_version(void);
  * Products of up to about one wave of tiles do the same in one kernel without a plan.  fp16 results with VS_PATH_CUDA_CORE take
  * the same formulations, with the CUDA-core kernel in the place of the gather kernels; fp16 operands with fp32 results there stay on the
  * CUDA cores.  fp32 products of 256 and more dense columns that are not too sparse are multiplied on the tensor cores from three bf16
- * parts of each operand, with sums in fp32 registers: no further from the exact result than the CUDA-core kernel's, which takes the
- * rest (sparser matrices, repeated columns, non-finite results, operands below 2^-100 or results below 2^-96 in magnitude).
+ * parts of each operand, with sums in fp32 registers: nearer to the exact result than the CUDA-core kernel's where a vector-row has many
+ * entries (2-norm over a row's results: 1.6e-7 against 4.1e-7 at 512 of 4096 columns).  That kernel takes the rest: vector-rows of fewer than
+ * max(24, n / 64 + 16) entries, sparser matrices, and the whole product where a vector-row names a column twice, a result is not
+ * finite, an operand other than 0 is below 2^-100 or a result other than 0 below 2^-96 in magnitude.  One such number is enough, and the
+ * time of the product is then spent on top (4096 x 4096 x 8192, 80 % sparse: 5.7 ms, not 0.96; 4.7 on the CUDA cores from the start).
  * Environment variable VSPARSE_B200_SPMM_F32 = "cores" | "split" forces one of the two.
  * Environment variable VSPARSE_B200_SPMM = "dense" | "gather" | "direct" (one kernel) forces one formulation.  The first call with a plan on a
  * stream allocates a scratch buffer with cudaMallocAsync on that stream (8 bytes per possible nonzero vector, m_vec * n
@@ -277,6 +280,9 @@ int vs_device_status(int clear, uint32_t *status);
  *                                                        thread put their plan in [ptr, ptr + bytes) when it
  *                                                        fits and run the row-gather formulation when it does
  *                                                        not: with a workspace set the library never allocates.
+ *                                                        (A matrix with vectors of 2 is laid out densely, see
+ *                                                        vs_spmm, only where that fits too: 2 bytes per element
+ *                                                        and problem with values of its own.)
  *                                                        Calls with VS_PATH_CUDA_CORE neither use it nor keep a
  *                                                        plan while one is set: they take the forms without.
  *                                                        (NULL, 0) returns to the library's own buffers.

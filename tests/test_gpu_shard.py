@@ -1,7 +1,7 @@
 """The two partitions of the operators over the GPUs of one box (columns of the dense operand for SpMM, batch x head for
 fixed-mask attention), run on ONE GPU: the G shards of a problem are computed one after another through
-vectorsparse_b200.shard on the real kernels and reassembled; since neither partition changes the order of any sum,
-the result must equal the unsharded one bit for bit, for G = 2, 4 and 8.  (The same helpers run one shard per rank
+vectorsparse_b200.shard on the real kernels and reassembled; since neither partition changes the order of any sum at these sizes
+(tests/test_gpu_shard_parts.py has those where it would), the result must equal the unsharded one bit for bit, for G = 2, 4 and 8.  (The same helpers run one shard per rank
 under torch.distributed; tests/test_shard_gloo.py covers the collectives on CPU.)"""
 import numpy as np
 import pytest

@@ -308,7 +308,7 @@ spmm_pair_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_a, 
                 const __half *vals = values0 + (int64_t)c_b * p.stride_values;
                 if constexpr (V == 1) {
                     // denser buckets, many batches of them: the entries of the next four are on their way while the values of these are
-                    // (64 x (1024 x 256 x 256), 80 / 50 %: 33.8 -> 32.3 and 57.7 -> 53.3 us; at V = 2 nothing)
+                    // (64 x (1024 x 256 x 256), 80 %, calls in a row on other inputs: 37.6 -> 36.1 us; 50 %, on the same: 57.7 -> 53.3; at V = 2 nothing)
                     constexpr int kAhead = kOverflowBatches;
                     int e0 = c_e0 + kStride * kFillBatches;
                     if (e0 - lane < c_e1) {

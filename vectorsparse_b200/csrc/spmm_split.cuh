@@ -18,7 +18,7 @@
 //
 // spmm_split_prepare writes A, zeros included, and B as three bf16 matrices each (scratch of 6 bytes per element), in the order in which
 // the tiles are read: a tile of a row-major matrix is 128-byte pieces kilobytes apart, and waiting for those took longer than multiplying
-// (4096 x 4096 x 256: 114 us of the product's 70).  The product is
+// (4096 x 4096 x 256: a product of 114 us, now 70).  The product is
 // a dense one in pairs of CTAs (tcgen05 cta_group::2) with the tiles and the protocol of spmm_pair.cuh: per stage of 64 columns six
 // times four 256 x 256 x 16 MMAs.  What it cannot do as well as the CUDA-core kernel, that kernel does behind it, from a
 // verdict: rows with few entries, and all of matrices too sparse, a column named twice in a vector-row, and numbers whose parts or products would leave the range of

@@ -1104,7 +1104,8 @@ template <int V> int launch_spmm_split(const SpmmParams &p, int64_t vectors, cud
     // at V = 1, 305 at V = 2, 301 at V = 4, 258 at V = 8 for 4096 x 4096 x 1024, 80 % sparse), or, where it takes the call otherwise, against that of the
     // kernel that stages tiles of B: per wave a start, the tiles, the entries of a vector-row (V = 8, 2048 x 4096 x 1024, 50 / 65 / 80 %
     // sparse: that kernel 228 / 165 / 103, this one 114 / 111 / 106; V = 1, 1024 x 1024 x 512: 54 / 41 / 29 and 38 / 37 / 36).  Below kMinDensity that kernel keeps every
-    // dense width, so that column shards of usual matrices (90 %, at V = 4 80 % sparse) have the bits of the whole product.
+    // dense width, so that column shards of usual matrices (90 %, at V = 4 80 % sparse) have the bits of the whole product; by cost the line would lie
+    // at 0.047 (V = 1) and 0.097 (V = 4) for 4096 x 4096 x 8192.
     constexpr double kCoresPs = V <= 2 ? 0.18 : V == 4 ? 0.35 : 0.6, kTileEntryUs = V == 1 ? 0.043 : V == 2 ? 0.047 : V == 4 ? 0.061 : 0.102, kMinDensity = V == 1 ? 0.102 : V == 2 ? 0.11 : V == 4 ? 0.205 : 0.13;
     // Nor does it take a matrix whose rows are about as short on average as those that the CUDA-core kernel computes behind it.
     q.few = forced ? 0 : splitspmm::few_entries(p.K);
