@@ -120,6 +120,138 @@ __global__ void __launch_bounds__(kCcThreads) spmm_cc_standby_kernel(const SpmmP
         spmm_cc_item<TIn, TOut, V, kChunks, kSlabs>(p, (int)(i / per), i % per, sizeof(TIn) == 4 && stands ? few : 0);
 }
 
+// The same sums for products that leave most of the GPU idle, where the threads above wait for one trip of gathers after another (72 x 205 x 48,
+// V = 8, 55 %: 41 us for 90 entries in a row, 8 here; what is left is one warp's latency, ~45 cycles an entry).  A warp takes a vector-row and 32 x kBytes bytes of its columns: the indices and values of 32 entries
+// come with one load per lane, 32 ahead, and are passed round through shared memory; the rows of B of kAhead entries are on their way while those of
+// the kAhead before are multiplied.  kBytes = 4 spreads a narrow product over four times the warps.  Entries in list order, as above: the same bits.
+constexpr int kFewThreads = 128, kFewWarps = kFewThreads / 32;
+template <typename T, int kBytes> struct Piece;   // kBytes of T as they lie in memory, widened on use
+template <> struct Piece<float, 16> {
+    static constexpr int kElems = 4;
+    float4 raw;
+    __device__ __forceinline__ void load(const float *p) { asm volatile("ld.global.nc.v4.f32 {%0,%1,%2,%3}, [%4];" : "=f"(raw.x), "=f"(raw.y), "=f"(raw.z), "=f"(raw.w) : "l"(p)); }
+    __device__ __forceinline__ void widen(float (&f)[4]) const { f[0] = raw.x; f[1] = raw.y; f[2] = raw.z; f[3] = raw.w; }
+};
+template <> struct Piece<float, 4> {
+    static constexpr int kElems = 1;
+    float raw;
+    __device__ __forceinline__ void load(const float *p) { raw = __ldg(p); }
+    __device__ __forceinline__ void widen(float (&f)[1]) const { f[0] = raw; }
+};
+template <> struct Piece<__half, 16> {
+    static constexpr int kElems = 8;
+    uint4 raw;
+    __device__ __forceinline__ void load(const __half *p) { asm volatile("ld.global.nc.v4.b32 {%0,%1,%2,%3}, [%4];" : "=r"(raw.x), "=r"(raw.y), "=r"(raw.z), "=r"(raw.w) : "l"(p)); }
+    __device__ __forceinline__ void widen(float (&f)[8]) const {
+        const __half2 *h = reinterpret_cast<const __half2 *>(&raw);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float2 t = __half22float2(h[i]);
+            f[2 * i] = t.x;
+            f[2 * i + 1] = t.y;
+        }
+    }
+};
+template <> struct Piece<__half, 4> {
+    static constexpr int kElems = 2;
+    __half2 raw;
+    __device__ __forceinline__ void load(const __half *p) { raw = __ldg(reinterpret_cast<const __half2 *>(p)); }
+    __device__ __forceinline__ void widen(float (&f)[2]) const {
+        const float2 t = __half22float2(raw);
+        f[0] = t.x;
+        f[1] = t.y;
+    }
+};
+template <typename TIn, typename TOut, int V, int kBytes>
+__global__ void __launch_bounds__(kFewThreads) spmm_cc_few_kernel(const SpmmParams p, int pieces) {
+    using B = Piece<TIn, kBytes>;
+    constexpr int E = B::kElems, kAhead = kBytes == 4 ? 16 : 8;
+    __shared__ __align__(16) float s_val[kFewWarps][2][32][V];
+    __shared__ int s_col[kFewWarps][2][32];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int64_t item = (int64_t)blockIdx.x * kFewWarps + warp;
+    if (item >= (int64_t)p.m_vec * pieces) return;
+    const int row = __ldg(p.row_indices + (int)(item / pieces)), b = blockIdx.y;
+    const int n = ((int)(item % pieces) * 32 + lane) * E;
+    const bool stored = n < p.N;   // lanes past the last column take part with the columns of the first lane
+    const TIn *values = static_cast<const TIn *>(p.values) + (int64_t)b * p.stride_values;
+    const TIn *rhs = static_cast<const TIn *>(p.rhs) + (int64_t)b * p.stride_rhs + (stored ? n : (int)(item % pieces) * 32 * E);
+
+    int j = __ldg(p.row_offsets + row);
+    const int end = __ldg(p.row_offsets + row + 1);
+    int col = 0;
+    float val[V];
+    auto fetch = [&](int at) {   // the lane's entry of the 32 from `at`; past the end the last one again, whose row of B is read and not used
+        const int from = min(at + lane, end - 1);
+        col = __ldg(p.col_indices + from);
+        VecLoad<TIn, V>::load(values + (int64_t)from * V, val);
+    };
+    auto stage = [&](int place) {
+        s_col[warp][place][lane] = col;
+#pragma unroll
+        for (int v = 0; v < V; ++v) s_val[warp][place][lane][v] = val[v];
+    };
+    float acc[V][E];
+#pragma unroll
+    for (int v = 0; v < V; ++v)
+#pragma unroll
+        for (int e = 0; e < E; ++e) acc[v][e] = 0.f;
+    B x[2][kAhead];
+    // kAhead entries from the u0-th of the 32 in `place`; unconditional, a load under a condition is waited for at once
+    auto request = [&](B (&to)[kAhead], int place, int u0) {
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) to[u].load(rhs + (int64_t)s_col[warp][place][u0 + u] * p.N);
+    };
+    auto multiply = [&](const B (&from)[kAhead], int place, int u0, int count) {
+#pragma unroll
+        for (int u = 0; u < kAhead; ++u) {
+            if (u0 + u < count) {
+                float a[V], f[E];
+                from[u].widen(f);
+#pragma unroll
+                for (int v = 0; v < V; ++v) a[v] = s_val[warp][place][u0 + u][v];
+#pragma unroll
+                for (int v = 0; v < V; ++v)
+#pragma unroll
+                    for (int e = 0; e < E; ++e) acc[v][e] = fmaf(a[v], f[e], acc[v][e]);
+            }
+        }
+    };
+    if (j < end) {
+        fetch(j);
+        stage(0);
+        __syncwarp();
+        fetch(j + 32);
+        request(x[0], 0, 0);
+    }
+    for (int place = 0; j < end; j += 32, place ^= 1) {
+        const int count = end - j;   // of the entries from here on
+        stage(place ^ 1);
+        __syncwarp();
+        fetch(j + 64);
+#pragma unroll
+        for (int u0 = 0; u0 < 32; u0 += kAhead) {
+            const int i = u0 / kAhead & 1;
+            if (u0 + kAhead < 32) request(x[i ^ 1], place, u0 + kAhead);
+            else request(x[i ^ 1], place ^ 1, 0);
+            multiply(x[i], place, u0, count);
+        }
+        __syncwarp();
+    }
+    if (!stored) return;
+    TOut *out = static_cast<TOut *>(p.out) + (int64_t)b * p.stride_out + n;
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        TOut *to = out + ((int64_t)row * V + v) * p.N;
+        if constexpr (E >= 4) {
+            store_chunk(to, acc[v]);
+        } else {
+#pragma unroll
+            for (int e = 0; e < E; ++e) store_scalar(to + e, acc[v][e]);
+        }
+    }
+}
+
 // ---- SDDMM --------------------------------------------------------------------------------------------------
 // Eight lanes share one mask entry j: lane g takes the 16-byte chunks g, g+8, ... of the contraction, keeps V
 // partial sums (one per real row of the vector), and the eight partials are folded with three xor-shuffles.

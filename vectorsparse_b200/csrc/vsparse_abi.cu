@@ -508,7 +508,7 @@ int64_t spmm_cc_tile_ctas(const SpmmParams &p) {
 // and a few entries per vector-row it lost, 5.5 against 4.3 us).  With two waves it still wins where the other kernel is
 // left with under eight warps per SM (1024 x 1024 x 1024 at V = 2, 50 / 90 / 98 % sparse: 60 / 23 / 12.5 against 131 / 39 / 12.5 us), and
 // loses where that has more (2048 x 512 x 256 at V = 1: 31 / 12.6 / 8.5 against 29 / 11.5 / 6.4).
-// VSPARSE_B200_SPMM_CC=rows|tiles chooses one.
+// VSPARSE_B200_SPMM_CC=rows|tiles|few chooses one.
 bool spmm_cc_tiles_chosen(int V, const SpmmParams &p, const DeviceInfo *d) {
     if (p.K < 1 || p.K > 1 << 30) return false;   // tile coordinates and column sums in 32 bits
     const int64_t ctas = spmm_cc_tile_ctas(p);
@@ -518,6 +518,21 @@ bool spmm_cc_tiles_chosen(int V, const SpmmParams &p, const DeviceInfo *d) {
     if (e && !std::strcmp(e, "tiles")) return true;
     const int64_t threads = (int64_t)p.m_vec * (p.N / 4) / spmm_cc_chunks(4 * V, 4, p.N) * p.batch;
     return p.K >= 128 && (ctas <= d->sm_count || (ctas <= 2 * d->sm_count && threads <= (int64_t)d->sm_count * 256));
+}
+// Bytes of a lane's columns in spmm_cc_few_kernel, or 0 where the others are the quicker ones: up to 20 of its warps per SM of 4-byte lanes at any V; where
+// rows would go to spmm_cc_kernel (no `tiles`) up to 96 at V = 2, and at V = 1 16-byte lanes up to 28.  us, as before / 4-byte / 16-byte lanes, warps of the
+// latter: fp16, V = 1, 132 rows x 4400 x 64, 55 % (66) 320 / 49 / 137, V = 2, 313 x 1019 x 48, 67 % (118) 78 / 18.5 / 51; fp32, V = 2, 110 x 4142 x 208, 59 %
+// (220) 134 / 68 / 220, V = 8, 50 x 2520 x 1784, 82 % (700) 72 / 55 / 116, V = 4, 68 x 1805 x 1940, 76 % (1088) 46 / 47 / 107; V = 1, 2416 x 1272 x 216, 60 %
+// (4832) 115 / 109 / 70, 575 x 139 x 1432, 78 % (6900) 12.3 / 22.6 / 13.1; V = 2, 200 x 1350 x 2100, 62 % (3400) 130 / 97 / 100, 147 x 130 x 3360, 54 %
+// (3969) 20.5 / 22.5 / 17.5.  VSPARSE_B200_SPMM_CC=few chooses the 4-byte lanes.
+int spmm_cc_few_bytes(int V, int chunk_elems, const SpmmParams &p, bool tiles, const DeviceInfo *d) {
+    const char *e = std::getenv("VSPARSE_B200_SPMM_CC");
+    if (e) return !std::strcmp(e, "few") ? 4 : 0;
+    const int64_t rows = (int64_t)p.m_vec * p.batch;
+    if (rows * ((p.N + 8 * chunk_elems - 1) / (8 * chunk_elems)) <= 20 * (int64_t)d->sm_count) return 4;
+    const int64_t wide = rows * ((p.N + 32 * chunk_elems - 1) / (32 * chunk_elems));
+    if (tiles || wide > 28 * (int64_t)d->sm_count) return 0;
+    return V == 1 ? 16 : V == 2 && wide <= 24 * (int64_t)d->sm_count ? 4 : 0;
 }
 // Leaves *taken false where no tensor map can be made.
 template <int V> int launch_spmm_cc_tile(const SpmmParams &p, DeviceInfo *d, cudaStream_t s, bool *taken) {
@@ -539,7 +554,7 @@ int spmm_cc_tile(int V, const SpmmParams &p, cudaStream_t s, bool *taken) {
     DeviceInfo *d = nullptr;
     const int rc = device_info(&d);
     if (rc != VS_OK) return rc;
-    if (!spmm_cc_tiles_chosen(V, p, d)) return VS_OK;
+    if (!spmm_cc_tiles_chosen(V, p, d) || spmm_cc_few_bytes(V, 4, p, true, d)) return VS_OK;
     switch (V) {
         case 1: return launch_spmm_cc_tile<1>(p, d, s, taken);
         case 2: return launch_spmm_cc_tile<2>(p, d, s, taken);
@@ -568,8 +583,23 @@ template <typename TIn, typename TOut, int V, int kChunks> void launch_spmm_cc_a
     }
     spmm_cc_kernel<TIn, TOut, V, kChunks><<<grid, kCcThreads, 0, s>>>(p);
 }
+template <typename TIn, typename TOut, int V, int kBytes> int launch_spmm_cc_few(const SpmmParams &p, cudaStream_t s) {
+    const int pieces = (p.N + 32 * Piece<TIn, kBytes>::kElems - 1) / (32 * Piece<TIn, kBytes>::kElems);
+    const int64_t blocks = ((int64_t)p.m_vec * pieces + kFewWarps - 1) / kFewWarps;
+    if (blocks > 0x7fffffffll) return VS_ERR_SHAPE;
+    spmm_cc_few_kernel<TIn, TOut, V, kBytes><<<dim3((unsigned)blocks, (unsigned)p.batch), kFewThreads, 0, s>>>(p, pieces);
+    return (int)cudaGetLastError();
+}
 template <typename TIn, typename TOut, int V> int launch_spmm_cc(const SpmmParams &p, cudaStream_t s) {
     constexpr int E = Chunk<TIn>::kElems;
+    DeviceInfo *d = nullptr;
+    const int rc = device_info(&d);
+    if (rc != VS_OK) return rc;
+    const int few = spmm_cc_few_bytes(V, E, p, false, d);
+    if (few == 4) return launch_spmm_cc_few<TIn, TOut, V, 4>(p, s);
+    if constexpr (V == 1) {
+        if (few == 16) return launch_spmm_cc_few<TIn, TOut, V, 16>(p, s);
+    }
     const int want = spmm_cc_chunks(V * E, E, p.N);
     const int64_t items = (int64_t)p.m_vec * (p.N / E) / want;
     const int64_t blocks = (items + kCcThreads - 1) / kCcThreads;
