@@ -14,10 +14,13 @@
 // Sampling.  The V rows of a vector-row are V CONSECUTIVE tensor-memory columns, so after a 32-column load lane c
 // holds, for each of the 32 / V vector-rows the load covers, exactly the V outputs of mask entry (vector-row, c) in
 // the order they have in memory: a lane that has such an entry writes them with one vector store.  Whether it has,
-// and which entry index j it is, comes from a column view of the mask that the plan kernel builds: per (block of 32
-// vector-rows, mask column) a 32-bit presence mask and the position of the cell's first entry in a list of entry
-// indices ordered by (block, column, vector-row).  No shared-memory boxes, no dynamic register indexing, nothing
-// outside the mask is ever stored, so non-finite products elsewhere in the tile cannot leak.  A presence bit holds
+// and which entry index j it is, comes from the mask as bits that the plan kernel lays out: per (vector-row, 32 columns) a word
+// with a bit for each column it names and the index of the first of them.  A warp samples 32 neighbouring columns, so a word
+// serves all its lanes, and j is that index plus the set bits below the lane's.  (Before, a lane looked up a word per (32 vector-rows, column)
+// and then the index of each entry in a list ordered by column, which the plan had to make: 137 -> 132 us at 256 x (2048 x 512), k = 256, V = 8,
+// 90 % sparse; 146 x (1008 x 1361), k = 128, V = 4 82 -> 78.)  Finding the entries ahead of the accumulator and without branches counts: by shuffles
+// between the stores 88 us in the latter, with a branch for each 100, from shared memory 94.  No shared-memory boxes, no dynamic register indexing, nothing
+// outside the mask is ever stored, so non-finite products elsewhere in the tile cannot leak.  A bit holds
 // one entry: when the same column appears twice in a vector-row the plan kernel says so and a fix-up kernel copies
 // the written entry's outputs to its twins (their values are equal by definition).
 //
@@ -38,8 +41,7 @@
 //
 // Organisation per CTA (both CTAs of a pair run the same roles on their own halves):
 //   warps 0-15  sampling epilogue: warp (quarter, part) owns accumulator lanes 32 quarter .. (32 mask columns) and
-//               tensor-memory columns 64 part .. + 63 (64 rows of lhs); cells are fetched two work items ahead, entry
-//               indices one
+//               tensor-memory columns 64 part .. + 63 (64 rows of lhs); words are fetched one work item ahead
 //   warp 16     one thread issuing the CTA's loads.  They are cta_group::2 loads: the tile lands in the issuing CTA, the
 //               bytes are counted on the FIRST CTA's barrier, which that CTA's loader arms with the bytes of both
 //   warp 17     first CTA: the MMA-issuing thread of the pair (idle in the second); its commits arrive on the barriers of
@@ -72,8 +74,8 @@ constexpr int kMmaWarp = kLoadWarp + 1;
 constexpr int kThreads = (kMmaWarp + 1) * 32;             // 576
 constexpr int kOperandBytes = kCtaRows * kBlockK * 2;     // 16 KiB: 128 rows of either operand, 64 contraction elements
 constexpr int kTmemCols = 2 * kTile;                      // two accumulator buffers
-constexpr int kBlockVecRows = 32;                         // vector-rows per presence mask
-constexpr int kPlanThreads = 1024;
+constexpr int kPlanWarps = 8, kPlanThreads = 32 * kPlanWarps;
+constexpr int kTwinThreads = 1024;
 constexpr int kMaxPlanColumns = 8192;                     // mask widths the plan kernel holds in shared memory
 constexpr int kSleepLoad = 32, kSleepMma = 0, kSleepEpilogue = 32;
 
@@ -87,7 +89,7 @@ struct Smem {  // offsets from the 1024-byte aligned base; identical in both CTA
     static constexpr int kAbort = kTmemHolder + 8;
     static constexpr int kTotal = kAbort + 8;
 };
-constexpr int kSmemBytes = Smem::kTotal + 1024;
+constexpr int kSmemBytes = Smem::kTotal;   // the dynamic segment is 1024-byte aligned (nothing static lies ahead of it)
 static_assert(kSmemBytes <= 227 * 1024, "shared memory budget");
 
 // The work items of one pair, as (batch entry, row tile of lhs, column tile of the mask).  With a resident rhs: a
@@ -120,134 +122,144 @@ struct ItemWalk {
 };
 
 // ---- plan -------------------------------------------------------------------------------------------------
-// One CTA per block of 32 vector-rows.  cells[block * n + c] = (presence mask over the block's vector-rows of an
-// entry in column c, position in `order` of the cell's first entry); order[] lists entry indices j by (block,
-// column, vector-row).  The entries of a block are one contiguous range of j, so a block's cells start at the
-// block's first j.  Columns outside [0, n) are dropped: their outputs are not written.  *twins is set when a
-// vector-row names a column twice (only one of the two reaches `order`).
+// The mask as bits: words[row * ceil(n / 32) + w] = (a bit per column 32 w .. 32 w + 31 that the vector-row names, the index of the first such
+// entry).  Where a vector-row's columns ascend, entry number r of the row is its r-th set bit, and that is all; the others (columns in another
+// order, named twice, or outside [0, n), which are dropped: their outputs are not written) have bit 31 of the index set, and the entry
+// itself stands in `order` at that index.  twins[CTA] is set where a vector-row names a column twice (only one of the two reaches `order`).
+//
+// kShare warps take a vector-row together, so the plan takes the whole GPU.  The form before, a CTA per 32 vector-rows that ordered their entries by
+// column, took 1.1 ns an entry of such a block: 80 us for 824 vector-rows of 1920 entries, 62 for 267 of 1520 skewed ones; now 10.5 and 6.4, of which 4 are a
+// launch by itself.  Lanes that first put the bits of a word together, by shuffles or by a match, take longer than atomics that wait for each other.
+template <int kShare>
 __global__ void __launch_bounds__(kPlanThreads)
 sddmm_cell_plan_kernel(const int32_t *__restrict__ row_offsets, const int32_t *__restrict__ col_indices, int m_vec, int n, int nnz_vec,
-                       uint2 *__restrict__ cells, int32_t *__restrict__ order, int32_t *__restrict__ twins) {
-    extern __shared__ uint32_t cell_sh[];   // [n] masks, then [n] positions
-    __shared__ int32_t offs[kBlockVecRows + 1];
-    __shared__ int32_t part_sum[32];
+                       uint2 *__restrict__ words, int32_t *__restrict__ order, int32_t *__restrict__ twins) {
+    static_assert(kShare == 1 || kShare == kPlanWarps, "a warp or the CTA");
+    extern __shared__ uint32_t plan_sh[];   // per vector-row: bits, then positions
+    __shared__ int warp_sum[kPlanWarps];
     pdl_launch_dependents();   // the multiplying kernel may set itself up while the plan is made
-    uint32_t *mask = cell_sh, *first = cell_sh + n;
-    const int t = threadIdx.x, blk = blockIdx.x, vr0 = blk * kBlockVecRows;
-    const int rows = min(kBlockVecRows, m_vec - vr0);
-    if (blk == 0 && t == 0) *twins = 0;
-    // the scratch holds nnz_vec entries (the caller's count): offsets that claim more are cut there
-    if (t <= kBlockVecRows) offs[t] = min(max(__ldg(row_offsets + vr0 + min(t, rows)), 0), nnz_vec);
-    for (int c = t; c < n; c += kPlanThreads) mask[c] = 0u;
-    __syncthreads();
-    const int j0 = offs[0], j1 = max(offs[rows], j0);
-    auto row_of = [&](int j) {   // the vector-row (0 .. rows - 1) whose range holds j
-        int lo = 0, hi = rows;
-        while (hi - lo > 1) {
-            const int mid = (lo + hi) >> 1;
-            if (offs[mid] <= j) lo = mid; else hi = mid;
-        }
-        return lo;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, n_words = (n + 31) / 32;
+    const int w0 = kShare == 1 ? 0 : warp, slot = kShare == 1 ? warp : 0;
+    uint32_t *bits = plan_sh + slot * 2 * n_words, *first = bits + n_words;
+    auto sync = [&]() {
+        if constexpr (kShare == 1) __syncwarp();
+        else __syncthreads();
     };
+    pdl_wait();
     bool twin = false;
-    for (int jb = j0 + t; jb < j1; jb += 4 * kPlanThreads) {   // four entries per thread and trip: their loads fly together
-        int c[4];
+    for (int row = blockIdx.x * (kPlanWarps / kShare) + slot; row < m_vec; row += gridDim.x * (kPlanWarps / kShare)) {
+        // the scratch holds nnz_vec entries (the caller's count): offsets that claim more are cut there
+        const int beg = min(max(__ldg(row_offsets + row), 0), nnz_vec), end = min(max(__ldg(row_offsets + row + 1), beg), nnz_vec);
+        for (int w = w0 * 32 + lane; w < n_words; w += 32 * kShare) bits[w] = 0u;
+        sync();
+        constexpr int kAhead = kShare == 1 ? 8 : 4;   // entries per lane whose loads fly together
+        bool plain = true;
+        for (int j0 = beg + w0 * 32 * kAhead; j0 < end; j0 += 32 * kAhead * kShare) {
+            int c[kAhead], before = j0 > beg ? __ldg(col_indices + j0 - 1) : -1;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) c[u] = jb + u * kPlanThreads < j1 ? __ldg(col_indices + jb + u * kPlanThreads) : -1;
+            for (int u = 0; u < kAhead; ++u) c[u] = __ldg(col_indices + min(j0 + 32 * u + lane, end - 1));
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            if ((unsigned)c[u] >= (unsigned)n) continue;
-            const uint32_t bit = 1u << row_of(jb + u * kPlanThreads);
-            twin |= (atomicOr(mask + c[u], bit) & bit) != 0u;
+            for (int u = 0; u < kAhead; ++u) {
+                int left = __shfl_up_sync(0xffffffffu, c[u], 1);
+                if (lane == 0) left = before;
+                before = __shfl_sync(0xffffffffu, c[u], 31);
+                if (j0 + 32 * u + lane < end) {
+                    plain = plain && c[u] > left && c[u] < n;
+                    if ((unsigned)c[u] < (unsigned)n) atomicOr(bits + (c[u] >> 5), 1u << (c[u] & 31));
+                }
+            }
         }
-    }
-    if (twin) atomicExch(twins, 1);
-    __syncthreads();
-    // exclusive scan of popc(mask[c]) over the columns: every thread sums a contiguous run, the runs are scanned with
-    // shuffles inside each warp and once more across the warps
-    const int per = (n + kPlanThreads - 1) / kPlanThreads;
-    const int c_lo = min(t * per, n), c_hi = min(c_lo + per, n);
-    int sum = 0;
-    for (int c = c_lo; c < c_hi; ++c) sum += __popc(mask[c]);
-    const int lane = t & 31, warp = t >> 5;
-    int incl = sum;
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const int up = __shfl_up_sync(0xffffffffu, incl, d);
-        if (lane >= d) incl += up;
-    }
-    if (lane == 31) part_sum[warp] = incl;
-    __syncthreads();
-    if (warp == 0) {
-        const int w_sum = lane < kPlanThreads / 32 ? part_sum[lane] : 0;
-        int w_incl = w_sum;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-            const int up = __shfl_up_sync(0xffffffffu, w_incl, d);
-            if (lane >= d) w_incl += up;
+        if constexpr (kShare == 1) {
+            plain = __all_sync(0xffffffffu, plain);
+            __syncwarp();
+        } else {
+            plain = __syncthreads_and(plain);
         }
-        if (lane < kPlanThreads / 32) part_sum[lane] = w_incl - w_sum;   // what the warps before this one hold
-    }
-    __syncthreads();
-    int run = j0 + part_sum[warp] + incl - sum;
-    uint2 *mine = cells + (int64_t)blk * n;
-    for (int c = c_lo; c < c_hi; ++c) {
-        first[c] = (uint32_t)run;
-        mine[c] = make_uint2(mask[c], (uint32_t)run);
-        run += __popc(mask[c]);
-    }
-    __syncthreads();
-    for (int jb = j0 + t; jb < j1; jb += 4 * kPlanThreads) {
-        int c[4];
+        int run = beg;
+        for (int x0 = 0; x0 < n_words; x0 += 32 * kShare) {
+            const int w = x0 + w0 * 32 + lane;
+            const uint32_t mine = w < n_words ? bits[w] : 0u;
+            int sum = __popc(mine);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) c[u] = jb + u * kPlanThreads < j1 ? __ldg(col_indices + jb + u * kPlanThreads) : -1;
+            for (int d = 1; d < 32; d <<= 1) {
+                const int up = __shfl_up_sync(0xffffffffu, sum, d);
+                if (lane >= d) sum += up;
+            }
+            int ahead = 0, total = __shfl_sync(0xffffffffu, sum, 31);
+            if constexpr (kShare > 1) {
+                if (lane == 0) warp_sum[warp] = total;
+                __syncthreads();
+                total = 0;
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-            if ((unsigned)c[u] >= (unsigned)n) continue;
-            const int j = jb + u * kPlanThreads;
-            const uint32_t below = (1u << row_of(j)) - 1u;
-            order[first[c[u]] + __popc(mask[c[u]] & below)] = j;   // twins write the same place: one of them stays
+                for (int x = 0; x < kShare; ++x) {
+                    if (x == warp) ahead = total;
+                    total += warp_sum[x];
+                }
+                __syncthreads();
+            }
+            if (w < n_words) {
+                const uint32_t at = (uint32_t)(run + ahead + sum - __popc(mine));
+                words[(int64_t)row * n_words + w] = make_uint2(mine, plain ? at : at | 0x80000000u);
+                first[w] = at;
+            }
+            run += total;
         }
+        sync();
+        if (!plain) {   // the same for all that share the row
+            int named = 0;   // entries with a column of the matrix; more than set bits where one is named twice
+            for (int j = beg + lane; j < end; j += 32) {
+                const int c = __ldg(col_indices + j);
+                if ((unsigned)c >= (unsigned)n) continue;
+                ++named;
+                if (w0 == 0) order[first[c >> 5] + __popc(bits[c >> 5] & ((1u << (c & 31)) - 1u))] = j;   // of twins one stays
+            }
+            twin = twin || (int)__reduce_add_sync(0xffffffffu, named) != run - beg;
+        }
+        sync();
     }
+    twin = __syncthreads_or(twin);
+    if (threadIdx.x == 0) twins[blockIdx.x] = twin;
 }
 
 // Runs behind the multiplying kernel; does nothing unless the plan kernel met a column twice in one vector-row.
 // Entry j whose place in `order` holds another entry j' is a twin of j': same vector-row, same column, same outputs.
 template <typename TOut, int V>
-__global__ void __launch_bounds__(kPlanThreads)
-sddmm_twin_kernel(const SddmmParams p, const uint2 *__restrict__ cells, const int32_t *__restrict__ order, const int32_t *__restrict__ twins) {
+__global__ void __launch_bounds__(kTwinThreads)
+sddmm_twin_kernel(const SddmmParams p, const uint2 *__restrict__ words, const int32_t *__restrict__ order, const int32_t *__restrict__ twins, int plan_ctas) {
     pdl_wait();
-    if (*twins == 0) return;
-    const int j = blockIdx.x * kPlanThreads + threadIdx.x;
-    if (j >= p.nnz_vec) return;
-    const int c = __ldg(p.col_indices + j);
-    if ((unsigned)c >= (unsigned)p.n) return;
-    int lo = 0, hi = p.m_vec;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (__ldg(p.row_offsets + mid) <= j) lo = mid; else hi = mid;
-    }
-    const uint2 cell = __ldg(cells + (int64_t)(lo / kBlockVecRows) * p.n + c);
-    const int other = __ldg(order + cell.y + __popc(cell.x & ((1u << (lo % kBlockVecRows)) - 1u)));
-    if (other == j) return;
-    for (int b = 0; b < p.batch; ++b) {
-        TOut *out = static_cast<TOut *>(p.out) + (int64_t)b * p.stride_out;
-        for (int v = 0; v < V; ++v) out[(int64_t)j * V + v] = out[(int64_t)other * V + v];
+    int any = 0;
+    for (int i = threadIdx.x; i < plan_ctas; i += kTwinThreads) any |= twins[i];
+    if (__syncthreads_or(any) == 0) return;
+    const int n_words = (p.n + 31) / 32;
+    for (int64_t j = (int64_t)blockIdx.x * kTwinThreads + threadIdx.x; j < p.nnz_vec; j += (int64_t)gridDim.x * kTwinThreads) {
+        const int c = __ldg(p.col_indices + j);
+        if ((unsigned)c >= (unsigned)p.n) continue;
+        int lo = 0, hi = p.m_vec;
+        while (hi - lo > 1) {
+            const int mid = (lo + hi) >> 1;
+            if (__ldg(p.row_offsets + mid) <= j) lo = mid; else hi = mid;
+        }
+        const uint2 word = __ldg(words + (int64_t)lo * n_words + (c >> 5));
+        if (!(word.y >> 31)) continue;
+        const int other = __ldg(order + (word.y & 0x7fffffffu) + __popc(word.x & ((1u << (c & 31)) - 1u)));
+        if (other == j) continue;
+        for (int b = 0; b < p.batch; ++b) {
+            TOut *out = static_cast<TOut *>(p.out) + (int64_t)b * p.stride_out;
+            for (int v = 0; v < V; ++v) out[(int64_t)j * V + v] = out[(int64_t)other * V + v];
+        }
     }
 }
 
 // map_lhs: {k, rows of lhs, batch}, map_rhs: {k, n, batch}; both box {64, 128, 1}, K-major with the 128-byte swizzle
-// and zero fill outside.  cells / order: see sddmm_cell_plan_kernel; blocks = number of 32-vector-row blocks.
+// and zero fill outside.  words / order: see sddmm_cell_plan_kernel.
 // resident: keep the rhs tiles of the current batch entry in shared memory (the host checks that they fit).
 template <typename TOut, int V>
 __global__ void __launch_bounds__(kThreads, 1)
 sddmm_pair_kernel(const SddmmParams p, const __grid_constant__ CUtensorMap map_lhs, const __grid_constant__ CUtensorMap map_rhs,
-                  const uint2 *__restrict__ cells, const int32_t *__restrict__ order, int blocks, int m_tiles, int n_tiles,
+                  const uint2 *__restrict__ words, const int32_t *__restrict__ order, int m_tiles, int n_tiles,
                   int resident, uint32_t *status) {
-    extern __shared__ uint8_t smem_raw[];
-    const uint32_t raw = tc::smem_u32(smem_raw);
-    const uint32_t base = (raw + 1023u) & ~1023u;   // the same offset in both CTAs: same kernel, same static layout
-    uint8_t *sm = smem_raw + (base - raw);
+    extern __shared__ __align__(1024) uint8_t sm[];
+    const uint32_t base = tc::smem_u32(sm);   // the same offset in both CTAs
 
     const int t = threadIdx.x;
     const int warp = t >> 5;
@@ -285,7 +297,7 @@ sddmm_pair_kernel(const SddmmParams p, const __grid_constant__ CUtensorMap map_l
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(sm + Smem::kTmemHolder);
 
     pdl_launch_dependents();
-    pdl_wait();   // the set-up above may have run beside the plan kernel; its cells are read from here on
+    pdl_wait();   // the set-up above may have run beside the plan kernel; its words are read from here on
     const int k_blocks = (p.k + kBlockK - 1) / kBlockK;   // the last one may be filled up with zeros by TMA
     const int64_t total_items = (int64_t)p.batch * n_tiles * m_tiles;
     // this pair's items: a contiguous run with a resident rhs, every pairs-th item otherwise
@@ -389,9 +401,11 @@ sddmm_pair_kernel(const SddmmParams p, const __grid_constant__ CUtensorMap map_l
         // =========================== sampling epilogue ===================================================
         // This lane's mask column is nt * 256 + 128 rank + 32 quarter + lane; the warp's 64 tensor-memory columns are
         // rows 64 part .. + 63 of the lhs tile = 64 / V vector-rows, read by two 32-column loads of 32 / V vector-rows
-        // each.  All of them lie in one block of 32 vector-rows, so the lane needs ONE cell per work item.
+        // each.  The warp's 32 mask columns are ONE word of each of those vector-rows: a lane fetches the word of vector-row `lane`
+        // (at V = 1 of `lane` + 32 too), an item ahead, and they are passed round when they are sampled.
         constexpr int kPerLoad = 32 / V;                 // vector-rows per 32-column load
-        constexpr bool kAheadEntries = 2 * kPerLoad <= 16;   // hold the next item's entry indices as well
+        constexpr int kHeld = 2 * kPerLoad > 32 ? 2 : 1; // words a lane holds
+        constexpr bool kAheadEntries = 2 * kPerLoad <= 16;   // the entries are found before the accumulator is waited for; at V <= 2 there are too many to hold
         constexpr int kElems = 16 / (int)sizeof(TOut);   // outputs per 16-byte store
         const int quarter = warp & 3, part = warp >> 2;
         const uint32_t lane_taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(part * 64);
@@ -400,56 +414,59 @@ sddmm_pair_kernel(const SddmmParams p, const __grid_constant__ CUtensorMap map_l
             tc::mbar_arrive_remote(acc_empty_first);        // both accumulator buffers start out free
             tc::mbar_arrive_remote(acc_empty_first + 8);
         }
-        auto cell_of = [&](const ItemWalk &w, bool valid, int &bit0) -> uint2 {
-            const int c = w.nt() * kTile + (int)rank * kCtaRows + quarter * 32 + lane;
-            const int vr = (w.mt() * kTile + part * 64) / V;   // first vector-row this warp samples
-            const int blk = vr / kBlockVecRows;
-            bit0 = vr % kBlockVecRows;
-            return (valid && c < p.n && blk < blocks) ? __ldg(cells + (int64_t)blk * p.n + c) : make_uint2(0u, 0u);
-        };
-        // the entry indices a lane needs for an item: 2 * kPerLoad bits of its cell, in vector-row order
-        auto entries_of = [&](const uint2 cell, int bit0, uint32_t &bits, int (&ent)[2 * kPerLoad]) {
-            bits = (cell.x >> bit0) & (uint32_t)((1ull << (2 * kPerLoad)) - 1ull);
-            const int pos0 = (int)cell.y + __popc(cell.x & ((1u << bit0) - 1u));
+        const int n_words = (p.n + 31) / 32;
+        auto words_of = [&](const ItemWalk &w, bool valid, uint2 (&held)[kHeld]) {
+            const int cw = (w.nt() * kTile + (int)rank * kCtaRows) / 32 + quarter;
+            const int vr = (w.mt() * kTile + part * 64) / V + lane;   // first vector-row this warp samples + lane
 #pragma unroll
-            for (int b = 0; b < 2 * kPerLoad; ++b)
-                ent[b] = ((bits >> b) & 1u) ? __ldg(order + pos0 + __popc(bits & ((1u << b) - 1u))) : -1;
+            for (int i = 0; i < kHeld; ++i)
+                held[i] = valid && cw < n_words && lane < 2 * kPerLoad && vr + 32 * i < p.m_vec ? __ldg(words + (int64_t)(vr + 32 * i) * n_words + cw) : make_uint2(0u, 0u);
         };
-        ItemWalk walk, ahead;   // `walk`: the item being sampled; `ahead`: two items further on
+        ItemWalk walk, ahead;   // `walk`: the item being sampled; `ahead`: one item further on
         walk.init(item0, item_stride, m_tiles, n_tiles, resident != 0);
         ahead = walk;
-        int bit0, n_bit0, f_bit0;
-        uint32_t bits, n_bits;
-        int ent[2 * kPerLoad], n_ent[kAheadEntries ? 2 * kPerLoad : 1];
-        uint2 n_cell, f_cell;
-        {
-            const uint2 c_cell = cell_of(ahead, my_items > 0, bit0);
-            ahead.next();
-            n_cell = cell_of(ahead, my_items > 1, n_bit0);
-            entries_of(c_cell, bit0, bits, ent);
-        }
+        uint2 held[kHeld], next[kHeld];
+        words_of(ahead, my_items > 0, held);
         bool ok_run = true;
         for (uint32_t i = 0; i < my_items && ok_run; ++i, walk.next()) {
             const uint32_t buf = i & 1u;
-            // requested now: the cell of item i + 2 and the entry indices of item i + 1 (its cell was requested an item ago);
-            // at V = 2 a lane may have 32 entries per item, too many to hold for two items: they are fetched when needed
             ahead.next();
-            f_cell = cell_of(ahead, i + 2 < my_items, f_bit0);
-            if constexpr (kAheadEntries) entries_of(n_cell, n_bit0, n_bits, n_ent);
-
+            words_of(ahead, i + 1 < my_items, next);
+            // entries named in `order`: rare, and the same for the whole warp
+            bool listed = false;
+#pragma unroll
+            for (int x = 0; x < kHeld; ++x) listed = listed || __any_sync(0xffffffffu, held[x].y >> 31);
+            auto entry_of = [&](uint32_t bits, uint32_t first) -> int {   // the lane's entry in a word, or -1; no branches, which the lanes would take one by one
+                const int j = (int)((first & 0x7fffffffu) + __popc(bits & ((1u << lane) - 1u)));
+                return bits >> lane & 1u ? j : -1;
+            };
+            int ent[kAheadEntries ? 2 * kPerLoad : 1];
+            if constexpr (kAheadEntries) {
+#pragma unroll
+                for (int b = 0; b < 2 * kPerLoad; ++b) ent[b] = entry_of(__shfl_sync(0xffffffffu, held[0].x, b), __shfl_sync(0xffffffffu, held[0].y, b));
+                if (listed) {
+#pragma unroll
+                    for (int b = 0; b < 2 * kPerLoad; ++b)
+                        if (__shfl_sync(0xffffffffu, held[0].y, b) >> 31 && ent[b] >= 0) ent[b] = __ldg(order + ent[b]);
+                }
+            }
             ok_run = __all_sync(0xffffffffu, wait_or_abort<kSleepEpilogue>(bar_acc_full + 8 * buf, (i >> 1) & 1u, abort_flag, abort_addr, peer));
             if (!ok_run) break;
             tc::tc_fence_after_sync();
             TOut *out = static_cast<TOut *>(p.out) + (int64_t)walk.b * p.stride_out;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                const uint32_t sub = (bits >> (h * kPerLoad)) & (uint32_t)((1u << kPerLoad) - 1u);
-                if (!__any_sync(0xffffffffu, sub != 0u)) continue;   // warp-uniform: nobody has an entry in these 32 rows
+                const uint2 half = held[kHeld == 2 ? h : 0];
+                const int row0 = kHeld == 2 ? 0 : h * kPerLoad;   // the lane that holds the half's first word
+                if (!__any_sync(0xffffffffu, half.x != 0u && lane >= row0 && lane < row0 + kPerLoad)) continue;   // no entry in these 32 rows
                 uint32_t r[32];
                 tc::tmem_ld_x32(lane_taddr + buf * kTile + (uint32_t)(h * 32), r);
 #pragma unroll
                 for (int b = 0; b < kPerLoad; ++b) {
-                    const int j = ent[h * kPerLoad + b];
+                    int j;
+                    if constexpr (kAheadEntries) j = ent[h * kPerLoad + b];
+                    else j = entry_of(__shfl_sync(0xffffffffu, half.x, row0 + b), __shfl_sync(0xffffffffu, half.y, row0 + b));
+                    if (!kAheadEntries && listed && __shfl_sync(0xffffffffu, half.y, row0 + b) >> 31 && j >= 0) j = __ldg(order + j);
                     if (j < 0) continue;
                     TOut *dst = out + (int64_t)j * V;
                     if constexpr (sizeof(TOut) == 2) {
@@ -466,16 +483,20 @@ sddmm_pair_kernel(const SddmmParams p, const __grid_constant__ CUtensorMap map_l
                             hh[0] = __floats2half2_rn(__uint_as_float(r[b * V]), __uint_as_float(r[b * V + 1]));
                             hh[1] = __floats2half2_rn(__uint_as_float(r[b * V + 2]), __uint_as_float(r[b * V + 3]));
                             *reinterpret_cast<uint2 *>(dst) = o;
-                        } else {
+                        } else if constexpr (V == 2) {
                             *reinterpret_cast<__half2 *>(dst) = __floats2half2_rn(__uint_as_float(r[b * V]), __uint_as_float(r[b * V + 1]));
+                        } else {
+                            *dst = __float2half_rn(__uint_as_float(r[b]));
                         }
                     } else {
                         if constexpr (V >= 4) {
 #pragma unroll
                             for (int e = 0; e < V / kElems; ++e)
                                 reinterpret_cast<uint4 *>(dst)[e] = make_uint4(r[b * V + 4 * e], r[b * V + 4 * e + 1], r[b * V + 4 * e + 2], r[b * V + 4 * e + 3]);
-                        } else {
+                        } else if constexpr (V == 2) {
                             *reinterpret_cast<uint2 *>(dst) = make_uint2(r[b * V], r[b * V + 1]);
+                        } else {
+                            *reinterpret_cast<uint32_t *>(dst) = r[b];
                         }
                     }
                 }
@@ -483,14 +504,8 @@ sddmm_pair_kernel(const SddmmParams p, const __grid_constant__ CUtensorMap map_l
             tc::tc_fence_before_sync();
             __syncwarp();
             if (lane == 0) tc::mbar_arrive_remote(acc_empty_first + 8 * buf);   // sampled: the buffer is free for the pair
-            if constexpr (kAheadEntries) {
-                bits = n_bits;
 #pragma unroll
-                for (int b = 0; b < 2 * kPerLoad; ++b) ent[b] = n_ent[b];
-            } else {
-                entries_of(n_cell, n_bit0, bits, ent);
-            }
-            n_cell = f_cell; n_bit0 = f_bit0;
+            for (int x = 0; x < kHeld; ++x) held[x] = next[x];
         }
     }
 

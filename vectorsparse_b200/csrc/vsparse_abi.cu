@@ -1276,37 +1276,20 @@ template <typename TOut, int V> int launch_sddmm_gather(const SddmmParams &p, cu
     return (int)cudaGetLastError();
 }
 
-// Which tensor-core SDDMM runs: dense tiles of lhs . rhs^T sampled at the mask cost the same whatever the sparsity,
-// the gather kernel a fixed amount per vector-row plus a little per mask entry.  The number of entries is an argument
-// here, so the choice is made on the host, in SM-cycles per product, fitted to measurements on B200 (lhs 2048 x 256,
-// rhs 512 x 256, 90 % and 98 % sparse; 4096 x 4096 masks of 410 entries per row at k = 64): gather ~306 per vector-row
-// and 64 contraction elements + ~4 per entry; dense ~2230 per 256 x 256 tile and 64 contraction elements over the two
-// SMs of a pair, and not less than ~4250 per tile (reading the accumulator out).
-// VSPARSE_B200_SDDMM = "dense" | "gather" (read at every call) forces one.
-bool sddmm_use_dense(const SddmmParams &p, int V) {
-    const char *e = std::getenv("VSPARSE_B200_SDDMM");
-    if (e && !std::strcmp(e, "dense")) return true;
-    if (e && !std::strcmp(e, "gather")) return false;
-    const double k_blocks = std::ceil((double)p.k / densesddmm::kBlockK);
-    const double tiles = std::ceil((double)p.m_vec * V / 256.0) * std::ceil((double)p.n / 256.0);
-    const double gather = (double)p.m_vec * 306.0 * k_blocks + (double)p.nnz_vec * 4.0;
-    const double dense = tiles * std::max(2230.0 * k_blocks, 4250.0);
-    return dense * 1.1 < gather;
-}
-
 // The dense SDDMM by pairs of CTAs (sddmm_pair.cuh) serves masks of up to pairsddmm::kMaxPlanColumns columns whose
 // outputs can be written with vector stores; VSPARSE_B200_SDDMM_PAIR=0 keeps the single-CTA kernel.
 inline bool sddmm_pair_enabled() {
     const char *e = std::getenv("VSPARSE_B200_SDDMM_PAIR");
     return !(e && !std::strcmp(e, "0"));
 }
-// Scratch of the pair kernel's plan: cells, entry order, the twins flag.
-int64_t sddmm_pair_plan_bytes(int m_vec, int n, int nnz_vec, int64_t *cells_out, int64_t *order_out) {
-    const int64_t blocks = (m_vec + pairsddmm::kBlockVecRows - 1) / pairsddmm::kBlockVecRows;
-    const int64_t cells_bytes = (blocks * n * 8 + 15) & ~15ll, order_bytes = ((int64_t)nnz_vec * 4 + 15) & ~15ll;
-    if (cells_out) *cells_out = cells_bytes;
+// Scratch of the pair kernel's plan: words, entry order, a twins flag per CTA of the plan.
+constexpr int kCellPlanCtas = 1024;
+inline int sddmm_cell_plan_ctas(int m_vec) { return std::min((m_vec + pairsddmm::kPlanWarps - 1) / pairsddmm::kPlanWarps, kCellPlanCtas); }
+int64_t sddmm_pair_plan_bytes(int m_vec, int n, int nnz_vec, int64_t *words_out, int64_t *order_out) {
+    const int64_t words_bytes = ((int64_t)m_vec * ((n + 31) / 32) * 8 + 15) & ~15ll, order_bytes = ((int64_t)nnz_vec * 4 + 15) & ~15ll;
+    if (words_out) *words_out = words_bytes;
     if (order_out) *order_out = order_bytes;
-    return cells_bytes + order_bytes + 16;
+    return words_bytes + order_bytes + 4 * (int64_t)std::min(m_vec, kCellPlanCtas);
 }
 // Plan, multiplying kernel and the fix-up for repeated columns; false if this call or this device cannot take them
 // (nothing has been enqueued then).
@@ -1316,17 +1299,12 @@ template <typename TOut, int V> bool launch_sddmm_pair(const SddmmParams &p, cud
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDevices) return false;
     if (resident[dev] == 0) {
-        if (set_smem(kernel, pairsddmm::kSmemBytes) != VS_OK ||
-            set_smem(pairsddmm::sddmm_cell_plan_kernel, 8 * pairsddmm::kMaxPlanColumns) != VS_OK) {
-            resident[dev] = -1;
-        } else {
-            const int n = max_resident_pairs(kernel, pairsddmm::kThreads, pairsddmm::kSmemBytes, d);
-            resident[dev] = n > 0 ? n : -1;
-        }
+        const int n = set_smem(kernel, pairsddmm::kSmemBytes) == VS_OK ? max_resident_pairs(kernel, pairsddmm::kThreads, pairsddmm::kSmemBytes, d) : 0;
+        resident[dev] = n > 0 ? n : -1;
     }
     if (resident[dev] < 0) return false;
-    int64_t cells_bytes = 0, order_bytes = 0;
-    const int64_t plan_bytes = sddmm_pair_plan_bytes(p.m_vec, p.n, p.nnz_vec, &cells_bytes, &order_bytes);
+    int64_t words_bytes = 0, order_bytes = 0;
+    const int64_t plan_bytes = sddmm_pair_plan_bytes(p.m_vec, p.n, p.nnz_vec, &words_bytes, &order_bytes);
     if (p.n > pairsddmm::kMaxPlanColumns || plan_bytes > kMaxPlanBytes || !aligned16(p.out) ||
         (p.batch > 1 && (p.stride_out * sizeof(TOut)) % 16 != 0))
         return false;
@@ -1339,13 +1317,15 @@ template <typename TOut, int V> bool launch_sddmm_pair(const SddmmParams &p, cud
     uint8_t *plan = nullptr;
     PlanScratch scratch;
     if (scratch.take(d, s, (size_t)plan_bytes, reinterpret_cast<void **>(&plan)) != VS_OK) return false;
-    uint2 *cells = reinterpret_cast<uint2 *>(plan);
-    int32_t *order = reinterpret_cast<int32_t *>(plan + cells_bytes);
-    int32_t *twins = reinterpret_cast<int32_t *>(plan + cells_bytes + order_bytes);
-    const int blocks = (p.m_vec + pairsddmm::kBlockVecRows - 1) / pairsddmm::kBlockVecRows;
-    pairsddmm::sddmm_cell_plan_kernel<<<blocks, pairsddmm::kPlanThreads, (size_t)8 * p.n, s>>>(p.row_offsets, p.col_indices, p.m_vec, p.n,
-                                                                                              p.nnz_vec, cells, order, twins);
-    int rc = (int)cudaGetLastError();
+    uint2 *words = reinterpret_cast<uint2 *>(plan);
+    int32_t *order = reinterpret_cast<int32_t *>(plan + words_bytes);
+    int32_t *twins = reinterpret_cast<int32_t *>(plan + words_bytes + order_bytes);
+    // a CTA per vector-row where the rows are long, a warp, whose 32 entries take 0.3 us, where they are short: 53 skewed rows of 960 entries 22 us / 5.5, 252 of
+    // 229 9.0 / 4.4; 256 of 51 4.5 with a warp
+    const bool shared_rows = (int64_t)p.nnz_vec > 192ll * p.m_vec;
+    const int plan_ctas = shared_rows ? std::min(p.m_vec, kCellPlanCtas) : sddmm_cell_plan_ctas(p.m_vec);
+    int rc = (int)launch_overlapped(shared_rows ? pairsddmm::sddmm_cell_plan_kernel<pairsddmm::kPlanWarps> : pairsddmm::sddmm_cell_plan_kernel<1>, (unsigned)plan_ctas, pairsddmm::kPlanThreads,
+                                    (size_t)(shared_rows ? 1 : pairsddmm::kPlanWarps) * ((p.n + 31) / 32) * 8, s, p.row_offsets, p.col_indices, p.m_vec, p.n, p.nnz_vec, words, order, twins);
     if (rc == VS_OK) {
         const int m_tiles = (p.m_vec * V + pairsddmm::kTile - 1) / pairsddmm::kTile;
         const int n_tiles = (p.n + pairsddmm::kTile - 1) / pairsddmm::kTile;
@@ -1355,12 +1335,12 @@ template <typename TOut, int V> bool launch_sddmm_pair(const SddmmParams &p, cud
         const char *res_env = std::getenv("VSPARSE_B200_SDDMM_RESIDENT");
         const int resident = (n_tiles * ((p.k + densesddmm::kBlockK - 1) / densesddmm::kBlockK) <= pairsddmm::kMaxResident && !(res_env && !std::strcmp(res_env, "0"))) ? 1 : 0;
         TimedLaunch timed(s);
-        rc = (int)launch_pairs(kernel, pairs, pairsddmm::kThreads, (size_t)pairsddmm::kSmemBytes, s, true, p, map_l, map_r, cells, order,
-                               blocks, m_tiles, n_tiles, resident, d->status);
+        rc = (int)launch_pairs(kernel, pairs, pairsddmm::kThreads, (size_t)pairsddmm::kSmemBytes, s, true, p, map_l, map_r, (const uint2 *)words, (const int32_t *)order,
+                               m_tiles, n_tiles, resident, d->status);
     }
     if (rc == VS_OK)
-        rc = (int)launch_overlapped(pairsddmm::sddmm_twin_kernel<TOut, V>, (unsigned)((p.nnz_vec + pairsddmm::kPlanThreads - 1) / pairsddmm::kPlanThreads),
-                                    pairsddmm::kPlanThreads, 0, s, p, cells, order, twins);
+        rc = (int)launch_overlapped(pairsddmm::sddmm_twin_kernel<TOut, V>, (unsigned)std::min<int64_t>((p.nnz_vec + pairsddmm::kTwinThreads - 1) / pairsddmm::kTwinThreads, d->sm_count),
+                                    pairsddmm::kTwinThreads, 0, s, p, (const uint2 *)words, (const int32_t *)order, (const int32_t *)twins, plan_ctas);
     *rc_out = rc;
     return true;
 }
@@ -1385,24 +1365,35 @@ template <typename TOut, int V> bool launch_sddmm_direct(const SddmmParams &p, c
                                      n_tiles, d->status);
     return true;
 }
-// Time each form of a sampled product takes (us, fitted to B200 at V = 1 to 8, 64 to 4096 rows and columns, contraction
-// lengths 64 to 1984, batches of 1 to 64).  Direct: waves of 128 x 128 tiles at two per SM, each paying for its contraction
-// (three times as much per block once both CTAs of an SM draw on L2) and for looking at every entry of its rows.  Dense:
-// the launches, the plan of 32 vector-rows per CTA, the tiles.  Gather: by the costs sddmm_use_dense() knows.
+// Time each form of a sampled product takes, us.  Direct: waves of 128 x 128 tiles at two per SM, each paying for its contraction (three times as much per
+// block once both CTAs of an SM draw on L2) and for looking at every entry of its rows.  Dense: the launches, waves of 256 x 256 tiles, each the longer of its
+// contraction and its sampling; the single-CTA kernel of wide masks takes 1.4 times as long.  Gather: rounds of a vector-row per CTA at two per SM, each entry
+// by itself for every 64 contraction elements.  Fitted to 87 sizes (V = 2 to 8, 64 to 4096 rows, 64 to 4608 columns, k = 64 to 1984, 50 to 98 % sparse, batches of
+// up to 256): 0.8 to 1.25 times the measured time in nine of ten, and the choice among the three within 1.4 % of the best in the mean.  (The costs
+// before counted an entry of the gather kernel once whatever k, which sent 3480 x 4231, k = 960, V = 8, 56 % there: 232 us instead of 32; 4 x (376 x 2817),
+// k = 1344, V = 4: 303 instead of 25.)
 struct SddmmTimes {
     double direct, dense, gather;
 };
 SddmmTimes sddmm_times(const SddmmParams &p, int V, const DeviceInfo *d) {
-    const double cycles_per_us = 1900.0 * d->sm_count;
-    const double k_blocks = std::ceil(p.k / 64.0), per_row = (double)p.nnz_vec / std::max(p.m_vec, 1);
-    const double tiles = std::ceil((double)p.m_vec * V / 128.0) * std::ceil(p.n / 128.0) * p.batch;
-    const double dense_tiles = std::ceil((double)p.m_vec * V / 256.0) * std::ceil(p.n / 256.0) * p.batch;
-    const double shared = std::min(1.0, std::max(0.0, tiles / d->sm_count - 1.0));
+    const double sms = d->sm_count, k_blocks = std::ceil(p.k / 64.0), per_row = (double)p.nnz_vec / std::max(p.m_vec, 1), m = (double)p.m_vec * V;
+    const double tiles = std::ceil(m / 128.0) * std::ceil(p.n / 128.0) * p.batch, items = std::max(1.0, std::ceil(m / 256.0) * std::ceil(p.n / 256.0) * p.batch);
+    const double shared = std::min(1.0, std::max(0.0, tiles / sms - 1.0)), pairs = sms / 2;
     SddmmTimes t;
-    t.direct = 2.0 + std::max(1.0, tiles / (2.0 * d->sm_count)) * (1.5 + (0.3 + 0.6 * shared) * k_blocks + 0.14 * (128.0 / V) * per_row / 256.0);
-    t.dense = 8.0 + 1.1e-3 * 32.0 * per_row + dense_tiles * std::max(2230.0 * k_blocks, 4250.0) / cycles_per_us;
-    t.gather = 4.5 + ((double)p.m_vec * 306.0 * k_blocks + (double)p.nnz_vec * 4.0) * p.batch / cycles_per_us;
+    t.direct = 2.0 + std::max(1.0, tiles / (2.0 * sms)) * (1.6 + (0.24 + 0.5 * shared) * k_blocks + (0.11 + 0.035 * shared) * std::min((double)p.m_vec, 128.0 / V) * per_row / 256.0);
+    const double waves = items > 4.0 * pairs ? items / pairs : std::ceil(items / pairs);
+    t.dense = 9.2 + waves * std::max(0.4 * k_blocks, 0.98 + 0.52e-3 * (double)p.nnz_vec * p.batch / items) * (p.n > pairsddmm::kMaxPlanColumns || !sddmm_pair_enabled() ? 1.4 : 1.0);
+    t.gather = 6.5 + std::max(1.0, (double)p.m_vec * p.batch / (2.0 * sms)) * (0.168 + 4.1e-3 * per_row) * k_blocks;
     return t;
+}
+// Which planned form runs (VSPARSE_B200_SDDMM = "dense" | "gather", read at every call, forces one).  The number of entries is an argument here, so the choice
+// is made on the host.
+bool sddmm_use_dense(const SddmmParams &p, int V, const DeviceInfo *d) {
+    const char *e = std::getenv("VSPARSE_B200_SDDMM");
+    if (e && !std::strcmp(e, "dense")) return true;
+    if (e && !std::strcmp(e, "gather")) return false;
+    const SddmmTimes t = sddmm_times(p, V, d);
+    return t.dense < 1.25 * t.gather;   // where the estimates are close, the one that long rows hold up least
 }
 // Small sampled products go to the one-kernel form.  lhs 512 x 256, rhs 2048 x 256, V = 4: 17.0 -> 7.8 us; 2048 x 512 x 256, V = 8,
 // 90 % sparse: one 11.1 -> 5.1, eight 14.4 -> 10.2, sixteen 18.9 -> 18.4.  VSPARSE_B200_SDDMM = "dense" and "gather" force those,
@@ -1411,7 +1402,7 @@ bool sddmm_direct_wanted(const SddmmParams &p, int V, const DeviceInfo *d) {
     const char *e = std::getenv("VSPARSE_B200_SDDMM");
     if (e) return !std::strcmp(e, "direct");
     const SddmmTimes t = sddmm_times(p, V, d);
-    return t.direct < (sddmm_use_dense(p, V) ? t.dense : t.gather);
+    return 1.07 * t.direct < (sddmm_use_dense(p, V, d) ? t.dense : t.gather);
 }
 
 template <typename TOut, int V> int launch_sddmm_tc(const SddmmParams &p, cudaStream_t s) {
@@ -1426,7 +1417,7 @@ template <typename TOut, int V> int launch_sddmm_tc(const SddmmParams &p, cudaSt
     const bool dense_ok = !t_no_scratch && p.n > 0 && p.m_vec > 0 && p.nnz_vec > 0 && p.k >= densesddmm::kBlockK && plan_bytes <= kMaxPlanBytes &&
                           plan_smem <= 40 * 1024 && aligned16(p.lhs) && aligned16(p.rhs) &&
                           (p.batch == 1 || ((p.stride_lhs * 2) % 16 == 0 && (p.stride_rhs * 2) % 16 == 0)) &&
-                          sddmm_use_dense(p, V);
+                          sddmm_use_dense(p, V, d);
     if (!dense_ok) return launch_sddmm_gather<TOut, V>(p, s, d);
     if (sddmm_pair_enabled() && launch_sddmm_pair<TOut, V>(p, s, d, &rc)) return rc;
     CUtensorMap map_l, map_r;
@@ -1486,15 +1477,6 @@ double sddmm_cores_time(const SddmmParams &p, int V) {
     constexpr double rows[4] = {2.27e-7, 3.66e-7, 4.90e-7, 8.99e-7}, chain[4] = {2.8e-3, 3.1e-3, 2.9e-3, 1.0e-2};
     return 2.5 + rows[v] * gathered + chain[v] * p.k;
 }
-// The planned form behind cudaSddmm, beside what sddmm_times() knows: a tile's contraction in series, 0.35 us for each 64 elements
-// (512 x 512, k = 1504: 17 us where the one-kernel form takes 9.6), and the sampling of a tile, which short vectors make the
-// longer part (4096 x 4096, k = 128, V = 2, 98 % sparse: 24.6 us, 14.9 without this).
-double sddmm_cores_dense_time(const SddmmParams &p, int V, const DeviceInfo *d, const SddmmTimes &t) {
-    const double per_row = (double)p.nnz_vec / std::max(p.m_vec, 1), launches = 8.0 + 1.1e-3 * 32.0 * per_row;
-    const double tiles = std::ceil((double)p.m_vec * V / 256.0) * std::ceil(p.n / 256.0) * p.batch;
-    const double sampling = (V == 2 ? 8000.0 : V == 4 ? 4400.0 : 4250.0) * tiles + (V == 2 ? 5.5 : V == 4 ? 2.0 : 1.0) * p.nnz_vec * p.batch;
-    return std::max(t.dense, launches + std::max(sampling / (1900.0 * d->sm_count), 0.35 * std::ceil(p.k / 64.0)));
-}
 template <int V> int launch_sddmm_cores(const SddmmParams &p, cudaStream_t s) {
     DeviceInfo *d;
     int rc = device_info(&d);
@@ -1505,14 +1487,12 @@ template <int V> int launch_sddmm_cores(const SddmmParams &p, cudaStream_t s) {
     const bool by_rule = !force_dense && !force_direct && sddmm_cores_wanted(p, V);
     if (!force_cores && !by_rule && strides && p.n > 0 && p.m_vec > 0) {
         const SddmmTimes t = sddmm_times(p, V, d);
-        const bool pair_ok = V > 1 && !t_no_scratch && sddmm_pair_enabled() && p.n <= pairsddmm::kMaxPlanColumns;
-        const double dense = pair_ok ? sddmm_cores_dense_time(p, V, d, t) : 0.0;
-        const bool pair = pair_ok && !force_direct && (force_dense || dense < t.direct);
+        const bool pair_ok = !t_no_scratch && sddmm_pair_enabled() && p.n <= pairsddmm::kMaxPlanColumns;
+        const bool pair = pair_ok && !force_direct && (force_dense || t.dense < t.direct);
         // The tile forms' estimates are up to 1.7 times too high where they are long; below, what the CUDA-core kernel is taken for is a clear gain.
-        const double tiled = pair ? dense : t.direct;
+        const double tiled = pair ? t.dense : t.direct;
         const bool sparse = !force_dense && !force_direct && sddmm_cores_time(p, V) + 1.2 < (tiled < 30.0 ? 1.0 : V == 1 ? 0.9 : 0.6) * tiled;
-        if constexpr (V > 1)
-            if (!sparse && pair && launch_sddmm_pair<__half, V>(p, s, d, &rc)) return rc;
+        if (!sparse && pair && launch_sddmm_pair<__half, V>(p, s, d, &rc)) return rc;
         if (!sparse && !force_dense && launch_sddmm_direct<__half, V>(p, s, d, &rc)) return rc;
     }
     return launch_sddmm_cc<__half, __half, V>(p, s);
@@ -2260,7 +2240,9 @@ VS_EXPORT int vs_sddmm_formulation(int m_vec, int k, int n, int nonzeros_vec, in
         return 0;
     SddmmParams p{};
     p.m_vec = m_vec; p.k = k; p.n = n; p.nnz_vec = nonzeros_vec;
-    return sddmm_use_dense(p, vec_length) ? 1 : 0;
+    DeviceInfo *d = nullptr;
+    if (device_info(&d) != VS_OK) return 0;
+    return sddmm_use_dense(p, vec_length, d) ? 1 : 0;
 }
 
 VS_EXPORT int vs_kernel_timing(int enable, double *total_ms, int *launches) {
