@@ -19,7 +19,12 @@
 // CVSE arrays on CUDA cores, entry by entry as the reference does.
 //
 // The K order of the MMAs is the one of the other densifying kernels (16 columns of A at a time, ascending), so that a product whose
-// columns ascend has the same bits whichever of them multiplies it; a row computed entry by entry has those of spmm_cc_kernel.
+// columns ascend has the same bits whichever of them multiplies it, where a tile is not shared (kSplit); a row computed entry by entry has those of spmm_cc_kernel.
+//
+// kSplit: a cluster of up to eight CTAs shares the tile, each with a part of A's columns, where few tiles have many chunks to walk (80 rows x 4023 columns x
+// 320, V = 8, 52 %: 32 chunks on 5 CTAs, 37 us; on 40 CTAs 13.8, a share of four chunks, its search and the sums of the others).  A group of lanes finds the first entry of its vector-row in each part by a search that assumes
+// ascending columns; the parts cover the row, and every entry is compared with the one before it, so that columns which do not ascend are
+// found out all the same.  The parts' sums meet in shared memory, in order, a share of the rows in each CTA.
 //
 // Roles (320 threads): warps 0-7 fill, then epilogue (TMEM lanes 32 (w % 4) .., columns 32 (w / 4) ..); warp 8 the MMA-issuing
 // thread; warp 9 the thread that loads B by TMA.  Rings: 2 chunks of A (32 KiB each), 3 of B (16 KiB each).  Every
@@ -54,6 +59,9 @@ constexpr int kAChunkBytes = 2 * kABlockBytes;
 constexpr int kBBlockBytes = 64 * kTileN * 2;             // 8 KiB: 64 rows of B x 64 columns
 constexpr int kBChunkBytes = 2 * kBBlockBytes;
 constexpr int kTmemCols = 64;
+constexpr int kPartPitch = kTileN + 4;                   // of a part's sums, fp32, in the place of the chunks of A
+constexpr int kMaxSplit = 8;                              // CTAs that share a tile
+static_assert(kTileM * kPartPitch * 4 <= kABuffers * kAChunkBytes && kTileM / kMaxSplit % 8 == 0, "a part's sums; whole vector-rows in a share");
 
 struct Smem {   // offsets from the 1024-byte aligned base
     static constexpr int kA = 0;
@@ -65,7 +73,7 @@ struct Smem {   // offsets from the 1024-byte aligned base
     static constexpr int kTmemHolder = kBarDone + kBBuffers * 8;
     static constexpr int kAbort = kTmemHolder + 8;
     static constexpr int kRedo = kAbort + 8;              // vector-rows of the tile to be computed entry by entry, a bit each
-    static constexpr int kTotal = kRedo + kTileM / 8;
+    static constexpr int kTotal = kRedo + 2 * (kTileM / 8);
 };
 constexpr int kSmemBytes = Smem::kTotal;   // the dynamic segment is 1024-byte aligned (nothing static lies ahead of it)
 static_assert(2 * (kSmemBytes + 1024) <= 228 * 1024, "two CTAs per SM");
@@ -172,7 +180,7 @@ __device__ __noinline__ void rows_by_entries(const SpmmParams &p, int b, int row
 // verdict: null when the densified product is the cheaper one whatever the number of nonzeros; otherwise the
 // kernel compares the costs the plan kernel compares (dense_cost for its `stages`, gather_per_row, gather_per_entry), writes
 // the answer there for the kernel enqueued behind this one, and returns at once when that kernel is to take the call.
-template <typename TOut, int V>
+template <typename TOut, int V, bool kSplit>
 __global__ void __launch_bounds__(kThreads, 2)
 spmm_direct_kernel(const __grid_constant__ SpmmParams p, const __grid_constant__ CUtensorMap map_b, int m_tiles, int n_tiles, float dense_cost,
                    float dense_per_entry, float gather_per_row, float gather_per_entry, int32_t *verdict, uint32_t *status) {
@@ -183,7 +191,7 @@ spmm_direct_kernel(const __grid_constant__ SpmmParams p, const __grid_constant__
     const uint32_t base = tc::smem_u32(sm);
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     volatile int *abort_flag = reinterpret_cast<volatile int *>(sm + Smem::kAbort);
-    uint32_t *redo_rows = reinterpret_cast<uint32_t *>(sm + Smem::kRedo);
+    uint32_t *redo_rows = reinterpret_cast<uint32_t *>(sm + Smem::kRedo), *own_redo = redo_rows + kTileM / 32;   // split: of this CTA's part of the columns; of its share of the rows
     const uint32_t bar_full = base + Smem::kBarFull, bar_done = base + Smem::kBarDone;
 
     pdl_launch_dependents();
@@ -195,7 +203,7 @@ spmm_direct_kernel(const __grid_constant__ SpmmParams p, const __grid_constant__
         *abort_flag = 0;
         tc::fence_mbar_init();
     }
-    if (t < kTileM / 32) redo_rows[t] = 0;
+    if (t < 2 * (kTileM / 32)) redo_rows[t] = 0;
     if (warp == kMmaWarp) {
         tc::tmem_alloc(base + Smem::kTmemHolder, kTmemCols);
         tc::tmem_relinquish();
@@ -212,10 +220,14 @@ spmm_direct_kernel(const __grid_constant__ SpmmParams p, const __grid_constant__
         mine = dense_cost + dense_per_entry * nnz < (float)p.m_vec * gather_per_row + gather_per_entry * nnz;
         if (blockIdx.x == 0 && t == 0) plan_publish(verdict, mine);
     }
-    const int mt = (int)(blockIdx.x % (unsigned)m_tiles);
-    const unsigned rest = blockIdx.x / (unsigned)m_tiles;
+    const int parts = kSplit ? (int)tc::cluster_nctarank() : 1, part = kSplit ? (int)tc::cluster_ctarank() : 0;
+    const unsigned tile = blockIdx.x / (unsigned)parts;
+    const int mt = (int)(tile % (unsigned)m_tiles);
+    const unsigned rest = tile / (unsigned)m_tiles;
     const int n0 = (int)(rest % (unsigned)n_tiles) * kTileN, b = (int)(rest / (unsigned)n_tiles);
-    const int chunks = mine ? (p.K + kChunkK - 1) / kChunkK : 0;
+    // this CTA's chunks: `chunk0` .. + chunks - 1
+    const int all_chunks = (p.K + kChunkK - 1) / kChunkK, chunk0 = kSplit ? part * all_chunks / parts : 0;
+    const int chunks = mine ? (kSplit ? (part + 1) * all_chunks / parts - chunk0 : all_chunks) : 0;
     bool bad = false;
 
     if (warp < kFillWarps) {
@@ -229,6 +241,30 @@ spmm_direct_kernel(const __grid_constant__ SpmmParams p, const __grid_constant__
             begin = __ldg(p.row_offsets + row);
             end = __ldg(p.row_offsets + row + 1);
         }
+        const int first = begin;   // of the vector-row
+        if constexpr (kSplit) {
+            // the first entry with a column of at least `bound`, for both ends of the part: every round cuts the range to one of kGroup + 1 pieces
+            auto search = [&](int bound) {
+                int lo = begin, hi = end;   // the answer lies in lo .. hi
+                while (__any_sync(0xffffffffu, lo < hi)) {
+                    const int at = lo + (int)((int64_t)(hi - lo) * (lane % kGroup) / kGroup);   // lane 0 of the group: lo itself
+                    const bool below = lo < hi && __ldg(p.col_indices + at) < bound;
+                    const uint32_t votes = __ballot_sync(0xffffffffu, below) >> (lane / kGroup * kGroup) & (uint32_t)((1ull << kGroup) - 1ull);
+                    const int n = __popc(votes);   // ascending: the lanes below are the first n
+                    const int new_lo = n ? lo + (int)((int64_t)(hi - lo) * (n - 1) / kGroup) + 1 : lo;
+                    const int new_hi = n < kGroup ? lo + (int)((int64_t)(hi - lo) * n / kGroup) : hi;
+                    if (lo < hi) {
+                        lo = n ? new_lo : lo;
+                        hi = max(new_hi, lo);
+                    }
+                }
+                return lo;
+            };
+            const int from = part > 0 ? search(chunk0 * kChunkK) : begin, to = part + 1 < parts ? search((chunk0 + chunks) * kChunkK) : end;
+            bad |= from > to;
+            begin = from;
+            end = max(from, to);
+        }
         next = begin + lane % kGroup;
         const __half *values = static_cast<const __half *>(p.values) + (int64_t)b * p.stride_values;
         int cols[2][kWindow], left[kWindow];
@@ -241,7 +277,7 @@ spmm_direct_kernel(const __grid_constant__ SpmmParams p, const __grid_constant__
                 left[e] = INT_MIN;
                 if (j < end) {
                     cols[1][e] = __ldg(p.col_indices + j);
-                    if (j > begin) left[e] = __ldg(p.col_indices + j - 1);
+                    if (j > first) left[e] = __ldg(p.col_indices + j - 1);
                     vals[1][e].load(values + (int64_t)j * V);
                 }
             }
@@ -274,7 +310,7 @@ spmm_direct_kernel(const __grid_constant__ SpmmParams p, const __grid_constant__
                                            ((piece ^ (k & 7u)) << 4)) = make_uint4(0, 0, 0, 0);
             }
             __syncwarp();
-            const int k0 = c * kChunkK, k1 = min(k0 + kChunkK, p.K);
+            const int k0 = (chunk0 + c) * kChunkK, k1 = min(k0 + kChunkK, p.K);
             auto scatter = [&]() {
 #pragma unroll
                 for (int e = 0; e < kWindow; ++e)
@@ -309,8 +345,13 @@ spmm_direct_kernel(const __grid_constant__ SpmmParams p, const __grid_constant__
             const int quarter = warp & 3, half = warp >> 2;
             uint32_t r[32];
             tc::tmem_ld_x32(tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(half * 32), r);
+            if constexpr (kSplit) {   // every MMA of this CTA is done: the chunks of A are read no more
+                float *sums = reinterpret_cast<float *>(sm + Smem::kA) + (quarter * 32 + lane) * kPartPitch + half * 32;
+#pragma unroll
+                for (int q = 0; q < 8; ++q) reinterpret_cast<uint4 *>(sums)[q] = make_uint4(r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+            }
             const int m = mt * kTileM + quarter * 32 + lane, n = n0 + half * 32;
-            if (m < p.m_vec * V) {
+            if (!kSplit && m < p.m_vec * V) {
                 TOut *out = static_cast<TOut *>(p.out) + (int64_t)b * p.stride_out + (int64_t)m * p.N + n;
                 float probe = 0.0f;   // x * 0 is NaN for a sum that is not finite
 #pragma unroll
@@ -338,7 +379,7 @@ spmm_direct_kernel(const __grid_constant__ SpmmParams p, const __grid_constant__
                 const int ab = c % kABuffers, bb = c % kBBuffers;
                 if (!wait_or_abort<0>(bar_full + 8 * bb, (c / kBBuffers) & 1, abort_flag)) break;
                 tc::tc_fence_after_sync();
-                const int k_left = p.K - c * kChunkK;
+                const int k_left = p.K - (chunk0 + c) * kChunkK;
                 const uint32_t a_lo = a_lo0 + ab * (kAChunkBytes >> 4), b_lo = b_lo0 + bb * (kBChunkBytes >> 4);
 #pragma unroll
                 for (int kk = 0; kk < kChunkK / 16; ++kk)
@@ -353,10 +394,10 @@ spmm_direct_kernel(const __grid_constant__ SpmmParams p, const __grid_constant__
             for (int c = 0; c < chunks; ++c) {
                 const int bb = c % kBBuffers;
                 if (c >= kBBuffers && !wait_or_abort<0>(bar_done + 8 * bb, ((c / kBBuffers) - 1) & 1, abort_flag)) break;
-                const int boxes = p.K - c * kChunkK > 64 ? 2 : 1;
+                const int boxes = p.K - (chunk0 + c) * kChunkK > 64 ? 2 : 1;
                 tc::mbar_expect_tx(bar_full + 8 * bb, (uint32_t)boxes * kBBlockBytes);
                 for (int s = 0; s < boxes; ++s)
-                    tc::tma_load_3d(base + Smem::kB + bb * kBChunkBytes + s * kBBlockBytes, &map_b, bar_full + 8 * bb, n0, c * kChunkK + 64 * s, b);
+                    tc::tma_load_3d(base + Smem::kB + bb * kBChunkBytes + s * kBBlockBytes, &map_b, bar_full + 8 * bb, n0, (chunk0 + c) * kChunkK + 64 * s, b);
             }
         }
         __syncwarp();
@@ -364,6 +405,54 @@ spmm_direct_kernel(const __grid_constant__ SpmmParams p, const __grid_constant__
 
     // ---- teardown, and the tiles that have to be computed entry by entry -----------------------------------
     tc::tc_fence_before_sync();
+    if constexpr (kSplit) {
+        // all parts' sums, and their rows to be computed anew, lie in shared memory: this CTA adds up its share of the rows
+        tc::cluster_sync();
+        const int share = kTileM / parts, row0 = part * share;
+        uint32_t theirs = 0;
+        if (t < kTileM / 32)
+            for (int r = 0; r < parts; ++r) theirs |= tc::ld_remote_u32(tc::map_to_cta(base + Smem::kRedo + 4 * t, r));
+        const bool failed = *abort_flag != 0;
+        if (mine && !failed) {
+            TOut *out = static_cast<TOut *>(p.out) + (int64_t)b * p.stride_out;
+            for (int i = t; i < share * (kTileN / 8); i += kThreads) {
+                const int row = row0 + i / (kTileN / 8), c = i % (kTileN / 8) * 8, m = mt * kTileM + row;
+                if (m >= p.m_vec * V || n0 + c >= p.N) continue;
+                float f[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) f[e] = 0.0f;
+                for (int r = 0; r < parts; ++r) {
+                    const uint32_t from = tc::map_to_cta(base + Smem::kA + (row * kPartPitch + c) * 4, r);
+#pragma unroll
+                    for (int q = 0; q < 2; ++q) {
+                        const float4 x = tc::ld_remote_f32x4(from + 16 * q);
+                        f[4 * q] += x.x; f[4 * q + 1] += x.y; f[4 * q + 2] += x.z; f[4 * q + 3] += x.w;
+                    }
+                }
+                float probe = 0.0f;
+#pragma unroll
+                for (int e = 0; e < 8; ++e) probe = fmaf(f[e], 0.0f, probe);
+                store_chunk(out + (int64_t)m * p.N + n0 + c, f);
+                if (probe != 0.0f) {
+                    atomicOr(own_redo + (row / V >> 5), 1u << (row / V & 31));
+                    bad = true;
+                }
+            }
+        }
+        // of the vector-rows found out by any part, those of this CTA's share
+        if (t < kTileM / 32) {
+            uint32_t share_bits = 0;
+            for (int x = 0; x < 32; ++x) {
+                const int vr = 32 * t + x;
+                if (vr * V >= row0 && vr * V < row0 + share) share_bits |= 1u << x;
+            }
+            theirs &= share_bits;
+            if (theirs) atomicOr(own_redo + t, theirs);
+            bad |= theirs != 0u;
+        }
+        if (!mine) bad = false;
+        tc::cluster_sync();   // nobody reads the others' shared memory any more
+    }
     const int redo = __syncthreads_or(bad ? 1 : 0);
     if (*abort_flag) {   // a bounded wait ran out: copies that may still be in flight get time to land
         for (int i = 0; i < 64; ++i) __nanosleep(1000);
@@ -373,7 +462,7 @@ spmm_direct_kernel(const __grid_constant__ SpmmParams p, const __grid_constant__
     if (warp == kMmaWarp) tc::tmem_dealloc(tmem_base, kTmemCols);
     if (redo) {
         const int row0 = mt * (kTileM / V);
-        rows_by_entries<TOut, V>(p, b, row0, min(kTileM / V, p.m_vec - row0), n0, redo_rows);
+        rows_by_entries<TOut, V>(p, b, row0, min(kTileM / V, p.m_vec - row0), n0, kSplit ? own_redo : redo_rows);
     }
 }
 

@@ -357,6 +357,30 @@ cudaError_t launch_overlapped(void (*kernel)(Exp...), unsigned grid, unsigned bl
     return cudaLaunchKernelEx(&cfg, kernel, std::forward<Act>(args)...);
 }
 
+// Launches clusters of `size` CTAs, `grid` CTAs in all, as a programmatic dependent.
+template <typename... Exp, typename... Act>
+cudaError_t launch_clusters(void (*kernel)(Exp...), unsigned grid, unsigned size, unsigned block, size_t smem, cudaStream_t s, Act &&...args) {
+    static const bool overlap = []() {
+        const char *e = std::getenv("VSPARSE_B200_PDL");
+        return !(e && !std::strcmp(e, "0"));
+    }();
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = size;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = overlap ? 2 : 1;
+    return cudaLaunchKernelEx(&cfg, kernel, std::forward<Act>(args)...);
+}
+
 // Launches `pairs` clusters of two CTAs (tcgen05 cta_group::2 kernels), optionally as a programmatic dependent.
 template <typename... Exp, typename... Act>
 cudaError_t launch_pairs(void (*kernel)(Exp...), unsigned pairs, unsigned block, size_t smem, cudaStream_t s, bool overlapped,
@@ -858,6 +882,20 @@ int launch_spmm_other(const SpmmParams &p, cudaStream_t s, DeviceInfo *d, const 
     }
 }
 
+// CTAs that share a tile of the one-kernel form: as many as the tiles leave room for, two from seven chunks of 128 columns on, up to eight with three or more
+// each.  By the sizes of the whole call, whose parts then have its bits (vs_set_part_of).  us, 1 / 2 / 4 / 8: 80 x 4023 x 320, V = 8, 52 % 37 / 23 / 15.5 / 13.8;
+// 1588 x 2035 x 104, V = 4, 57 % 36 / 27 / 21; 172 x 2995 x 64, V = 2, 52 % 64 / 39 / 26 / 19; 158 x 1018 x 128, V = 2, 93 % 12.6 / 10.5; but six chunks,
+// 15 x (232 x 986 x 64) and alike, V = 8, 91 %: 8.3 to 9.0 / 8.7 to 10.1.  VSPARSE_B200_SPMM_SPLIT sets the most.
+int spmm_direct_split(const SpmmParams &p, int V, const DeviceInfo *d) {
+    const char *e = std::getenv("VSPARSE_B200_SPMM_SPLIT");
+    const int most = e ? std::atoi(e) : directspmm::kMaxSplit;
+    const int64_t tiles = ((int64_t)p.m_vec * V + directspmm::kTileM - 1) / directspmm::kTileM *
+                          ((std::max(p.N, t_whole_columns) + directspmm::kTileN - 1) / directspmm::kTileN) * std::max(p.batch, t_whole_batch);
+    const int chunks = (p.K + directspmm::kChunkK - 1) / directspmm::kChunkK;
+    int split = 1;
+    while (2 * split <= std::min(most, directspmm::kMaxSplit) && 2 * split * tiles <= 2 * d->sm_count && std::max(7, 6 * split) <= chunks) split *= 2;
+    return split;
+}
 // Small products in one kernel (spmm_direct.cuh); false if this call or this device cannot take it.  When the densified
 // product is the cheaper one whatever the number of nonzeros, nothing else is enqueued; otherwise the kernel leaves its
 // verdict where the gather kernel behind it looks for the plan kernel's.
@@ -876,19 +914,35 @@ template <typename TOut, int V, bool kCores> bool launch_spmm_direct(const SpmmP
     // V > 2: only past 4096 columns, where a product whose rows hold a few entries waits for 32 and more chunks, and with scratch.
     const bool by_density = kCores && !forced && (V <= 2 ? p.K > 1024 : p.K > 4096 && !t_no_scratch);
     if (by_density) cost = {(V > 2 ? 0.018f : V == 2 ? 0.03f : tiles > 48 ? 0.045f : 0.035f) * (float)p.K * (float)p.m_vec / stages, 0.0f, 0.0f, 1.0f};
-    const bool always = forced || (kCores && !by_density) || (!kCores && cost.dense_per_entry == 0.0f && cost.dense_per_stage * stages < cost.gather_per_row * (float)p.m_vec);
+    bool always = forced || (kCores && !by_density) || (!kCores && cost.dense_per_entry == 0.0f && cost.dense_per_stage * stages < cost.gather_per_row * (float)p.m_vec);
+    // A caller that says how many values there are is spared the kernel that would return at once (10 x (4 to 16 rows of tiles), 700 to 1600 columns: 2 to 3 of
+    // 8 to 16 us).
+    if (!always && p.stride_values > 0) {
+        const float nnz = (float)(p.stride_values / V);
+        if (!(cost.dense_per_stage * stages + cost.dense_per_entry * nnz < cost.gather_per_row * (float)p.m_vec + cost.gather_per_entry * nnz)) {
+            *rc_out = launch_spmm_other<TOut, V, kCores>(p, s, d, nullptr, 0);
+            return true;
+        }
+        always = true;
+    }
     CUtensorMap map;
-    static DeviceBits smem_set;
-    auto kernel = directspmm::spmm_direct_kernel<TOut, V>;
-    if (make_tile_map(&map, p.rhs, false, (uint64_t)p.K, (uint64_t)p.N, (uint64_t)p.batch, (uint64_t)p.stride_rhs, 64, 64) != VS_OK ||
-        set_smem_once(kernel, directspmm::kSmemBytes, smem_set) != VS_OK)
+    static DeviceBits smem_set, smem_set_split;
+    const int split = spmm_direct_split(p, V, d);
+    auto kernel = split > 1 ? directspmm::spmm_direct_kernel<TOut, V, true> : directspmm::spmm_direct_kernel<TOut, V, false>;
+    if (tiles * split > 0x7fffffffll || make_tile_map(&map, p.rhs, false, (uint64_t)p.K, (uint64_t)p.N, (uint64_t)p.batch, (uint64_t)p.stride_rhs, 64, 64) != VS_OK ||
+        set_smem_once(kernel, directspmm::kSmemBytes, split > 1 ? smem_set_split : smem_set) != VS_OK)
         return false;
     void *verdict = nullptr;
     PlanScratch scratch;
     if (!always && (t_no_scratch || scratch.take(d, s, 16, &verdict) != VS_OK)) return false;
-    *rc_out = (int)launch_overlapped(kernel, (unsigned)tiles, directspmm::kThreads, directspmm::kSmemBytes, s, p, map, m_tiles, n_tiles,
-                                     cost.dense_per_stage * stages, cost.dense_per_entry, cost.gather_per_row, cost.gather_per_entry,
-                                     static_cast<int32_t *>(verdict), d->status);
+    if (split > 1)
+        *rc_out = (int)launch_clusters(kernel, (unsigned)(tiles * split), (unsigned)split, directspmm::kThreads, directspmm::kSmemBytes, s, p, map, m_tiles, n_tiles,
+                                       cost.dense_per_stage * stages, cost.dense_per_entry, cost.gather_per_row, cost.gather_per_entry,
+                                       static_cast<int32_t *>(verdict), d->status);
+    else
+        *rc_out = (int)launch_overlapped(kernel, (unsigned)tiles, directspmm::kThreads, directspmm::kSmemBytes, s, p, map, m_tiles, n_tiles,
+                                         cost.dense_per_stage * stages, cost.dense_per_entry, cost.gather_per_row, cost.gather_per_entry,
+                                         static_cast<int32_t *>(verdict), d->status);
     if (*rc_out == VS_OK && !always) {
         // Not overlapped: CTAs that become resident beside a grid of under one wave crowd onto the SMs it leaves free, and where the
         // CUDA-core kernel then does the work that cost it half its speed (V = 1, 4096 x 4096 x 256, 98 % sparse: 31 -> 46 us).
@@ -910,7 +964,11 @@ bool spmm_direct_wanted(const SpmmParams &p, int V, bool cores, const DeviceInfo
     const int64_t tiles = m_tiles * ((p.N + directspmm::kTileN - 1) / directspmm::kTileN) * p.batch;
     const int chunks = (p.K + directspmm::kChunkK - 1) / directspmm::kChunkK;
     if (cores && p.N <= 256 && ((V == 1 && tiles <= 2 * d->sm_count) || (V == 2 && tiles <= 64))) return true;
-    if (tiles <= 2 * d->sm_count) return chunks <= (V == 8 ? 64 : V == 4 ? 32 : 16);
+    // Few tiles share their columns among CTAs, which puts the line at so many times the K; at V <= 2 with a laid-out matrix on the other side of it, up to five
+    // chunks each (194 x 2678 x 768, V = 2, 77 %: 26.9 us against 24.6, 426 x 2547 x 256, 93 %: 19.8 against 24.3; without one, 172 x 2995 x 64, V = 2, 52 %
+    // 19 against 164, 16 x (1062 x 2224 x 32) 36 against 80, 884 x 2710 x 968 33 against 78).
+    const int split = spmm_direct_split(p, V, d), each = (chunks + split - 1) / split, most = V == 8 ? 64 : V == 4 ? 32 : 16;
+    if (tiles <= 2 * d->sm_count) return chunks <= most || (each <= most && (V > 2 || each <= 5 || p.N < 128 || p.N % 64 != 0));
     return tiles <= 4 * d->sm_count && chunks <= (V >= 4 ? 4 : 1);
 }
 
