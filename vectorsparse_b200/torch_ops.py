@@ -16,6 +16,9 @@ of fixed-mask sparse attention into torch.autograd, so that the pair can sit ins
 
     c = sparse_dense_product(values, b, mask)                 # [m, N] = A(values) @ b, differentiable in values and b
     # backward: d b = A^T @ d c (vs_spmm_t), d values = (d c @ b^T) sampled at the structure (vs_sddmm)
+
+On plain contiguous fp16 CUDA tensors both are recorded in torch's graph by the binding, without a Python function per pass; the two
+torch.autograd.Function classes take everything else (modes, tracers, transforms, subclasses) and say what the gradients are.
 """
 from __future__ import annotations
 
@@ -102,6 +105,20 @@ class AttentionMask:
         self.t_offsets, self.t_rows, self.t_src = (torch.from_numpy(x).to(device) for x in _cvse.transpose(a))
 
 
+def _native(which, operands, mask, path, scale):
+    """The operator recorded in torch's graph by the binding (csrc/binding.cpp), or None where torch has to see more than that: modes, tracers, functorch
+    transforms, forward-mode levels, a compiler, a profiler, tensor subclasses; the binding itself declines what is not plain, contiguous and fp16."""
+    if (torch._C._len_torch_dispatch_stack() or _len_pre_dispatch() or torch._C._len_torch_function_stack()
+            or torch._C._get_tracing_state() is not None or torch.autograd.profiler._is_profiler_enabled
+            or torch._C._are_functorch_transforms_active() or torch.autograd.forward_ad._current_level >= 0 or torch.compiler.is_compiling()):
+        return None
+    for t in operands:
+        if type(t) is not torch.Tensor and type(t) is not torch.nn.Parameter:
+            return None
+    return ops._binding.differentiable(which, path, mask.m_vec, mask.V, mask.n, mask.nnz_vec, scale, mask.row_indices, mask.row_offsets,
+                                       mask.col_indices, mask.t_offsets, mask.t_rows, mask.t_src, mask, *operands)
+
+
 class FixedMaskAttention(torch.autograd.Function):
     """softmax(scale * Q K^T at the mask) V with the library's forward and backward operators (the probabilities are
     recomputed in the backward pass, not kept)."""
@@ -117,18 +134,22 @@ class FixedMaskAttention(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_out):
-        q, k, v = ctx.saved_tensors
-        m = ctx.mask
-        batch = q.shape[0] if q.dim() == 3 else 1
-        gq, gk, gv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
-        ws_p, ws_g = (torch.empty((batch, m.nnz_vec * m.V), dtype=torch.float16, device=q.device) for _ in range(2))
-        ops.attention_cvse_backward(ctx.path, m.m_vec, m.V, m.n, k.shape[-1], m.nnz_vec, m.row_indices, m.row_offsets, m.col_indices,
-                                    m.t_offsets, m.t_rows, m.t_src, q, k, v, grad_out.contiguous(), gq, gk, gv, ws_p, ws_g, ctx.scale)
-        return gq, gk, gv, None, None, None
+        return (*_attention_backward(ctx.mask, ctx.path, ctx.scale, ctx.saved_tensors, grad_out), None, None, None)
+
+
+def _attention_backward(m, path, scale, saved, grad_out):
+    q, k, v = saved
+    batch = q.shape[0] if q.dim() == 3 else 1
+    gq, gk, gv = torch.empty_like(q), torch.empty_like(k), torch.empty_like(v)
+    ws_p, ws_g = (torch.empty((batch, m.nnz_vec * m.V), dtype=torch.float16, device=q.device) for _ in range(2))
+    ops.attention_cvse_backward(path, m.m_vec, m.V, m.n, k.shape[-1], m.nnz_vec, m.row_indices, m.row_offsets, m.col_indices,
+                                m.t_offsets, m.t_rows, m.t_src, q, k, v, grad_out.contiguous(), gq, gk, gv, ws_p, ws_g, scale)
+    return gq, gk, gv
 
 
 def fixed_mask_attention(q, k, v, mask: AttentionMask, scale: float, path: int = VS_PATH_TENSOR):
-    return FixedMaskAttention.apply(q, k, v, mask, scale, path)
+    out = _native(1, (q, k, v), mask, path, float(scale))
+    return FixedMaskAttention.apply(q, k, v, mask, scale, path) if out is None else out
 
 
 class SparseDenseProduct(torch.autograd.Function):
@@ -148,19 +169,31 @@ class SparseDenseProduct(torch.autograd.Function):
 
     @staticmethod
     def backward(ctx, grad_c):
-        values, b = ctx.saved_tensors
-        m = ctx.mask
-        grad_c = grad_c.contiguous()
-        grad_values = grad_b = None
-        if ctx.needs_input_grad[1]:
-            grad_b = torch.empty_like(b)
-            ops.spmm_t(m.m_vec, m.V, b.shape[-1], m.n, m.t_offsets, m.t_rows, m.t_src, values, grad_c, grad_b, m.nnz_vec)
-        if ctx.needs_input_grad[0]:
-            g = _through(_sddmm, torch.ops.vsparse.sddmm, (grad_c, b), ctx.path, m.m_vec, m.V, m.nnz_vec, m.row_indices, m.row_offsets,
-                         m.col_indices, grad_c, b)
-            grad_values = g.sum(0) if (g.dim() == 2 and values.dim() == 1) else g
-        return grad_values, grad_b, None, None
+        return (*_product_backward(ctx.mask, ctx.path, ctx.saved_tensors, grad_c, ctx.needs_input_grad[:2]), None, None)
+
+
+def _product_backward(m, path, saved, grad_c, wanted):
+    values, b = saved
+    grad_c = grad_c.contiguous()
+    grad_values = grad_b = None
+    if wanted[1]:
+        grad_b = torch.empty_like(b)
+        ops.spmm_t(m.m_vec, m.V, b.shape[-1], m.n, m.t_offsets, m.t_rows, m.t_src, values, grad_c, grad_b, m.nnz_vec)
+    if wanted[0]:
+        g = _through(_sddmm, torch.ops.vsparse.sddmm, (grad_c, b), path, m.m_vec, m.V, m.nnz_vec, m.row_indices, m.row_offsets,
+                     m.col_indices, grad_c, b)
+        grad_values = g.sum(0) if (g.dim() == 2 and values.dim() == 1) else g
+    return grad_values, grad_b
 
 
 def sparse_dense_product(values, b, mask: AttentionMask, path: int = VS_PATH_TENSOR):
-    return SparseDenseProduct.apply(values, b, mask, path)
+    c = _native(0, (values, b), mask, path, 0.0)
+    return SparseDenseProduct.apply(values, b, mask, path) if c is None else c
+
+
+def _backward(which, mask, path, scale, saved, grad, wanted):
+    """The backward pass of a node of the binding where it does not make it itself."""
+    return _attention_backward(mask, path, scale, saved, grad) if which else _product_backward(mask, path, saved, grad, wanted)
+
+
+ops._binding.bind_backward(_backward)
