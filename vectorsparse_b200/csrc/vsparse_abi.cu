@@ -887,11 +887,12 @@ int launch_spmm_other(const SpmmParams &p, cudaStream_t s, DeviceInfo *d, const 
 // 1588 x 2035 x 104, V = 4, 57 % 36 / 27 / 21; 172 x 2995 x 64, V = 2, 52 % 64 / 39 / 26 / 19; 158 x 1018 x 128, V = 2, 93 % 12.6 / 10.5; but six chunks,
 // 15 x (232 x 986 x 64) and alike, V = 8, 91 %: 8.3 to 9.0 / 8.7 to 10.1.  VSPARSE_B200_SPMM_SPLIT sets the most.
 int spmm_direct_split(const SpmmParams &p, int V, const DeviceInfo *d) {
+    const int chunks = (p.K + directspmm::kChunkK - 1) / directspmm::kChunkK;
+    if (chunks < 7) return 1;
     const char *e = std::getenv("VSPARSE_B200_SPMM_SPLIT");
     const int most = e ? std::atoi(e) : directspmm::kMaxSplit;
     const int64_t tiles = ((int64_t)p.m_vec * V + directspmm::kTileM - 1) / directspmm::kTileM *
                           ((std::max(p.N, t_whole_columns) + directspmm::kTileN - 1) / directspmm::kTileN) * std::max(p.batch, t_whole_batch);
-    const int chunks = (p.K + directspmm::kChunkK - 1) / directspmm::kChunkK;
     int split = 1;
     while (2 * split <= std::min(most, directspmm::kMaxSplit) && 2 * split * tiles <= 2 * d->sm_count && std::max(7, 6 * split) <= chunks) split *= 2;
     return split;
@@ -1259,10 +1260,16 @@ int spmm_split(int V, const SpmmParams &p, cudaStream_t s, bool *taken) {
 // 32 chunks of 16 bytes (k <= 256 in fp16, 128 in fp32), a group of eight lanes per mask entry otherwise.
 // VSPARSE_B200_SDDMM_CC=entry keeps the latter.
 template <typename TIn, typename TOut, int V, int L> int launch_sddmm_cc_row(const SddmmParams &p, cudaStream_t s) {
-    const int64_t blocks = ((int64_t)p.m_vec * L + kCcThreads - 1) / kCcThreads;
+    // groups of lanes that share a vector-row: until there are 16 warps per SM, with eight entries each or more
+    DeviceInfo *d = nullptr;
+    const int rc = device_info(&d);
+    if (rc != VS_OK) return rc;
+    int pieces = 1;
+    while ((int64_t)p.m_vec * p.batch * pieces * L < 16ll * 32 * d->sm_count && p.nnz_vec / p.m_vec >= 16 * pieces && pieces < 64) pieces *= 2;
+    const int64_t blocks = ((int64_t)p.m_vec * pieces * L + kCcThreads - 1) / kCcThreads;
     if (blocks > 0x7fffffffll) return VS_ERR_SHAPE;
     dim3 grid((unsigned)blocks, (unsigned)p.batch, 1);
-    sddmm_cc_row_kernel<TIn, TOut, V, L><<<grid, kCcThreads, 0, s>>>(p);
+    sddmm_cc_row_kernel<TIn, TOut, V, L><<<grid, kCcThreads, 0, s>>>(p, pieces);
     return (int)cudaGetLastError();
 }
 template <typename TIn, typename TOut, int V> int launch_sddmm_cc(const SddmmParams &p, cudaStream_t s) {
