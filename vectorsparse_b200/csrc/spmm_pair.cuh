@@ -1,6 +1,6 @@
 // Tensor-core SpMM on densified tiles of the sparse matrix, computed by PAIRS of CTAs (a cluster of two SMs,
 // tcgen05 cta_group::2): the `wmmaSpmm` entry point of the reference (src/wmma_spmm.cu:388-409) for dense widths
-// that are multiples of 64.  Same formulation, plan and semantics as spmm_dense.cuh next to this file (see there
+// above 128 that are multiples of 8.  Same formulation, plan and semantics as spmm_dense.cuh next to this file (see there
 // for why a zero-filled tile of A beats a row gather on this part); what changes is who multiplies what:
 //
 //     C[256 rows x tn cols] += A_dense[256 x 64] * B[64 x tn]        per 64-wide block of A's columns, tn = 256 or 128
@@ -152,7 +152,7 @@ struct Walk {
 // map_b: the dense operand as {N, K, batch}, box {64, 64, 1}; map_b2: the same memory as {64, K, N / 64, batch},
 // box {64, 64, 2, 1} (both 64-column slabs of a CTA's half of a 256-column tile in one copy); map_out: the output
 // as {N, rows, batch}, box {32, 32, 1}.  All with zero fill / clipping outside the matrix; no multicast anywhere.
-// tn: columns per work item (256 or 128), N % 64 == 0; the last tile of a row may be wider than what is left of the matrix.
+// tn: columns per work item (256 or 128); the last tile of a row may be wider than what is left of the matrix.  map_b2 only where N % 64 == 0.
 // kPrepared: the tiles of A have been laid out in memory, 128 rows by 64 columns with the columns contiguous (densify_kernel), and come
 // through map_a, {64, 128, 1, tiles}, box {64, 128, 1, 1}, beside those of B; batch_a == 1: one matrix for the whole batch; no fill warps.
 template <typename TOut, int V, bool kTransposed, bool kPrepared = false>
@@ -387,6 +387,7 @@ spmm_pair_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_a, 
         // them can arrive after the CTA has gone.
         if (lane == 0) {
             bool ok_run = true;
+            const bool blocked = p.N % 64 == 0;   // else map_b2 is not there
             const uint32_t full_first = tc::map_to_cta(bar_full, 0);
             Walk walk;
             walk.init(pair, pairs, 0u, total_stages, m_tiles, n_tiles, k_blocks);
@@ -405,10 +406,11 @@ spmm_pair_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_a, 
                 if constexpr (kPrepared)
                     tc::tma_load_4d_pair(base + Smem::kA + slot * kAStageBytes, &map_a, bar, 0, 0, 0,
                                          ((batch_a == 1 ? 0 : walk.b) * row_tiles + 2 * walk.mt + (int)rank) * k_blocks + walk.kb);
-                if (slabs == 2) {
+                if (slabs == 2 && blocked) {
                     tc::tma_load_4d_pair(base + Smem::kB + slot * kBStageBytes, &map_b2, bar, 0, walk.kb * kBlockK, n0 >> 6, walk.b);
                 } else {
-                    tc::tma_load_3d_pair(base + Smem::kB + slot * kBStageBytes, &map_b, bar, n0, walk.kb * kBlockK, walk.b);
+                    for (int h = 0; h < slabs; ++h)
+                        tc::tma_load_3d_pair(base + Smem::kB + slot * kBStageBytes + h * kBSlabBytes, &map_b, bar, n0 + 64 * h, walk.kb * kBlockK, walk.b);
                 }
             }
             const uint32_t tail0 = total_stages > (uint32_t)kBarStages ? total_stages - kBarStages : 0u;

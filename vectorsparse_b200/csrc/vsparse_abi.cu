@@ -804,13 +804,15 @@ template <typename K> int max_resident_pairs(K kernel, int block, size_t smem, D
     return n;
 }
 
-// The densified product by pairs of CTAs (spmm_pair.cuh) takes dense widths from 128 up that are multiples of 64, the single-CTA
-// kernel (spmm_dense.cuh) the others, and 128 where there are more row tiles than its CTAs.  us, single CTAs / pairs, product with the matrix
+// The densified product by pairs of CTAs (spmm_pair.cuh) takes dense widths from 128 up, the single-CTA kernel (spmm_dense.cuh) the narrower ones, and 128 where
+// there are more row tiles than its CTAs.  us, single CTAs / pairs, product with the matrix
 // and with its transpose: 64 x (2048 x 512 x N), V = 8, 90 % sparse: N = 128 28 / 33 and 33 / 39, 192 38 / 35 and 51 / 41, 448 65 / 59 and 85 / 64;
-// 4096 x 4096 x 1984, V = 2, 70 %: 261 / 149 and 281 / 161.  VSPARSE_B200_SPMM_PAIR=0 keeps every width on the former, =1 on the latter.
-inline bool spmm_pair_takes(int N, int64_t row_items, const DeviceInfo *d) {
+// 4096 x 4096 x 1984, V = 2, 70 %: 261 / 149 and 281 / 161; widths that are no multiple of 64: 64 x (2048 x 512 x 200), V = 8 45.6 / 40.0, x 264 63 / 59,
+// 17 x (2062 x 1310 x 560), V = 2 (laid out) 241 / 148, 4 x (3958 x 1750 x 584), V = 1 (laid out) 195 / 81.  VSPARSE_B200_SPMM_PAIR=0 keeps every width on the former, =1 on the latter.
+inline bool spmm_pair_takes(int N, int V, int64_t row_items, const DeviceInfo *d, bool from_plan = false) {
     const char *e = std::getenv("VSPARSE_B200_SPMM_PAIR");
-    if (N % 64 != 0 || N < 128 || (e && !std::strcmp(e, "0"))) return false;
+    if (N % 8 != 0 || N < 128 || (e && !std::strcmp(e, "0"))) return false;
+    if (from_plan && V <= 2 && N % 64 != 0 && !e) return false;   // scattering short vectors for the rest of a wide tile costs more than the pair saves (V = 1 41 / 34 for 64 x (1024 x 256 x 256) already)
     return N > 128 || row_items <= d->sm_count || e;
 }
 // Columns of B per work item of the pair kernel.  An item of 128 columns costs 0.9 of one of 256 (both fill the same tile of A), so
@@ -965,11 +967,14 @@ bool spmm_direct_wanted(const SpmmParams &p, int V, bool cores, const DeviceInfo
     const int64_t tiles = m_tiles * ((p.N + directspmm::kTileN - 1) / directspmm::kTileN) * p.batch;
     const int chunks = (p.K + directspmm::kChunkK - 1) / directspmm::kChunkK;
     if (cores && p.N <= 256 && ((V == 1 && tiles <= 2 * d->sm_count) || (V == 2 && tiles <= 64))) return true;
-    // Few tiles share their columns among CTAs, which puts the line at so many times the K; at V <= 2 with a laid-out matrix on the other side of it, up to five
-    // chunks each (194 x 2678 x 768, V = 2, 77 %: 26.9 us against 24.6, 426 x 2547 x 256, 93 %: 19.8 against 24.3; without one, 172 x 2995 x 64, V = 2, 52 %
-    // 19 against 164, 16 x (1062 x 2224 x 32) 36 against 80, 884 x 2710 x 968 33 against 78).
-    const int split = spmm_direct_split(p, V, d), each = (chunks + split - 1) / split, most = V == 8 ? 64 : V == 4 ? 32 : 16;
-    if (tiles <= 2 * d->sm_count) return chunks <= most || (each <= most && (V > 2 || each <= 5 || p.N < 128 || p.N % 64 != 0));
+    // Few tiles share their columns among CTAs, which puts the line at so many times the K.  At V <= 2 a matrix laid out first is on the other side of it where
+    // B is wide enough to pay for that.  us, one kernel / laid out, V = 2: 657 x 1460 x 1320, 78 % (12 chunks) 38 / 22, 909 x 1511 x 872, 57 % 50 / 25, 1180 x
+    // 1966 x 640, 81 % (8 each) 29 / 24, 506 x 765 x 704, 71 % (6) 18.5 / 16.2, 1906 x 569 x 528, 76 % (5) 20.6 / 26.9; 1984 x 1031 x 320, 87 % (9) 24 / 28, 8 x (97 x
+    // 762 x 192), 88 % (6) 17 / 22, 1762 x 1938 x 192, 87 % (4) 21.6 / 26, 1984 x 3120 x 192, 61 % (13) 120 / 110; one kernel / a plan, 172 x 2995 x 64 19 / 164, 16 x
+    // (1062 x 2224 x 32) (9) 36 / 80, V = 1, 2 x (2792 x 4032 x 112) (16) 165 / 157.
+    const int split = spmm_direct_split(p, V, d), each = (chunks + split - 1) / split;
+    const int short_vectors = p.N >= 512 && !t_no_scratch ? (tiles > 40 ? 5 : 6) : split > 1 ? 10 : 16;
+    if (tiles <= 2 * d->sm_count) return each <= (V == 8 ? 64 : V == 4 ? 32 : short_vectors);
     return tiles <= 4 * d->sm_count && chunks <= (V >= 4 ? 4 : 1);
 }
 
@@ -989,7 +994,10 @@ template <typename TOut, int V, bool kCores> bool launch_spmm_laid_out(const Spm
     const int m_tiles = (int)((M + pairspmm::kTileM - 1) / pairspmm::kTileM), row_tiles = (int)((M + 127) / 128);
     const int Kp = (p.K + 63) / 64 * 64, k_blocks = Kp / 64, batch_a = p.batch > 1 && p.stride_values ? p.batch : 1;
     const int64_t row_items = (int64_t)p.batch * m_tiles, a_bytes = (int64_t)batch_a * row_tiles * 128 * Kp * 2;
-    if (capacity < 0 || !spmm_pair_takes(p.N, row_items, d) || a_bytes > (128ll << 20)) return false;
+    if (capacity < 0 || !spmm_pair_takes(p.N, V, row_items, d) || a_bytes > (128ll << 20)) return false;
+    // Widths that are no multiple of 64: where there is work for the tiles, six blocks of 64 columns and 5 % of the vectors (68 x (3960 x 66 x 1128), V = 1 218 us on
+    // single CTAs, 312 laid out; 49 x (160 x 1166 x 336), V = 1, 96 % 26 and 32)
+    if (!e && p.N % 64 != 0 && (k_blocks < 6 || (p.stride_values > 0 && (double)(p.stride_values / V) < 0.05 * p.m_vec * p.K))) return false;
     const int tn = spmm_pair_width(p.N, row_items, capacity), n_tiles = (p.N + tn - 1) / tn;
     const int64_t items = row_items * n_tiles;
     if (items * k_blocks > 0x7fffffffll) return false;
@@ -1005,12 +1013,13 @@ template <typename TOut, int V, bool kCores> bool launch_spmm_laid_out(const Spm
     const int64_t header = ((4 + checks) * 4 + 255) / 256 * 256;
     CUtensorMap map_a, map_b, map_b2, map_out;
     if (make_tile_map(&map_b, p.rhs, false, (uint64_t)p.K, (uint64_t)p.N, (uint64_t)p.batch, (uint64_t)p.stride_rhs, 64, 64) != VS_OK ||
-        make_blocked_map(&map_b2, p.rhs, (uint64_t)p.K, (uint64_t)p.N, (uint64_t)p.batch, (uint64_t)p.stride_rhs, 2) != VS_OK ||
+        (p.N % 64 == 0 && make_blocked_map(&map_b2, p.rhs, (uint64_t)p.K, (uint64_t)p.N, (uint64_t)p.batch, (uint64_t)p.stride_rhs, 2) != VS_OK) ||
         make_tile_map(&map_out, p.out, sizeof(TOut) == 4, (uint64_t)M, (uint64_t)p.N, (uint64_t)p.batch, (uint64_t)p.stride_out, pairspmm::kStoreCols, 32) != VS_OK)
         return false;
     uint8_t *mem = nullptr;
     PlanScratch scratch;
     if (scratch.take(d, s, (size_t)(header + a_bytes), reinterpret_cast<void **>(&mem)) != VS_OK) return false;
+    if (p.N % 64 != 0) map_b2 = map_b;
     if (make_packed_map(&map_a, mem + header, 64, 128, 1, (uint64_t)batch_a * row_tiles * k_blocks, 1) != VS_OK) return false;
     int32_t *verdict = reinterpret_cast<int32_t *>(mem);
     int rc = (int)launch_overlapped(densify::densify_kernel<V>, (unsigned)checks, densify::kPrepThreads, 0, s, p, batch_a, Kp, min_vectors,
@@ -1082,7 +1091,7 @@ template <typename TOut, int V, bool kCores> int launch_spmm_tc(const SpmmParams
     const int force_dense = mode == SpmmMode::kDense ? 1 : 0;
     SpmmCosts planned = cost;
     if constexpr (kCores) {
-        const bool pairs = use_b4 && spmm_pair_takes(p.N, (int64_t)p.batch * m_tiles, d);
+        const bool pairs = (use_b4 || p.N % 64 != 0) && spmm_pair_takes(p.N, V, (int64_t)p.batch * m_tiles, d, true);
         const int tn = spmm_pair_width(p.N, (int64_t)p.batch * m_tiles, d->sm_count / 2);
         const int64_t widths = pairs ? (p.N + tn - 1) / tn : n_tiles;
         planned = cores_costs_of(p, V, (int64_t)p.batch * m_tiles * widths, pairs ? d->sm_count / 2 : d->sm_count, d);
@@ -1098,7 +1107,7 @@ template <typename TOut, int V, bool kCores> int launch_spmm_tc(const SpmmParams
     rc = (int)cudaGetLastError();
     if (rc == VS_OK) {
         int rc_pair = VS_OK;
-        if (use_b4 && spmm_pair_takes(p.N, (int64_t)p.batch * m_tiles, d) &&
+        if ((use_b4 || p.N % 64 != 0) && spmm_pair_takes(p.N, V, (int64_t)p.batch * m_tiles, d, true) &&
             launch_spmm_pair<TOut, V, false>(p, s, d, map, map_out, map_b4, blk_offsets, blk_entries, m_tiles, k_blocks, flag, checks, flag + kPlanRedo, &rc_pair))
             rc = rc_pair;
         else
@@ -1759,7 +1768,7 @@ template <typename TOut, int V> int launch_spmm_t(const spmmt::Params *list, int
     for (int i = 0; i < count && rc == VS_OK; ++i) {
         q.values = list[i].values; q.rhs = list[i].rhs; q.out = list[i].out;
         int rc_pair = VS_OK;
-        if (use_b4 && spmm_pair_takes(q.N, (int64_t)q.batch * m_tiles, d) &&
+        if ((use_b4 || q.N % 64 != 0) && spmm_pair_takes(q.N, V, (int64_t)q.batch * m_tiles, d, true) &&
             launch_spmm_pair<TOut, V, true>(q, s, d, map[i], map_out[i], map_b4[i], blk_offsets, blk_entries, m_tiles, k_blocks, flag, checks, flag + kPlanRedo + i, &rc_pair))
             rc = rc_pair;
         else
