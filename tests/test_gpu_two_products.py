@@ -1,0 +1,33 @@
+"""The two transposed products of attention's backward (dV = P^T dO, dK = dS^T Q) in one launch: bit for bit what each gives by itself,
+with one tile in all, a ragged last tile, and more tiles than the SMs that a product gets."""
+import numpy as np
+import pytest
+import torch
+
+from gpu_util import DEV, captured_kernels, custom, dev, structure
+from vectorsparse_b200 import VS_PATH_TENSOR, cvse, ops
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("V", [2, 4, 8])
+@pytest.mark.parametrize("heads,n,d", [(1, 64, 64), (3, 520, 64), (2, 264, 64), (100, 264, 64)])
+@pytest.mark.parametrize("cores", [False, True])
+def test_each_as_by_itself(monkeypatch, V, heads, n, d, cores):
+    monkeypatch.setenv("VSPARSE_B200_SPMM_T", "gather" if cores else "dense")
+    monkeypatch.setenv("VSPARSE_B200_ATTENTION", "fused")
+    a = custom([4 * (7 * i % (n // 16)) for i in range(n // V)], n, V, seed=n + V)
+    q, k, v, go = (dev(cvse.fill_random((heads, n, d), np.float16, cvse.DIST_NORMAL, 10 + i, 1.0)) for i in range(4))
+    gq, gk, gv, want_k, want_v = (torch.full((heads, n, d), float("nan"), dtype=torch.float16, device=DEV) for _ in range(5))
+    ws_p, ws_g = (torch.zeros(heads, a.nnz_vec * V, dtype=torch.float16, device=DEV) for _ in range(2))
+    s, t = structure(a), [dev(x) for x in cvse.transpose(a)]
+    launches = captured_kernels(lambda: ops.attention_cvse_backward(VS_PATH_TENSOR, a.m_vec, V, n, d, a.nnz_vec, *s, *t, q, k, v, go, gq, gk, gv,
+                                                                    ws_p, ws_g, 0.125))
+    assert launches.count("spmm_dense_kernel") == (0 if cores else 1), launches
+    assert launches.count("spmm_t_kernel") == (2 if cores else 1), launches
+    ops.attention_cvse_backward(VS_PATH_TENSOR, a.m_vec, V, n, d, a.nnz_vec, *s, *t, q, k, v, go, gq, gk, gv, ws_p, ws_g, 0.125)
+    for values, rhs, out in ((ws_g, q, want_k), (ws_p, go, want_v)):
+        ops.spmm_t(a.m_vec, V, d, n, *t, values, rhs, out, a.nnz_vec)
+    torch.cuda.synchronize()
+    assert ops.device_status() == 0
+    assert torch.equal(gk, want_k) and torch.equal(gv, want_v)

@@ -265,20 +265,20 @@ __device__ __forceinline__ Item decode_item(int64_t w, int m_tiles, int n_tiles,
 // (batch entry, column tile, row tile, column block) of stage g, advanced by a fixed number of stages.
 struct StageIter {
     int b, nt, mt, kb;
-    int d_mt, d_nt, d_b;   // one step of gridDim.x work items, as digits of (b, nt, mt)
+    int d_mt, d_nt, d_b;   // one step of G work items, as digits of (b, nt, mt)
     int m_tiles, n_tiles, k_blocks;
     uint32_t g, total;
-    __device__ __forceinline__ void init(uint32_t g0, uint32_t total_stages, int m_tiles_, int n_tiles_, int k_blocks_) {
+    __device__ __forceinline__ void init(uint32_t cta, uint32_t G, uint32_t g0, uint32_t total_stages, int m_tiles_, int n_tiles_,
+                                         int k_blocks_) {   // CTA `cta` of the G that share the items
         m_tiles = m_tiles_; n_tiles = n_tiles_; k_blocks = k_blocks_;
         g = g0; total = total_stages;
-        const uint32_t G = gridDim.x;
         d_mt = (int)(G % (uint32_t)m_tiles);
         const uint32_t r = G / (uint32_t)m_tiles;
         d_nt = (int)(r % (uint32_t)n_tiles);
         d_b = (int)(r / (uint32_t)n_tiles);
         const uint32_t i0 = g0 / (uint32_t)k_blocks;       // divisions once, here
         kb = (int)(g0 - i0 * (uint32_t)k_blocks);
-        const int64_t w = blockIdx.x + (int64_t)i0 * G;
+        const int64_t w = cta + (int64_t)i0 * G;
         mt = (int)(w % m_tiles);
         const int64_t rr = w / m_tiles;
         nt = (int)(rr % n_tiles);
@@ -297,12 +297,12 @@ struct StageIter {
     }
 };
 
-// The items of this CTA one after the other (blockIdx.x, + gridDim.x, ...), again without divisions per step.
+// The items of this CTA one after the other (cta, + G, ...), again without divisions per step.
 struct ItemIter {
     StageIter w;
     int N;
-    __device__ __forceinline__ void init(int m_tiles, int n_tiles, int N_) {
-        w.init(0u, 0xffffffffu, m_tiles, n_tiles, 1);
+    __device__ __forceinline__ void init(uint32_t cta, uint32_t G, int m_tiles, int n_tiles, int N_) {
+        w.init(cta, G, 0u, 0xffffffffu, m_tiles, n_tiles, 1);
         N = N_;
     }
     __device__ __forceinline__ Item get() const {
@@ -352,13 +352,26 @@ template <> struct ValueVec<1> { typedef unsigned short Raw; unsigned short raw;
 // {64, 64, 2, 1}, i.e. both boxes of a stage in one copy (the TMA unit works through copies one after the
 // other, and two 8 KiB copies per stage were what the MMAs waited for).  map_out: the output, dimensions {N, rows, batch}, box {32, 32, 1}, swizzle span =
 // the 64 (fp16) or 128 (fp32) bytes of a box row (stores clip at the edges of the matrix).
-template <typename TOut, int V, bool kTransposed>
+//
+// kTwo: two products that share the structure, the sizes and the strides (the two transposed products of attention's
+// backward) in one launch.  The upper half of the grid works on the second; its redo word follows the first's.  A
+// CTA belongs to one product, so its roles walk the items as they do for one, and the waves of the launch are never
+// more than those of two launches one after the other.  (Few heads left those nearly empty: one head of 3000, 64
+// wide, V = 4, has 12 tiles a product.  Its forward and backward: 168.4 -> 118.1 us; 5 heads of 2656 174.8 -> 137.8;
+// 16 heads of 2048, V = 8, with 128 tiles each, 154.5 -> 142.6; 123 heads of 1880 1059.8 -> 1016.0.)
+template <bool kTwo> struct Second {};
+template <> struct Second<true> {
+    CUtensorMap map_b, map_out, map_b4;
+    const void *values, *rhs;
+};
+
+template <typename TOut, int V, bool kTransposed, bool kTwo = false>
 __global__ void __launch_bounds__(kThreads, 1)
-spmm_dense_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b,
-                  const __grid_constant__ CUtensorMap map_out, const __grid_constant__ CUtensorMap map_b4, int use_b4,
+spmm_dense_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b_,
+                  const __grid_constant__ CUtensorMap map_out_, const __grid_constant__ CUtensorMap map_b4_, int use_b4,
                   const int32_t *__restrict__ blk_offsets,
                   const uint2 *__restrict__ blk_entries, int m_tiles, int n_tiles, int k_blocks, uint32_t *status,
-                  const int32_t *use_dense, int plan_checks, int32_t *redo) {
+                  const int32_t *use_dense, int plan_checks, int32_t *redo, const __grid_constant__ Second<kTwo> two) {
     pdl_launch_dependents();   // the gather kernel behind this one may queue up
     pdl_wait();                // launched while the plan kernel may still be at work: nothing it writes is read before here
     // Not chosen (the gather kernel behind this one takes the call): the CTA still sets itself up and tears itself
@@ -367,6 +380,18 @@ spmm_dense_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b,
     // set-up, is also what the compiler likes best: taken after it — which would let the set-up overlap the plan
     // kernel — the same code ran 14 % slower at 50 % sparsity and 8 % slower at width 64.)
     const bool chosen = plan_dense_chosen(use_dense, plan_checks);
+    uint32_t cta = blockIdx.x, G = gridDim.x;
+    const CUtensorMap *map_b = &map_b_, *map_out = &map_out_, *map_b4 = &map_b4_;
+    const void *p_values = p.values, *p_rhs = p.rhs;
+    if constexpr (kTwo) {
+        G >>= 1;
+        if (cta >= G) {
+            cta -= G;
+            map_b = &two.map_b; map_out = &two.map_out; map_b4 = &two.map_b4;
+            p_values = two.values; p_rhs = two.rhs;
+            ++redo;
+        }
+    }
     extern __shared__ uint8_t smem_raw[];
     const uint32_t raw = tc::smem_u32(smem_raw);
     const uint32_t base = (raw + 1023u) & ~1023u;
@@ -407,8 +432,7 @@ spmm_dense_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b,
     const uint32_t tmem_base = *reinterpret_cast<volatile uint32_t *>(sm + Smem::kTmemHolder);
 
     const int64_t total_items = chosen ? (int64_t)p.batch * n_tiles * m_tiles : 0;
-    const int64_t G = gridDim.x;
-    const uint32_t my_items = (total_items > blockIdx.x) ? (uint32_t)((total_items - blockIdx.x + G - 1) / G) : 0u;
+    const uint32_t my_items = (total_items > cta) ? (uint32_t)((total_items - cta + G - 1) / G) : 0u;
     const uint32_t total_stages = my_items * (uint32_t)k_blocks;
     const int m_rows = kTransposed ? p.m_vec : p.m_vec * V;   // rows of the output (for A^T, p.m_vec counts its rows)
 
@@ -430,7 +454,7 @@ spmm_dense_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b,
         // the first 64 entries one stage ahead, their values before the wait for the slot.
         struct Pos { int b, mt, kb; bool valid; };
         StageIter walk;
-        walk.init(a_slot, total_stages, m_tiles, n_tiles, k_blocks);
+        walk.init(cta, G, a_slot, total_stages, m_tiles, n_tiles, k_blocks);
         auto locate = [&]() {   // the walker's position, then kAStages further on
             Pos q;
             q.valid = walk.valid(); q.b = walk.b; q.mt = walk.mt; q.kb = walk.kb;
@@ -461,7 +485,7 @@ spmm_dense_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b,
         uint32_t p_pos[kFillBatches] = {};
         bool ok_run = true;
         for (uint32_t g = a_slot; g < total_stages && ok_run; g += kAStages) {
-            const __half *vals = static_cast<const __half *>(p.values) + (int64_t)cur.b * p.stride_values;
+            const __half *vals = static_cast<const __half *>(p_values) + (int64_t)cur.b * p.stride_values;
             // values of the first 64 entries, entries of the next stage, bounds of the one after: all in flight
             // while this warp waits for its slot
             ValueVec<V> c_val[kFillBatches];
@@ -543,7 +567,7 @@ spmm_dense_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b,
             uint32_t g = 0;
             bool ok_run = true;
             ItemIter items;
-            items.init(m_tiles, n_tiles, p.N);
+            items.init(cta, G, m_tiles, n_tiles, p.N);
             for (uint32_t i = 0; i < my_items && ok_run; ++i, items.next()) {
                 const Item it = items.get();
                 const int slabs = (it.tn + 63) >> 6;
@@ -555,10 +579,10 @@ spmm_dense_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b,
                     const uint32_t bar = bar_full + 8 * slot;
                     tc::mbar_expect_tx(bar, (uint32_t)slabs * kBSlabBytes);   // arrives and arms the byte count
                     if (use_b4 && slabs == kTileN / 64) {   // both boxes with one instruction
-                        tc::tma_load_4d(base + Smem::kB + slot * kBStageBytes, &map_b4, bar, 0, kb * kBlockK, it.n0 >> 6, it.b);
+                        tc::tma_load_4d(base + Smem::kB + slot * kBStageBytes, map_b4, bar, 0, kb * kBlockK, it.n0 >> 6, it.b);
                     } else {
                         for (int s = 0; s < slabs; ++s)
-                            tc::tma_load_3d(base + Smem::kB + slot * kBStageBytes + s * kBSlabBytes, &map_b, bar, it.n0 + 64 * s,
+                            tc::tma_load_3d(base + Smem::kB + slot * kBStageBytes + s * kBSlabBytes, map_b, bar, it.n0 + 64 * s,
                                             kb * kBlockK, it.b);
                     }
                     *progress = g + 1;
@@ -571,11 +595,11 @@ spmm_dense_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b,
         // through the TMA queue would hold up the loads queued behind them.  This warp asks each tile into L2
         // with plain prefetches about one work item before the loader wants it, paced by the loader's counter.
         volatile uint32_t *progress = reinterpret_cast<volatile uint32_t *>(sm + Smem::kLoaderProgress);
-        const __half *rhs = static_cast<const __half *>(p.rhs);
+        const __half *rhs = static_cast<const __half *>(p_rhs);
         uint32_t g = (uint32_t)k_blocks;   // the stage being prefetched
         bool ok_run = true;
         ItemIter items;
-        items.init(m_tiles, n_tiles, p.N);
+        items.init(cta, G, m_tiles, n_tiles, p.N);
         for (uint32_t i = 1; i < my_items && ok_run; ++i) {
             items.next();
             const Item it = items.get();
@@ -613,7 +637,7 @@ spmm_dense_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b,
             uint32_t a_slot = 0, b_slot = 0, b_parity = 0;
             bool ok_run = true;
             ItemIter items;
-            items.init(m_tiles, n_tiles, p.N);
+            items.init(cta, G, m_tiles, n_tiles, p.N);
             bool ready = false;   // whether the next stage was already seen full
             for (uint32_t i = 0; i < my_items && ok_run; ++i, items.next()) {
                 const Item it = items.get();
@@ -674,7 +698,7 @@ spmm_dense_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b,
         tc::mbar_arrive(bar_acc_empty);
         tc::mbar_arrive(bar_acc_empty + 8);
         ItemIter items;
-        items.init(m_tiles, n_tiles, p.N);
+        items.init(cta, G, m_tiles, n_tiles, p.N);
         for (uint32_t i = 0; i < my_items && ok_run; ++i, items.next()) {
             const Item it = items.get();
             const uint32_t buf = i & 1u;
@@ -716,7 +740,7 @@ spmm_dense_kernel(const SpmmParams p, const __grid_constant__ CUtensorMap map_b,
                     tc::fence_proxy_async();
                     __syncwarp();
                     if (lane == 0) {
-                        tc::tma_store_3d(&map_out, stg_u32 + box * kBoxBytes, it.n0 + c0, row0, it.b);
+                        tc::tma_store_3d(map_out, stg_u32 + box * kBoxBytes, it.n0 + c0, row0, it.b);
                         tc::bulk_commit_group();
                     }
                     ++box_count;

@@ -79,16 +79,21 @@ __device__ __forceinline__ void store8(float *dst, const float (&acc)[8]) {
 
 // Work item = (batch entry, 256-column chunk, group of kWarps output rows); items are walked grid-stride so that
 // a launch never needs more CTAs than fit the machine a few times over.
-template <typename TOut, int V>
-__global__ void __launch_bounds__(kThreads) spmm_t_kernel(const Params p, int64_t items, int row_groups, int chunks,
-                                                          const int32_t *plan_hdr, int plan_checks, int redo) {
+// Behind a launch that served two products (kTwo) the upper half of the grid stands by for the second, whose redo
+// word follows the first's.
+template <typename TOut, int V, bool kTwo = false>
+__global__ void __launch_bounds__(kThreads) spmm_t_kernel(const Params first, const Params second, int64_t items, int row_groups,
+                                                          int chunks, const int32_t *plan_hdr, int plan_checks, int redo) {
     // Enqueued behind the tensor-core kernel (plan_hdr != null): wait for its end, then leave unless it handed the
     // call over (a matrix it cannot hold, or a non-finite sum it would not vouch for).
     pdl_launch_dependents();   // the next call's plan kernel may queue up behind this one
     pdl_wait();
-    if (plan_hdr && plan_dense_stands(plan_hdr, plan_checks, redo)) return;
+    const bool upper = kTwo && blockIdx.x >= gridDim.x / 2;
+    const Params &p = upper ? second : first;
+    const unsigned cta = upper ? blockIdx.x - gridDim.x / 2 : blockIdx.x, ctas = kTwo ? gridDim.x / 2 : gridDim.x;
+    if (plan_hdr && plan_dense_stands(plan_hdr, plan_checks, redo + (upper ? 1 : 0))) return;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int64_t w = blockIdx.x; w < items; w += gridDim.x) {
+    for (int64_t w = cta; w < items; w += ctas) {
         const int rg = (int)(w % row_groups);
         const int64_t rest = w / row_groups;
         const int chunk = (int)(rest % chunks);

@@ -1112,7 +1112,8 @@ template <typename TOut, int V, bool kCores> int launch_spmm_tc(const SpmmParams
             rc = rc_pair;
         else
             rc = (int)launch_overlapped(kernel, grid, densespmm::kThreads, densespmm::kSmemBytes, s, p, map, map_out, map_b4, use_b4,
-                                        blk_offsets, blk_entries, m_tiles, n_tiles, k_blocks, d->status, flag, checks, flag + kPlanRedo);
+                                        blk_offsets, blk_entries, m_tiles, n_tiles, k_blocks, d->status, flag, checks, flag + kPlanRedo,
+                                        densespmm::Second<false>());
     }
     if (rc == VS_OK) rc = launch_spmm_other<TOut, V, kCores>(p, s, d, flag, checks);
     return rc;
@@ -1669,8 +1670,10 @@ VS_EXPORT int vs_spmm(int path, int in_dtype, int out_dtype, int m_vec, int vec_
 namespace {
 // CUDA-core kernel.  With `plan_hdr` it is enqueued behind the dense kernel and returns at once unless that kernel
 // left the call to it.
+// `second`: another product of the same structure and sizes, served by the same launch (only behind the dense kernel).
 template <typename TOut, int V>
-int launch_spmm_t_cc(const spmmt::Params &p, cudaStream_t s, DeviceInfo *d, const int32_t *plan_hdr, int plan_checks, int redo = kPlanRedo) {
+int launch_spmm_t_cc(const spmmt::Params &p, cudaStream_t s, DeviceInfo *d, const int32_t *plan_hdr, int plan_checks, int redo = kPlanRedo,
+                     const spmmt::Params *second = nullptr) {
     const int row_groups = (p.n + spmmt::kWarps - 1) / spmmt::kWarps;
     const int chunks = (p.N + spmmt::kChunk - 1) / spmmt::kChunk;
     const int64_t items = (int64_t)p.batch * chunks * row_groups;
@@ -1679,8 +1682,13 @@ int launch_spmm_t_cc(const spmmt::Params &p, cudaStream_t s, DeviceInfo *d, cons
                                                       // took 14 us to do so, a quarter of them a quarter of that)
     const unsigned grid = (unsigned)(items < cap ? items : cap);
     auto kernel = spmmt::spmm_t_kernel<TOut, V>;
-    if (plan_hdr) return (int)launch_overlapped(kernel, grid, spmmt::kThreads, 0, s, p, items, row_groups, chunks, plan_hdr, plan_checks, redo);
-    kernel<<<grid, spmmt::kThreads, 0, s>>>(p, items, row_groups, chunks, plan_hdr, plan_checks, redo);
+    if (second) {
+        const int64_t half = cap / 2;
+        return (int)launch_overlapped(spmmt::spmm_t_kernel<TOut, V, (V > 1)>, 2 * (unsigned)(items < half ? items : half), spmmt::kThreads, 0, s,
+                                      p, *second, items, row_groups, chunks, plan_hdr, plan_checks, redo);
+    }
+    if (plan_hdr) return (int)launch_overlapped(kernel, grid, spmmt::kThreads, 0, s, p, p, items, row_groups, chunks, plan_hdr, plan_checks, redo);
+    kernel<<<grid, spmmt::kThreads, 0, s>>>(p, p, items, row_groups, chunks, plan_hdr, plan_checks, redo);
     return (int)cudaGetLastError();
 }
 
@@ -1749,8 +1757,10 @@ template <typename TOut, int V> int launch_spmm_t(const spmmt::Params *list, int
             use_b4 = 0;
     }
     auto kernel = densespmm::spmm_dense_kernel<TOut, V, true>;
-    static DeviceBits smem_set;
+    auto kernel_two = densespmm::spmm_dense_kernel<TOut, V, true, (V > 1)>;   // attention's vectors are longer than 1
+    static DeviceBits smem_set, smem_set_two;
     rc = set_smem_once(kernel, densespmm::kSmemBytes, smem_set);
+    if (rc == VS_OK && count == 2) rc = set_smem_once(kernel_two, densespmm::kSmemBytes, smem_set_two);
     if (rc != VS_OK) return rc;
     uint8_t *plan = nullptr;
     PlanScratch scratch;
@@ -1765,15 +1775,30 @@ template <typename TOut, int V> int launch_spmm_t(const spmmt::Params *list, int
                                 blk_entries, capacity, mode == SpmmTMode::kDense ? 1 : 0, 1100.0f, 0.0f, 5.0f * V, 1.5f, flag);
     const int64_t items = (int64_t)q.batch * n_tiles * m_tiles;
     const unsigned grid = (unsigned)(items < d->sm_count ? items : d->sm_count);   // one persistent CTA per SM
+    const bool pairs = (use_b4 || q.N % 64 != 0) && spmm_pair_takes(q.N, V, (int64_t)q.batch * m_tiles, d, true);
+    if constexpr (V > 1) {
+        if (count == 2 && !pairs && d->sm_count > 1 && rc == VS_OK) {   // half of the SMs each: never more waves than one product after the other
+            densespmm::Second<true> two;
+            two.map_b = map[1]; two.map_out = map_out[1]; two.map_b4 = map_b4[1];
+            two.values = list[1].values; two.rhs = list[1].rhs;
+            const int64_t half = d->sm_count / 2;
+            rc = (int)launch_overlapped(kernel_two, 2 * (unsigned)(items < half ? items : half), densespmm::kThreads, densespmm::kSmemBytes, s, q,
+                                        map[0], map_out[0], map_b4[0], use_b4, blk_offsets, blk_entries, m_tiles, n_tiles, k_blocks, d->status,
+                                        flag, checks, flag + kPlanRedo, two);
+            if (rc == VS_OK) rc = launch_spmm_t_cc<TOut, V>(list[0], s, d, flag, checks, kPlanRedo, &list[1]);
+            return rc;
+        }
+    }
     for (int i = 0; i < count && rc == VS_OK; ++i) {
         q.values = list[i].values; q.rhs = list[i].rhs; q.out = list[i].out;
         int rc_pair = VS_OK;
-        if ((use_b4 || q.N % 64 != 0) && spmm_pair_takes(q.N, V, (int64_t)q.batch * m_tiles, d, true) &&
+        if (pairs &&
             launch_spmm_pair<TOut, V, true>(q, s, d, map[i], map_out[i], map_b4[i], blk_offsets, blk_entries, m_tiles, k_blocks, flag, checks, flag + kPlanRedo + i, &rc_pair))
             rc = rc_pair;
         else
             rc = (int)launch_overlapped(kernel, grid, densespmm::kThreads, densespmm::kSmemBytes, s, q, map[i], map_out[i], map_b4[i], use_b4,
-                                        blk_offsets, blk_entries, m_tiles, n_tiles, k_blocks, d->status, flag, checks, flag + kPlanRedo + i);
+                                        blk_offsets, blk_entries, m_tiles, n_tiles, k_blocks, d->status, flag, checks, flag + kPlanRedo + i,
+                                        densespmm::Second<false>());
         if (rc == VS_OK) rc = launch_spmm_t_cc<TOut, V>(list[i], s, d, flag, checks, kPlanRedo + i);
     }
     return rc;
