@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 
 
 @pytest.mark.parametrize("V", [2, 4, 8])
-@pytest.mark.parametrize("heads,n,d", [(1, 64, 64), (3, 520, 64), (2, 264, 64), (100, 264, 64)])
+@pytest.mark.parametrize("heads,n,d", [(3, 264, 128), (1, 64, 64), (3, 520, 64), (2, 264, 64), (100, 264, 64)])
 @pytest.mark.parametrize("cores", [False, True])
 def test_each_as_by_itself(monkeypatch, V, heads, n, d, cores):
     monkeypatch.setenv("VSPARSE_B200_SPMM_T", "gather" if cores else "dense")

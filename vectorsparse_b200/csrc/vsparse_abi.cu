@@ -1777,7 +1777,11 @@ template <typename TOut, int V> int launch_spmm_t(const spmmt::Params *list, int
     const unsigned grid = (unsigned)(items < d->sm_count ? items : d->sm_count);   // one persistent CTA per SM
     const bool pairs = (use_b4 || q.N % 64 != 0) && spmm_pair_takes(q.N, V, (int64_t)q.batch * m_tiles, d, true);
     if constexpr (V > 1) {
-        if (count == 2 && !pairs && d->sm_count > 1 && rc == VS_OK) {   // half of the SMs each: never more waves than one product after the other
+        // Half of the SMs each: never more waves than one product after the other.  Up to 128 columns wide that also beats pairs of CTAs
+        // for one product after the other, in every size that the pairs took there: attention forward and backward of 12 heads x 2280,
+        // d = 128, V = 8 244.4 -> 217.3 us, of 24 x 664, V = 4 116.2 -> 101.8, of one head of 2856, V = 8 92.4 -> 81.5.
+        const char *forced = std::getenv("VSPARSE_B200_SPMM_PAIR");
+        if (count == 2 && (!pairs || (q.N <= 128 && !forced)) && d->sm_count > 1 && rc == VS_OK) {
             densespmm::Second<true> two;
             two.map_b = map[1]; two.map_out = map_out[1]; two.map_b4 = map_b4[1];
             two.values = list[1].values; two.rhs = list[1].rhs;
