@@ -324,7 +324,8 @@ int vs_measure_fp32_fma(double *tflops);
 
 /* Which tensor-path SDDMM formulation vs_sddmm / vs_sddmm_batched would run for this problem: 1 = dense tiles
  * sampled at the mask, 0 = row gather (environment override included).  Diagnostic, no counterpart in the
- * reference; lets a benchmark name the kernels it measures.  Needs no device. */
+ * reference; lets a benchmark name the kernels it measures.  Answers for a batch large enough to fill a B200 (a few
+ * small products may take another form) and needs no device. */
 int vs_sddmm_formulation(int m_vec, int k, int n, int nonzeros_vec, int vec_length);
 
 /* ------------------------------------------------------------------------------------------------------

@@ -1450,8 +1450,8 @@ template <typename TOut, int V> bool launch_sddmm_direct(const SddmmParams &p, c
 struct SddmmTimes {
     double direct, dense, gather;
 };
-SddmmTimes sddmm_times(const SddmmParams &p, int V, const DeviceInfo *d) {
-    const double sms = d->sm_count, k_blocks = std::ceil(p.k / 64.0), per_row = (double)p.nnz_vec / std::max(p.m_vec, 1), m = (double)p.m_vec * V;
+SddmmTimes sddmm_times(const SddmmParams &p, int V, int sm_count) {
+    const double sms = sm_count, k_blocks = std::ceil(p.k / 64.0), per_row = (double)p.nnz_vec / std::max(p.m_vec, 1), m = (double)p.m_vec * V;
     const double tiles = std::ceil(m / 128.0) * std::ceil(p.n / 128.0) * p.batch, items = std::max(1.0, std::ceil(m / 256.0) * std::ceil(p.n / 256.0) * p.batch);
     const double shared = std::min(1.0, std::max(0.0, tiles / sms - 1.0)), pairs = sms / 2;
     SddmmTimes t;
@@ -1463,11 +1463,11 @@ SddmmTimes sddmm_times(const SddmmParams &p, int V, const DeviceInfo *d) {
 }
 // Which planned form runs (VSPARSE_B200_SDDMM = "dense" | "gather", read at every call, forces one).  The number of entries is an argument here, so the choice
 // is made on the host.
-bool sddmm_use_dense(const SddmmParams &p, int V, const DeviceInfo *d) {
+bool sddmm_use_dense(const SddmmParams &p, int V, int sm_count) {
     const char *e = std::getenv("VSPARSE_B200_SDDMM");
     if (e && !std::strcmp(e, "dense")) return true;
     if (e && !std::strcmp(e, "gather")) return false;
-    const SddmmTimes t = sddmm_times(p, V, d);
+    const SddmmTimes t = sddmm_times(p, V, sm_count);
     return t.dense < 1.25 * t.gather;   // where the estimates are close, the one that long rows hold up least
 }
 // Small sampled products go to the one-kernel form.  lhs 512 x 256, rhs 2048 x 256, V = 4: 17.0 -> 7.8 us; 2048 x 512 x 256, V = 8,
@@ -1476,8 +1476,8 @@ bool sddmm_use_dense(const SddmmParams &p, int V, const DeviceInfo *d) {
 bool sddmm_direct_wanted(const SddmmParams &p, int V, const DeviceInfo *d) {
     const char *e = std::getenv("VSPARSE_B200_SDDMM");
     if (e) return !std::strcmp(e, "direct");
-    const SddmmTimes t = sddmm_times(p, V, d);
-    return 1.07 * t.direct < (sddmm_use_dense(p, V, d) ? t.dense : t.gather);
+    const SddmmTimes t = sddmm_times(p, V, d->sm_count);
+    return 1.07 * t.direct < (sddmm_use_dense(p, V, d->sm_count) ? t.dense : t.gather);
 }
 
 template <typename TOut, int V> int launch_sddmm_tc(const SddmmParams &p, cudaStream_t s) {
@@ -1492,7 +1492,7 @@ template <typename TOut, int V> int launch_sddmm_tc(const SddmmParams &p, cudaSt
     const bool dense_ok = !t_no_scratch && p.n > 0 && p.m_vec > 0 && p.nnz_vec > 0 && p.k >= densesddmm::kBlockK && plan_bytes <= kMaxPlanBytes &&
                           plan_smem <= 40 * 1024 && aligned16(p.lhs) && aligned16(p.rhs) &&
                           (p.batch == 1 || ((p.stride_lhs * 2) % 16 == 0 && (p.stride_rhs * 2) % 16 == 0)) &&
-                          sddmm_use_dense(p, V, d);
+                          sddmm_use_dense(p, V, d->sm_count);
     if (!dense_ok) return launch_sddmm_gather<TOut, V>(p, s, d);
     if (sddmm_pair_enabled() && launch_sddmm_pair<TOut, V>(p, s, d, &rc)) return rc;
     CUtensorMap map_l, map_r;
@@ -1561,7 +1561,7 @@ template <int V> int launch_sddmm_cores(const SddmmParams &p, cudaStream_t s) {
     const bool strides = p.batch == 1 || ((p.stride_lhs * 2) % 16 == 0 && (p.stride_rhs * 2) % 16 == 0);
     const bool by_rule = !force_dense && !force_direct && sddmm_cores_wanted(p, V);
     if (!force_cores && !by_rule && strides && p.n > 0 && p.m_vec > 0) {
-        const SddmmTimes t = sddmm_times(p, V, d);
+        const SddmmTimes t = sddmm_times(p, V, d->sm_count);
         const bool pair_ok = !t_no_scratch && sddmm_pair_enabled() && p.n <= pairsddmm::kMaxPlanColumns;
         const bool pair = pair_ok && !force_direct && (force_dense || t.dense < t.direct);
         // The tile forms' estimates are up to 1.7 times too high where they are long; below, what the CUDA-core kernel is taken for is a clear gain.
@@ -2357,9 +2357,8 @@ VS_EXPORT int vs_sddmm_formulation(int m_vec, int k, int n, int nonzeros_vec, in
         return 0;
     SddmmParams p{};
     p.m_vec = m_vec; p.k = k; p.n = n; p.nnz_vec = nonzeros_vec;
-    DeviceInfo *d = nullptr;
-    if (device_info(&d) != VS_OK) return 0;
-    return sddmm_use_dense(p, vec_length, d) ? 1 : 0;
+    p.batch = 4096;   // no batch is given and no device needed: the answer for as many products as fill a B200 many times over
+    return sddmm_use_dense(p, vec_length, 148) ? 1 : 0;
 }
 
 VS_EXPORT int vs_kernel_timing(int enable, double *total_ms, int *launches) {
