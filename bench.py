@@ -90,16 +90,15 @@ NCU_TRAFFIC_BYTES = {
 def kernels_per_step(w, a=None):
     """Names of the library's kernels one step launches (the count is what `gpu_launches` reports)."""
     tensor = w.get("path") != 1
-    # the densified product runs on pairs of CTAs for dense widths above 128 that are multiples of 64, on single CTAs otherwise (128 itself
+    # the densified product runs on pairs of CTAs for dense widths above 128, on single CTAs otherwise (128 itself
     # on pairs where the products are few, which the streams here are not)
-    pair = w["N"] % 64 == 0 and w["N"] > 128 and os.environ.get("VSPARSE_B200_SPMM_PAIR") != "0"
+    pair = w["N"] > 128 and os.environ.get("VSPARSE_B200_SPMM_PAIR") != "0"
     dense = "spmm_pair_kernel" if pair else "spmm_dense_kernel"
     if w["op"] == "attention":
         return ["attention_kernel"]
     if w["op"] == "attention_bwd":
-        plan3 = ["dense_plan_kernel", dense,
-                 "fallback kernel (returns at once unless the plan kernel chose it)"]
-        return ["attention_kernel"] + plan3 + plan3
+        return ["attention_kernel", "dense_plan_kernel<transposed>", dense + "<transposed> (both products)",
+                "spmm_t_kernel (returns at once unless the plan kernel chose it)"]
     if w["op"] == "spmm_t":
         if os.environ.get("VSPARSE_B200_SPMM_T") == "gather":
             return ["spmm_t_kernel"]
