@@ -1738,7 +1738,13 @@ template <typename TOut, int V> int launch_spmm_t(const spmmt::Params *list, int
         }
         return (int)VS_OK;
     };
-    const bool dense_ok = !t_no_scratch && mode != SpmmTMode::kGather && q.K > 0 && q.m_vec > 0 && plan_bytes <= kMaxPlanBytes &&
+    // One small product: plan, tiles and stand-by are 20 us at the least, and few tiles leave most SMs idle, where the CUDA-core kernel is one
+    // launch of many warps.  The host does not know the number of entries, so the line is drawn where even a full matrix is small, and rows of A^T
+    // are short (a warp walks one).  Forward and backward of a training product, tiles / entries, us (vector-rows first): 73 x 719 x 192, V = 4, 73 % sparse
+    // 69 / 63; 462 x 174 x 64, V = 8, 60 % 94 / 74; 125 x 88 x 128, V = 4, 67 % 89 / 64; 229 x 94 x 1216, V = 2, 62 % 69 / 63; past the line
+    // 182 x 1232 x 192, V = 8, 58 % 69 / 72, 154 x 926 x 512, V = 8, 52 % 71 / 81 and 367 x 847 x 192, V = 8, 53 % 74 / 99.
+    const bool small = mode == SpmmTMode::kAuto && count == 1 && m_vec <= 512 && (double)M * p.n * p.N * p.batch <= 100e6;
+    const bool dense_ok = !t_no_scratch && !small && mode != SpmmTMode::kGather && q.K > 0 && q.m_vec > 0 && plan_bytes <= kMaxPlanBytes &&
                           plan_smem <= 40 * 1024 && (q.batch == 1 || (q.stride_rhs * 2) % 16 == 0) &&
                           (q.batch == 1 || (q.stride_out * sizeof(TOut)) % 16 == 0);
     if (!dense_ok) return by_cores();
