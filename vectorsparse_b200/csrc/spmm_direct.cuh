@@ -22,9 +22,10 @@
 // columns ascend has the same bits whichever of them multiplies it, where a tile is not shared (kSplit); a row computed entry by entry has those of spmm_cc_kernel.
 //
 // kSplit: a cluster of up to eight CTAs shares the tile, each with a part of A's columns, where few tiles have many chunks to walk (80 rows x 4023 columns x
-// 320, V = 8, 52 %: 32 chunks on 5 CTAs, 37 us; on 40 CTAs 13.8, a share of four chunks, its search and the sums of the others).  A group of lanes finds the first entry of its vector-row in each part by a search that assumes
-// ascending columns; the parts cover the row, and every entry is compared with the one before it, so that columns which do not ascend are
-// found out all the same.  The parts' sums meet in shared memory, in order, a share of the rows in each CTA.
+// 320, V = 8, 52 %: 32 chunks on 5 CTAs, 37 us; on 40 CTAs 13.8, a share of four chunks, its search and the sums of the others).  Each takes a run of chunks.  A group of lanes finds the first entry of its vector-row in each part by a search
+// that assumes ascending columns; the parts cover the row whatever its order.  Columns which do not ascend are found out all the same: a lane compares every
+// entry that it looks at with the one before it, and it either looks at all of its entries or stops at a column past the end of its part, where an
+// ascending row has none.  The parts' sums meet in shared memory, in order, a share of the rows in each CTA.
 //
 // Roles (320 threads): warps 0-7 fill, then epilogue (TMEM lanes 32 (w % 4) .., columns 32 (w / 4) ..); warp 8 the MMA-issuing
 // thread; warp 9 the thread that loads B by TMA.  Rings: 2 chunks of A (32 KiB each), 3 of B (16 KiB each).  Every
@@ -332,8 +333,11 @@ spmm_direct_kernel(const __grid_constant__ SpmmParams p, const __grid_constant__
             if (lane == 0) tc::mbar_arrive(bar_full + 8 * (c % kBBuffers));
             if (used_up) load_window();   // behind the fence, which waits for outstanding loads as well as for stores
         }
+        // A column at or past the end of this CTA's part: beyond the matrix, or of a row that does not ascend.  What stands behind it in the lane's list was
+        // not looked at.
+        const int part_end = min((chunk0 + chunks) * kChunkK, p.K);
 #pragma unroll
-        for (int e = 0; e < kWindow; ++e) bad |= cols[0][e] != INT_MAX && cols[0][e] >= p.K;   // columns beyond the matrix
+        for (int e = 0; e < kWindow; ++e) bad |= cols[0][e] != INT_MAX && cols[0][e] >= part_end;
         const int fill_row = warp * kRows + lane / kGroup;
         if (bad) atomicOr(redo_rows + (fill_row >> 5), 1u << (fill_row & 31));
 
