@@ -884,8 +884,15 @@ int launch_spmm_other(const SpmmParams &p, cudaStream_t s, DeviceInfo *d, const 
     }
 }
 
+// The sizes of the whole call that `p` is a part of (vs_set_part_of); its own where it is a part of none.
+SpmmParams whole_call(const SpmmParams &p) {
+    SpmmParams whole = p;
+    whole.N = std::max(p.N, t_whole_columns);
+    whole.batch = std::max(p.batch, t_whole_batch);
+    return whole;
+}
 // CTAs that share a tile of the one-kernel form: as many as the tiles leave room for, two from seven chunks of 128 columns on, up to eight with three or more
-// each.  By the sizes of the whole call, whose parts then have its bits (vs_set_part_of).  us, 1 / 2 / 4 / 8: 80 x 4023 x 320, V = 8, 52 % 37 / 23 / 15.5 / 13.8;
+// each.  us, 1 / 2 / 4 / 8: 80 x 4023 x 320, V = 8, 52 % 37 / 23 / 15.5 / 13.8;
 // 1588 x 2035 x 104, V = 4, 57 % 36 / 27 / 21; 172 x 2995 x 64, V = 2, 52 % 64 / 39 / 26 / 19; 158 x 1018 x 128, V = 2, 93 % 12.6 / 10.5; but six chunks,
 // 15 x (232 x 986 x 64) and alike, V = 8, 91 %: 8.3 to 9.0 / 8.7 to 10.1.  VSPARSE_B200_SPMM_SPLIT sets the most.
 int spmm_direct_split(const SpmmParams &p, int V, const DeviceInfo *d) {
@@ -893,17 +900,16 @@ int spmm_direct_split(const SpmmParams &p, int V, const DeviceInfo *d) {
     if (chunks < 7) return 1;
     const char *e = std::getenv("VSPARSE_B200_SPMM_SPLIT");
     const int most = e ? std::atoi(e) : directspmm::kMaxSplit;
-    const int64_t tiles = ((int64_t)p.m_vec * V + directspmm::kTileM - 1) / directspmm::kTileM *
-                          ((std::max(p.N, t_whole_columns) + directspmm::kTileN - 1) / directspmm::kTileN) * std::max(p.batch, t_whole_batch);
+    const int64_t tiles = ((int64_t)p.m_vec * V + directspmm::kTileM - 1) / directspmm::kTileM * ((p.N + directspmm::kTileN - 1) / directspmm::kTileN) * p.batch;
     int split = 1;
     while (2 * split <= std::min(most, directspmm::kMaxSplit) && 2 * split * tiles <= 2 * d->sm_count && std::max(7, 6 * split) <= chunks) split *= 2;
     return split;
 }
-// Small products in one kernel (spmm_direct.cuh); false if this call or this device cannot take it.  When the densified
+// Small products in one kernel (spmm_direct.cuh), `split` CTAs to a tile; false if this call or this device cannot take it.  When the densified
 // product is the cheaper one whatever the number of nonzeros, nothing else is enqueued; otherwise the kernel leaves its
 // verdict where the gather kernel behind it looks for the plan kernel's.
 template <typename TOut, int V, bool kCores> bool launch_spmm_direct(const SpmmParams &p, cudaStream_t s, DeviceInfo *d, SpmmCosts cost,
-                                                                     bool forced, int *rc_out) {
+                                                                     bool forced, int split, int *rc_out) {
     const int m_tiles = (int)(((int64_t)p.m_vec * V + directspmm::kTileM - 1) / directspmm::kTileM);
     const int n_tiles = (p.N + directspmm::kTileN - 1) / directspmm::kTileN;
     const int64_t tiles = (int64_t)p.batch * m_tiles * n_tiles;
@@ -916,7 +922,9 @@ template <typename TOut, int V, bool kCores> bool launch_spmm_direct(const SpmmP
     // with 256 dense columns 34 / 31 / 25 against 72 / 41 / 23.
     // V > 2: only past 4096 columns, where a product whose rows hold a few entries waits for 32 and more chunks, and with scratch.
     const bool by_density = kCores && !forced && (V <= 2 ? p.K > 1024 : p.K > 4096 && !t_no_scratch);
-    if (by_density) cost = {(V > 2 ? 0.018f : V == 2 ? 0.03f : tiles > 48 ? 0.045f : 0.035f) * (float)p.K * (float)p.m_vec / stages, 0.0f, 0.0f, 1.0f};
+    const SpmmParams whole = split > 1 ? whole_call(p) : p;   // its parts share tiles where it does
+    const bool many = (int64_t)whole.batch * m_tiles * ((whole.N + directspmm::kTileN - 1) / directspmm::kTileN) > 48;
+    if (by_density) cost = {(V > 2 ? 0.018f : V == 2 ? 0.03f : many ? 0.045f : 0.035f) * (float)p.K * (float)p.m_vec / stages, 0.0f, 0.0f, 1.0f};
     bool always = forced || (kCores && !by_density) || (!kCores && cost.dense_per_entry == 0.0f && cost.dense_per_stage * stages < cost.gather_per_row * (float)p.m_vec);
     // A caller that says how many values there are is spared the kernel that would return at once (10 x (4 to 16 rows of tiles), 700 to 1600 columns: 2 to 3 of
     // 8 to 16 us).
@@ -930,7 +938,6 @@ template <typename TOut, int V, bool kCores> bool launch_spmm_direct(const SpmmP
     }
     CUtensorMap map;
     static DeviceBits smem_set, smem_set_split;
-    const int split = spmm_direct_split(p, V, d);
     auto kernel = split > 1 ? directspmm::spmm_direct_kernel<TOut, V, true> : directspmm::spmm_direct_kernel<TOut, V, false>;
     if (tiles * split > 0x7fffffffll || make_tile_map(&map, p.rhs, false, (uint64_t)p.K, (uint64_t)p.N, (uint64_t)p.batch, (uint64_t)p.stride_rhs, 64, 64) != VS_OK ||
         set_smem_once(kernel, directspmm::kSmemBytes, split > 1 ? smem_set_split : smem_set) != VS_OK)
@@ -962,7 +969,7 @@ template <typename TOut, int V, bool kCores> bool launch_spmm_direct(const SpmmP
 // kernels' 256-row tiles leave most SMs idle there (V = 1, 4096 x 4096 x 64, 80 / 95 % sparse: 272 -> 114 and 94 -> 53 us; 128 x 4096 x
 // 256: 136 -> 109 and 51 -> 50), at V = 2 up to 64 tiles (2048 vector-rows x 4096 x 64: 143 -> 71 and 58 -> 46; with 256 dense columns
 // 82 -> 93 and 47 -> 60).
-bool spmm_direct_wanted(const SpmmParams &p, int V, bool cores, const DeviceInfo *d) {
+bool spmm_direct_wanted(const SpmmParams &p, int V, bool cores, int split, const DeviceInfo *d) {
     const int64_t m_tiles = ((int64_t)p.m_vec * V + directspmm::kTileM - 1) / directspmm::kTileM;
     const int64_t tiles = m_tiles * ((p.N + directspmm::kTileN - 1) / directspmm::kTileN) * p.batch;
     const int chunks = (p.K + directspmm::kChunkK - 1) / directspmm::kChunkK;
@@ -972,10 +979,20 @@ bool spmm_direct_wanted(const SpmmParams &p, int V, bool cores, const DeviceInfo
     // 1966 x 640, 81 % (8 each) 29 / 24, 506 x 765 x 704, 71 % (6) 18.5 / 16.2, 1906 x 569 x 528, 76 % (5) 20.6 / 26.9; 1984 x 1031 x 320, 87 % (9) 24 / 28, 8 x (97 x
     // 762 x 192), 88 % (6) 17 / 22, 1762 x 1938 x 192, 87 % (4) 21.6 / 26, 1984 x 3120 x 192, 61 % (13) 120 / 110; one kernel / a plan, 172 x 2995 x 64 19 / 164, 16 x
     // (1062 x 2224 x 32) (9) 36 / 80, V = 1, 2 x (2792 x 4032 x 112) (16) 165 / 157.
-    const int split = spmm_direct_split(p, V, d), each = (chunks + split - 1) / split;
+    const int each = (chunks + split - 1) / split;
     const int short_vectors = p.N >= 512 && !t_no_scratch ? (tiles > 40 ? 5 : 6) : split > 1 ? 10 : 16;
     if (tiles <= 2 * d->sm_count) return each <= (V == 8 ? 64 : V == 4 ? 32 : short_vectors);
     return tiles <= 4 * d->sm_count && chunks <= (V >= 4 ? 4 : 1);
+}
+// Whether a call takes that form, and how many CTAs share a tile.  Shared tiles add up in another order than every other kernel of the tensor cores, so a part of a
+// call (vs_set_part_of) has them where, and as, the whole does; where the whole has not, a part takes what is quickest for its own sizes.
+bool spmm_direct_chosen(const SpmmParams &p, int V, bool cores, bool forced, const DeviceInfo *d, int *split) {
+    const SpmmParams whole = whole_call(p);
+    *split = spmm_direct_split(whole, V, d);
+    const bool chosen = forced || spmm_direct_wanted(whole, V, cores, *split, d);
+    if ((chosen && *split > 1) || (whole.N == p.N && whole.batch == p.batch)) return chosen;
+    *split = 1;
+    return forced || spmm_direct_wanted(p, V, cores, 1, d);
 }
 
 // The same product with A laid out densely in memory first (densify.cuh), at V <= 2, where filling the tiles from a plan is what the pair
@@ -1043,8 +1060,10 @@ template <typename TOut, int V, bool kCores> int launch_spmm_tc(const SpmmParams
     if (rc != VS_OK) return rc;
     const SpmmMode mode = spmm_mode();
     constexpr SpmmCosts cost = kCores ? cores_costs(V) : kGatherCosts;
-    if ((mode == SpmmMode::kDirect || (mode == SpmmMode::kAuto && spmm_direct_wanted(p, V, kCores, d))) &&
-        launch_spmm_direct<TOut, V, kCores>(p, s, d, cost, mode == SpmmMode::kDirect, &rc))
+    const bool direct = mode == SpmmMode::kDirect;
+    int split = 1;
+    if ((direct || mode == SpmmMode::kAuto) && spmm_direct_chosen(p, V, kCores, direct, d, &split) &&
+        launch_spmm_direct<TOut, V, kCores>(p, s, d, cost, direct, split, &rc))
         return rc;
     if constexpr (V <= 2) {
         if (!t_no_scratch && mode != SpmmMode::kGather && p.K > 0 && (p.batch == 1 || (p.stride_rhs * 2) % 16 == 0) &&
@@ -1190,9 +1209,7 @@ template <int V> int launch_spmm_split(const SpmmParams &p, int64_t vectors, cud
     }
     if (resident[dev] < 0) return VS_OK;
     const int64_t M = (int64_t)p.m_vec * V;
-    SpmmParams whole = p;
-    whole.N = std::max(p.N, t_whole_columns);
-    whole.batch = std::max(p.batch, t_whole_batch);
+    const SpmmParams whole = whole_call(p);
     const SplitSizes z = split_sizes(p, V, p.N, p.batch, resident[dev]), zw = split_sizes(p, V, whole.N, whole.batch, resident[dev]);
     splitspmm::PrepParams q;
     q.batch_a = z.batch_a; q.batch_b = z.batch_b; q.Kp = z.Kp; q.Np = z.Np;
