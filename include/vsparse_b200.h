@@ -295,10 +295,10 @@ int64_t vs_sddmm_workspace_bytes(int m_vec, int n, int nonzeros_vec);
 int64_t vs_spmm_t_workspace_bytes(int m_vec, int vec_length, int n, int batch, int64_t stride_values);
 int vs_set_workspace(void *workspace, int64_t bytes);
 
-/* The calls of this host thread are parts of one call with `columns` dense columns (SpMM by column shards) or `batch` problems
- * (SpMM and attention by batch shards); 0: of none, the state of every thread at its start.  Where the order of sums depends on a choice between
+/* The calls of this host thread are parts of one call with `columns` dense columns (SpMM and the transposed product by column shards) or `batch` problems
+ * (those and attention by batch shards); 0: of none, the state of every thread at its start.  Where the order of sums depends on a choice between
  * kernels - fp32 SpMM on the CUDA cores or from bf16 parts, fp16 SpMM of few tiles and 769 columns of the matrix and more with one to eight CTAs to a
- * tile, attention in one kernel or in steps and with one, two or four warps to a row - it is made as for the whole call, so that the parts have its bits. */
+ * tile, small transposed products on the CUDA cores or on tiles, attention in one kernel or in steps and with one, two or four warps to a row - it is made as for the whole call, so that the parts have its bits. */
 int vs_set_part_of(int columns, int batch);
 
 /* Frees the plan scratch the library keeps on the current device for `stream` (stream-ordered: behind the work

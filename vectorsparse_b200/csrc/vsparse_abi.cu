@@ -1723,8 +1723,8 @@ SpmmTMode spmm_t_mode() {   // read at every call, so that a test can switch ker
 // plan kernel's units (SM-cycles per 128 columns): the CUDA-core kernel ~5 per value (0.92 ms for 256 products of
 // 2048 x 512, 90 % sparse, V = 8), the dense kernel ~1100 per stage plus ~1.5 per vector of fill work (0.170 ms on
 // the same problem against 0.137 for the forward product with the same tiles).
-// `count` products (at most kPlanProducts) with the same structure, sizes and strides: one plan serves them.
-template <typename TOut, int V> int launch_spmm_t(const spmmt::Params *list, int count, int m_vec, cudaStream_t s) {
+// `count` products (at most kPlanProducts) with the same structure, sizes and strides: one plan serves them.  `alone`: the caller has no other with that structure.
+template <typename TOut, int V> int launch_spmm_t(const spmmt::Params *list, int count, int m_vec, cudaStream_t s, bool alone) {
     const spmmt::Params &p = list[0];
     DeviceInfo *d;
     int rc = device_info(&d);
@@ -1755,12 +1755,13 @@ template <typename TOut, int V> int launch_spmm_t(const spmmt::Params *list, int
         }
         return (int)VS_OK;
     };
-    // One small product: plan, tiles and stand-by are 20 us at the least, and few tiles leave most SMs idle, where the CUDA-core kernel is one
+    // One small product, by the sizes of the whole call that it is a part of (the CUDA-core kernel adds up in another order than the tiles): plan, tiles and stand-by are 20 us at the least, and few tiles leave most SMs idle, where the CUDA-core kernel is one
     // launch of many warps.  The host does not know the number of entries, so the line is drawn where even a full matrix is small, and rows of A^T
     // are short (a warp walks one).  Forward and backward of a training product, tiles / entries, us (vector-rows first): 73 x 719 x 192, V = 4, 73 % sparse
     // 69 / 63; 462 x 174 x 64, V = 8, 60 % 94 / 74; 125 x 88 x 128, V = 4, 67 % 89 / 64; 229 x 94 x 1216, V = 2, 62 % 69 / 63; past the line
     // 182 x 1232 x 192, V = 8, 58 % 69 / 72, 154 x 926 x 512, V = 8, 52 % 71 / 81 and 367 x 847 x 192, V = 8, 53 % 74 / 99.
-    const bool small = mode == SpmmTMode::kAuto && count == 1 && m_vec <= 512 && (double)M * p.n * p.N * p.batch <= 100e6;
+    const SpmmParams whole = whole_call(q);
+    const bool small = mode == SpmmTMode::kAuto && alone && m_vec <= 512 && (double)M * p.n * whole.N * whole.batch <= 100e6;
     const bool dense_ok = !t_no_scratch && !small && mode != SpmmTMode::kGather && q.K > 0 && q.m_vec > 0 && plan_bytes <= kMaxPlanBytes &&
                           plan_smem <= 40 * 1024 && (q.batch == 1 || (q.stride_rhs * 2) % 16 == 0) &&
                           (q.batch == 1 || (q.stride_out * sizeof(TOut)) % 16 == 0);
@@ -1830,12 +1831,12 @@ template <typename TOut, int V> int launch_spmm_t(const spmmt::Params *list, int
     }
     return rc;
 }
-template <typename TOut> int spmm_t_by_v(int V, const spmmt::Params *p, int count, int m_vec, cudaStream_t s) {
+template <typename TOut> int spmm_t_by_v(int V, const spmmt::Params *p, int count, int m_vec, cudaStream_t s, bool alone) {
     switch (V) {
-        case 1: return launch_spmm_t<TOut, 1>(p, count, m_vec, s);
-        case 2: return launch_spmm_t<TOut, 2>(p, count, m_vec, s);
-        case 4: return launch_spmm_t<TOut, 4>(p, count, m_vec, s);
-        case 8: return launch_spmm_t<TOut, 8>(p, count, m_vec, s);
+        case 1: return launch_spmm_t<TOut, 1>(p, count, m_vec, s, alone);
+        case 2: return launch_spmm_t<TOut, 2>(p, count, m_vec, s, alone);
+        case 4: return launch_spmm_t<TOut, 4>(p, count, m_vec, s, alone);
+        case 8: return launch_spmm_t<TOut, 8>(p, count, m_vec, s, alone);
     }
     return VS_ERR_VEC_LENGTH;
 }
@@ -1877,7 +1878,7 @@ VS_EXPORT int vs_spmm_t_batched(int in_dtype, int out_dtype, int m_vec, int vec_
                                  stride_values, stride_rhs, stride_out, p, empty);
     if (rc != VS_OK || empty) return rc;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    return out_dtype == VS_F16 ? spmm_t_by_v<__half>(vec_length, &p, 1, m_vec, s) : spmm_t_by_v<float>(vec_length, &p, 1, m_vec, s);
+    return out_dtype == VS_F16 ? spmm_t_by_v<__half>(vec_length, &p, 1, m_vec, s, true) : spmm_t_by_v<float>(vec_length, &p, 1, m_vec, s, true);
 }
 
 VS_EXPORT int vs_spmm_t(int in_dtype, int out_dtype, int m_vec, int vec_length, int k, int n, const int32_t *t_offsets,
@@ -2087,7 +2088,7 @@ VS_EXPORT int vs_attention_cvse_backward(int path, int m_vec, int vec_length, in
         if (rc == VS_OK && !empty)
             rc = spmm_t_params(VS_F16, VS_F16, m_vec, vec_length, d, n, t_offsets, t_rows, t_src, grad_workspace, q, grad_k, batch, s_ws, s_q, s_k, both[1], empty);
         if (rc != VS_OK || empty) return rc;
-        return spmm_t_by_v<__half>(vec_length, both, 2, m_vec, st);
+        return spmm_t_by_v<__half>(vec_length, both, 2, m_vec, st, false);
     }
     // P = softmax(scale * Q K^T) at the mask, recomputed rather than kept from the forward pass
     int rc = vs_sddmm_batched(path, VS_F16, VS_F16, m_vec, d, n, nonzeros_vec, row_indices, row_offsets, col_indices, q, kmat,
@@ -2109,7 +2110,7 @@ VS_EXPORT int vs_attention_cvse_backward(int path, int m_vec, int vec_length, in
     bool empty;
     rc = spmm_t_params(VS_F16, VS_F16, m_vec, vec_length, d, n, t_offsets, t_rows, t_src, probs_workspace, grad_out, grad_v, batch, s_ws, s_q, s_k,
                        both[0], empty);
-    if (rc == VS_OK && !empty && apart) rc = spmm_t_by_v<__half>(vec_length, both, 1, m_vec, static_cast<cudaStream_t>(stream));
+    if (rc == VS_OK && !empty && apart) rc = spmm_t_by_v<__half>(vec_length, both, 1, m_vec, static_cast<cudaStream_t>(stream), false);
     if (rc != VS_OK) return rc;
     // dP = dO V^T at the mask; dS = scale * P o (dP - rowsum(P o dP))
     rc = vs_sddmm_batched(path, VS_F16, VS_F16, m_vec, d, n, nonzeros_vec, row_indices, row_offsets, col_indices, grad_out, vmat,
@@ -2125,8 +2126,8 @@ VS_EXPORT int vs_attention_cvse_backward(int path, int m_vec, int vec_length, in
         rc = spmm_t_params(VS_F16, VS_F16, m_vec, vec_length, d, n, t_offsets, t_rows, t_src, grad_workspace, q, grad_k, batch, s_ws, s_q, s_k,
                            both[1], empty);
     if (rc != VS_OK || empty) return rc;
-    return apart ? spmm_t_by_v<__half>(vec_length, both + 1, 1, m_vec, static_cast<cudaStream_t>(stream))
-                 : spmm_t_by_v<__half>(vec_length, both, 2, m_vec, static_cast<cudaStream_t>(stream));
+    return apart ? spmm_t_by_v<__half>(vec_length, both + 1, 1, m_vec, static_cast<cudaStream_t>(stream), false)
+                 : spmm_t_by_v<__half>(vec_length, both, 2, m_vec, static_cast<cudaStream_t>(stream), false);
 }
 
 VS_EXPORT int vs_attention_cvse(int path, int m_vec, int vec_length, int n, int d, int nonzeros_vec,

@@ -25,7 +25,7 @@ _scope = threading.local()
 def part_of(columns: int = 0, batch: int = 0):
     """Calls of this host thread inside the block are parts of one call with that many dense columns or problems, and choose the order of their sums
     as that call would (vs_set_part_of): fp32 SpMM between the CUDA cores and the tensor cores, fp16 SpMM of few tiles among the CTAs that share one,
-    attention between its forms and the warps that share a row.  A part then has the bits of the whole, at the price of a kernel that may not be the quickest for the part alone."""
+    small transposed products between the CUDA cores and tiles, attention between its forms and the warps that share a row.  A part then has the bits of the whole, at the price of a kernel that may not be the quickest for the part alone."""
     from . import _lib
     outer = getattr(_scope, "value", (0, 0))
     _scope.value = (columns, batch)
