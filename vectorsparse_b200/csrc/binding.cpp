@@ -385,14 +385,14 @@ struct MaskNode : torch::autograd::Node {
             std::lock_guard<std::mutex> guard(lock);
             for (auto &x : saved) kept.push_back(x.unpack(shared_from_this()));
         }
-        if (!in[0].defined()) return torch::autograd::variable_list(num_outputs());
-        bool fast = !c10::GradMode::is_enabled() && c10::impl::TorchDispatchModeTLS::stack_len() == 0 && !at::hasCallbacks() && plain(in[0]);
-        for (const at::Tensor &t : kept) fast = fast && plain(t) && t.is_contiguous() && t.device() == in[0].device();
-        if (!fast) return in_python(kept, in[0]);
-        c10::cuda::CUDAGuard guard(in[0].device());
-        const at::Tensor grad = in[0].contiguous();
+        const at::Tensor given = in[0].defined() ? in[0] : input_metadata(0).zeros_like();   // no gradient counts as zeros, as in the Python function
+        bool fast = !c10::GradMode::is_enabled() && c10::impl::TorchDispatchModeTLS::stack_len() == 0 && !at::hasCallbacks() && plain(given);
+        for (const at::Tensor &t : kept) fast = fast && plain(t) && t.is_contiguous() && t.device() == given.device();
+        if (!fast) return in_python(kept, given);
+        c10::cuda::CUDAGuard guard(given.device());
+        const at::Tensor grad = given.contiguous();
         torch::autograd::variable_list out(num_outputs());
-        return (which ? attention(kept, grad, out) : product(kept, grad, out)) == 0 ? out : in_python(kept, in[0]);
+        return (which ? attention(kept, grad, out) : product(kept, grad, out)) == 0 ? out : in_python(kept, given);
     }
 
     int product(const std::vector<at::Tensor> &kept, const at::Tensor &grad, torch::autograd::variable_list &out) {
