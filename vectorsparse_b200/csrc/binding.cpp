@@ -10,11 +10,13 @@
 // that vectorsparse_b200._lib has loaded is the one that is called.
 #include <Python.h>
 
+#include <ATen/PythonTorchFunctionTLS.h>
 #include <ATen/core/Tensor.h>
 #include <ATen/ops/empty.h>
 #include <ATen/ops/empty_like.h>
 #include <ATen/record_function.h>
 #include <c10/core/SafePyObject.h>
+#include <c10/core/impl/LocalDispatchKeySet.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAGuard.h>
@@ -23,6 +25,7 @@
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 #include <torch/csrc/PyInterpreter.h>
 #include <torch/csrc/Exceptions.h>
 
@@ -329,6 +332,11 @@ bool plain(const at::Tensor &t) {
            !t.key_set().has_any(c10::DispatchKeySet({c10::DispatchKey::Python, c10::DispatchKey::FuncTorchBatched, c10::DispatchKey::FuncTorchGradWrapper,
                                                      c10::DispatchKey::Functionalize, c10::DispatchKey::Conjugate, c10::DispatchKey::Negative}));
 }
+// Whether modes of either kind, a tracer or a profiler listen to this thread's operators (torch_ops._through asks the same).
+bool heard() {
+    return c10::impl::TorchDispatchModeTLS::stack_len() != 0 || at::impl::PythonTorchFunctionTLS::stack_len() != 0 || torch::jit::tracer::isTracing() ||
+           c10::impl::tls_is_dispatch_key_included(c10::DispatchKey::PreDispatch) || at::hasCallbacks();
+}
 template <typename F> int enqueue_on(const at::Tensor &t, F &&f) { return f((void *)c10::cuda::getCurrentCUDAStream(t.get_device()).stream()); }
 
 struct MaskNode : torch::autograd::Node {
@@ -386,7 +394,7 @@ struct MaskNode : torch::autograd::Node {
             for (auto &x : saved) kept.push_back(x.unpack(shared_from_this()));
         }
         const at::Tensor given = in[0].defined() ? in[0] : input_metadata(0).zeros_like();   // no gradient counts as zeros, as in the Python function
-        bool fast = !c10::GradMode::is_enabled() && c10::impl::TorchDispatchModeTLS::stack_len() == 0 && !at::hasCallbacks() && plain(given);
+        bool fast = !c10::GradMode::is_enabled() && !heard() && plain(given);
         for (const at::Tensor &t : kept) fast = fast && plain(t) && t.is_contiguous() && t.device() == given.device();
         if (!fast) return in_python(kept, given);
         c10::cuda::CUDAGuard guard(given.device());
