@@ -103,7 +103,9 @@ int vs_spmm(int path, int in_dtype, int out_dtype, int m_vec, int vec_length, in
 /* `batch` independent products that share one CVSE structure (row_indices/row_offsets/col_indices) and differ
  * in values, rhs and output, found at element strides stride_values / stride_rhs / stride_out from the first
  * (a stride of 0 shares that operand; stride_out must not be 0).  Strides must keep 16-byte alignment.  With batch 1 stride_values may
- * say how many values there are, or an upper bound: calls too sparse for the tensor-core form of fp32 products then skip its kernels.
+ * say how many values there are, or an upper bound: calls too sparse for the tensor-core form of fp32 products then skip its kernels, and fp16
+ * products choose between their forms by it, on the host, where otherwise (0, or a batch that it does not already show to be sparse) the device looks at
+ * row_offsets and a second kernel stands by.  No result depends on it but for the order of sums; a bound far above the number costs time.
  * One launch covers the whole batch.  The reference has no batched call; this is the batch x head form of its
  * SpMM for fixed-mask sparse attention. */
 int vs_spmm_batched(int path, int in_dtype, int out_dtype, int m_vec, int vec_length, int k, int n,

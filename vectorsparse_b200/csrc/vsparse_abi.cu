@@ -927,14 +927,15 @@ template <typename TOut, int V, bool kCores> bool launch_spmm_direct(const SpmmP
     if (by_density) cost = {(V > 2 ? 0.018f : V == 2 ? 0.03f : many ? 0.045f : 0.035f) * (float)p.K * (float)p.m_vec / stages, 0.0f, 0.0f, 1.0f};
     bool always = forced || (kCores && !by_density) || (!kCores && cost.dense_per_entry == 0.0f && cost.dense_per_stage * stages < cost.gather_per_row * (float)p.m_vec);
     // A caller that says how many values there are is spared the kernel that would return at once (10 x (4 to 16 rows of tiles), 700 to 1600 columns: 2 to 3 of
-    // 8 to 16 us).
+    // 8 to 16 us).  The distance between the matrices of a batch is no such number, only a bound: too few for the tiles by that are too few, enough by that the
+    // device has to say.
     if (!always && p.stride_values > 0) {
         const float nnz = (float)(p.stride_values / V);
         if (!(cost.dense_per_stage * stages + cost.dense_per_entry * nnz < cost.gather_per_row * (float)p.m_vec + cost.gather_per_entry * nnz)) {
             *rc_out = launch_spmm_other<TOut, V, kCores>(p, s, d, nullptr, 0);
             return true;
         }
-        always = true;
+        always = whole_call(p).batch == 1;
     }
     CUtensorMap map;
     static DeviceBits smem_set, smem_set_split;
@@ -1012,7 +1013,8 @@ template <typename TOut, int V, bool kCores> bool launch_spmm_laid_out(const Spm
     const int Kp = (p.K + 63) / 64 * 64, k_blocks = Kp / 64, batch_a = p.batch > 1 && p.stride_values ? p.batch : 1;
     const int64_t row_items = (int64_t)p.batch * m_tiles, a_bytes = (int64_t)batch_a * row_tiles * 128 * Kp * 2;
     if (capacity < 0 || !spmm_pair_takes(p.N, V, row_items, d) || a_bytes > (128ll << 20)) return false;
-    // Widths that are no multiple of 64: where there is work for the tiles, six blocks of 64 columns and 5 % of the vectors (68 x (3960 x 66 x 1128), V = 1 218 us on
+    // Widths that are no multiple of 64: where there is work for the tiles, six blocks of 64 columns and not, by the count or its bound,
+    // under 5 % of the vectors (68 x (3960 x 66 x 1128), V = 1 218 us on
     // single CTAs, 312 laid out; 49 x (160 x 1166 x 336), V = 1, 96 % 26 and 32)
     if (!e && p.N % 64 != 0 && (k_blocks < 6 || (p.stride_values > 0 && (double)(p.stride_values / V) < 0.05 * p.m_vec * p.K))) return false;
     const int tn = spmm_pair_width(p.N, row_items, capacity), n_tiles = (p.N + tn - 1) / tn;
