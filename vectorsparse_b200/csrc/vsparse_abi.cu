@@ -1725,6 +1725,15 @@ SpmmTMode spmm_t_mode() {   // read at every call, so that a test can switch ker
 // plan kernel's units (SM-cycles per 128 columns): the CUDA-core kernel ~5 per value (0.92 ms for 256 products of
 // 2048 x 512, 90 % sparse, V = 8), the dense kernel ~1100 per stage plus ~1.5 per vector of fill work (0.170 ms on
 // the same problem against 0.137 for the forward product with the same tiles).
+struct Span {
+    const void *at;
+    int64_t elems;   // fp16, of each problem
+};
+// Whether two of them share memory.
+bool overlap(const Span &x, const Span &y, int batch) {
+    const uintptr_t a = reinterpret_cast<uintptr_t>(x.at), b = reinterpret_cast<uintptr_t>(y.at);
+    return a < b + 2 * (uintptr_t)(y.elems * batch) && b < a + 2 * (uintptr_t)(x.elems * batch);
+}
 // `count` products (at most kPlanProducts) with the same structure, sizes and strides: one plan serves them.  `alone`: the caller has no other with that structure.
 template <typename TOut, int V> int launch_spmm_t(const spmmt::Params *list, int count, int m_vec, cudaStream_t s, bool alone) {
     const spmmt::Params &p = list[0];
@@ -1807,7 +1816,9 @@ template <typename TOut, int V> int launch_spmm_t(const spmmt::Params *list, int
         // for one product after the other, in every size that the pairs took there: attention forward and backward of 12 heads x 2280,
         // d = 128, V = 8 244.4 -> 217.3 us, of 24 x 664, V = 4 116.2 -> 101.8, of one head of 2856, V = 8 92.4 -> 81.5.
         const char *forced = std::getenv("VSPARSE_B200_SPMM_PAIR");
-        if (count == 2 && (!pairs || (q.N <= 128 && !forced)) && d->sm_count > 1 && rc == VS_OK) {
+        // Results that share memory are written one after the other.
+        const int64_t elems = (int64_t)q.m_vec * q.N;
+        if (count == 2 && (!pairs || (q.N <= 128 && !forced)) && d->sm_count > 1 && rc == VS_OK && !overlap({list[0].out, elems}, {list[1].out, elems}, q.batch)) {
             densespmm::Second<true> two;
             two.map_b = map[1]; two.map_out = map_out[1]; two.map_b4 = map_b4[1];
             two.values = list[1].values; two.rhs = list[1].rhs;
@@ -2009,10 +2020,6 @@ template <int D, bool kBackward> int launch_attention_rows(const attention::Para
     if (warps == 2) return launch_attention<D, 2, kBackward>(p, batch, s);
     return launch_attention<D, 4, kBackward>(p, batch, s);
 }
-struct Span {
-    const void *at;
-    int64_t elems;   // fp16
-};
 // Whether the one-kernel form takes a call; what it does not take, and every refusal, is the operators' own.  Their steps read an operand for the
 // last time before a later step writes (grad_q in the place of grad_out, out in the place of kmat): where a result lies on an operand, they stay.
 // VSPARSE_B200_ATTENTION=steps|fused.
@@ -2037,9 +2044,8 @@ bool attention_fused(int path, int m_vec, int V, int n, int d, int nnz_vec, int 
         if (!x.at || reinterpret_cast<uintptr_t>(x.at) % 32 != 0) return false;
     for (const Span &x : results) {
         if (!x.at || !aligned16(x.at)) return false;
-        const uintptr_t first = reinterpret_cast<uintptr_t>(x.at), end = first + 2 * (uintptr_t)x.elems * batch;
         for (const Span &y : sources)
-            if (first < reinterpret_cast<uintptr_t>(y.at) + 2 * (uintptr_t)y.elems * batch && reinterpret_cast<uintptr_t>(y.at) < end) return false;
+            if (overlap(x, y, batch)) return false;
     }
     return (int64_t)nnz_vec * V % 8 == 0;
 }
@@ -2100,14 +2106,11 @@ VS_EXPORT int vs_attention_cvse_backward(int path, int m_vec, int vec_length, in
                          s_ws, stream);
     if (rc != VS_OK) return rc;
     // dV = P^T dO together with dK = dS^T Q, from one plan and (spmm_dense_kernel<kTwo>) in one launch, unless dQ or dK is to stand where
-    // dO or P is still to be read.  Forward and backward of 10 heads x 2152, d = 128, V = 4: 305.3 -> 277.2 us; 16 x 3400,
+    // dO or P is still to be read, or shares dV's memory.  Forward and backward of 10 heads x 2152, d = 128, V = 4: 305.3 -> 277.2 us; 16 x 3400,
     // V = 2 658.7 -> 639.6.
-    auto over = [&](const void *x, int64_t x_elems, const void *y, int64_t y_elems) {
-        const uintptr_t a = reinterpret_cast<uintptr_t>(x), b = reinterpret_cast<uintptr_t>(y);
-        return a < b + 2 * (uintptr_t)(y_elems * batch) && b < a + 2 * (uintptr_t)(x_elems * batch);
-    };
-    const bool apart = over(grad_q, s_q, grad_out, s_q) || over(grad_q, s_q, probs_workspace, s_ws) ||
-                       over(grad_k, s_k, grad_out, s_q) || over(grad_k, s_k, probs_workspace, s_ws);
+    bool apart = false;
+    for (const Span &x : {Span{grad_q, s_q}, Span{grad_k, s_k}})
+        for (const Span &y : {Span{grad_out, s_q}, Span{probs_workspace, s_ws}, Span{grad_v, s_k}}) apart = apart || overlap(x, y, batch);
     spmmt::Params both[2];
     bool empty;
     rc = spmm_t_params(VS_F16, VS_F16, m_vec, vec_length, d, n, t_offsets, t_rows, t_src, probs_workspace, grad_out, grad_v, batch, s_ws, s_q, s_k,
