@@ -240,7 +240,8 @@ sddmm_twin_kernel(const SddmmParams p, const uint2 *__restrict__ words, const in
             if (__ldg(p.row_offsets + mid) <= j) lo = mid; else hi = mid;
         }
         const uint2 word = __ldg(words + (int64_t)lo * n_words + (c >> 5));
-        if (!(word.y >> 31)) continue;
+        // an entry behind the last row's (the caller may count more than the offsets do) need not be in the row found: `order` names none there
+        if (!(word.y >> 31) || !(word.x >> (c & 31) & 1u)) continue;
         const int other = __ldg(order + (word.y & 0x7fffffffu) + __popc(word.x & ((1u << (c & 31)) - 1u)));
         if (other == j) continue;
         for (int b = 0; b < p.batch; ++b) {
