@@ -324,10 +324,10 @@ int vs_kernel_timing(int enable, double *total_ms, int *launches);
  * no counterpart in the reference. */
 int vs_measure_fp32_fma(double *tflops);
 
-/* Which tensor-path SDDMM formulation vs_sddmm / vs_sddmm_batched would run for this problem: 1 = dense tiles
- * sampled at the mask, 0 = row gather (environment override included).  Diagnostic, no counterpart in the
- * reference; lets a benchmark name the kernels it measures.  Answers for a batch large enough to fill a B200 (a few
- * small products may take another form) and needs no device. */
+/* Which tensor-path SDDMM formulation vs_sddmm_batched runs for a batch of such problems that is large enough to fill a B200 many
+ * times over: 1 = dense tiles sampled at the mask, 0 = row gather (environment override included).  One product or a few may take
+ * another form, which depends on their number.  Diagnostic, no counterpart in the reference; lets a benchmark name the kernels it
+ * measures.  Needs no device. */
 int vs_sddmm_formulation(int m_vec, int k, int n, int nonzeros_vec, int vec_length);
 
 /* ------------------------------------------------------------------------------------------------------

@@ -36,7 +36,7 @@ def test_each_as_by_itself(monkeypatch, V, heads, n, d, cores):
 def test_of_the_composed_steps(monkeypatch):
     """The operators one after the other give the same two products, and still do where dQ or dK is written over dO or P."""
     monkeypatch.setenv("VSPARSE_B200_ATTENTION", "steps")
-    monkeypatch.setenv("VSPARSE_B200_SPMM_T", "dense")   # one small product by itself needs no plan
+    monkeypatch.setenv("VSPARSE_B200_SPMM_T", "dense")   # tiles, whatever the density
     V, heads, n, d = 4, 2, 264, 64
     a = custom([4 * (7 * i % (n // 16)) for i in range(n // V)], n, V, seed=n + V)
     q, k, v, go = (dev(cvse.fill_random((heads, n, d), np.float16, cvse.DIST_NORMAL, 10 + i, 1.0)) for i in range(4))

@@ -17,7 +17,7 @@
 // and which entry index j it is, comes from the mask as bits that the plan kernel lays out: per (vector-row, 32 columns) a word
 // with a bit for each column it names and the index of the first of them.  A warp samples 32 neighbouring columns, so a word
 // serves all its lanes, and j is that index plus the set bits below the lane's.  (Before, a lane looked up a word per (32 vector-rows, column)
-// and then the index of each entry in a list ordered by column, which the plan had to make: 137 -> 132 us at 256 x (2048 x 512), k = 256, V = 8,
+// and then the index of each entry in a list ordered by column, which the plan had to make: 160 -> 156 us at 256 x (2048 x 512), k = 256, V = 8,
 // 90 % sparse; 146 x (1008 x 1361), k = 128, V = 4 82 -> 78.)  Finding the entries ahead of the accumulator and without branches counts: by shuffles
 // between the stores 88 us in the latter, with a branch for each 100, from shared memory 94.  No shared-memory boxes, no dynamic register indexing, nothing
 // outside the mask is ever stored, so non-finite products elsewhere in the tile cannot leak.  A bit holds

@@ -1220,7 +1220,7 @@ template <int V> int launch_spmm_split(const SpmmParams &p, int64_t vectors, cud
     // us: 64 columns of an item by a pair, the preparation at 4.6 TB/s, launches (180 estimated, 165 to 180 measured at 4096 x 4096 x 1024; 36
     // and 36 at 1024 cubed; 25 and 25 at 512 cubed); against the CUDA-core kernel's time per vector and column (611 us
     // at V = 1, 305 at V = 2, 301 at V = 4, 258 at V = 8 for 4096 x 4096 x 1024, 80 % sparse), or, where it takes the call otherwise, against that of the
-    // kernel that stages tiles of B: per wave a start, the tiles, the entries of a vector-row (V = 8, 2048 x 4096 x 1024, 50 / 65 / 80 %
+    // kernel that stages tiles of B (also where few vector-rows then go to spmm_cc_few_kernel, whose time is not fitted): per wave a start, the tiles, the entries of a vector-row (V = 8, 2048 x 4096 x 1024, 50 / 65 / 80 %
     // sparse: that kernel 228 / 165 / 103, this one 114 / 111 / 106; V = 1, 1024 x 1024 x 512: 54 / 41 / 29 and 38 / 37 / 36).  Below kMinDensity that kernel keeps every
     // dense width, so that column shards of usual matrices (90 %, at V = 4 80 % sparse) have the bits of the whole product; by cost the line would lie
     // at 0.047 (V = 1) and 0.097 (V = 4) for 4096 x 4096 x 8192.
